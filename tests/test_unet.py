@@ -130,6 +130,52 @@ def test_gradients_match_oracle(shape):
         assert np.abs(gbb - rbb).max() <= 3e-2 * max(float(np.abs(rbb).max()), 1e-12), (i, gbb[:4], rbb[:4])
 
 
+def _exact_case(B, H, W):
+    """A network of 0, 1/2 and 1 at the centre taps on inputs 0, 64, 128, 192, and a target that makes every
+    error a small integer or half: with B H W a power of two every sum of the forward and the dX passes is exact in
+    FP32 in any order, so the bf16 roundings agree with the oracle's bit for bit; and all values are >= 0."""
+    offs, nw, nb = U.offsets()
+    w, b = np.zeros(nw, np.float32), np.zeros(nb, np.float32)
+    for i, (_, _, c1, _, _, c2, co, _, _) in enumerate(U.LAYERS):
+        wl = np.zeros((9, co, c1 + c2), np.float32)
+        outs, live = (1 if i == len(U.LAYERS) - 1 else co), (3 if i == 0 else c1)
+        for o in range(outs):
+            wl[4, o, [k % live for k in range(o, max(live, outs), outs)]] = 0.5 if o % 2 else 1.0
+            if c2:
+                wl[4, o, c1 + o % c2] = 0.5
+        w[offs[i][0]:offs[i][0] + wl.size] = wl.ravel()
+    rng = np.random.default_rng(31)
+    inp = np.zeros((B, H, W, 32), np.float32)
+    inp[..., :3] = 64.0 * rng.integers(0, 4, (B, H, W, 3))
+    return w, b, inp, np.zeros((B, H, W), np.float32), -rng.integers(0, 4, (B, H, W)).astype(np.float32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 8, 8), (1, 8, 64), (2, 16, 32), (1, 256, 256)])
+def test_weight_gradient_sums_are_the_products_over_all_pixels(shape):
+    """The weight and bias gradients where their tiling can go wrong: partial 16 x 8 tiles, one tile a CTA, and
+    more than two tiles a CTA (the staging buffers used again). On _exact_case every product is exact and >= 0, so
+    an FP32 sum over n pixels, whatever its order, is within n 2^-23 of the oracle's f64 sum, element by element."""
+    import lapstack_b200 as L
+    B, H, W = shape
+    w, b, inp, d_in, tgt = _exact_case(B, H, W)
+    net = L.UNet(seed=0)
+    net.set_params(w, b)
+    net.train_step(*_to_gpu(inp, d_in, tgt), lr=0.0)
+    gw, gb = net.grads()
+    net.close()
+    act, out0 = U.forward(inp, w, b)
+    _, rgw, rgb = U.backward(act, out0, d_in, tgt, w)
+    assert np.count_nonzero(rgw) > (0.9 if H > 8 else 0.1) * (rgw.size - 9 * 32 * (29 + 31))  # the live weights
+    offs, _, _ = U.offsets()
+    for i, (wo, bo) in enumerate(offs):
+        c1, c2, co, lv = U.LAYERS[i][2], U.LAYERS[i][5], U.LAYERS[i][6], U.LAYERS[i][7]
+        n = max(B * (H >> lv) * (W >> lv), 1)
+        for g, r in ((gw[wo:wo + 9 * co * (c1 + c2)], rgw[wo:wo + 9 * co * (c1 + c2)]), (gb[bo:bo + co], rgb[bo:bo + co])):
+            bad = np.abs(g - r) > n * 2.0 ** -23 * r
+            assert not bad.any(), (i, int(bad.sum()), g[bad][:3], r[bad][:3])
+
+
 @pytest.mark.gpu
 def test_training_fits_a_fixed_batch():
     """Adam on the library's gradients learns a correction that depends on the guide channel."""
