@@ -46,6 +46,7 @@ struct ConvArgs {
     int c2s, mode2;      // source 2 (channels c1..cin-1), its channel stride
     int cin, cout;
     const __nv_bfloat16* w;  // [9][cout][cin]
+    const __nv_bfloat16* wp;  // the same packed for the tcgen05 path: [cout / N][cin / 32][9][4][N][8]
     const float* bias;       // [cout] or null
     int relu;
     __nv_bfloat16* out;      // [B][H][W][cout] bf16, or null
@@ -197,27 +198,54 @@ __global__ void __launch_bounds__(UN_THREADS) conv3x3_kernel(const ConvArgs a) {
 }
 
 // ------------------------------------------------- the same conv on tcgen05
-// conv3x3_tc_kernel: the implicit GEMM on the 5th-generation tensor cores. A CTA of 4 warps owns a
-// 16 x 8 tile of output pixels (M = 128, one TMEM lane per pixel) and N = cout output channels (one
-// fp32 TMEM column each). Per 32-channel input chunk every thread stages the 18 x 10 input halo and
-// the chunk's 9 x N x 32 weights in shared memory in the canonical no-swizzle K-major layout of the
-// UMMA operand descriptors (8 rows of 16 bytes per core matrix): the halo as [k8][pixel][8 channels],
-// so that the tap (ky, kx) of the A operand is the same layout started (ky * 10 + kx) pixels later
-// (rows of 8 pixels 10 pixels apart: SBO = 160 B, the next 8 channels LBO = 180 pixels further);
-// the weights as [tap][k8][n][8]. One thread issues the 9 taps x 2 K-steps of tcgen05.mma
-// (kind::f16, BF16 x BF16 -> FP32 in TMEM) and commits them to an mbarrier that every thread waits
-// on (bounded) before the staging of the next chunk; the epilogue reads the accumulator with
-// tcgen05.ld (warp w: lanes 32w..32w+31), adds the bias, applies ReLU and stores NHWC.
+// conv3x3_tc_kernel: the implicit GEMM on the 5th-generation tensor cores. A tile is 16 x 8 output pixels
+// (M = 128, one TMEM lane per pixel) x N output channels (one fp32 TMEM column each); cin goes by chunks of
+// 32. The operands lie in shared memory in the canonical no-swizzle K-major layout of the UMMA descriptors
+// (8 rows of 16 bytes per core matrix): the 18 x 10 halo of a chunk as [k8][pixel][8 channels], so that the
+// tap (ky, kx) of the A operand is the same layout started (ky * 10 + kx) pixels later (rows of 8 pixels 10
+// pixels apart: SBO = 160 B, the next 8 channels LBO = one plane further); the weights as [tap][k8][n][8],
+// which is how cast_weights_kernel packs them, so that a chunk's weights are one bulk copy.
+// One persistent CTA per SM, its warps split by role: up to eight load halos into two rings of stages, the
+// even and the odd tiles' (cp.async, zero-filled outside the image; a pooled source by registers), one thread
+// copies weights, two warps issue 9 taps x 2 K-steps of tcgen05.mma (kind::f16, BF16 x BF16 -> FP32) per tile
+// and chunk, the even tiles and the odd ones, and commit them to mbarriers, two sets of four warps read finished
+// accumulators (tcgen05.ld, a lane quarter each), add the bias, apply ReLU and store NHWC while the next tiles
+// multiply: the TMEM holds 4 or 8 accumulators. Every product is added in the order chunk, tap, K-step.
+// A layer whose weights fit the weight buffers (two chunks, four at N = 32) keeps them for the whole launch and
+// takes its tiles one by one; a larger one streams them, chunk by chunk, over groups of as many tiles as
+// there are accumulators.
+// What bounds it: an MMA of M = 128, K = 16 reads 4 KB of A from shared memory, 32 cycles, whatever N is, so a
+// tile and chunk takes 576 cycles at least; measured 1300 to 1500 at N = 32, where each role's own instructions
+// (about 130 a tile in the epilogue, 330 a halo in a loader) are what is left, 3 TB/s. One MMA warp instead of
+// two took 1800, one set of epilogue warps 1600, MMAs issued by one divergent lane 2400 (56 cycles each to move
+// their operands to the uniform registers). The 15 layers on a 2064 x 1376 grid (1.02 TFLOP): 3.7 ms as CTAs of
+// one tile that staged, multiplied and stored in turn, 1.55 ms here.
 constexpr int TC_TH = 16, TC_TW = 8;
 constexpr int TC_HP = TC_TH + 2, TC_WP = TC_TW + 2, TC_PIX = TC_HP * TC_WP;  // 18 x 10 halo
 // try_wait polls per wait: far beyond a chunk's MMAs (microseconds); a CTA that meets a set error word
 // (an earlier wait ran out) does nothing
 constexpr unsigned TC_SPIN_LIMIT = 1u << 20;
 
-__host__ __device__ constexpr size_t tc_a_bytes() { return (size_t)4 * TC_PIX * 16; }
-__host__ __device__ constexpr size_t tc_b_bytes(int n) { return (size_t)9 * 4 * n * 16; }
-// A, B, the mbarrier and the TMEM address slot
-__host__ __device__ constexpr size_t tc_smem_bytes(int n) { return tc_a_bytes() + tc_b_bytes(n) + 16; }
+constexpr int TC_PLANE = TC_PIX * 16 + 32;  // bytes of 8 channels of a halo (+32: bank spread of the stores)
+constexpr int TC_STAGE = 4 * TC_PLANE;      // a chunk's halo
+// The warps of a CTA by role. Warp w issues on scheduler w % 4: the two MMA warps (which take the tiles in
+// turn, so that one's waits and commits hide behind the other's MMAs) share theirs with little else.
+constexpr int TC_EW = 4;                                // 0-3, 12-15: the epilogue of the even and the odd tiles, a TMEM lane quarter each
+constexpr int TC_MMA0 = 4, TC_MMA1 = 5, TC_WW = 8;      // the MMAs, the weights
+constexpr int TC_LW = 8;                                // 6, 7, 9-11, 17-19: the loaders
+__device__ __forceinline__ int tc_loader(int w) { return w < 6 || w == 8 || (w > 11 && w < 17) ? -1 : w > 16 ? w - 12 : w - 6 - (w > 8); }
+constexpr int TC_THREADS = 32 * 20;
+__host__ __device__ constexpr int tc_chunk(int n) { return 9 * 4 * n * 16; }
+__host__ __device__ constexpr int tc_wbufs(int n) { return n == 32 ? 4 : 2; }  // weight buffers (chunks)
+// accumulators in TMEM: even, so that each belongs to the even or to the odd tiles (a wait by parity then never
+// meets a phase of the other role's)
+__host__ __device__ constexpr int tc_accs(int n) { return n >= 96 ? 4 : 8; }
+__host__ __device__ constexpr int tc_depth(int n) { return n == 128 ? 6 : n == 96 ? 8 : 12; }  // halos, in two rings
+__host__ __device__ constexpr size_t tc_smem(int n) {
+    return (size_t)tc_wbufs(n) * tc_chunk(n) + tc_depth(n) * TC_STAGE + 8 * (2 * tc_depth(n) + 2 * 4 + 2 * 8 + 2) + 16 + 4 * n;
+}
+static_assert(tc_smem(32) <= 227 * 1024 && tc_smem(64) <= 227 * 1024 && tc_smem(96) <= 227 * 1024 && tc_smem(128) <= 227 * 1024,
+              "shared memory");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // the UMMA shared-memory descriptor, no swizzle (layout type 0), version 1; addresses and offsets in bytes
@@ -230,133 +258,332 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    uint32_t done = 0;
+    for (unsigned it = 0; it < TC_SPIN_LIMIT && !done; it++)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                     : "=r"(done)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// The output channels one CTA takes (N): the largest of 128, 96, 64 and 32 that divides cout.
+__host__ __device__ constexpr int tc_block(int cout) {
+    return cout % 128 == 0 ? 128 : cout % 96 == 0 ? 96 : cout % 64 == 0 ? 64 : cout % 32 == 0 ? 32 : 0;
+}
+// A bounded wait that also gives up once another role of the CTA has. A poll may suspend the warp for up to
+// TC_WAIT_NS, so that waiting warps do not crowd the shared-memory pipe the others work through.
+constexpr unsigned TC_WAIT_NS = 1000;
+__device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t parity, volatile int* abort) {
+    uint32_t done = 0;
+    for (unsigned it = 0; it < TC_SPIN_LIMIT; it++) {
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                     : "=r"(done)
+                     : "r"(bar), "r"(parity), "r"(TC_WAIT_NS)
+                     : "memory");
+        if (done) return true;
+        if (*abort) return false;
+    }
+    *abort = 1;
+    return false;
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+// 32 bytes in one store (whole sectors)
+__device__ __forceinline__ void st32(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+                 "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
+// A CTA's tiles, one gridDim.x apart, walked without divisions.
+struct TileWalk {
+    int b, ty, tx;
+    __device__ __forceinline__ void step(int sb, int sy, int sx, int tiles_y, int tiles_x) {
+        tx += sx;
+        if (tx >= tiles_x) tx -= tiles_x, ty++;
+        ty += sy;
+        if (ty >= tiles_y) ty -= tiles_y, b++;
+        b += sb;
+    }
+};
+
 template <int N>
-__global__ void __launch_bounds__(UN_THREADS) conv3x3_tc_kernel(const ConvArgs a, int* status) {
-    extern __shared__ __align__(128) unsigned char tc_smem[];
-    unsigned char* As = tc_smem;
-    unsigned char* Bs = tc_smem + tc_a_bytes();
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(Bs + tc_b_bytes(N));
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
-    const int tiles_x = (a.W + TC_TW - 1) / TC_TW;
-    const int x0 = (blockIdx.x % tiles_x) * TC_TW, y0 = (blockIdx.x / tiles_x) * TC_TH;
-    const int n0 = blockIdx.y * N, b = blockIdx.z;
+__global__ void __launch_bounds__(TC_THREADS, 1) conv3x3_tc_kernel(const ConvArgs a, int* status) {
+    extern __shared__ __align__(128) unsigned char tc_smem_[];
+    constexpr int NB = tc_wbufs(N), NACC = tc_accs(N), CB = tc_chunk(N), DEPTH = tc_depth(N);
+    unsigned char* Ws = tc_smem_;
+    unsigned char* As = tc_smem_ + NB * CB;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(As + DEPTH * TC_STAGE);
+    constexpr int RING = DEPTH / 2;  // halos of the even tiles, then of the odd ones: one consumer each
+    const uint32_t a_full = smem_u32(bars), a_empty = a_full + 8 * DEPTH, w_full = a_empty + 8 * DEPTH, w_empty = w_full + 32,
+                   d_full = w_empty + 32, d_empty = d_full + 64, fin = d_empty + 64;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2 * DEPTH + 26);
+    volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);
+    float* bs = reinterpret_cast<float*>(bars + 2 * DEPTH + 28);  // the bias
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr uint32_t COLS = N < 32 ? 32 : N;
-    if (*(volatile int*)status) return;  // an earlier CTA's wait ran out: nothing is allocated yet
+    const int tiles_x = (a.W + TC_TW - 1) / TC_TW, tiles_y = (a.H + TC_TH - 1) / TC_TH, ntiles = tiles_x * tiles_y * a.B;
+    const int nloc = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // this CTA's tiles
+    const int n0 = blockIdx.y * N, nch = a.cin / UN_CH;
+    const bool resident = nch <= NB;
+    const int G = resident ? 1 : NACC;
+    if (__syncthreads_or(*(volatile int*)status)) return;  // an earlier CTA's wait ran out: nothing is allocated yet
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(COLS));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(512u));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar)), "r"(1));
+        for (int q = 0; q < DEPTH; q++) mbar_init(a_full + 8 * q, 1), mbar_init(a_empty + 8 * q, 1);
+        for (int q = 0; q < 4; q++) mbar_init(w_full + 8 * q, 1), mbar_init(w_empty + 8 * q, 2);
+        for (int q = 0; q < 8; q++) mbar_init(d_full + 8 * q, 1), mbar_init(d_empty + 8 * q, TC_EW);
+        mbar_init(fin, 1), mbar_init(fin + 8, 1);
+        *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
+    for (int q = tid; q < N; q += TC_THREADS) bs[q] = a.bias ? a.bias[n0 + q] : 0.f;
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = *tslot;
-    const uint32_t a_base = smem_u32(As), b_base = smem_u32(Bs);
-    constexpr uint32_t IDESC = umma_idesc_bf16(N);
-    bool ok = true;
-    int chunk = 0;
-    for (int c0 = 0; c0 < a.cin; c0 += UN_CH, chunk++) {
-        const bool first = c0 < a.c1;
-        const __nv_bfloat16* src = first ? a.src1 : a.src2;
-        const int cs = first ? a.c1s : a.c2s, mode = first ? a.mode1 : a.mode2, cb = first ? c0 : c0 - a.c1;
-        // the halo: [k8][pixel][8 channels], zero outside the image
-        for (int i = tid; i < TC_PIX * 4; i += UN_THREADS) {
-            const int pix = i >> 2, v = i & 3;
-            const int yy = y0 - 1 + pix / TC_WP, xx = x0 - 1 + pix % TC_WP;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (yy >= 0 && yy < a.H && xx >= 0 && xx < a.W) val = load8(src, cs, mode, b, yy, xx, a.H, a.W, cb + 8 * v);
-            *reinterpret_cast<uint4*>(As + ((size_t)v * TC_PIX + pix) * 16) = val;
-        }
-        // the weights: [tap][k8][n][8]
-        for (int i = tid; i < 9 * N * 4; i += UN_THREADS) {
-            const int v = i & 3, row = i >> 2, tap = row / N, n = row % N;
-            const uint4 val = *reinterpret_cast<const uint4*>(a.w + ((size_t)tap * a.cout + n0 + n) * a.cin + c0 + 8 * v);
-            *reinterpret_cast<uint4*>(Bs + (((size_t)tap * 4 + v) * N + n) * 16) = val;
-        }
-        // the generic-proxy stores, visible to the tensor cores' async proxy
-        asm volatile("fence.proxy.async.shared::cta;");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll 1
-            for (int tap = 0; tap < 9; tap++) {
-                const int ky = tap / 3, kx = tap % 3;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tslot, 0);
+    const int sx = (int)gridDim.x % tiles_x, sy = (int)gridDim.x / tiles_x % tiles_y, sb = (int)gridDim.x / (tiles_x * tiles_y);
+    TileWalk at{(int)blockIdx.x / (tiles_x * tiles_y), (int)blockIdx.x / tiles_x % tiles_y, (int)blockIdx.x % tiles_x};
+    if (const int lw = tc_loader(warp); lw >= 0) {
+        // ---- the loaders, half of them for each ring (the even and the odd tiles): a warp takes every LW-th halo of
+        // its ring, 180 pixels x 4 vectors of 8 channels: lane l the vector l % 4 of the pixels l / 4, l / 4 + 8, ...
+        constexpr int Q = (TC_PIX + 7) / 8;
+        // a warp waits for its slot by parity, having last seen the halo LW + RING back consumed: with LW > RING
+        // the slot could be two phases behind, which a parity cannot tell from free
+        constexpr int LW = TC_LW / 2 < RING ? TC_LW / 2 : RING;
+        static_assert(LW <= RING, "a loader warp's stride");
+        const int ring = lw & 1;
+        const int v = lane & 3, pix0 = lane >> 2;
+        int seq = 0, held = -1;
+        bool ok = lw / 2 < LW;
+        auto hand_over = [&]() {  // the copies into slot `held` are done: visible to the tensor cores, then full
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(a_full + 8 * held);
+        };
+        for (int k0 = 0; k0 < nloc && ok; k0 += G) {
+            const int gn = min(G, nloc - k0);
+            TileWalk t = at;
+            for (int ch = 0; ch < nch && ok; ch++) {
+                const int c0 = ch * UN_CH;
+                const bool first = c0 < a.c1;
+                const int cs = first ? a.c1s : a.c2s, mode = first ? a.mode1 : a.mode2;
+                const int up = mode == SRC_UP ? 1 : 0, hs = a.H >> up, ws = a.W >> up;
+                const __nv_bfloat16* src = (first ? a.src1 : a.src2) + (first ? c0 : c0 - a.c1) + 8 * v;
+                t = at;
+                for (int g = 0; g < gn; g++, t.step(sb, sy, sx, tiles_y, tiles_x)) {
+                    if (((k0 + g) & 1) != ring) continue;
+                    const int mine = seq++;  // this halo's place in its ring's order
+                    if (mine % LW != lw / 2) continue;
+                    const int st = ring * RING + mine % RING;
+                    if (held >= 0) {
+                        asm volatile("cp.async.wait_group 0;" ::: "memory");
+                        hand_over();
+                    }
+                    if (mine >= RING) ok = mbar_wait_or(a_empty + 8 * st, (uint32_t)((mine / RING - 1) & 1), abort);
+                    ok = __all_sync(0xffffffffu, ok);
+                    held = -1;
+                    if (!ok) break;
+                    unsigned char* S = As + st * TC_STAGE + v * TC_PLANE + pix0 * 16;
+                    const int yb = t.ty * TC_TH - 1, xb = t.tx * TC_TW - 1;
+                    int c = pix0, y = yb;  // pixel pix0 of the halo: row 0, column pix0 (pix0 < 8 < TC_WP)
+                    if (mode == SRC_POOL) {
+#pragma unroll 4
+                        for (int q = 0; q < Q; q++) {
+                            const int x = xb + c;
+                            uint4 val = make_uint4(0u, 0u, 0u, 0u);
+                            if ((unsigned)y < (unsigned)a.H && (unsigned)x < (unsigned)a.W) val = load8(src, cs, SRC_POOL, t.b, y, x, a.H, a.W, 0);
+                            if (8 * q + pix0 < TC_PIX) *reinterpret_cast<uint4*>(S + q * 128) = val;
+                            c += 8;
+                            if (c >= TC_WP) c -= TC_WP, y++;
+                        }
+                    } else {
+                        const __nv_bfloat16* img = src + (size_t)t.b * hs * ws * cs;
+                        const uint32_t d0 = smem_u32(S);
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const uint64_t da = umma_desc(a_base + (uint32_t)((2 * j * TC_PIX + ky * TC_WP + kx) * 16), TC_PIX * 16, TC_WP * 16);
-                    const uint64_t db = umma_desc(b_base + (uint32_t)(((tap * 4 + 2 * j) * N) * 16), N * 16, 8 * 16);
-                    const uint32_t acc = (chunk > 0 || tap > 0 || j > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-                        "l"(da), "l"(db), "r"(IDESC), "r"(acc));
+                        for (int q = 0; q < Q; q++) {
+                            const int x = xb + c;
+                            const bool in = (unsigned)y < (unsigned)a.H && (unsigned)x < (unsigned)a.W;
+                            const __nv_bfloat16* p = in ? img + ((size_t)(y >> up) * ws + (x >> up)) * cs : src;
+                            if (8 * q + pix0 < TC_PIX)
+                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d0 + q * 128), "l"(p), "r"(in ? 16 : 0)
+                                             : "memory");
+                            c += 8;
+                            if (c >= TC_WP) c -= TC_WP, y++;
+                        }
+                    }
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                    held = st;
                 }
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar)) : "memory");
+            at = t;
         }
-        // every thread: the chunk's MMAs are done (their shared-memory reads too) before the next staging
-        uint32_t done = 0;
-        for (unsigned it = 0; it < TC_SPIN_LIMIT && !done; it++)
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                         : "=r"(done)
-                         : "r"(smem_u32(mbar)), "r"((uint32_t)(chunk & 1)));
-        if (!done) {
-            ok = false;
-            break;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (ok && held >= 0) hand_over();
+    } else if (warp == TC_WW) {
+        // ---- the weights: one bulk copy per chunk; the resident ones once
+        if (lane == 0) {
+            const unsigned char* wp = reinterpret_cast<const unsigned char*>(a.wp) + (size_t)blockIdx.y * nch * CB;
+            const int total = resident ? nch : nch * ((nloc + G - 1) / G);
+            int seq = 0;
+            for (; seq < total; seq++) {
+                const int buf = seq % NB;
+                if (seq >= NB && !mbar_wait_or(w_empty + 8 * buf, (uint32_t)((seq / NB - 1) & 1), abort)) break;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(w_full + 8 * buf), "r"(CB) : "memory");
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 smem_u32(Ws + buf * CB)),
+                             "l"(wp + (size_t)(seq % nch) * CB), "r"(CB), "r"(w_full + 8 * buf)
+                             : "memory");
+            }
+            for (int q = max(0, seq - NB); q < seq; q++) mbar_wait(w_full + 8 * (q % NB), (uint32_t)((q / NB) & 1));  // none left in flight
         }
-    }
-    if (!ok) {
-        // the wait ran out: flag it, give the MMAs in flight a second bounded wait, free the TMEM, return
-        if (tid == 0) atomicOr(status, 0x100);
-        uint32_t done = 0;
-        for (unsigned it = 0; it < TC_SPIN_LIMIT && !done; it++)
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                         : "=r"(done)
-                         : "r"(smem_u32(mbar)), "r"((uint32_t)(chunk & 1)));
-    } else {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        // epilogue: pixel m = 32 warp + lane = (row m / 8, column m % 8); 8 channels per load
-        const int m = 32 * warp + lane, y = y0 + m / TC_TW, x = x0 + m % TC_TW;
-        const bool in = y < a.H && x < a.W;
-        const size_t pix = ((size_t)b * a.H + y) * a.W + x;
+    } else if (warp == TC_MMA0 || warp == TC_MMA1) {
+        // ---- the MMAs: 9 taps x 2 K-steps per tile and chunk. The whole warp walks the loop, so that descriptors
+        // and addresses stay warp-uniform (issued from one divergent lane, every operand of every MMA is moved
+        // to the uniform registers by itself: 56 cycles an MMA); one elected lane issues.
+        constexpr uint32_t IDESC = umma_idesc_bf16(N);
+        const bool leader = elect_one();
+        const uint64_t da0 = umma_desc(smem_u32(As), TC_PLANE, TC_WP * 16), db0 = umma_desc(smem_u32(Ws), N * 16, 8 * 16);
+        int st = 0, buf = 0;
+        const int mw = warp - TC_MMA0;
+        uint32_t aph = 0, wph = 0;
+        bool ok = true;
+        for (int k0 = 0; k0 < nloc && ok; k0 += G) {
+            const int gn = min(G, nloc - k0);
+            for (int ch = 0; ch < nch && ok; ch++) {
+                if (resident) buf = ch;
+                if (!resident || k0 == 0) ok = mbar_wait_or(w_full + 8 * buf, wph, abort);
+                const uint64_t dbc = db0 + (uint32_t)(buf * (CB >> 4));
+                for (int g = 0; g < gn && ok; g++) {
+                    const int k = k0 + g, acc = k % NACC;
+                    if ((k & 1) != mw) continue;  // the other MMA warp's tile
+                    if (ch == 0 && k >= NACC) ok = mbar_wait_or(d_empty + 8 * acc, (uint32_t)((k / NACC - 1) & 1), abort);
+                    const int slot = mw * RING + st;
+                    ok = ok && mbar_wait_or(a_full + 8 * slot, aph, abort);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;");
+                    const uint64_t dac = da0 + (uint32_t)(slot * (TC_STAGE >> 4));
+                    const uint32_t d = tmem + acc * N;
+                    if (leader) {
+#pragma unroll
+                        for (int tap = 0; tap < 9; tap++)
+#pragma unroll
+                            for (int j = 0; j < 2; j++)
+                                umma_bf16(d, dac + ((2 * j * TC_PLANE) >> 4) + (tap / 3) * TC_WP + tap % 3, dbc + (tap * 4 + 2 * j) * N, IDESC,
+                                          (tap > 0 || j > 0) ? 1u : ch > 0);
+                        umma_commit(a_empty + 8 * slot);
+                        if (ch == nch - 1) umma_commit(d_full + 8 * acc);
+                    }
+                    __syncwarp();
+                    if (++st == RING) st = 0, aph ^= 1;
+                }
+                if (!resident) {  // this warp's MMAs on the chunk's weights, if any
+                    if (ok && leader) umma_commit(w_empty + 8 * buf);
+                    if (++buf == NB) buf = 0, wph ^= 1;
+                }
+            }
+        }
+        if (!ok) {  // the MMAs in flight get a bounded wait before the TMEM goes
+            if (leader) umma_commit(fin + 8 * mw);
+            __syncwarp();
+            mbar_wait(fin + 8 * mw, 0);
+        }
+    } else if (warp < TC_EW || (warp >= 12 && warp < 16)) {
+        // ---- the epilogue: pixel m = 32 quarter + lane = (row m / 8, column m % 8)
+        const int quarter = warp & 3, m = 32 * quarter + lane, set = warp >= 12;
+        bool ok = true;
+        for (int k = 0; k < nloc && ok; k++, at.step(sb, sy, sx, tiles_y, tiles_x)) {
+            if ((k & 1) != set) continue;
+            const int acc = k % NACC;
+            ok = __all_sync(0xffffffffu, mbar_wait_or(d_full + 8 * acc, (uint32_t)((k / NACC) & 1), abort));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const int y = at.ty * TC_TH + m / TC_TW, x = at.tx * TC_TW + m % TC_TW;
+            const bool in = y < a.H && x < a.W;
+            const size_t pix = ((size_t)at.b * a.H + y) * a.W + x;
 #pragma unroll 1
-        for (int c = 0; c < N; c += 8) {
-            uint32_t r[8];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                         : "r"(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c));
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
-            if (!in) continue;
-            float v[8];
+            for (int c = 0; c < N; c += 32) {
+                uint32_t r[32];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+                    "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                      "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+                      "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+                      "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                    : "r"(tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(acc * N + c)));
+                asm volatile("tcgen05.wait::ld.sync.aligned;");
+                if (c + 32 == N) {  // the accumulator is read: the next tile may take it
+                    asm volatile("tcgen05.fence::before_thread_sync;");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(d_empty + 8 * acc);
+                }
+                if (!in) continue;
+                const int n = n0 + c;
+                if (a.bias) {
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                v[q] = __uint_as_float(r[q]);
-                if (a.bias) v[q] += a.bias[n0 + c + q];
-                if (a.relu) v[q] = fmaxf(v[q], 0.f);
-            }
-            const int n = n0 + c;
-            if (a.out) {
-                uint4 o;
-                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
+                    for (int q = 0; q < 32; q += 4) {
+                        const float4 b4 = *reinterpret_cast<const float4*>(bs + c + q);
+                        r[q] = __float_as_uint(__uint_as_float(r[q]) + b4.x);
+                        r[q + 1] = __float_as_uint(__uint_as_float(r[q + 1]) + b4.y);
+                        r[q + 2] = __float_as_uint(__uint_as_float(r[q + 2]) + b4.z);
+                        r[q + 3] = __float_as_uint(__uint_as_float(r[q + 3]) + b4.w);
+                    }
+                }
+                if (a.relu) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-                *reinterpret_cast<uint4*>(a.out + pix * a.cout + n) = o;
+                    for (int q = 0; q < 32; q++) r[q] = __float_as_uint(fmaxf(__uint_as_float(r[q]), 0.f));
+                }
+                if (a.out_c0 && n == 0) a.out_c0[pix] = __uint_as_float(r[0]);
+                if (a.out) {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        uint32_t o[8];
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+                            o[q] = bf2_as_u32(__floats2bfloat162_rn(__uint_as_float(r[16 * h + 2 * q]), __uint_as_float(r[16 * h + 2 * q + 1])));
+                        st32(a.out + pix * a.cout + n + 16 * h, o);
+                    }
+                }
+                if (a.out_f32) {
+#pragma unroll
+                    for (int h = 0; h < 4; h++) {
+                        uint32_t o[8];
+#pragma unroll
+                        for (int q = 0; q < 8; q++) o[q] = r[8 * h + q];
+                        st32(a.out_f32 + pix * a.cout + n + 8 * h, o);
+                    }
+                }
             }
-            if (a.out_f32) {
-                float4* o = reinterpret_cast<float4*>(a.out_f32 + pix * a.cout + n);
-                o[0] = make_float4(v[0], v[1], v[2], v[3]);
-                o[1] = make_float4(v[4], v[5], v[6], v[7]);
-            }
-            if (a.out_c0 && n == 0) a.out_c0[pix] = v[0];
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS));
+    if (tid == 0 && *abort) atomicOr(status, 0x100);  // a wait ran out: the output is not whole
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
 // ------------------------------------------------------------ backward parts
@@ -426,22 +653,6 @@ static_assert(dw_stage(32) >= 16 * dw_zplane(32) && dw_stage(64) >= 16 * dw_zpla
               "A's planes stay inside the stage");
 constexpr uint32_t DW_COLS = 512, DW_DB_COL = 288;
 
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    uint32_t done = 0;
-    for (unsigned it = 0; it < TC_SPIN_LIMIT && !done; it++)
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                     : "=r"(done)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-    return done != 0;
-}
-__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
-}
 __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
     asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
@@ -593,14 +804,22 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ gw,
         w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     }
 }
+// The tcgen05 path's packing of a [tap][n][c] weight: [n / N][c / 32][tap][c % 32 / 8][n % N][c % 8], N = tc_block(nn).
+__device__ __forceinline__ size_t pack_at(int tap, int n, int c, int nn, int cc) {
+    const int N = tc_block(nn);
+    return ((((size_t)(n / N) * (cc / 32) + c / 32) * 9 + tap) * 4 + c % 32 / 8) * N * 8 + (size_t)(n % N) * 8 + c % 8;
+}
+// wb = w, wt its flipped transpose for dX, and both packed (wp, wtp)
 __global__ void cast_weights_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wt,
-                                    int cout, int cin) {
+                                    __nv_bfloat16* __restrict__ wp, __nv_bfloat16* __restrict__ wtp, int cout, int cin) {
     const size_t n = (size_t)9 * cout * cin;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int ci = (int)(i % cin), co = (int)((i / cin) % cout), tap = (int)(i / ((size_t)cin * cout));
         const __nv_bfloat16 v = __float2bfloat16_rn(w[i]);
         wb[i] = v;
         wt[((size_t)(8 - tap) * cin + ci) * cout + co] = v;
+        wp[pack_at(tap, co, ci, cout, cin)] = v;
+        wtp[pack_at(8 - tap, ci, co, cin, cout)] = v;
     }
 }
 
@@ -713,7 +932,7 @@ struct lsb_unet {
     float *b = nullptr, *gb = nullptr, *mb = nullptr, *vb = nullptr;
     unsigned char* wmask = nullptr;  // trainable weights (the output layer keeps channels 1.. at zero)
     unsigned char* bmask = nullptr;
-    __nv_bfloat16 *wb = nullptr, *wt = nullptr;
+    __nv_bfloat16 *wb = nullptr, *wt = nullptr, *wp = nullptr, *wtp = nullptr;
     int step = 0;
     // activations for the current shape
     int B = 0, H = 0, W = 0;
@@ -801,22 +1020,22 @@ static cudaError_t ensure_shape(lsb_unet* u, int B, int H, int W, bool train) {
 
 template <int N>
 static cudaError_t conv_tc_launch(const ConvArgs& a, int* status, cudaStream_t s) {
-    const size_t smem = tc_smem_bytes(N);
-    cudaError_t e = cudaFuncSetAttribute(conv3x3_tc_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(conv3x3_tc_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem(N));
     if (e != cudaSuccess) return e;
-    const dim3 grid(((a.W + TC_TW - 1) / TC_TW) * ((a.H + TC_TH - 1) / TC_TH), a.cout / N, a.B);
-    lsb_launched(), conv3x3_tc_kernel<N><<<grid, UN_THREADS, smem, s>>>(a, status);
+    const int ntiles = ((a.W + TC_TW - 1) / TC_TW) * ((a.H + TC_TH - 1) / TC_TH) * a.B, nblk = a.cout / N;
+    const dim3 grid(std::min(ntiles, std::max(1, 148 / nblk)), nblk);
+    lsb_launched(), conv3x3_tc_kernel<N><<<grid, TC_THREADS, tc_smem(N), s>>>(a, status);
     return cudaGetLastError();
 }
 
 static cudaError_t conv_launch(const ConvArgs& a, cudaStream_t s, int* status = nullptr, bool tc = false) {
-    // tcgen05: every layer's cin is a multiple of 32 and its cout 32, 64, 128 or 256 (one CTA takes them all)
-    if (tc && status && a.cin % UN_CH == 0) {
-        switch (a.cout) {
+    // tcgen05: every layer's cin is a multiple of 32 and its cout a multiple of one of the kernel's N
+    if (tc && status && a.wp && a.cin % UN_CH == 0) {
+        switch (tc_block(a.cout)) {
             case 32: return conv_tc_launch<32>(a, status, s);
             case 64: return conv_tc_launch<64>(a, status, s);
+            case 96: return conv_tc_launch<96>(a, status, s);
             case 128: return conv_tc_launch<128>(a, status, s);
-            case 256: return conv_tc_launch<256>(a, status, s);
             default: break;
         }
     }
@@ -863,6 +1082,7 @@ static ConvArgs layer_args(const lsb_unet* u, int i) {
     a.cin = l.c1 + l.c2;
     a.cout = l.cout;
     a.w = u->wb + l.woff;
+    a.wp = u->wp + l.woff;
     a.bias = u->b + l.boff;
     a.relu = l.relu;
     a.B = u->B;
@@ -886,8 +1106,9 @@ static cudaError_t unet_forward(lsb_unet* u) {
 
 static cudaError_t cast_all(lsb_unet* u) {
     for (auto& l : u->layers) {
-        lsb_launched(), cast_weights_kernel<<<ugrid((size_t)9 * l.cout * (l.c1 + l.c2)), 256, 0, u->s>>>(u->w + l.woff, u->wb + l.woff,
-                                                                                                      u->wt + l.woff, l.cout, l.c1 + l.c2);
+        lsb_launched(), cast_weights_kernel<<<ugrid((size_t)9 * l.cout * (l.c1 + l.c2)), 256, 0, u->s>>>(u->w + l.woff, u->wb + l.woff, u->wt + l.woff,
+                                                                                                      u->wp + l.woff, u->wtp + l.woff, l.cout,
+                                                                                                      l.c1 + l.c2);
     }
     return cudaGetLastError();
 }
@@ -933,6 +1154,7 @@ extern "C" char* lsb_unet_create(int32_t device, uint64_t seed, lsb_unet** out) 
               alloc((void**)&u->vw, u->nw * 4) && alloc((void**)&u->b, u->nb * 4) && alloc((void**)&u->gb, u->nb * 4) &&
               alloc((void**)&u->mb, u->nb * 4) && alloc((void**)&u->vb, u->nb * 4) && alloc((void**)&u->wmask, u->nw) &&
               alloc((void**)&u->bmask, u->nb) && alloc((void**)&u->wb, u->nw * 2) && alloc((void**)&u->wt, u->nw * 2) &&
+              alloc((void**)&u->wp, u->nw * 2) && alloc((void**)&u->wtp, u->nw * 2) &&
               alloc((void**)&u->loss, 8) && alloc((void**)&u->status, 4) &&
               cudaHostAlloc((void**)&u->loss_host, 8, cudaHostAllocDefault) == cudaSuccess &&
               cudaStreamCreateWithFlags(&u->s, cudaStreamNonBlocking) == cudaSuccess;
@@ -959,7 +1181,7 @@ extern "C" void lsb_unet_destroy(lsb_unet* u) {
     if (u->s) cudaStreamSynchronize(u->s);
     free_shape(u);
     for (void* p : {(void*)u->w, (void*)u->gw, (void*)u->mw, (void*)u->vw, (void*)u->b, (void*)u->gb, (void*)u->mb, (void*)u->vb,
-                    (void*)u->wmask, (void*)u->bmask, (void*)u->wb, (void*)u->wt, (void*)u->loss, (void*)u->status})
+                    (void*)u->wmask, (void*)u->bmask, (void*)u->wb, (void*)u->wt, (void*)u->wp, (void*)u->wtp, (void*)u->loss, (void*)u->status})
         if (p) cudaFree(p);
     if (u->loss_host) cudaFreeHost(u->loss_host);
     for (cudaEvent_t v : u->fev)
@@ -1066,6 +1288,7 @@ static cudaError_t unet_backward(lsb_unet* u) {
         d.cin = l.cout;
         d.cout = cin;
         d.w = u->wt + l.woff;
+        d.wp = u->wtp + l.woff;
         d.out_f32 = u->dxbuf;
         d.B = a.B;
         d.H = a.H;

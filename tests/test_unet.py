@@ -177,6 +177,31 @@ def test_weight_gradient_sums_are_the_products_over_all_pixels(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 8, 8), (3, 40, 56), (1, 512, 512)])
+def test_tcgen05_pipeline_gives_the_mma_sync_values_on_exact_sums(shape):
+    """On _exact_case every convolution sum is exact in any order, so the pipelined tcgen05 kernel and the mma.sync
+    one agree bit for bit: from one tile a CTA to so many that every ring of stages, weight buffers and
+    accumulators is used again. With B H W a power of two the gradients' operands agree too, and the sums of
+    equal per-CTA parts differ by the order of at most 148 additions."""
+    import lapstack_b200 as L
+    B, H, W = shape
+    w, b, inp, d_in, tgt = _exact_case(B, H, W)
+    outs, grads = {}, {}
+    for path in ("tcgen05", "mma.sync"):
+        net = L.UNet(seed=0)
+        net.set_conv(path)
+        net.set_params(w, b)
+        t = _to_gpu(inp, d_in, tgt)
+        outs[path] = net.forward(*t[:2]).cpu().numpy()
+        net.train_step(*t, lr=0.0)
+        grads[path] = net.grads()[0]
+        net.close()
+    assert np.array_equal(outs["tcgen05"], outs["mma.sync"]) and outs["tcgen05"].max() > 0
+    if (B * H * W) & (B * H * W - 1) == 0:
+        assert np.all(np.abs(grads["tcgen05"] - grads["mma.sync"]) <= 2 * 148 * 2.0 ** -24 * grads["mma.sync"])
+
+
+@pytest.mark.gpu
 def test_training_fits_a_fixed_batch():
     """Adam on the library's gradients learns a correction that depends on the guide channel."""
     import lapstack_b200 as L
