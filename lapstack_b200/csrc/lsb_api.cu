@@ -13,10 +13,13 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <list>
 #include <map>
+#include <functional>
 #include <future>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -55,17 +58,19 @@ static std::string fmt(const char* f, ...) {
 
 struct DevPool {
     std::vector<void*> ptrs;
+    size_t bytes = 0;
     template <class T>
     cudaError_t get(T** p, size_t n) {
         void* q = nullptr;
         cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
-        if (e == cudaSuccess) ptrs.push_back(q);
+        if (e == cudaSuccess) ptrs.push_back(q), bytes += std::max<size_t>(n, 1) * sizeof(T);
         *p = (T*)q;
         return e;
     }
     void release() {
         for (void* p : ptrs) cudaFree(p);
         ptrs.clear();
+        bytes = 0;
     }
     ~DevPool() { release(); }
 };
@@ -76,6 +81,57 @@ constexpr int BRIGHT_PARTS = 512;
 constexpr int SEL_CHUNK = 10;
 // Frames of the last selection chunk (it folds after the last frame lands).
 constexpr int SEL_TAIL = 4;
+
+// Page-locked staging for copies between device memory and pageable host arrays: STAGE_BUFS buffers in turn, filled
+// or emptied by several host threads while the link moves the others. A pageable cudaMemcpyAsync goes through one
+// driver thread's copy: 11 GB/s, 2 to 5 GB/s into memory not yet touched (three planes of 12 Mpx in and one out:
+// 23 ms); through these buffers, see host_in and host_out.
+constexpr int STAGE_BUFS = 4;
+constexpr size_t STAGE_BYTES = (size_t)4 << 20;
+struct HostStage {
+    std::mutex mu;
+    char* buf[STAGE_BUFS] = {};
+    cudaEvent_t ev[STAGE_BUFS] = {};
+    int next = 0;
+    cudaError_t ready() {
+        for (int i = 0; i < STAGE_BUFS; i++) {
+            if (!buf[i]) {
+                cudaError_t e = cudaHostAlloc((void**)&buf[i], STAGE_BYTES, cudaHostAllocDefault);
+                if (e != cudaSuccess) return buf[i] = nullptr, cudaGetLastError(), e;
+            }
+            if (!ev[i]) {
+                cudaError_t e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+                if (e != cudaSuccess) return ev[i] = nullptr, e;
+            }
+        }
+        return cudaSuccess;
+    }
+    void release() {
+        for (int i = 0; i < STAGE_BUFS; i++) {
+            if (ev[i]) cudaEventDestroy(ev[i]), ev[i] = nullptr;
+            if (buf[i]) cudaFreeHost(buf[i]), buf[i] = nullptr;
+        }
+    }
+    ~HostStage() { release(); }
+};
+
+// What a standalone call (a WLS solve, a depth pass over given slices, a registered pair) works in, kept by the engine
+// for the next call of the same kind and size: allocating and freeing it (and the solver's captured graphs) cost
+// 25 to 40 ms a call, the solve of a 3 Mpx grid 6. A call takes its entry out of the list while it runs, so that no two
+// calls share one; the engine keeps at most SOLO_MAX entries and SOLO_BYTES, newest first, and frees all of them when
+// an allocation fails and when it is destroyed.
+struct Solo {
+    int kind = 0;
+    uint32_t key[4] = {};
+    DevPool pool;
+    WlsSolver* ws = nullptr;
+    lsb_stack* st = nullptr;  // a depth-only stack
+    std::vector<float*> planes;
+    size_t bytes() const;
+    ~Solo();
+};
+enum { SOLO_WLS = 1, SOLO_DEPTH = 2, SOLO_PAIR = 3 };
+constexpr size_t SOLO_MAX = 8, SOLO_BYTES = (size_t)4 << 30;
 
 struct lsb_engine {
     lsb_config cfg;
@@ -93,6 +149,9 @@ struct lsb_engine {
     float* scal;  // [floor, p90, max, ...]
     AlignCtx actx;
     cudaEvent_t ev[12];
+    HostStage stage;
+    std::mutex solo_mu;
+    std::list<Solo*> solos;  // idle workspaces, newest first
     void log(const std::string& line) {
         if (cfg.log) cfg.log(line.c_str(), cfg.user);
     }
@@ -218,6 +277,138 @@ struct lsb_stack {
     }
 };
 
+Solo::~Solo() {
+    wls_destroy(ws);
+    delete st;
+}
+size_t Solo::bytes() const { return pool.bytes + wls_bytes(ws) + (st ? st->pool.bytes + wls_bytes(st->ws) : 0); }
+
+static void solo_flush(lsb_engine* e) {
+    std::list<Solo*> all;
+    {
+        std::lock_guard<std::mutex> lk(e->solo_mu);
+        all.swap(e->solos);
+    }
+    for (Solo* s : all) delete s;
+}
+// The workspace of one call, out of the engine's list (or a new one: fresh) and back into it when the call is done.
+struct SoloHold {
+    lsb_engine* e;
+    Solo* s = nullptr;
+    bool fresh = false, keep = false;
+    SoloHold(lsb_engine* e_, int kind, uint32_t a, uint32_t b, uint32_t c = 0, uint32_t d = 0) : e(e_) {
+        const uint32_t key[4] = {a, b, c, d};
+        {
+            std::lock_guard<std::mutex> lk(e->solo_mu);
+            for (auto it = e->solos.begin(); it != e->solos.end(); ++it)
+                if ((*it)->kind == kind && !memcmp((*it)->key, key, sizeof key)) {
+                    s = *it;
+                    e->solos.erase(it);
+                    break;
+                }
+        }
+        if (s) return;
+        fresh = true;
+        s = new Solo();
+        s->kind = kind;
+        memcpy(s->key, key, sizeof key);
+    }
+    ~SoloHold() {
+        if (!keep) {  // an error on the way: nothing of it is kept
+            cudaStreamSynchronize(e->s);
+            cudaGetLastError();
+            delete s;
+            return;
+        }
+        std::vector<Solo*> out;
+        {
+            std::lock_guard<std::mutex> lk(e->solo_mu);
+            e->solos.push_front(s);
+            size_t sum = 0, n = 0;
+            for (auto it = e->solos.begin(); it != e->solos.end();) {
+                sum += (*it)->bytes();
+                if (++n > SOLO_MAX || sum > SOLO_BYTES) out.push_back(*it), it = e->solos.erase(it);
+                else ++it;
+            }
+        }
+        for (Solo* q : out) delete q;
+    }
+};
+// f(), and once more without the idle workspaces if the device has no room for it beside them.
+template <class F>
+static cudaError_t with_room(lsb_engine* e, F f) {
+    cudaError_t r = f();
+    if (r != cudaErrorMemoryAllocation) return r;
+    cudaGetLastError();
+    solo_flush(e);
+    return f();
+}
+
+static bool pageable(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+static void copy_threads(char* dst, const char* src, size_t bytes) {
+    constexpr size_t PIECE = (size_t)512 << 10;
+    const long n = (long)((bytes + PIECE - 1) / PIECE);
+    static const int workers = std::max(1, std::min(8, (int)std::thread::hardware_concurrency()));
+#pragma omp parallel for num_threads(workers) schedule(static) if (n > 1)
+    for (long i = 0; i < n; i++) memcpy(dst + i * PIECE, src + i * PIECE, std::min(PIECE, bytes - (size_t)i * PIECE));
+}
+// Host -> device on st; src may be reused on return when it is pageable, as with cudaMemcpyAsync. From 1 MB on, a
+// pageable source goes through the staging buffers (below that the driver's own copy is as fast).
+static cudaError_t host_in(lsb_engine* e, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    if (bytes < ((size_t)1 << 20) || !pageable(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    std::lock_guard<std::mutex> lk(e->stage.mu);
+    if (e->stage.ready() != cudaSuccess) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    for (size_t at = 0; at < bytes; at += STAGE_BYTES) {
+        const size_t n = std::min(STAGE_BYTES, bytes - at);
+        const int b = e->stage.next;
+        e->stage.next = (b + 1) % STAGE_BUFS;
+        cudaError_t r = cudaEventSynchronize(e->stage.ev[b]);  // the copy that last read this buffer
+        if (r != cudaSuccess) return r;
+        copy_threads(e->stage.buf[b], (const char*)src + at, n);
+        r = cudaMemcpyAsync((char*)dst + at, e->stage.buf[b], n, cudaMemcpyHostToDevice, st);
+        if (r == cudaSuccess) r = cudaEventRecord(e->stage.ev[b], st);
+        if (r != cudaSuccess) return r;
+    }
+    return cudaSuccess;
+}
+// Device -> host behind the work on st; a pageable dst of 1 MB or more is written when it returns.
+static cudaError_t host_out(lsb_engine* e, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    if (bytes < ((size_t)1 << 20) || !pageable(dst)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    std::lock_guard<std::mutex> lk(e->stage.mu);
+    if (e->stage.ready() != cudaSuccess) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    size_t sent = 0, done = 0;
+    int order[STAGE_BUFS], head = 0, flying = 0;
+    while (done < bytes) {
+        while (sent < bytes && flying < STAGE_BUFS) {
+            const size_t n = std::min(STAGE_BYTES, bytes - sent);
+            const int b = e->stage.next;
+            e->stage.next = (b + 1) % STAGE_BUFS;
+            cudaError_t r = cudaEventSynchronize(e->stage.ev[b]);
+            if (r == cudaSuccess) r = cudaMemcpyAsync(e->stage.buf[b], (const char*)src + sent, n, cudaMemcpyDeviceToHost, st);
+            if (r == cudaSuccess) r = cudaEventRecord(e->stage.ev[b], st);
+            if (r != cudaSuccess) return cudaStreamSynchronize(st), r;
+            order[(head + flying++) % STAGE_BUFS] = b;
+            sent += n;
+        }
+        const int b = order[head];
+        const size_t n = std::min(STAGE_BYTES, bytes - done);
+        cudaError_t r = cudaEventSynchronize(e->stage.ev[b]);
+        if (r != cudaSuccess) return cudaStreamSynchronize(st), r;
+        copy_threads((char*)dst + done, e->stage.buf[b], n);
+        done += n;
+        head = (head + 1) % STAGE_BUFS;
+        flying--;
+    }
+    return cudaSuccess;
+}
+
 namespace lsb {
 cudaError_t unet_warm_start(lsb_unet* u, const float* guide, const float* d, const float* conf, int dw, int dh, float dmax, float* x0,
                             cudaStream_t st);
@@ -332,6 +523,7 @@ void lsb_engine_destroy(lsb_engine* e) {
     for (auto& v : e->ev)
         if (v) cudaEventDestroy(v);
     if (e->actx.sums_host) cudaFreeHost(e->actx.sums_host);
+    solo_flush(e);
     e->pool.release();
     if (e->cs) cudaStreamSynchronize(e->cs), cudaStreamDestroy(e->cs);
     if (e->s_mark) cudaEventDestroy(e->s_mark);
@@ -371,9 +563,13 @@ static std::vector<float> focus_taps(uint32_t r_in, uint32_t r_out) {
     return out;
 }
 
-static char* stack_alloc(lsb_stack* s) {
+// Every buffer of a stack; depth_only: what the depth pass over given slices needs of them.
+static char* stack_alloc(lsb_stack* s, bool depth_only) {
     DevPool& P = s->pool;
     const size_t W = s->w, H = s->h, N = s->n;
+    if (depth_only) {
+        TRY(P.get(&s->img, 3 * W * H));
+    } else {
     // fold inputs carry 64 bytes of tail padding: the async tile copies read whole words
     TRY(P.get(&s->frames, N * W * H * 3 + 32));
     s->g.assign(s->levels + 1, nullptr);
@@ -406,14 +602,14 @@ static char* stack_alloc(lsb_stack* s) {
     s->gsel_floats = (size_t)16 << 20;  // 64 MB: the small levels' frame-group states
     TRY(P.get(&s->gsel, s->gsel_floats));
     TRY(P.get(&s->xf_dev, N));
+    }
     if (s->dp.enabled) {
         s->bk = 1 << s->dp.scale;
         s->dw = (int)((W + s->bk - 1) / s->bk);
         s->dh = (int)((H + s->bk - 1) / s->bk);
         const size_t m = (size_t)s->dw * s->dh;
-        void* p = nullptr;
-        TRY(cudaMalloc(&p, N * m * gs_bytes(s)));
-        P.ptrs.push_back(p);
+        char* p = nullptr;
+        TRY(P.get(&p, N * m * gs_bytes(s)));
         s->slices = p;
         for (float** q : {&s->guide, &s->mi, &s->vi, &s->tmp, &s->draw, &s->dmed, &s->conf, &s->mins, &s->u, &s->w2, &s->t0,
                           &s->t1, &s->t2, &s->abar, &s->bbar})
@@ -469,6 +665,7 @@ static char* stack_alloc(lsb_stack* s) {
         s->chunk_ev.assign(3 * ((N + SEL_CHUNK - 1) / SEL_CHUNK + 1), nullptr);
         for (auto& v : s->chunk_ev) TRY(cudaEventCreate(&v));
     }
+    if (depth_only) return nullptr;
     s->copied.assign(N, nullptr);
     for (auto& v : s->copied) TRY(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
     return nullptr;
@@ -517,9 +714,8 @@ extern "C" char* lsb_check_params(const lsb_fuse_params* fuse, const lsb_align_p
     return bad ? dup_err(bad) : nullptr;
 }
 
-extern "C" char* lsb_stack_begin(lsb_engine* e, uint32_t w, uint32_t h, uint32_t n_frames, const lsb_fuse_params* fuse,
-                                 const lsb_align_params* align, const lsb_depth_params* depth, int32_t brightness, int32_t crop,
-                                 lsb_stack** out) {
+static char* stack_make(lsb_engine* e, uint32_t w, uint32_t h, uint32_t n_frames, const lsb_fuse_params* fuse, const lsb_align_params* align,
+                        const lsb_depth_params* depth, int32_t brightness, int32_t crop, int storage, bool depth_only, lsb_stack** out) {
     *out = nullptr;
     if (!e) return dup_err("no engine");
     if (w == 0 || h == 0 || n_frames == 0) return dup_err("a stack needs a size and at least one frame");
@@ -536,7 +732,7 @@ extern "C" char* lsb_stack_begin(lsb_engine* e, uint32_t w, uint32_t h, uint32_t
     s->dp = depth ? *depth : lsb_depth_params{};
     s->brightness = brightness != 0;
     s->crop = crop != 0;
-    s->storage = e->cfg.storage;
+    s->storage = storage;
     if (s->storage < 0 || s->storage > 2) {
         delete s;
         return dup_err("storage must be 0 (FP32), 1 (UNORM16 levels, FP16 slices) or 2 (FP16)");
@@ -565,7 +761,7 @@ extern "C" char* lsb_stack_begin(lsb_engine* e, uint32_t w, uint32_t h, uint32_t
         s->lw.push_back((s->lw.back() + 1) / 2);
         s->lh.push_back((s->lh.back() + 1) / 2);
     }
-    char* err = stack_alloc(s);
+    char* err = stack_alloc(s, depth_only);
     if (err) {
         delete s;
         return err;
@@ -578,6 +774,24 @@ extern "C" char* lsb_stack_begin(lsb_engine* e, uint32_t w, uint32_t h, uint32_t
     s->gains.assign((size_t)n_frames * 3, 1.f);
     *out = s;
     return nullptr;
+}
+
+extern "C" char* lsb_stack_begin(lsb_engine* e, uint32_t w, uint32_t h, uint32_t n_frames, const lsb_fuse_params* fuse,
+                                 const lsb_align_params* align, const lsb_depth_params* depth, int32_t brightness, int32_t crop,
+                                 lsb_stack** out) {
+    *out = nullptr;
+    if (!e) return dup_err("no engine");
+    char* err = stack_make(e, w, h, n_frames, fuse, align, depth, brightness, crop, e->cfg.storage, false, out);
+    if (!err || cudaGetLastError() != cudaErrorMemoryAllocation) return err;
+    bool idle;
+    {
+        std::lock_guard<std::mutex> lk(e->solo_mu);
+        idle = !e->solos.empty();
+    }
+    if (!idle) return err;
+    lsb_free_str(err);  // again without the idle workspaces of standalone calls
+    solo_flush(e);
+    return stack_make(e, w, h, n_frames, fuse, align, depth, brightness, crop, e->cfg.storage, false, out);
 }
 
 static bool is_device_ptr(const void* p) {
@@ -609,7 +823,11 @@ extern "C" char* lsb_stack_push_u16(lsb_stack* s, const uint16_t* rgb, size_t st
         TRY(cudaEventRecord(e->s_mark, e->s));
         TRY(cudaStreamWaitEvent(e->cs, e->s_mark, 0));
     }
-    if (stride_px == s->w) TRY(cudaMemcpyAsync(dst, rgb, sizeof(uint16_t) * 3 * (size_t)s->w * s->h, kind, e->cs));
+    if (stride_px == s->w) {
+        const size_t bytes = sizeof(uint16_t) * 3 * (size_t)s->w * s->h;
+        if (kind == cudaMemcpyHostToDevice) TRY(host_in(e, dst, rgb, bytes, e->cs));
+        else TRY(cudaMemcpyAsync(dst, rgb, bytes, kind, e->cs));
+    }
     else TRY(cudaMemcpy2DAsync(dst, 6 * (size_t)s->w, rgb, 6 * stride_px, 6 * (size_t)s->w, s->h, kind, e->cs));
     TRY(cudaEventRecord(s->copied[i], e->cs));
     TRY(cudaStreamWaitEvent(e->s, s->copied[i], 0));
@@ -689,8 +907,8 @@ extern "C" char* lsb_stack_push_u16_sized(lsb_stack* s, const uint16_t* rgb, uin
     }
     TRY(cudaStreamWaitEvent(cs, s->stage_free[b], 0));
     uint16_t* raw = s->stage[b];
-    cudaMemcpyKind kind = is_device_ptr(rgb) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    TRY(cudaMemcpyAsync(raw, rgb, sizeof(uint16_t) * 3 * px, kind, cs));
+    if (is_device_ptr(rgb)) TRY(cudaMemcpyAsync(raw, rgb, sizeof(uint16_t) * 3 * px, cudaMemcpyDeviceToDevice, cs));
+    else TRY(host_in(e, raw, rgb, sizeof(uint16_t) * 3 * px, cs));
     if (s->dust && (int)w == s->dust->W && (int)h == s->dust->H) TRY(dust_apply_rgb16(s->dust, raw, cs));
     int pw = (int)w, ph = (int)h;
     const uint16_t* cur = raw;
@@ -744,16 +962,15 @@ extern "C" char* lsb_prep_frame_u16(lsb_engine* e, const lsb_frame_prep* p, cons
     cudaError_t ce = cudaMalloc(&raw, sizeof(uint16_t) * 3 * (size_t)w * h);
     if (ce == cudaSuccess) ce = cudaMalloc(&mid, sizeof(uint16_t) * 3 * (size_t)pw * ph);
     if (ce == cudaSuccess) ce = cudaMalloc(&res, sizeof(uint16_t) * 3 * (size_t)ow * oh);
-    const cudaMemcpyKind ki = is_device_ptr(in) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    const cudaMemcpyKind ko = is_device_ptr(out) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(raw, in, sizeof(uint16_t) * 3 * (size_t)w * h, ki, cs);
+    const size_t bi = sizeof(uint16_t) * 3 * (size_t)w * h, bo = sizeof(uint16_t) * 3 * (size_t)ow * oh;
+    if (ce == cudaSuccess) ce = is_device_ptr(in) ? cudaMemcpyAsync(raw, in, bi, cudaMemcpyDeviceToDevice, cs) : host_in(e, raw, in, bi, cs);
     if (ce == cudaSuccess && d && (int)w == d->W && (int)h == d->H) ce = dust_apply_rgb16(d, raw, cs);
     if (ce == cudaSuccess) ce = turn_draft_rgb16(raw, (int)w, (int)h, (int)p->rotate, (int)p->draft, mid, cs);
     if (ce == cudaSuccess) {
         if (ow != pw || oh != ph) ce = resize_rgb16(mid, pw, ph, res, ow, oh, cs);
         else ce = cudaMemcpyAsync(res, mid, sizeof(uint16_t) * 3 * (size_t)ow * oh, cudaMemcpyDeviceToDevice, cs);
     }
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(out, res, sizeof(uint16_t) * 3 * (size_t)ow * oh, ko, cs);
+    if (ce == cudaSuccess) ce = is_device_ptr(out) ? cudaMemcpyAsync(out, res, bo, cudaMemcpyDeviceToDevice, cs) : host_out(e, out, res, bo, cs);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(cs);
     cudaStreamSynchronize(cs);
     cudaFree(raw);
@@ -778,8 +995,9 @@ extern "C" char* lsb_stack_push_f32(lsb_stack* s, const float* const planes[3]) 
     }
     const size_t np = (size_t)s->w * s->h;
     for (int c = 0; c < 3; c++) {
-        cudaMemcpyKind kind = is_device_ptr(planes[c]) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-        TRY(cudaMemcpyAsync(s->frames_f32 + ((size_t)s->count * 3 + c) * np, planes[c], sizeof(float) * np, kind, s->e->s));
+        float* dst = s->frames_f32 + ((size_t)s->count * 3 + c) * np;
+        if (is_device_ptr(planes[c])) TRY(cudaMemcpyAsync(dst, planes[c], sizeof(float) * np, cudaMemcpyDeviceToDevice, s->e->s));
+        else TRY(host_in(s->e, dst, planes[c], sizeof(float) * np, s->e->s));
     }
     s->count++;
     s->folded = false;
@@ -1504,6 +1722,9 @@ static void common_area(const std::vector<double>& sims, int n, int w, int h, in
             hi = std::min(hi, rows[y1].second);
             if (lo > hi) break;
             size_t rw = (size_t)(hi - lo + 1), rh = (size_t)(y1 - y0 + 1);
+            // the rows below only narrow it: no rectangle from y0 on can beat the best any more (without this the
+            // search is quadratic in the height, 15 M steps for 5504 rows, and outlasts the device work)
+            if (rw * (size_t)(h - y0) <= bw * bh) break;
             if (rw * rh > bw * bh) {
                 bx = (size_t)lo;
                 by = (size_t)y0;
@@ -1664,12 +1885,19 @@ extern "C" char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint3
     lsb_fuse_params fp{1, 1, 2, 2, 256, 0, 0, 0.f};
     lsb_depth_params dp = *p;
     dp.enabled = 1;
-    lsb_stack* s = nullptr;
-    lsb_config saved = e->cfg;
-    e->cfg.storage = 0;
-    char* err = lsb_stack_begin(e, w, h, n, &fp, nullptr, &dp, 0, 0, &s);
-    e->cfg = saved;
-    if (err) return err;
+    if (const char* bad = params_error(&fp, nullptr, &dp)) return dup_err(bad);
+    SoloHold hold(e, SOLO_DEPTH, w, h, n, dp.scale);
+    if (hold.fresh) {
+        char* err = stack_make(e, w, h, n, &fp, nullptr, &dp, 0, 0, STORE_F32, true, &hold.s->st);
+        if (err && cudaGetLastError() == cudaErrorMemoryAllocation) {
+            lsb_free_str(err);
+            solo_flush(e);
+            err = stack_make(e, w, h, n, &fp, nullptr, &dp, 0, 0, STORE_F32, true, &hold.s->st);
+        }
+        if (err) return err;
+    }
+    lsb_stack* s = hold.s->st;
+    s->dp = dp;
     cudaStream_t st = e->s;
     const int k = s->bk, dw = s->dw, dh = s->dh;
     const size_t m = (size_t)dw * dh;
@@ -1678,7 +1906,6 @@ extern "C" char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint3
         cudaStreamSynchronize(st);
         cudaGetLastError();
         lsb_result_free(out);
-        lsb_stack_destroy(s);
         return m_;
     };
 #define TRYS(x)                                                                                        \
@@ -1686,8 +1913,8 @@ extern "C" char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint3
         cudaError_t _e = (x);                                                                          \
         if (_e != cudaSuccess) return fail(dup_err(fmt("%s: %s", #x, cudaGetErrorString(_e))));       \
     } while (0)
-    TRYS(cudaMemcpyAsync(s->img, fused, sizeof(float) * 3 * w * h, cudaMemcpyHostToDevice, st));
-    TRYS(cudaMemcpyAsync(s->slices, slices, sizeof(float) * n * m, cudaMemcpyHostToDevice, st));
+    TRYS(host_in(e, s->img, fused, sizeof(float) * 3 * w * h, st));
+    TRYS(host_in(e, s->slices, slices, sizeof(float) * n * m, st));
     TRYS(luma_and_guide(s->img, (int)w, (int)h, k, s->yfull, s->guide, dw, dh, st));
     if (dp.agg_radius > 0) gf_stats(s->guide, dw, dh, (int)dp.agg_radius, s->tmp, s->mi, s->vi, st);
     AggArgs ag{s->slices, (int)n, dw, dh, (int)dp.agg_radius, dp.agg_eps, s->guide, s->mi, s->vi, s->state, 0, 0};
@@ -1705,7 +1932,8 @@ extern "C" char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint3
     double rel64 = 0.0;
     if (dp.lambda > 0.f) {
         cudaError_t ce;
-        WlsSolver* ws = stack_solver(s, dw, dh, dp, st, &ce);
+        WlsSolver* ws = nullptr;
+        with_room(e, [&] { return ws = stack_solver(s, dw, dh, dp, st, &ce), ce; });
         if (ce == cudaSuccess) ce = wls_set_weights(ws, s->conf, st);
         if (ce == cudaSuccess) ce = wls_solve(ws, s->dmed, (int)dp.cg_iters, s->u, &rel, &it, st, (int)dp.vcycle_mode, false, &rel64);
         it1 = it;
@@ -1730,9 +1958,9 @@ extern "C" char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint3
     out->n_frames = n;
     out->dw = dw;
     out->dh = dh;
-    out->depth = (float*)malloc(sizeof(float) * w * h);
-    out->conf = (float*)malloc(sizeof(float) * w * h);
-    out->floor_cells = (float*)malloc(sizeof(float) * m);
+    out->depth = (float*)hb_get(sizeof(float) * w * h);
+    out->conf = (float*)hb_get(sizeof(float) * w * h);
+    out->floor_cells = (float*)hb_get(sizeof(float) * m);
     if (!out->depth || !out->conf || !out->floor_cells) return fail(dup_err("out of host memory"));
     TRYS(cudaMemcpyAsync(out->depth, s->dfull, sizeof(float) * w * h, cudaMemcpyDeviceToHost, st));
     TRYS(cudaMemcpyAsync(out->conf, s->cfull, sizeof(float) * w * h, cudaMemcpyDeviceToHost, st));
@@ -1746,7 +1974,7 @@ extern "C" char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint3
     out->wls_rel64 = rel64;
     out->wls_iters = it;
     out->wls_iters_first = it1;
-    lsb_stack_destroy(s);
+    hold.keep = true;
     return nullptr;
 #undef TRYS
 }
@@ -1759,32 +1987,37 @@ extern "C" char* lsb_wls_solve(lsb_engine* e, const float* d, const float* conf,
     if (const char* bad = size_error(w, h)) return dup_err(bad);
     cudaStream_t st = e->s;
     const size_t m = (size_t)w * h;
-    DevPool P;
-    float *dd, *cc, *gg, *uu;
-    TRY(P.get(&dd, m));
-    TRY(P.get(&cc, m));
-    TRY(P.get(&gg, m));
-    TRY(P.get(&uu, m));
-    TRY(cudaMemcpyAsync(dd, d, sizeof(float) * m, cudaMemcpyHostToDevice, st));
-    TRY(cudaMemcpyAsync(cc, conf, sizeof(float) * m, cudaMemcpyHostToDevice, st));
-    TRY(cudaMemcpyAsync(gg, guide, sizeof(float) * m, cudaMemcpyHostToDevice, st));
+    SoloHold hold(e, SOLO_WLS, w, h);
+    Solo& S = *hold.s;
+    if (hold.fresh) {
+        S.planes.assign(4, nullptr);
+        for (float*& q : S.planes) TRY(with_room(e, [&] { return S.pool.get(&q, m); }));
+        TRY(with_room(e, [&] {  // planes first: the timed part is the solve
+            cudaError_t ce;
+            wls_destroy(S.ws);
+            S.ws = wls_alloc((int)w, (int)h, &ce);
+            return ce;
+        }));
+    }
+    float *dd = S.planes[0], *cc = S.planes[1], *gg = S.planes[2], *uu = S.planes[3];
+    TRY(host_in(e, dd, d, sizeof(float) * m, st));
+    TRY(host_in(e, cc, conf, sizeof(float) * m, st));
+    TRY(host_in(e, gg, guide, sizeof(float) * m, st));
     TRY(cudaMemsetAsync(uu, 0, sizeof(float) * m, st));
-    cudaError_t ce;
-    WlsSolver* ws = wls_alloc((int)w, (int)h, &ce);  // planes first: the timed part is the solve
-    if (ce == cudaSuccess) ce = cudaEventRecord(e->ev[0], st);
-    if (ce == cudaSuccess) ce = wls_prepare(ws, gg, lambda, sigma_c, (int)edge_mode, st);
-    if (ce == cudaSuccess) ce = wls_set_weights(ws, cc, st);
+    cudaError_t ce = cudaEventRecord(e->ev[0], st);
+    if (ce == cudaSuccess) ce = wls_prepare(S.ws, gg, lambda, sigma_c, (int)edge_mode, st);
+    if (ce == cudaSuccess) ce = wls_set_weights(S.ws, cc, st);
     float r = 0.f;
     int it = 0;
-    if (ce == cudaSuccess) ce = wls_solve(ws, dd, (int)max_iters, uu, &r, &it, st, (int)vcycle_mode, false, nullptr);
+    if (ce == cudaSuccess) ce = wls_solve(S.ws, dd, (int)max_iters, uu, &r, &it, st, (int)vcycle_mode, false, nullptr);
     TRY(cudaEventRecord(e->ev[1], st));
-    wls_destroy(ws);
     if (ce != cudaSuccess) return dup_err(fmt("wls: %s", cudaGetErrorString(ce)));
-    TRY(cudaMemcpyAsync(u, uu, sizeof(float) * m, cudaMemcpyDeviceToHost, st));
+    TRY(host_out(e, u, uu, sizeof(float) * m, st));
     TRY(cudaStreamSynchronize(st));
     if (rel) *rel = r;
     if (iters) *iters = (uint32_t)it;
     if (ms) *ms = ms_between(e->ev[0], e->ev[1]);
+    hold.keep = true;
     return nullptr;
 }
 
@@ -1793,22 +2026,22 @@ extern "C" char* lsb_align_pair(lsb_engine* e, const float* rf, const float* tg,
     if (!e || !rf || !tg || !out8) return dup_err("null argument");
     if (const char* bad = size_error(w, h)) return dup_err(bad);
     cudaStream_t st = e->s;
-    DevPool P;
-    float *a, *b;
-    TRY(P.get(&a, (size_t)w * h));
-    TRY(P.get(&b, (size_t)w * h));
-    TRY(cudaMemcpyAsync(a, rf, sizeof(float) * w * h, cudaMemcpyHostToDevice, st));
-    TRY(cudaMemcpyAsync(b, tg, sizeof(float) * w * h, cudaMemcpyHostToDevice, st));
     std::vector<std::pair<int, int>> dims;
     gauss_dims((int)w, (int)h, dims);
-    std::vector<float*> pr, pt;
-    for (auto& dd : dims) {
-        float *x, *y;
-        TRY(P.get(&x, (size_t)dd.first * dd.second));
-        TRY(P.get(&y, (size_t)dd.first * dd.second));
-        pr.push_back(x);
-        pt.push_back(y);
+    SoloHold hold(e, SOLO_PAIR, w, h);
+    Solo& S = *hold.s;
+    if (hold.fresh) {  // the two planes, then each level of the one and the other
+        S.planes.assign(2 + 2 * dims.size(), nullptr);
+        for (size_t q = 0; q < S.planes.size(); q++) {
+            const size_t cells = q < 2 ? (size_t)w * h : (size_t)dims[q / 2 - 1].first * dims[q / 2 - 1].second;
+            TRY(with_room(e, [&] { return S.pool.get(&S.planes[q], cells); }));
+        }
     }
+    float *a = S.planes[0], *b = S.planes[1];
+    std::vector<float*> pr, pt;
+    for (size_t q = 2; q < S.planes.size(); q += 2) pr.push_back(S.planes[q]), pt.push_back(S.planes[q + 1]);
+    TRY(host_in(e, a, rf, sizeof(float) * w * h, st));
+    TRY(host_in(e, b, tg, sizeof(float) * w * h, st));
     TRY(gauss_levels(a, (int)w, (int)h, pr, st));
     TRY(gauss_levels(b, (int)w, (int)h, pt, st));
     const double id[8] = {0, 0, 1, 0, 1, 0, 0, 0};
@@ -1818,6 +2051,7 @@ extern "C" char* lsb_align_pair(lsb_engine* e, const float* rf, const float* tg,
     e->actx.device_search = e->coop;
     TRY(multiscale_align(e->actx, a, pr, b, pt, (int)w, (int)h, init8 ? init8 : id, fr, (int)coarsen, out8));
     if (evals) *evals = (uint32_t)e->actx.evals;
+    hold.keep = true;
     return nullptr;
 }
 
@@ -1869,7 +2103,7 @@ extern "C" char* lsb_stack_weighted_average(lsb_stack* s, const lsb_wav_params* 
     const bool aligned = s->ap.enabled && n > 1 && !s->f32src;
     FoldArgs a = level_args(s, 0, aligned, false, &focus, &src);
     TRY(wav_accumulate(a, src, s->wav_w, n, dw, dh, s->bk, s->img_tmp, st));
-    TRY(cudaMemcpyAsync(out, s->img_tmp, sizeof(float) * 3 * (size_t)s->w * s->h, cudaMemcpyDeviceToHost, st));
+    TRY(host_out(e, out, s->img_tmp, sizeof(float) * 3 * (size_t)s->w * s->h, st));
     TRY(cudaStreamSynchronize(st));
     return nullptr;
 }
@@ -1998,7 +2232,7 @@ extern "C" char* lsb_stack_fuse_range(lsb_stack* s, uint32_t lo, uint32_t hi, co
     }
     TRY(resize_planes(s->slab_img, s->w, (size_t)s->w * s->h, 3, (int)r[0], (int)r[1], (int)r[2], (int)r[3], (int)ow, (int)oh, (int)interp,
                       s->slab_out, st));
-    TRY(cudaMemcpyAsync(out, s->slab_out, sizeof(float) * of, cudaMemcpyDeviceToHost, st));
+    TRY(host_out(s->e, out, s->slab_out, sizeof(float) * of, st));
     TRY(cudaStreamSynchronize(st));
     int status = 0;
     TRY(cudaMemcpy(&status, s->status, sizeof(int), cudaMemcpyDeviceToHost));
@@ -2018,9 +2252,9 @@ extern "C" char* lsb_resize(lsb_engine* e, const float* src, uint32_t planes, ui
     float *di = nullptr, *dout = nullptr;
     cudaError_t ce = cudaMalloc(&di, sizeof(float) * ni);
     if (ce == cudaSuccess) ce = cudaMalloc(&dout, sizeof(float) * no);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(di, src, sizeof(float) * ni, cudaMemcpyHostToDevice, e->s);
+    if (ce == cudaSuccess) ce = host_in(e, di, src, sizeof(float) * ni, e->s);
     if (ce == cudaSuccess) ce = resize_planes(di, pw, (size_t)pw * ph, (int)planes, 0, 0, (int)pw, (int)ph, (int)w, (int)h, (int)interp, dout, e->s);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(out, dout, sizeof(float) * no, cudaMemcpyDeviceToHost, e->s);
+    if (ce == cudaSuccess) ce = host_out(e, out, dout, sizeof(float) * no, e->s);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->s);
     cudaFree(di);
     cudaFree(dout);

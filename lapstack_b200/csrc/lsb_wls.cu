@@ -33,20 +33,14 @@ struct WlsSolver {
     double *part, *scal;  // scal: [rz, pap, rr, bnorm2, rz_new]
     float* alpha_beta;    // [alpha, beta]
     float* host_rel;      // pinned: [rel, stop]
-    std::vector<void*> allocs;
+    void* slab = nullptr;  // every plane: one allocation
+    size_t bytes = 0;
     // the CG iteration as two CUDA graphs (A: A p, alpha, the updates, |r|; B: the preconditioner,
     // beta, the new direction), captured on the first solve for this u and V-cycle mode
     cudaGraphExec_t gA = nullptr, gB = nullptr;
     const float* g_u = nullptr;
     int g_mode = -1;
     long long kA = 0, kB = 0;
-    float* alloc(size_t n, cudaError_t* e) {
-        void* p = nullptr;
-        cudaError_t r = cudaMalloc(&p, n * sizeof(float));
-        if (r != cudaSuccess) *e = r;
-        else allocs.push_back(p);
-        return (float*)p;
-    }
 };
 
 static int g1(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 16); }
@@ -918,39 +912,37 @@ WlsSolver* wls_alloc(int w, int h, cudaError_t* err) {
     WlsSolver* S = new WlsSolver();
     S->w = w;
     S->h = h;
-    size_t n = (size_t)w * h;
-    S->ex = S->alloc(n, err);
-    S->ey = S->alloc(n, err);
-    int cw = w, ch = h;
-    while (true) {
-        WlsLevel L;
+    const size_t n = (size_t)w * h;
+    for (int cw = w, ch = h;; cw = (cw + 1) / 2, ch = (ch + 1) / 2) {
+        WlsLevel L{};
         L.w = cw;
         L.h = ch;
-        size_t m = (size_t)cw * ch;
-        L.wd = S->alloc(m, err);
-        L.ax = S->alloc(m, err);
-        L.ay = S->alloc(m, err);
-        L.dinv = S->alloc(m, err);
-        L.x = S->alloc(m, err);
-        L.b = S->alloc(m, err);
-        L.r = S->alloc(m, err);
-        uint16_t** hs[7] = {&L.hwd, &L.hax, &L.hay, &L.hdinv, &L.hx, &L.hb, &L.hr};
-        for (uint16_t** h : hs) *h = (uint16_t*)S->alloc((m + 1) / 2, err);
         S->lv.push_back(L);
         if (std::max(cw, ch) <= MG_MIN) break;
-        cw = (cw + 1) / 2;
-        ch = (ch + 1) / 2;
     }
-    S->cp = S->alloc(n, err);
-    S->dp = S->alloc(n, err);
-    S->f = S->alloc(n, err);
-    S->r = S->alloc(n, err);
-    S->z = S->alloc(n, err);
-    S->p = S->alloc(n, err);
-    S->ap = S->alloc(n, err);
-    S->part = (double*)S->alloc(2 * DOT_BLOCKS, err);
-    S->scal = (double*)S->alloc(16, err);
-    S->alpha_beta = S->alloc(4, err);
+    // the planes laid out in one slab, 256-byte aligned: first their total, then their places
+    for (int pass = 0; pass < 2; pass++) {
+        size_t at = 0;
+        auto put = [&](auto** p, size_t count) {
+            using T = std::remove_pointer_t<std::remove_reference_t<decltype(*p)>>;
+            if (pass) *p = (T*)((char*)S->slab + at);
+            at += (count * sizeof(T) + 255) / 256 * 256;
+        };
+        for (WlsLevel& L : S->lv) {
+            const size_t m = (size_t)L.w * L.h;
+            for (float** q : {&L.wd, &L.ax, &L.ay, &L.dinv, &L.x, &L.b, &L.r}) put(q, m);
+            for (uint16_t** q : {&L.hwd, &L.hax, &L.hay, &L.hdinv, &L.hx, &L.hb, &L.hr}) put(q, m);
+        }
+        for (float** q : {&S->ex, &S->ey, &S->cp, &S->dp, &S->f, &S->r, &S->z, &S->p, &S->ap}) put(q, n);
+        put(&S->part, (size_t)DOT_BLOCKS);
+        put(&S->scal, 8);
+        put(&S->alpha_beta, 4);
+        if (pass == 0) {
+            S->bytes = at;
+            *err = cudaMalloc(&S->slab, at);
+            if (*err != cudaSuccess) return S;
+        }
+    }
     if (cudaHostAlloc((void**)&S->host_rel, 64, cudaHostAllocDefault) != cudaSuccess) *err = cudaErrorMemoryAllocation;
     return S;
 }
@@ -968,22 +960,15 @@ cudaError_t wls_prepare(WlsSolver* S, const float* guide, float lambda, float si
     return cudaGetLastError();
 }
 
-WlsSolver* wls_create(const float* guide, int w, int h, float lambda, float sigma_c, int edge_mode, cudaStream_t s,
-                      cudaError_t* err) {
-    WlsSolver* S = wls_alloc(w, h, err);
-    if (*err != cudaSuccess) return S;
-    *err = wls_prepare(S, guide, lambda, sigma_c, edge_mode, s);
-    return S;
-}
-
 int wls_width(const WlsSolver* s) { return s->w; }
 int wls_height(const WlsSolver* s) { return s->h; }
+size_t wls_bytes(const WlsSolver* s) { return s ? s->bytes : 0; }
 
 void wls_destroy(WlsSolver* s) {
     if (!s) return;
     if (s->gA) cudaGraphExecDestroy(s->gA);
     if (s->gB) cudaGraphExecDestroy(s->gB);
-    for (void* p : s->allocs) cudaFree(p);
+    if (s->slab) cudaFree(s->slab);
     if (s->host_rel) cudaFreeHost(s->host_rel);
     delete s;
 }

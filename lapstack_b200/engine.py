@@ -593,12 +593,10 @@ def depth_from_slices(slices, fused, params: DepthParams | None = None, engine: 
     r = Result()
     check(e._L.lsb_depth_from_slices(e._h, C.c_void_p(sl.ctypes.data), sl.shape[0], C.c_void_p(fu.ctypes.data), w, h,
                                      C.byref(dp), C.byref(r)))
-    try:
-        return DepthMap(_arr(r.depth, w * h, np.float32).reshape(h, w), _arr(r.conf, w * h, np.float32).reshape(h, w), w, h, r.dw,
-                        r.dh, _arr(r.floor_cells, r.dw * r.dh, np.float32).reshape(r.dh, r.dw), r.floor_value, r.p90, r.wls_rel,
-                        r.wls_rel64, r.wls_iters, r.wls_iters_first)
-    finally:
-        e._L.lsb_result_free(C.byref(r))
+    own = _ResultOwner(e._L, r)  # the planes are views of the library's buffers, as Stack.finish's
+    return DepthMap(_view(own, r.depth, w * h, np.float32).reshape(h, w), _view(own, r.conf, w * h, np.float32).reshape(h, w), w, h, r.dw,
+                    r.dh, _view(own, r.floor_cells, r.dw * r.dh, np.float32).reshape(r.dh, r.dw), r.floor_value, r.p90, r.wls_rel,
+                    r.wls_rel64, r.wls_iters, r.wls_iters_first)
 
 
 def wls_solve(d, conf, guide, lam, sigma_c, max_iters=200, edge_mode=0, vcycle_mode=0, engine: Engine | None = None):
