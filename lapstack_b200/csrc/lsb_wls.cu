@@ -528,129 +528,188 @@ __global__ void __launch_bounds__(32 * P) pthomas_kernel(float* __restrict__ u, 
 }
 constexpr int PT_ROWS = 8, PT_COLS = 16;
 
-// depth.rs:677 `solve_rows`: the row sweep with one row per warp held in shared memory (the partition
-// method of pthomas_kernel with 32 segments, lane = segment): a row's
-// coefficients are read once, coalesced, and every step of the segments'
-// sweeps hits shared memory (segments start w/32 floats apart: no bank
-// conflicts when that is odd, at most two-way otherwise). The reduced system
-// is solved by lane 0 from the segments' end coefficients gathered with
-// shuffles.
-constexpr int PTR_SEGS = 32;
-__global__ void __launch_bounds__(32) pthomas_rows_kernel(float* __restrict__ u, const float* __restrict__ f, const float* __restrict__ wd,
-                                                          int unit_wd, const float* __restrict__ a, int w, int h, float lam) {
-    extern __shared__ float sm[];
-    __shared__ float X[PTR_SEGS];
-    const int line = blockIdx.x, lane = threadIdx.x;
-    if (line >= h) return;
-    float* A = sm;
-    float* WD = A + w;
-    float* F = WD + w;
-    float* S0 = F + w;
-    float* S1 = S0 + w;
-    float* S2 = S1 + w;
-    const size_t row = (size_t)line * w;
-    for (int i = lane; i < w; i += 32) {
-        A[i] = a[row + i];
-        F[i] = f[row + i];
-        WD[i] = unit_wd ? 1.f : wd[row + i];
+// The same partition method with a line's data in shared memory and many short segments (up to 128 a line): a
+// CTA holds LC lines (rows: one; columns: up to 8, a 32-byte sector of each image row), thread = (segment, line),
+// segments of `ept` elements (odd: conflict-free). (1) Each segment eliminates forward to its last equation
+// g X_{s-1} + d X_s + u x_next = r, and backward to its first unknown x_b = rho + sig X_{s-1} + tau X_s. (2) The
+// segments' last unknowns X_s form a tridiagonal system, solved by parallel cyclic reduction across the threads
+// (log2 steps; the system is diagonally dominant, as the line's is). (3) With X_{s-1} and X_s known each segment
+// solves its unknowns in place. Elements past the line's end are decoupled unknowns (a = 0, weight 1, right-hand
+// side 0), so that every segment is whole.
+// What bounds it: the divisions' latency along a segment (three a cell) and one read and one write of each plane;
+// the earlier forms walked 32 segments of a row per warp, or 16 of a column through global memory, 17 words a cell:
+// 0.46 and 0.38 ms a sweep on 4128 x 2752, 0.08 to 0.11 and 0.135 here.
+constexpr int PTRI_SEGS = 128;
+__host__ __device__ constexpr size_t ptri_smem(int segs, int ept, int lc, bool unit) {
+    return sizeof(float) * ((size_t)segs * ept * lc * (unit ? 2 : 3) + (size_t)4 * segs * lc);
+}
+template <bool ROWS, bool UNIT, int lc>
+__global__ void __launch_bounds__(ROWS ? 128 : 1024) ptri_kernel(float* __restrict__ u, const float* __restrict__ f, const float* __restrict__ wd,
+                                                                 const float* __restrict__ a, int w, int h, float lam, int segs, int ept) {
+    extern __shared__ float ptri_sm[];
+    const int nlines = ROWS ? h : w, len = ROWS ? w : h, cells = segs * ept * lc, nt = segs * lc;
+    float* A = ptri_sm;          // a, then the backward elimination's x_{i-1} coefficients
+    float* F = A + cells;        // the right-hand side, then the solution
+    float* WD = F + cells;       // weights (UNIT: none)
+    float* red = UNIT ? WD : WD + cells;  // [4][segs][lc]
+    const int tid = threadIdx.x, l0 = blockIdx.x * lc, col = tid % lc, seg = tid / lc;
+    // this thread's elements of the load and the store: line l0 + col, from element seg on, segs apart (w h < 2^31)
+    const bool mine = l0 + col < nlines;
+    const unsigned k0 = ROWS ? (unsigned)l0 * w + seg : (unsigned)seg * w + l0 + col, dk = ROWS ? segs : (unsigned)segs * w;
+    {
+        unsigned k = k0;
+#pragma unroll 4
+        for (int i = seg, e = tid; i < segs * ept; i += segs, e += nt, k += dk) {
+            const bool in = mine && i < len;
+            A[e] = in && i + 1 < len ? a[k] : 0.f;
+            const float wv = UNIT ? 1.f : (in ? wd[k] : 1.f), fv = in ? f[k] : 0.f;
+            F[e] = UNIT ? fv : wv * fv;
+            if (!UNIT) WD[e] = wv;
+        }
     }
-    __syncwarp();
-    const int len = w, b = (int)((long long)lane * len / PTR_SEGS), e = (int)((long long)(lane + 1) * len / PTR_SEGS);
+    __syncthreads();
     const float nl = -lam;
-    float a_prev = b > 0 ? A[b - 1] : 0.f;
-    float dprev = 1.f, gprev = 0.f, rprev = 0.f, uprev = 0.f;
-    for (int i = b; i < e; i++) {
-        const float ai = i + 1 < len ? A[i] : 0.f;
-        const float wdi = WD[i];
-        const float diag = wdi + lam * (a_prev + ai);
-        const float lower = nl * a_prev, upper = nl * ai;
-        const float ri = wdi * F[i];
-        float dd = diag, gg = lower, rv = ri;
-        if (i > b) {
-            const float mlt = lower / dprev;
-            dd = diag - mlt * uprev;
-            gg = -(mlt * gprev);
-            rv = ri - mlt * rprev;
-        }
-        if (fabsf(dd) < 1e-12f) dd = 1e-12f;
-        S0[i] = dd;
-        S1[i] = gg;
-        S2[i] = rv;
-        dprev = dd;
-        gprev = gg;
-        rprev = rv;
-        uprev = upper;
-        a_prev = ai;
+    const int base = seg * ept * lc + col;  // element j of the segment: base + j lc
+    const float a_before = seg > 0 ? A[base - lc] : 0.f;
+    auto guard = [](float d) { return fabsf(d) < 1e-12f ? 1e-12f : d; };
+    // (1) forward: the segment's last equation
+    float dp = 1.f, gp = 0.f, rp = 0.f, up = 0.f, ap = a_before;
+#pragma unroll 2
+    for (int j = 0; j < ept; j++) {
+        const int k = base + j * lc;
+        const float ai = A[k], wi = UNIT ? 1.f : WD[k], ri = F[k];
+        const float diag = wi + lam * (ap + ai), lower = nl * ap;
+        const float mlt = j > 0 ? lower * (1.f / dp) : 0.f;
+        gp = j > 0 ? -(mlt * gp) : lower;
+        rp = ri - mlt * rp;
+        dp = guard(diag - mlt * up);
+        up = nl * ai;
+        ap = ai;
     }
-    const float dL = dprev, gL = gprev, rL = rprev, uL = uprev;  // the segment's last equation
-    float rn = 0.f, sn = 0.f, tn = 1.f;
-    S0[e - 1] = 0.f;
-    S1[e - 1] = 0.f;
-    S2[e - 1] = 1.f;
-    for (int i = e - 2; i >= b; i--) {
-        const float upper = nl * A[i];
-        const float inv = 1.f / S0[i];
-        const float rho = (S2[i] - upper * rn) * inv, sig = (-S1[i] - upper * sn) * inv, tau = -(upper * tn) * inv;
-        S0[i] = rho;
-        S1[i] = sig;
-        S2[i] = tau;
-        rn = rho;
-        sn = sig;
-        tn = tau;
-    }
-    // the reduced system on lane 0, the coefficients of segment q (and q + 1) by shuffle
-    float cprev = 0.f, rprev2 = 0.f;
-    float rc[PTR_SEGS], rr[PTR_SEGS];
-#pragma unroll
-    for (int q = 0; q < PTR_SEGS; q++) {
-        const float dq = __shfl_sync(0xffffffffu, dL, q), gq = __shfl_sync(0xffffffffu, gL, q);
-        const float rq = __shfl_sync(0xffffffffu, rL, q), uq = __shfl_sync(0xffffffffu, uL, q);
-        const int nq = q + 1 < PTR_SEGS ? q + 1 : q;
-        const float rF = __shfl_sync(0xffffffffu, rn, nq), sF = __shfl_sync(0xffffffffu, sn, nq), tF = __shfl_sync(0xffffffffu, tn, nq);
-        const bool nx = q + 1 < PTR_SEGS;
-        const float Aq = q > 0 ? gq : 0.f;
-        const float Bq = nx ? dq + uq * sF : dq;
-        const float Cq = nx ? uq * tF : 0.f;
-        const float Rq = nx ? rq - uq * rF : rq;
-        float den = Bq - Aq * cprev;
-        if (fabsf(den) < 1e-12f) den = 1e-12f;
-        cprev = Cq / den;
-        rprev2 = (Rq - Aq * rprev2) / den;
-        rc[q] = cprev;
-        rr[q] = rprev2;
-    }
-    if (lane == 0) {
-        float xn = 0.f;
-#pragma unroll
-        for (int q = PTR_SEGS - 1; q >= 0; q--) {
-            xn = q == PTR_SEGS - 1 ? rr[q] : rr[q] - rc[q] * xn;
-            X[q] = xn;
+    // ... and backward: its first unknown
+    float P = 0.f, Q = 1.f, T = 0.f;
+    {
+        float ai = ept > 1 ? A[base + (ept - 2) * lc] : 0.f;
+#pragma unroll 2
+        for (int j = ept - 2; j >= 0; j--) {
+            const int k = base + j * lc;
+            const float al = j > 0 ? A[k - lc] : a_before, wi = UNIT ? 1.f : WD[k], ri = F[k];
+            const float upper = nl * ai, lower = nl * al;
+            const float inv = 1.f / guard(wi + lam * (al + ai) + upper * T);
+            P = (ri - upper * P) * inv;
+            Q = -(upper * Q) * inv;
+            T = -lower * inv;
+            ai = al;
         }
     }
-    __syncwarp();
-    const float xl = lane > 0 ? X[lane - 1] : 0.f, xs = X[lane];
-    for (int i = b; i < e; i++) S0[i] = S0[i] + S1[i] * xl + S2[i] * xs;
-    __syncwarp();
-    for (int i = lane; i < w; i += 32) u[row + i] = S0[i];
+    // (2) the reduced system
+    auto R = [&](int q, int sg) -> float& { return red[(q * segs + sg) * lc + col]; };
+    R(0, seg) = P;
+    R(1, seg) = T;
+    R(2, seg) = Q;
+    __syncthreads();
+    const bool nx = seg + 1 < segs;
+    const float nP = nx ? R(0, seg + 1) : 0.f, nS = nx ? R(1, seg + 1) : 0.f, nT = nx ? R(2, seg + 1) : 0.f;
+    float ra = gp, rb = guard(dp + up * nS), rc = up * nT, rr = rp - up * nP;
+    for (int d = 1; d < segs; d *= 2) {
+        __syncthreads();
+        R(0, seg) = ra;
+        R(1, seg) = rb;
+        R(2, seg) = rc;
+        R(3, seg) = rr;
+        __syncthreads();
+        const int lo = seg - d, hi = seg + d;
+        float na = 0.f, nc = 0.f, b2 = rb, r2 = rr;
+        if (lo >= 0) {
+            const float q = ra * (1.f / R(1, lo));
+            b2 -= R(2, lo) * q;
+            r2 -= R(3, lo) * q;
+            na = -(R(0, lo) * q);
+        }
+        if (hi < segs) {
+            const float q = rc * (1.f / R(1, hi));
+            b2 -= R(0, hi) * q;
+            r2 -= R(3, hi) * q;
+            nc = -(R(2, hi) * q);
+        }
+        ra = na;
+        rb = guard(b2);
+        rc = nc;
+        rr = r2;
+    }
+    __syncthreads();
+    const float xs = rr / rb;
+    R(0, seg) = xs;
+    __syncthreads();
+    // (3) the segment's unknowns between X_{s-1} and X_s
+    {
+        float y = xs, ai = ept > 1 ? A[base + (ept - 2) * lc] : 0.f;
+        T = 0.f;
+        for (int j = ept - 2; j >= 0; j--) {
+            const int k = base + j * lc;
+            const float al = j > 0 ? A[k - lc] : a_before, wi = UNIT ? 1.f : WD[k], ri = F[k];
+            const float upper = nl * ai, lower = nl * al;
+            const float inv = 1.f / guard(wi + lam * (al + ai) + upper * T);
+            y = (ri - upper * y) * inv;
+            T = -lower * inv;
+            F[k] = y;
+            A[k] = T;
+            ai = al;
+        }
+        F[base + (ept - 1) * lc] = xs;
+        float x = seg > 0 ? R(0, seg - 1) : 0.f;
+#pragma unroll 2
+        for (int j = 0; j + 1 < ept; j++) {
+            const int k = base + j * lc;
+            x = F[k] + A[k] * x;
+            F[k] = x;
+        }
+    }
+    __syncthreads();
+    unsigned k = k0;
+#pragma unroll 4
+    for (int i = seg, e = tid; i < len; i += segs, e += nt, k += dk)
+        if (mine) u[k] = F[e];
+}
+// The sweep's shape for lines of `len`: as many segments as give them about 8 elements, 32 to 128; columns by 8, or by
+// fewer where 8 do not fit shared memory. False: no shape fits (a line longer than the shared memory).
+constexpr size_t PTRI_MAX_SMEM = 220 * 1024;
+static bool ptri_shape(bool rows, bool unit, int len, int& lc, int& segs, int& ept) {
+    segs = 32;
+    while (segs < PTRI_SEGS && len > segs * 8) segs *= 2;
+    ept = ((len + segs - 1) / segs) | 1;
+    for (lc = rows || !unit ? 1 : 8; lc >= 1; lc /= 2)  // weighted columns: only the solve of a single one
+        if (ptri_smem(segs, ept, lc, unit) <= PTRI_MAX_SMEM) return true;
+    return false;
 }
 
-static void thomas(bool rows, float* u, const float* f, const float* wd, int unit_wd, const float* a, int w, int h, float lam,
-                   float* cp, float* dp, float* sc, cudaStream_t s) {
+// cp, dp, sc: scratch of the one-thread kernel and the global-memory partition.
+static cudaError_t thomas(bool rows, float* u, const float* f, const float* wd, int unit_wd, const float* a, int w, int h, float lam,
+                          float* cp, float* dp, float* sc, cudaStream_t s) {
     const int nlines = rows ? h : w, len = rows ? w : h;
-    if (rows && len >= PTR_SEGS * 8 && (size_t)6 * len * sizeof(float) <= 200 * 1024) {
-        const size_t smem = (size_t)6 * len * sizeof(float);
-        cudaFuncSetAttribute(pthomas_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        lsb_launched(), pthomas_rows_kernel<<<nlines, 32, smem, s>>>(u, f, wd, unit_wd, a, w, h, lam);
-        return;
+    int lc, segs, ept;
+    if (len >= 64 && ptri_shape(rows, unit_wd != 0, len, lc, segs, ept)) {
+        const size_t smem = ptri_smem(segs, ept, lc, unit_wd != 0);
+        auto go = [&](auto kern) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PTRI_MAX_SMEM);
+            if (e != cudaSuccess) return e;
+            lsb_launched(), kern<<<(nlines + lc - 1) / lc, segs * lc, smem, s>>>(u, f, wd, a, w, h, lam, segs, ept);
+            return cudaGetLastError();
+        };
+        if (rows) return unit_wd ? go(ptri_kernel<true, true, 1>) : go(ptri_kernel<true, false, 1>);
+        if (!unit_wd) return go(ptri_kernel<false, false, 1>);
+        return lc == 8 ? go(ptri_kernel<false, true, 8>) : lc == 4 ? go(ptri_kernel<false, true, 4>)
+               : lc == 2 ? go(ptri_kernel<false, true, 2>) : go(ptri_kernel<false, true, 1>);
     }
     if (sc && len >= (rows ? PT_ROWS : PT_COLS) * 8) {
         const int g = (nlines + 31) / 32;
         if (rows) lsb_launched(), pthomas_kernel<true, PT_ROWS><<<g, 32 * PT_ROWS, 0, s>>>(u, f, wd, unit_wd, a, w, h, lam, cp, dp, sc);
         else lsb_launched(), pthomas_kernel<false, PT_COLS><<<g, 32 * PT_COLS, 0, s>>>(u, f, wd, unit_wd, a, w, h, lam, cp, dp, sc);
-        return;
+        return cudaGetLastError();
     }
     if (rows) lsb_launched(), thomas_kernel<true><<<(nlines + TT - 1) / TT, TT, 0, s>>>(u, f, wd, unit_wd, a, w, h, lam, cp, dp);
     else lsb_launched(), thomas_kernel<false><<<(nlines + TT - 1) / TT, TT, 0, s>>>(u, f, wd, unit_wd, a, w, h, lam, cp, dp);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------ the BF16 V-cycle (mode 1)
@@ -1115,15 +1174,16 @@ cudaError_t wls_solve(WlsSolver* S, const float* d, int max_iters, float* u, flo
     }
     if (!x0_given) {
         // depth.rs:1022-1034: three separable sweeps, the first confidence-weighted
-        cudaMemcpyAsync(S->f, d, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
+        const float* from = d;
         for (int t = 1; t <= 3; t++) {
             float p4 = 1.f;
             for (int q = 0; q < 3 - t; q++) p4 *= 4.f;
             const float lam_t = (1.5f * S->lambda * p4) / (64.f - 1.f);
-            thomas(true, u, S->f, L0.wd, t == 1 ? 0 : 1, S->ex, w, h, lam_t, S->cp, S->dp, S->z, s);
-            cudaMemcpyAsync(S->f, u, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
-            thomas(false, u, S->f, L0.wd, 1, S->ey, w, h, lam_t, S->cp, S->dp, S->z, s);
-            cudaMemcpyAsync(S->f, u, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
+            // rows into f, columns into u: no sweep reads what it writes
+            cudaError_t e = thomas(true, S->f, from, L0.wd, t == 1 ? 0 : 1, S->ex, w, h, lam_t, S->cp, S->dp, S->z, s);
+            if (e == cudaSuccess) e = thomas(false, u, S->f, L0.wd, 1, S->ey, w, h, lam_t, S->cp, S->dp, S->z, s);
+            if (e != cudaSuccess) return e;
+            from = u;
         }
     }
     // b = W d, |b|, r = b - A u, z = M r, p = z
