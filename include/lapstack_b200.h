@@ -356,8 +356,9 @@ char* lsb_stack_autotune(lsb_stack* s, lsb_tuning* out);
  * focus measure and its radii. On an error every result is freed and the
  * message names the stack. */
 char* lsb_batch_run(lsb_stack* const* stacks, uint32_t n_stacks, lsb_result* outs);
-/* Use the network's prediction as the x0 of this stack's WLS solves (NULL: the
- * reference's FGS start). The stack does not own the network. */
+/* Use the network's prediction as the x0 of this stack's WLS solve (the robust
+ * solve after it goes on from its solution; NULL: the reference's FGS start for
+ * both). The stack does not own the network. */
 char* lsb_stack_set_warm_start(lsb_stack* s, lsb_unet* u);
 /* Device planes of the last run's depth grid (dw x dh, valid until the next
  * run; no counterpart in the reference): the guide luma, the median-filtered raw depth, the normalised

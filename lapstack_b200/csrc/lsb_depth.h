@@ -53,14 +53,16 @@ struct WlsLevel {
 struct WlsSolver;
 // The planes of a w x h solver (allocated once, reused by every solve of that size) ...
 WlsSolver* wls_alloc(int w, int h, cudaError_t* err);
-// ... and the edge weights of one guide (depth.rs:653), down the hierarchy.
+// ... and the guide and settings of the edge weights (depth.rs:653) that the next wls_set_weights makes: the guide is
+// read by that call's kernels.
 cudaError_t wls_prepare(WlsSolver* s, const float* guide, float lambda, float sigma_c, int edge_mode, cudaStream_t st);
 int wls_width(const WlsSolver* s);
 int wls_height(const WlsSolver* s);
 size_t wls_bytes(const WlsSolver* s);
 void wls_destroy(WlsSolver* s);
-// wd = max(conf, 0) + 1e-4, aggregated down the hierarchy, diagonals taken
-cudaError_t wls_set_weights(WlsSolver* s, const float* conf, cudaStream_t st);
+// wd = max(conf, 0) + 1e-4, aggregated down the hierarchy, diagonals taken; the edges too after a wls_prepare. mode: the
+// V-cycle of the solves to come (as wls_solve's).
+cudaError_t wls_set_weights(WlsSolver* s, const float* conf, int mode, cudaStream_t st);
 // Solve for d into u; returns (rel, iters) through the pointers. mode 0: the
 // reference FP32 V-cycle; 1: BF16 smoother/restriction inside FP32 CG.
 // x0_given: u holds a start (the FGS guess is skipped). coarse_corr: optional

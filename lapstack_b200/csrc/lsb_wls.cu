@@ -22,71 +22,113 @@ constexpr float MG_OMEGA = 0.8f;
 constexpr int MG_COARSE = 32, MG_MIN = 16;
 // the BF16 V-cycle: levels, and Jacobi sweeps before and after the coarse correction
 constexpr int MG_H_LEVELS = 6, MG_H_SWEEPS = 2;
-constexpr int DOT_BLOCKS = 592;
+// blocks of a kernel that reduces (persistent: each takes every so many tiles): 8 of 256 threads an SM
+constexpr int RED_BLOCKS = 148 * 8;
 
 struct WlsSolver {
     int w, h;
     float lambda;
     float *ex, *ey;
     std::vector<WlsLevel> lv;
-    float *cp, *dp, *f, *r, *z, *p, *ap;
-    double *part, *scal;  // scal: [rz, pap, rr, bnorm2, rz_new]
+    float *cp, *dp, *f, *r, *z, *p, *p2, *ap;  // p, p2: the search direction, in turn (f: the start sweeps' row results)
+    double *part, *scal;  // partial sums of the reductions; scal: [rz, |b|]
     float* alpha_beta;    // [alpha, beta]
-    float* host_rel;      // pinned: [rel, stop]
+    int* ctl;             // [stop, iterations done, blocks of a reduction that are done, p.Ap <= 0]
+    bool ctl_zero = false;
+    float* host_rel;      // page-locked: [rel, stop, iterations, -, rel as a double]
+    const float* guide = nullptr;  // of the last wls_prepare, its edge weights made by the next wls_set_weights
+    float inv = 0.f, inv2s2 = 0.f;
+    int edge_mode = 0;
     void* slab = nullptr;  // every plane: one allocation
     size_t bytes = 0;
-    // the CG iteration as two CUDA graphs (A: A p, alpha, the updates, |r|; B: the preconditioner,
-    // beta, the new direction), captured on the first solve for this u and V-cycle mode
-    cudaGraphExec_t gA = nullptr, gB = nullptr;
+    // one CG iteration as a graph, captured on the first solve for this u and V-cycle mode
+    cudaGraphExec_t g = nullptr;
     const float* g_u = nullptr;
-    int g_mode = -1;
-    long long kA = 0, kB = 0;
+    int g_mode = -1, g_max = 0;
+    long long g_kernels = 0;
+    cudaEvent_t done[2] = {nullptr, nullptr};  // the last two iterations queued
 };
 
 static int g1(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 16); }
 static dim3 g2(int w, int h) { return dim3((w + 31) / 32, (h + 7) / 8); }
 static const dim3 B2(32, 8);
 
-// depth.rs:653 `edge_weights`: e = exp(-|dI| / sigma) right and below (mode 0);
-// mode 1, the Gaussian-of-gradient weight exp(-dI^2 / (2 sigma^2)).
-__global__ void edge_kernel(const float* __restrict__ g, int w, int h, float inv, float inv2s2, int mode, float lambda,
-                            float* ex, float* ey, float* ax, float* ay) {
+// BF16 copies of a level's operators (wd, ax, ay, dinv), for the mixed-precision V-cycle; null: none.
+struct HOps {
+    uint16_t *wd, *ax, *ay, *dinv;
+};
+typedef __nv_bfloat16 bf;
+__device__ __forceinline__ float ldh(const uint16_t* p, size_t k) { return __bfloat162float(((const bf*)p)[k]); }
+__device__ __forceinline__ void sth(uint16_t* p, size_t k, float v) { ((bf*)p)[k] = __float2bfloat16_rn(v); }
+__device__ __forceinline__ void put_ops(const HOps& H, size_t k, float wd, float ax, float ay, float dinv) {
+    if (!H.wd) return;
+    sth(H.wd, k, wd);
+    sth(H.ax, k, ax);
+    sth(H.ay, k, ay);
+    sth(H.dinv, k, dinv);
+}
+// depth.rs:812 `set_dinv` of one cell: its weight and the edges that leave it (0 past the border: adding it changes nothing)
+__device__ __forceinline__ float dinv_of(float wd, bool l, float axl, bool r, float axr, bool t, float ayt, bool b, float ayb) {
+    float v = wd;
+    if (l) v = __fadd_rn(v, axl);
+    if (r) v = __fadd_rn(v, axr);
+    if (t) v = __fadd_rn(v, ayt);
+    if (b) v = __fadd_rn(v, ayb);
+    return __fdiv_rn(1.f, fmaxf(v, 1e-12f));
+}
+// Level 0 of a solve in one pass: depth.rs:653 `edge_weights`, e = exp(-|dI| / sigma) right and below (mode 0; mode 1:
+// the Gaussian-of-gradient weight exp(-dI^2 / (2 sigma^2))) times lambda, depth.rs:994 wd = max(conf, 0) + 1e-4 and
+// depth.rs:812 the diagonal, the left and upper edges computed again by the cell that needs them. EDGES false: other
+// weights on the same edges (the robust solve).
+template <bool EDGES>
+__global__ void level0_kernel(const float* __restrict__ g, const float* __restrict__ conf, int w, int h, float inv, float inv2s2, int mode,
+                              float lambda, float* __restrict__ ex, float* __restrict__ ey, float* __restrict__ ax, float* __restrict__ ay,
+                              float* __restrict__ wd, float* __restrict__ dinv, const HOps H) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= w || y >= h) return;
     const size_t k = (size_t)y * w + x;
-    float vx = 0.f, vy = 0.f;
-    if (x + 1 < w) {
-        const float d = fabsf(__fsub_rn(g[k], g[k + 1]));
-        vx = mode == 0 ? expf(__fmul_rn(d, inv)) : expf(-__fmul_rn(__fmul_rn(d, d), inv2s2));
+    const bool L = x > 0, R = x + 1 < w, T = y > 0, B = y + 1 < h;
+    const float wv = __fadd_rn(fmaxf(conf[k], 0.f), 1e-4f);
+    float al, ar, at, ab;
+    if (EDGES) {
+        const float gc = g[k];
+        auto edge = [&](float a, float b) {
+            const float d = fabsf(__fsub_rn(a, b));
+            return mode == 0 ? expf(__fmul_rn(d, inv)) : expf(-__fmul_rn(__fmul_rn(d, d), inv2s2));
+        };
+        const float vx = R ? edge(gc, g[k + 1]) : 0.f, vy = B ? edge(gc, g[k + w]) : 0.f;
+        al = L ? __fmul_rn(lambda, edge(g[k - 1], gc)) : 0.f;
+        at = T ? __fmul_rn(lambda, edge(g[k - w], gc)) : 0.f;
+        ar = __fmul_rn(lambda, vx);
+        ab = __fmul_rn(lambda, vy);
+        ex[k] = vx;
+        ey[k] = vy;
+        ax[k] = ar;
+        ay[k] = ab;
+    } else {
+        al = L ? ax[k - 1] : 0.f;
+        ar = ax[k];
+        at = T ? ay[k - w] : 0.f;
+        ab = ay[k];
     }
-    if (y + 1 < h) {
-        const float d = fabsf(__fsub_rn(g[k], g[k + w]));
-        vy = mode == 0 ? expf(__fmul_rn(d, inv)) : expf(-__fmul_rn(__fmul_rn(d, d), inv2s2));
-    }
-    ex[k] = vx;
-    ey[k] = vy;
-    ax[k] = __fmul_rn(lambda, vx);
-    ay[k] = __fmul_rn(lambda, vy);
+    wd[k] = wv;
+    const float dv = dinv_of(wv, L, al, R, ar, T, at, B, ab);
+    dinv[k] = dv;
+    put_ops(H, k, wv, ar, ab, dv);
 }
-
-// depth.rs:852 `coarsen` (edges) and :886 `coarsen_wd_into` (data weights)
-__global__ void coarsen_edges_kernel(const float* __restrict__ ax, const float* __restrict__ ay, int w, int h, float* cax,
-                                     float* cay, int cw, int ch) {
-    const int xx = blockIdx.x * blockDim.x + threadIdx.x, yy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (xx >= cw || yy >= ch) return;
+// depth.rs:852 `coarsen`, one coarse cell's right and lower edge from the finer level's
+__device__ __forceinline__ float coarse_ax(const float* ax, int w, int h, int xx, int yy) {
     float a = 0.f;
-    if (xx + 1 < cw)
-        for (int y = 2 * yy; y < min(2 * yy + 2, h); y++) a = __fadd_rn(a, ax[(size_t)y * w + 2 * xx + 1]);
-    cax[(size_t)yy * cw + xx] = a;
-    float b = 0.f;
-    if (yy + 1 < ch) {
-        const int y = 2 * yy + 1;
-        for (int x = 2 * xx; x < min(2 * xx + 2, w); x++) b = __fadd_rn(b, ay[(size_t)y * w + x]);
-    }
-    cay[(size_t)yy * cw + xx] = b;
+    for (int y = 2 * yy; y < min(2 * yy + 2, h); y++) a = __fadd_rn(a, ax[(size_t)y * w + 2 * xx + 1]);
+    return a;
 }
-// b_c = P^T r (depth.rs:911 `restrict`), the same block sum as the data weights
-__device__ __forceinline__ float block_sum_at(const float* __restrict__ src, int w, int h, int xx, int yy) {
+__device__ __forceinline__ float coarse_ay(const float* ay, int w, int h, int xx, int yy) {
+    float b = 0.f;
+    for (int x = 2 * xx; x < min(2 * xx + 2, w); x++) b = __fadd_rn(b, ay[(size_t)(2 * yy + 1) * w + x]);
+    return b;
+}
+// depth.rs:886 `coarsen_wd_into`, depth.rs:911 `restrict`: 2x2 block sums
+__device__ __forceinline__ float block_sum_at(const float* src, int w, int h, int xx, int yy) {
     float o = 0.f;
     for (int y = 2 * yy; y < min(2 * yy + 2, h); y++) {
         float rs = 0.f;
@@ -95,24 +137,55 @@ __device__ __forceinline__ float block_sum_at(const float* __restrict__ src, int
     }
     return o;
 }
-// depth.rs:911 `restrict` (and the 2x2 aggregation of depth.rs:852 `coarsen`): 2x2 block sums.
 __global__ void block_sum_kernel(const float* __restrict__ src, int w, int h, float* __restrict__ dst, int cw, int ch) {
     const int xx = blockIdx.x * blockDim.x + threadIdx.x, yy = blockIdx.y * blockDim.y + threadIdx.y;
     if (xx >= cw || yy >= ch) return;
     dst[(size_t)yy * cw + xx] = block_sum_at(src, w, h, xx, yy);
 }
-// depth.rs:812 `set_dinv`
-__global__ void dinv_kernel(const float* __restrict__ wd, const float* __restrict__ ax, const float* __restrict__ ay, int w, int h,
-                            float* __restrict__ dinv) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= w || y >= h) return;
-    const size_t k = (size_t)y * w + x;
-    float v = wd[k];
-    if (x > 0) v = __fadd_rn(v, ax[k - 1]);
-    if (x + 1 < w) v = __fadd_rn(v, ax[k]);
-    if (y > 0) v = __fadd_rn(v, ay[k - w]);
-    if (y + 1 < h) v = __fadd_rn(v, ay[k]);
-    dinv[k] = __fdiv_rn(1.f, fmaxf(v, 1e-12f));
+// One coarse cell of the hierarchy: its edges (EDGES; else those that are there), weight and diagonal from the finer level F.
+template <bool EDGES>
+__device__ __forceinline__ void coarse_cell(const WlsLevel& F, const WlsLevel& C, const HOps& H, int xx, int yy) {
+    const size_t k = (size_t)yy * C.w + xx;
+    const bool L = xx > 0, R = xx + 1 < C.w, T = yy > 0, B = yy + 1 < C.h;
+    float al, ar, at, ab;
+    if (EDGES) {
+        al = L ? coarse_ax(F.ax, F.w, F.h, xx - 1, yy) : 0.f;
+        ar = R ? coarse_ax(F.ax, F.w, F.h, xx, yy) : 0.f;
+        at = T ? coarse_ay(F.ay, F.w, F.h, xx, yy - 1) : 0.f;
+        ab = B ? coarse_ay(F.ay, F.w, F.h, xx, yy) : 0.f;
+        C.ax[k] = ar;
+        C.ay[k] = ab;
+    } else {
+        al = L ? C.ax[k - 1] : 0.f;
+        ar = C.ax[k];
+        at = T ? C.ay[k - C.w] : 0.f;
+        ab = C.ay[k];
+    }
+    const float wv = block_sum_at(F.wd, F.w, F.h, xx, yy);
+    C.wd[k] = wv;
+    const float dv = dinv_of(wv, L, al, R, ar, T, at, B, ab);
+    C.dinv[k] = dv;
+    put_ops(H, k, wv, ar, ab, dv);
+}
+template <bool EDGES>
+__global__ void coarse_level_kernel(const WlsLevel F, const WlsLevel C, const HOps H) {
+    const int xx = blockIdx.x * blockDim.x + threadIdx.x, yy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (xx < C.w && yy < C.h) coarse_cell<EDGES>(F, C, H, xx, yy);
+}
+// The small levels, one after another in one CTA (each reads what the one before wrote, behind a block barrier).
+constexpr int MG_TAIL_CELLS = 8192, MG_TAIL_MAX = 16;
+struct MgSetup {
+    WlsLevel lv[MG_TAIL_MAX + 1];  // the last large level, then the small ones
+    HOps H[MG_TAIL_MAX + 1];
+    int n;
+};
+template <bool EDGES>
+__global__ void __launch_bounds__(1024) coarse_tail_kernel(const MgSetup T) {
+    for (int l = 1; l < T.n; l++) {
+        const WlsLevel& C = T.lv[l];
+        for (int k = threadIdx.x; k < C.w * C.h; k += blockDim.x) coarse_cell<EDGES>(T.lv[l - 1], C, T.H[l], k % C.w, k / C.w);
+        __syncthreads();
+    }
 }
 // depth.rs:786 `apply`: mode 0 out = A x; 1 out = b - A x; 2 out = x + w D^-1 (b - A x)
 __device__ __forceinline__ float stencil_at(const float* __restrict__ x, const float* __restrict__ b, const float* __restrict__ wd,
@@ -129,34 +202,182 @@ __device__ __forceinline__ float stencil_at(const float* __restrict__ x, const f
     if (mode == 1) return __fsub_rn(b[k], v);
     return __fadd_rn(xk, __fmul_rn(__fmul_rn(MG_OMEGA, dinv[k]), __fsub_rn(b[k], v)));
 }
-// depth.rs:786 `MgLevel::apply` (mode 0: A x; 1: b - A x) and :837 `jacobi` (mode 2).
-__global__ void stencil_kernel(const float* __restrict__ x, const float* __restrict__ b, const float* __restrict__ wd,
-                               const float* __restrict__ ax, const float* __restrict__ ay, const float* __restrict__ dinv,
-                               float* __restrict__ out, int w, int h, int mode) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= w || y >= h) return;
-    const size_t k = (size_t)y * w + i;
-    const float xk = x[k];
-    float v = __fmul_rn(wd[k], xk);
-    if (i > 0) v = __fadd_rn(v, __fmul_rn(ax[k - 1], __fsub_rn(xk, x[k - 1])));
-    if (i + 1 < w) v = __fadd_rn(v, __fmul_rn(ax[k], __fsub_rn(xk, x[k + 1])));
-    if (y > 0) v = __fadd_rn(v, __fmul_rn(ay[k - w], __fsub_rn(xk, x[k - w])));
-    if (y + 1 < h) v = __fadd_rn(v, __fmul_rn(ay[k], __fsub_rn(xk, x[k + w])));
-    if (mode == 0) out[k] = v;
-    else if (mode == 1) out[k] = __fsub_rn(b[k], v);
-    else out[k] = __fadd_rn(xk, __fmul_rn(__fmul_rn(MG_OMEGA, dinv[k]), __fsub_rn(b[k], v)));
+// Sums over the grid of the CG's dot products (depth.rs:1037 `dot`: f64 products, each exact), taken by the kernel
+// that has the factors in registers: each thread's sum, the block's in a fixed tree, its place in `part`; the last
+// block to arrive adds the blocks' parts in a fixed order (the same values every run). True in that block, whose
+// thread 0 then has the sums.
+template <int NS>
+__device__ __forceinline__ bool reduce_last(double (&v)[NS], double* part, int* ticket) {
+    __shared__ double red[NS][8];
+    __shared__ int last;
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    auto block_sum = [&]() {  // 256 threads
+#pragma unroll
+        for (int q = 0; q < NS; q++)
+            for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+        __syncthreads();
+        if (lane == 0)
+            for (int q = 0; q < NS; q++) red[q][wid] = v[q];
+        __syncthreads();
+        if (tid == 0)
+            for (int q = 0; q < NS; q++) {
+                double t = red[q][0];
+                for (int i = 1; i < 8; i++) t += red[q][i];
+                v[q] = t;
+            }
+    };
+    block_sum();
+    if (tid == 0) {
+        for (int q = 0; q < NS; q++) part[(size_t)q * gridDim.x + blockIdx.x] = v[q];
+        __threadfence();
+        last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    for (int q = 0; q < NS; q++) {
+        double t = 0.0;
+        for (int i = tid; i < (int)gridDim.x; i += 256) t += __ldcg(part + (size_t)q * gridDim.x + i);
+        v[q] = t;
+    }
+    block_sum();
+    if (tid == 0) *ticket = 0;
+    return true;
 }
-// depth.rs:840 zero-start Jacobi: x = w * D^-1 * b
-__global__ void jac0_kernel(const float* __restrict__ b, const float* __restrict__ dinv, float* __restrict__ x, size_t n) {
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-        x[k] = __fmul_rn(__fmul_rn(MG_OMEGA, dinv[k]), b[k]);
+// The CG's scalars on the device and what the host reads.
+struct CgOut {
+    float rel;
+    int stop, iters, pad;
+    double rel64;
+};
+struct CgRef {
+    double *part, *scal;
+    float* ab;
+    int* ctl;
+    CgOut* host;
+};
+// depth.rs:1074 beta = r.z / the one before (the first direction is z), behind the preconditioner's last pass
+__device__ __forceinline__ void cg_rz(const CgRef& C, double rz) {
+    C.ab[1] = C.ctl[1] > 0 ? (float)(rz / C.scal[0]) : 0.f;
+    C.scal[0] = rz;
 }
-// depth.rs:901 `prolong_add`
-__global__ void prolong_kernel(float* __restrict__ x, int w, int h, const float* __restrict__ xc, int cw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= w || y >= h) return;
-    const size_t k = (size_t)y * w + i;
-    x[k] = __fadd_rn(x[k], xc[(size_t)(y / 2) * cw + i / 2]);
+__device__ __forceinline__ void cg_rel(const CgRef& C, double rr, int iters, bool stop) {
+    const double rel = sqrt(rr) / C.scal[1];
+    const float relf = (float)rel;
+    stop = stop || relf < 1e-5f;
+    C.ctl[0] = stop;
+    C.ctl[1] = iters;
+    C.host->rel = relf;
+    C.host->rel64 = rel;
+    C.host->iters = iters;
+    C.host->stop = stop;
+}
+// depth.rs:1039: b = W d, r = b - A u, |b| and |r|.
+__global__ void __launch_bounds__(256) cg_start_kernel(const float* __restrict__ d, const float* __restrict__ u, const float* __restrict__ wd,
+                                                       const float* __restrict__ ax, const float* __restrict__ ay, float* __restrict__ r, int w,
+                                                       int h, const CgRef C) {
+    const int tx = (w + 31) / 32, nt = tx * ((h + 7) / 8);
+    double v[2] = {0.0, 0.0};
+    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+        const int i = t % tx * 32 + threadIdx.x, y = t / tx * 8 + threadIdx.y;
+        if (i >= w || y >= h) continue;
+        const size_t k = (size_t)y * w + i;
+        const float bk = __fmul_rn(wd[k], d[k]);
+        const float rv = __fsub_rn(bk, stencil_at(u, nullptr, wd, ax, ay, nullptr, w, h, i, y, 0));
+        r[k] = rv;
+        v[0] += (double)bk * (double)bk;
+        v[1] += (double)rv * (double)rv;
+    }
+    if (reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0 && threadIdx.y == 0) {
+        C.scal[1] = fmax(sqrt(v[0]), 1e-30);
+        cg_rel(C, v[1], 0, false);
+    }
+}
+// depth.rs:1074 p = z + beta p, then depth.rs:1056 A p and p.Ap -> alpha: the direction of a tile and its ring computed
+// into shared memory from z and the last direction, which stays in the other buffer (neighbours read it).
+__global__ void __launch_bounds__(256) cg_dir_kernel(const float* __restrict__ z, float* p0, float* p1, const float* __restrict__ wd,
+                                                     const float* __restrict__ ax, const float* __restrict__ ay, float* __restrict__ ap, int w,
+                                                     int h, const CgRef C) {
+    if (C.ctl[0]) return;
+    __shared__ float P[10][34];
+    const int it = C.ctl[1], tx = (w + 31) / 32, nt = tx * ((h + 7) / 8), tid = threadIdx.y * 32 + threadIdx.x;
+    const bool first = it == 0;
+    const float beta = C.ab[1];
+    const float* old = it & 1 ? p1 : p0;
+    float* now = it & 1 ? p0 : p1;
+    double v[1] = {0.0};
+    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+        const int x0 = t % tx * 32, y0 = t / tx * 8;
+        const int i = x0 + threadIdx.x, y = y0 + threadIdx.y;
+        const bool in = i < w && y < h;
+        const size_t k = in ? (size_t)y * w + i : 0;
+        const float wk = wd[k], ar = ax[k], al = k > 0 ? ax[k - 1] : 0.f, ab = ay[k], at = k >= (size_t)w ? ay[k - w] : 0.f;
+        __syncthreads();  // the tile before is done with P
+        for (int e = tid; e < 10 * 34; e += 256) {
+            const int rr = e / 34, c = e - rr * 34, gx = x0 - 1 + c, gy = y0 - 1 + rr;
+            float pv = 0.f;
+            if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
+                const size_t q = (size_t)gy * w + gx;
+                pv = first ? z[q] : __fadd_rn(z[q], __fmul_rn(beta, old[q]));
+            }
+            P[rr][c] = pv;
+        }
+        __syncthreads();
+        if (!in) continue;
+        const int r = threadIdx.y + 1, c = threadIdx.x + 1;
+        const float xk = P[r][c];
+        float a = __fmul_rn(wk, xk);
+        if (i > 0) a = __fadd_rn(a, __fmul_rn(al, __fsub_rn(xk, P[r][c - 1])));
+        if (i + 1 < w) a = __fadd_rn(a, __fmul_rn(ar, __fsub_rn(xk, P[r][c + 1])));
+        if (y > 0) a = __fadd_rn(a, __fmul_rn(at, __fsub_rn(xk, P[r - 1][c])));
+        if (y + 1 < h) a = __fadd_rn(a, __fmul_rn(ab, __fsub_rn(xk, P[r + 1][c])));
+        now[k] = xk;
+        ap[k] = a;
+        v[0] += (double)xk * (double)a;
+    }
+    if (reduce_last(v, C.part, C.ctl + 2) && tid == 0) {
+        // p.Ap <= 0: alpha 0, u and r stay as they are and the iteration ends (depth.rs:1060)
+        C.ab[0] = v[0] <= 0.0 ? 0.f : (float)(C.scal[0] / v[0]);
+        C.ctl[3] = v[0] <= 0.0;
+    }
+}
+// depth.rs:1064-1065: u += alpha p, r -= alpha Ap, |r| -> the residual; the end of an iteration.
+__global__ void __launch_bounds__(256) cg_step_kernel(float* __restrict__ u, const float* __restrict__ p0, const float* __restrict__ p1,
+                                                      float* __restrict__ r, const float* __restrict__ ap, size_t n, int max_iters, const CgRef C) {
+    if (C.ctl[0]) return;  // an iteration queued ahead of the last one's result
+    const float alpha = C.ab[0];
+    const float* p = C.ctl[1] & 1 ? p0 : p1;
+    double v[1] = {0.0};
+    const size_t t0 = blockIdx.x * (size_t)256 + threadIdx.x, nt = (size_t)gridDim.x * 256;
+    auto one = [&](float& uv, float pv, float& rv, float av) {
+        uv = __fadd_rn(uv, __fmul_rn(alpha, pv));
+        rv = __fsub_rn(rv, __fmul_rn(alpha, av));
+        v[0] += (double)rv * (double)rv;
+    };
+    const bool vec = ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(r) |
+                       reinterpret_cast<uintptr_t>(ap)) & 15) == 0;
+    const size_t n4 = vec ? n / 4 : 0;
+    for (size_t i = t0; i < n4; i += nt) {
+        float4 uv = reinterpret_cast<float4*>(u)[i], rv = reinterpret_cast<float4*>(r)[i];
+        const float4 pv = reinterpret_cast<const float4*>(p)[i], av = reinterpret_cast<const float4*>(ap)[i];
+        one(uv.x, pv.x, rv.x, av.x);
+        one(uv.y, pv.y, rv.y, av.y);
+        one(uv.z, pv.z, rv.z, av.z);
+        one(uv.w, pv.w, rv.w, av.w);
+        reinterpret_cast<float4*>(u)[i] = uv;
+        reinterpret_cast<float4*>(r)[i] = rv;
+    }
+    for (size_t i = 4 * n4 + t0; i < n; i += nt) one(u[i], p[i], r[i], ap[i]);
+    if (reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0) {
+        const int it = C.ctl[1] + 1;
+        cg_rel(C, v[0], it, C.ctl[3] != 0 || it >= max_iters);
+    }
+}
+// r.z alone, for a preconditioner that ends in a copy (a grid small enough for one CTA).
+__global__ void __launch_bounds__(256) cg_rz_kernel(const float* __restrict__ r, const float* __restrict__ z, size_t n, const CgRef C) {
+    double v[1] = {0.0};
+    for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) v[0] += (double)r[i] * (double)z[i];
+    if (reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0) cg_rz(C, v[0]);
 }
 
 // One fine level's way down the V-cycle in one pass (depth.rs:924-930): the zero-start Jacobi sweep
@@ -207,29 +428,41 @@ __global__ void __launch_bounds__(256) vc_down_kernel(const float* __restrict__ 
 __device__ __forceinline__ float prolonged_at(const float* __restrict__ x, const float* __restrict__ xc, int w, int cw, int i, int y) {
     return __fadd_rn(x[(size_t)y * w + i], xc[(size_t)(y >> 1) * cw + (i >> 1)]);
 }
-// The block's 32 x 8 corrected x and a one-cell ring are computed once into shared memory.
+// The block's 32 x 8 corrected x and a one-cell ring are computed once into shared memory, the cell's own operands
+// loaded before. DOT (level 0): persistent over the tiles, r.z taken on the way (b is the CG's r).
+template <bool DOT>
 __global__ void __launch_bounds__(256) vc_up_kernel(const float* __restrict__ x, const float* __restrict__ xc, int cw,
                                                     const float* __restrict__ b, const float* __restrict__ wd,
                                                     const float* __restrict__ ax, const float* __restrict__ ay,
-                                                    const float* __restrict__ dinv, float* __restrict__ out, int w, int h) {
+                                                    const float* __restrict__ dinv, float* __restrict__ out, int w, int h, const CgRef C) {
+    if (DOT && C.ctl[0]) return;
     __shared__ float X[8 + 2][32 + 2];
-    const int x0 = blockIdx.x * blockDim.x - 1, y0 = blockIdx.y * blockDim.y - 1;
-    for (int e = threadIdx.y * blockDim.x + threadIdx.x; e < 10 * 34; e += blockDim.x * blockDim.y) {
-        const int r = e / 34, c = e - r * 34, gx = x0 + c, gy = y0 + r;
-        X[r][c] = gx >= 0 && gx < w && gy >= 0 && gy < h ? prolonged_at(x, xc, w, cw, gx, gy) : 0.f;
+    const int tx = (w + 31) / 32, nt = tx * ((h + 7) / 8), tid = threadIdx.y * 32 + threadIdx.x;
+    double v[1] = {0.0};
+    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+        const int x0 = t % tx * 32, y0 = t / tx * 8, i = x0 + threadIdx.x, y = y0 + threadIdx.y;
+        const bool in = i < w && y < h;
+        const size_t k = in ? (size_t)y * w + i : 0;
+        const float bk = b[k], wk = wd[k], dk = dinv[k], ar = ax[k], al = k > 0 ? ax[k - 1] : 0.f, ab = ay[k], at = k >= (size_t)w ? ay[k - w] : 0.f;
+        if (DOT) __syncthreads();  // the tile before is done with X
+        for (int e = tid; e < 10 * 34; e += 256) {
+            const int r = e / 34, c = e - r * 34, gx = x0 - 1 + c, gy = y0 - 1 + r;
+            X[r][c] = gx >= 0 && gx < w && gy >= 0 && gy < h ? prolonged_at(x, xc, w, cw, gx, gy) : 0.f;
+        }
+        __syncthreads();
+        if (!in) continue;
+        const int r = threadIdx.y + 1, c = threadIdx.x + 1;
+        const float xk = X[r][c];
+        float a = __fmul_rn(wk, xk);
+        if (i > 0) a = __fadd_rn(a, __fmul_rn(al, __fsub_rn(xk, X[r][c - 1])));
+        if (i + 1 < w) a = __fadd_rn(a, __fmul_rn(ar, __fsub_rn(xk, X[r][c + 1])));
+        if (y > 0) a = __fadd_rn(a, __fmul_rn(at, __fsub_rn(xk, X[r - 1][c])));
+        if (y + 1 < h) a = __fadd_rn(a, __fmul_rn(ab, __fsub_rn(xk, X[r + 1][c])));
+        const float o = __fadd_rn(xk, __fmul_rn(__fmul_rn(MG_OMEGA, dk), __fsub_rn(bk, a)));
+        out[k] = o;
+        if (DOT) v[0] += (double)bk * (double)o;
     }
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= w || y >= h) return;
-    const size_t k = (size_t)y * w + i;
-    const int r = threadIdx.y + 1, c = threadIdx.x + 1;
-    const float xk = X[r][c];
-    float v = __fmul_rn(wd[k], xk);
-    if (i > 0) v = __fadd_rn(v, __fmul_rn(ax[k - 1], __fsub_rn(xk, X[r][c - 1])));
-    if (i + 1 < w) v = __fadd_rn(v, __fmul_rn(ax[k], __fsub_rn(xk, X[r][c + 1])));
-    if (y > 0) v = __fadd_rn(v, __fmul_rn(ay[k - w], __fsub_rn(xk, X[r - 1][c])));
-    if (y + 1 < h) v = __fadd_rn(v, __fmul_rn(ay[k], __fsub_rn(xk, X[r + 1][c])));
-    out[k] = __fadd_rn(xk, __fmul_rn(__fmul_rn(MG_OMEGA, dinv[k]), __fsub_rn(b[k], v)));
+    if (DOT && reduce_last(v, C.part, C.ctl + 2) && tid == 0) cg_rz(C, v[0]);
 }
 
 // The coarse end of the V-cycle (depth.rs:924 `vcycle` from level 0 of `T`
@@ -238,7 +471,6 @@ __global__ void __launch_bounds__(256) vc_up_kernel(const float* __restrict__ x,
 // sweep back up; __syncthreads between steps. The per-element arithmetic is
 // the separate kernels'. Each level's solution ends in its lv[].x (a sweep
 // writes r, then copies back), as the host-driven levels above expect.
-constexpr int MG_TAIL_CELLS = 8192, MG_TAIL_MAX = 16;
 struct MgTail {
     WlsLevel lv[MG_TAIL_MAX];
     int n;
@@ -278,12 +510,6 @@ __global__ void __launch_bounds__(1024) vcycle_tail_kernel(const MgTail T) {
         tail_sweep(L, false);
     }
 }
-// depth.rs:994 wd = max(conf, 0) + 1e-4
-__global__ void wd_kernel(const float* __restrict__ conf, float* __restrict__ wd, size_t n) {
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-        wd[k] = __fadd_rn(fmaxf(conf[k], 0.f), 1e-4f);
-}
-
 // depth.rs:677 `solve_rows` / :707 `solve_cols`: the Thomas algorithm along
 // every line, one thread per line, 32 lines per warp. The warp stages 32x32
 // tiles of the coefficients through shared memory with coalesced row-segment
@@ -717,10 +943,6 @@ static cudaError_t thomas(bool rows, float* u, const float* f, const float* wd, 
 // BF16 copies of the level operators and vectors, arithmetic in FP32; the
 // outer CG stays FP32 with FP64 dot products. No reference counterpart: the
 // reference's V-cycle is FP32 (vcycle_mode 0 here).
-typedef __nv_bfloat16 bf;
-__device__ __forceinline__ float ldh(const uint16_t* p, size_t k) { return __bfloat162float(((const bf*)p)[k]); }
-__device__ __forceinline__ void sth(uint16_t* p, size_t k, float v) { ((bf*)p)[k] = __float2bfloat16_rn(v); }
-
 __global__ void to_bf16_kernel(const float* __restrict__ a, uint16_t* __restrict__ o, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) sth(o, i, a[i]);
 }
@@ -817,29 +1039,38 @@ __global__ void __launch_bounds__(256) vc_down_h_kernel(const BT* __restrict__ b
 // Up: x2 = x1 + P x_c, then two sweeps; the result -> out (BF16, or level 0's FP32 z).
 // A 32 x 8 block of fine cells: x2 with a 2-cell ring, the first sweep with a 1-cell ring.
 constexpr int VH_U2W = 32 + 4, VH_U2H = 8 + 4, VH_U3W = 32 + 2, VH_U3H = 8 + 2;
-template <class BT, class OT>
+template <class BT, class OT, bool DOT>
 __global__ void __launch_bounds__(256) vc_up_h_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ xc, int cw,
                                                       const BT* __restrict__ b, const uint16_t* __restrict__ wd,
                                                       const uint16_t* __restrict__ ax, const uint16_t* __restrict__ ay,
-                                                      const uint16_t* __restrict__ dinv, OT* __restrict__ out, int w, int h) {
+                                                      const uint16_t* __restrict__ dinv, OT* __restrict__ out, int w, int h, const CgRef C) {
+    if (DOT && C.ctl[0]) return;
     __shared__ float X2[VH_U2H * VH_U2W], X3[VH_U3H * VH_U3W];
-    const int tid = threadIdx.y * 32 + threadIdx.x, fx = 32 * blockIdx.x, fy = 8 * blockIdx.y;
-    for (int e = tid; e < VH_U2W * VH_U2H; e += 256) {
-        const int r = e / VH_U2W, c = e - r * VH_U2W, gx = fx - 2 + c, gy = fy - 2 + r;
-        X2[e] = gx >= 0 && gx < w && gy >= 0 && gy < h ? rbf(ldh(x, (size_t)gy * w + gx) + ldh(xc, (size_t)(gy / 2) * cw + gx / 2)) : 0.f;
+    const int tx = (w + 31) / 32, nt = tx * ((h + 7) / 8), tid = threadIdx.y * 32 + threadIdx.x;
+    double v[1] = {0.0};
+    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
+        const int fx = t % tx * 32, fy = t / tx * 8;
+        if (DOT) __syncthreads();  // the tile before is done with X2 and X3
+        for (int e = tid; e < VH_U2W * VH_U2H; e += 256) {
+            const int r = e / VH_U2W, c = e - r * VH_U2W, gx = fx - 2 + c, gy = fy - 2 + r;
+            X2[e] = gx >= 0 && gx < w && gy >= 0 && gy < h ? rbf(ldh(x, (size_t)gy * w + gx) + ldh(xc, (size_t)(gy / 2) * cw + gx / 2)) : 0.f;
+        }
+        __syncthreads();
+        for (int e = tid; e < VH_U3W * VH_U3H; e += 256) {
+            const int r = e / VH_U3W, c = e - r * VH_U3W, gx = fx - 1 + c, gy = fy - 1 + r;
+            X3[e] = gx >= 0 && gx < w && gy >= 0 && gy < h
+                        ? rbf(sweep_tile<VH_U2W>(X2, r + 1, c + 1, ldv(b, (size_t)gy * w + gx), wd, ax, ay, dinv, w, h, gx, gy, 2))
+                        : 0.f;
+        }
+        __syncthreads();
+        const int i = fx + threadIdx.x, y = fy + threadIdx.y;
+        if (i >= w || y >= h) continue;
+        const size_t k = (size_t)y * w + i;
+        const float bk = ldv(b, k), o = sweep_tile<VH_U3W>(X3, threadIdx.y + 1, threadIdx.x + 1, bk, wd, ax, ay, dinv, w, h, i, y, 2);
+        stv(out, k, o);
+        if (DOT) v[0] += (double)bk * (double)o;
     }
-    __syncthreads();
-    for (int e = tid; e < VH_U3W * VH_U3H; e += 256) {
-        const int r = e / VH_U3W, c = e - r * VH_U3W, gx = fx - 1 + c, gy = fy - 1 + r;
-        X3[e] = gx >= 0 && gx < w && gy >= 0 && gy < h
-                    ? rbf(sweep_tile<VH_U2W>(X2, r + 1, c + 1, ldv(b, (size_t)gy * w + gx), wd, ax, ay, dinv, w, h, gx, gy, 2))
-                    : 0.f;
-    }
-    __syncthreads();
-    const int i = fx + threadIdx.x, y = fy + threadIdx.y;
-    if (i >= w || y >= h) return;
-    const size_t k = (size_t)y * w + i;
-    stv(out, k, sweep_tile<VH_U3W>(X3, threadIdx.y + 1, threadIdx.x + 1, ldv(b, k), wd, ax, ay, dinv, w, h, i, y, 2));
+    if (DOT && reduce_last(v, C.part, C.ctl + 2) && tid == 0) cg_rz(C, v[0]);
 }
 
 // The coarsest level's sweeps in one CTA of 32 x 32 threads with the level's planes in shared memory:
@@ -877,89 +1108,6 @@ __global__ void __launch_bounds__(1024) coarse_h_kernel(uint16_t* __restrict__ x
     __syncthreads();
     for (int k = tid; k < n; k += 1024) x[k] = src[k];
 }
-// depth.rs:1037 `dot`, f64 products: per-block partials, then the partials in order.
-// Each thread's products (exact in f64) summed in a fixed order: 16-byte loads of four elements
-// at a time when both planes allow them (more bytes in flight), the elements past the last four
-// by the first threads.
-__global__ void dot_partial_kernel(const float* __restrict__ a, const float* __restrict__ b, size_t n, double* part) {
-    double s = 0.0;
-    const size_t t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
-    const bool vec = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
-    const size_t n4 = vec ? n / 4 : 0;
-    const float4* a4 = reinterpret_cast<const float4*>(a);
-    const float4* b4 = reinterpret_cast<const float4*>(b);
-    for (size_t i = t0; i < n4; i += nt) {
-        const float4 x = __ldg(a4 + i), y = __ldg(b4 + i);
-        s += (double)x.x * (double)y.x;
-        s += (double)x.y * (double)y.y;
-        s += (double)x.z * (double)y.z;
-        s += (double)x.w * (double)y.w;
-    }
-    for (size_t i = 4 * n4 + t0; i < n; i += nt) s += (double)a[i] * (double)b[i];
-    __shared__ double red[256];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int st = 128; st > 0; st >>= 1) {
-        if (threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
-}
-// depth.rs:1039-1072, the CG scalars. mode: 0 rz; 1 pap -> alpha; 2 rz_new -> beta; 3 rr -> rel; 4 bb -> bnorm
-__global__ void dot_final_kernel(const double* part, int nparts, double* scal, float* ab, float* host_rel, int mode) {
-    // the partials summed by 256 threads (each a fixed stride of them), then a fixed tree
-    __shared__ double red[256];
-    double t = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += 256) t += part[i];
-    red[threadIdx.x] = t;
-    __syncthreads();
-    for (int st = 128; st > 0; st >>= 1) {
-        if (threadIdx.x < st) red[threadIdx.x] += red[threadIdx.x + st];
-        __syncthreads();
-    }
-    if (threadIdx.x != 0) return;
-    const double s = red[0];
-    if (mode == 0) scal[0] = s;
-    else if (mode == 1) {
-        scal[1] = s;
-        host_rel[1] = s <= 0.0 ? 1.f : 0.f;
-        ab[0] = s <= 0.0 ? 0.f : (float)(scal[0] / s);
-    } else if (mode == 2) {
-        ab[1] = (float)(s / scal[0]);
-        scal[0] = s;
-    } else if (mode == 3) {
-        scal[2] = s;
-        host_rel[0] = (float)(sqrt(s) / scal[3]);
-        host_rel[2] = 0.f;
-        ((double*)(host_rel + 4))[0] = sqrt(s) / scal[3];
-    } else {
-        scal[3] = fmax(sqrt(s), 1e-30);
-    }
-}
-// depth.rs:1064-1065: u += alpha p, r -= alpha Ap.
-__global__ void axpy2_kernel(float* __restrict__ u, const float* __restrict__ p, float* __restrict__ r, const float* __restrict__ ap,
-                             const float* ab, size_t n) {
-    const float alpha = ab[0];
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        u[i] = __fadd_rn(u[i], __fmul_rn(alpha, p[i]));
-        r[i] = __fsub_rn(r[i], __fmul_rn(alpha, ap[i]));
-    }
-}
-// depth.rs:1074: p = z + beta p.
-__global__ void pupd_kernel(float* __restrict__ p, const float* __restrict__ z, const float* ab, size_t n) {
-    const float beta = ab[1];
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        p[i] = __fadd_rn(z[i], __fmul_rn(beta, p[i]));
-}
-// depth.rs:1039: b = w d.
-__global__ void mul_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ o, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        o[i] = __fmul_rn(a[i], b[i]);
-}
-__global__ void fill_kernel(float* o, float v, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) o[i] = v;
-}
-
 WlsSolver* wls_alloc(int w, int h, cudaError_t* err) {
     *err = cudaSuccess;
     // set here, outside the graph captures of the CG iteration that launch it
@@ -992,10 +1140,11 @@ WlsSolver* wls_alloc(int w, int h, cudaError_t* err) {
             for (float** q : {&L.wd, &L.ax, &L.ay, &L.dinv, &L.x, &L.b, &L.r}) put(q, m);
             for (uint16_t** q : {&L.hwd, &L.hax, &L.hay, &L.hdinv, &L.hx, &L.hb, &L.hr}) put(q, m);
         }
-        for (float** q : {&S->ex, &S->ey, &S->cp, &S->dp, &S->f, &S->r, &S->z, &S->p, &S->ap}) put(q, n);
-        put(&S->part, (size_t)DOT_BLOCKS);
-        put(&S->scal, 8);
+        for (float** q : {&S->ex, &S->ey, &S->cp, &S->dp, &S->f, &S->r, &S->z, &S->p, &S->p2, &S->ap}) put(q, n);
+        put(&S->part, (size_t)2 * RED_BLOCKS);
+        put(&S->scal, 4);
         put(&S->alpha_beta, 4);
+        put(&S->ctl, 4);
         if (pass == 0) {
             S->bytes = at;
             *err = cudaMalloc(&S->slab, at);
@@ -1003,20 +1152,18 @@ WlsSolver* wls_alloc(int w, int h, cudaError_t* err) {
         }
     }
     if (cudaHostAlloc((void**)&S->host_rel, 64, cudaHostAllocDefault) != cudaSuccess) *err = cudaErrorMemoryAllocation;
+    for (cudaEvent_t& v : S->done)
+        if (*err == cudaSuccess) *err = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
     return S;
 }
 
-cudaError_t wls_prepare(WlsSolver* S, const float* guide, float lambda, float sigma_c, int edge_mode, cudaStream_t s) {
-    const int w = S->w, h = S->h;
+cudaError_t wls_prepare(WlsSolver* S, const float* guide, float lambda, float sigma_c, int edge_mode, cudaStream_t) {
     S->lambda = lambda;
-    const float inv = -1.0f / std::max(sigma_c, 1e-6f);
-    const float inv2s2 = 1.0f / (2.0f * sigma_c * sigma_c);
-    lsb_launched(), edge_kernel<<<g2(w, h), B2, 0, s>>>(guide, w, h, inv, inv2s2, edge_mode, lambda, S->ex, S->ey, S->lv[0].ax, S->lv[0].ay);
-    for (size_t l = 1; l < S->lv.size(); l++) {
-        const WlsLevel &F = S->lv[l - 1], &C = S->lv[l];
-        lsb_launched(), coarsen_edges_kernel<<<g2(C.w, C.h), B2, 0, s>>>(F.ax, F.ay, F.w, F.h, C.ax, C.ay, C.w, C.h);
-    }
-    return cudaGetLastError();
+    S->inv = -1.0f / std::max(sigma_c, 1e-6f);
+    S->inv2s2 = 1.0f / (2.0f * sigma_c * sigma_c);
+    S->edge_mode = edge_mode;
+    S->guide = guide;
+    return cudaSuccess;
 }
 
 int wls_width(const WlsSolver* s) { return s->w; }
@@ -1025,8 +1172,9 @@ size_t wls_bytes(const WlsSolver* s) { return s ? s->bytes : 0; }
 
 void wls_destroy(WlsSolver* s) {
     if (!s) return;
-    if (s->gA) cudaGraphExecDestroy(s->gA);
-    if (s->gB) cudaGraphExecDestroy(s->gB);
+    if (s->g) cudaGraphExecDestroy(s->g);
+    for (cudaEvent_t v : s->done)
+        if (v) cudaEventDestroy(v);
     if (s->slab) cudaFree(s->slab);
     if (s->host_rel) cudaFreeHost(s->host_rel);
     delete s;
@@ -1034,59 +1182,51 @@ void wls_destroy(WlsSolver* s) {
 
 int wls_levels(const WlsSolver* s) { return (int)s->lv.size(); }
 
-cudaError_t wls_set_weights(WlsSolver* S, const float* conf, cudaStream_t s) {
-    lsb_launched(), wd_kernel<<<g1((size_t)S->w * S->h), 256, 0, s>>>(conf, S->lv[0].wd, (size_t)S->w * S->h);
-    for (size_t l = 0; l < S->lv.size(); l++) {
+static bool tail_level(const WlsSolver* S, size_t l) {
+    return (size_t)S->lv[l].w * S->lv[l].h <= (size_t)MG_TAIL_CELLS && S->lv.size() - l <= (size_t)MG_TAIL_MAX;
+}
+static CgRef cg_ref(const WlsSolver* S) { return CgRef{S->part, S->scal, S->alpha_beta, S->ctl, (CgOut*)S->host_rel}; }
+
+// Every level's operators: level 0 in one pass, each large level in one from the finer one, the small ones in one CTA;
+// the edges too after a wls_prepare. mode 1: their BF16 copies on the levels its V-cycle visits. (As one kernel per
+// quantity and level, with the copies made in both modes, this was 44 launches of a few us for a 1024 x 768 grid.)
+cudaError_t wls_set_weights(WlsSolver* S, const float* conf, int mode, cudaStream_t s) {
+    const float* guide = S->guide;
+    S->guide = nullptr;
+    auto ops = [&](size_t l) {
         const WlsLevel& C = S->lv[l];
-        if (l > 0) {
-            const WlsLevel& F = S->lv[l - 1];
-            lsb_launched(), block_sum_kernel<<<g2(C.w, C.h), B2, 0, s>>>(F.wd, F.w, F.h, C.wd, C.w, C.h);
-        }
-        lsb_launched(), dinv_kernel<<<g2(C.w, C.h), B2, 0, s>>>(C.wd, C.ax, C.ay, C.w, C.h, C.dinv);
+        return mode == 1 && l < (size_t)MG_H_LEVELS ? HOps{C.hwd, C.hax, C.hay, C.hdinv} : HOps{};
+    };
+    const WlsLevel& Z = S->lv[0];
+    auto level0 = [&](auto k) {
+        lsb_launched(), k<<<g2(Z.w, Z.h), B2, 0, s>>>(guide, conf, Z.w, Z.h, S->inv, S->inv2s2, S->edge_mode, S->lambda, S->ex, S->ey, Z.ax, Z.ay,
+                                                    Z.wd, Z.dinv, ops(0));
+    };
+    if (guide) level0(level0_kernel<true>);
+    else level0(level0_kernel<false>);
+    size_t l = 1;
+    for (; l < S->lv.size() && !tail_level(S, l); l++) {
+        const WlsLevel &F = S->lv[l - 1], &C = S->lv[l];
+        if (guide) lsb_launched(), coarse_level_kernel<true><<<g2(C.w, C.h), B2, 0, s>>>(F, C, ops(l));
+        else lsb_launched(), coarse_level_kernel<false><<<g2(C.w, C.h), B2, 0, s>>>(F, C, ops(l));
     }
-    // the BF16 V-cycle's operators (levels 0 .. MG_H_LEVELS-1)
-    for (size_t l = 0; l < S->lv.size() && l < (size_t)MG_H_LEVELS; l++) {
-        const WlsLevel& C = S->lv[l];
-        const size_t m = (size_t)C.w * C.h;
-        const float* src[4] = {C.wd, C.ax, C.ay, C.dinv};
-        uint16_t* dst[4] = {C.hwd, C.hax, C.hay, C.hdinv};
-        for (int q = 0; q < 4; q++) lsb_launched(), to_bf16_kernel<<<g1(m), 256, 0, s>>>(src[q], dst[q], m);
+    if (l < S->lv.size()) {
+        MgSetup T;
+        T.n = 0;
+        for (size_t q = l - 1; q < S->lv.size(); q++, T.n++) T.lv[T.n] = S->lv[q], T.H[T.n] = ops(q);
+        if (guide) lsb_launched(), coarse_tail_kernel<true><<<1, 1024, 0, s>>>(T);
+        else lsb_launched(), coarse_tail_kernel<false><<<1, 1024, 0, s>>>(T);
     }
     return cudaGetLastError();
 }
 
-static void jacobi(WlsLevel& L, bool zero, cudaStream_t s) {
-    if (zero) {
-        lsb_launched(), jac0_kernel<<<g1((size_t)L.w * L.h), 256, 0, s>>>(L.b, L.dinv, L.x, (size_t)L.w * L.h);
-        return;
-    }
-    lsb_launched(), stencil_kernel<<<g2(L.w, L.h), B2, 0, s>>>(L.x, L.b, L.wd, L.ax, L.ay, L.dinv, L.r, L.w, L.h, 2);
-    std::swap(L.x, L.r);
-}
+static int red_grid(int w, int h) { return std::min(RED_BLOCKS, ((w + 31) / 32) * ((h + 7) / 8)); }
 
-static bool tail_level(const WlsSolver* S, size_t l) {
-    return (size_t)S->lv[l].w * S->lv[l].h <= (size_t)MG_TAIL_CELLS && S->lv.size() - l <= (size_t)MG_TAIL_MAX;
-}
-// depth.rs:924 `vcycle` on a level with a coarser one (MG_PRE = MG_POST = 1): down and up in one pass
-// each. The right-hand side is bin (null: the level's b); the result lands in xout (null: the level's
-// x, through its r buffer).
-static void vcycle(WlsSolver* S, size_t l, cudaStream_t s);
-static void vcycle_fused(WlsSolver* S, size_t l, const float* bin, float* xout, cudaStream_t s) {
+// depth.rs:924 `vcycle` (MG_PRE = MG_POST = 1): a level's way down and its way up in one pass each, the small levels in
+// one CTA (every chain of levels ends in them: the coarsest has at most 16 x 16 cells). The right-hand side is bin
+// (null: the level's b); the result lands in xout (null: the level's x, through its r buffer), with r.z at level 0.
+static void vcycle(WlsSolver* S, size_t l, const float* bin, float* xout, cudaStream_t s) {
     WlsLevel& T = S->lv[l];
-    WlsLevel& C = S->lv[l + 1];
-    const float* b = bin ? bin : T.b;
-    lsb_launched(), vc_down_kernel<<<g2(C.w, C.h), B2, 0, s>>>(b, T.wd, T.ax, T.ay, T.dinv, T.x, T.w, T.h, C.b, C.w, C.h);
-    vcycle(S, l + 1, s);
-    float* out = xout ? xout : T.r;
-    lsb_launched(), vc_up_kernel<<<g2(T.w, T.h), B2, 0, s>>>(T.x, C.x, C.w, b, T.wd, T.ax, T.ay, T.dinv, out, T.w, T.h);
-    if (!xout) std::swap(T.x, T.r);
-}
-static void vcycle(WlsSolver* S, size_t l, cudaStream_t s) {
-    WlsLevel& T = S->lv[l];
-    if (l + 1 < S->lv.size() && !tail_level(S, l)) {
-        vcycle_fused(S, l, nullptr, nullptr, s);
-        return;
-    }
     if (tail_level(S, l)) {
         MgTail tl;
         tl.n = (int)(S->lv.size() - l);
@@ -1094,17 +1234,17 @@ static void vcycle(WlsSolver* S, size_t l, cudaStream_t s) {
         lsb_launched(), vcycle_tail_kernel<<<1, 1024, 0, s>>>(tl);
         return;
     }
-    if (l + 1 == S->lv.size()) {
-        for (int k = 0; k < MG_COARSE; k++) jacobi(T, k == 0, s);
+    WlsLevel& C = S->lv[l + 1];
+    const float* b = bin ? bin : T.b;
+    lsb_launched(), vc_down_kernel<<<g2(C.w, C.h), B2, 0, s>>>(b, T.wd, T.ax, T.ay, T.dinv, T.x, T.w, T.h, C.b, C.w, C.h);
+    vcycle(S, l + 1, nullptr, nullptr, s);
+    if (xout) {
+        lsb_launched(), vc_up_kernel<true><<<red_grid(T.w, T.h), B2, 0, s>>>(T.x, C.x, C.w, b, T.wd, T.ax, T.ay, T.dinv, xout, T.w, T.h, cg_ref(S));
         return;
     }
-    jacobi(T, true, s);
-    lsb_launched(), stencil_kernel<<<g2(T.w, T.h), B2, 0, s>>>(T.x, T.b, T.wd, T.ax, T.ay, T.dinv, T.r, T.w, T.h, 1);
-    WlsLevel& C = S->lv[l + 1];
-    lsb_launched(), block_sum_kernel<<<g2(C.w, C.h), B2, 0, s>>>(T.r, T.w, T.h, C.b, C.w, C.h);
-    vcycle(S, l + 1, s);
-    lsb_launched(), prolong_kernel<<<g2(T.w, T.h), B2, 0, s>>>(T.x, T.w, T.h, C.x, C.w);
-    jacobi(T, false, s);
+    const int nt = ((T.w + 31) / 32) * ((T.h + 7) / 8);
+    lsb_launched(), vc_up_kernel<false><<<nt, B2, 0, s>>>(T.x, C.x, C.w, b, T.wd, T.ax, T.ay, T.dinv, T.r, T.w, T.h, cg_ref(S));
+    std::swap(T.x, T.r);
 }
 
 // A damped Jacobi sweep on level L (zero: the zero-start one) against its BF16 right-hand side:
@@ -1142,21 +1282,16 @@ static void vcycle_h(WlsSolver* S, size_t l, cudaStream_t s, const float* b32 = 
         lsb_launched(), vc_down_h_kernel<BT><<<g2(C.w, C.h), B2, 0, s>>>(b, T.hwd, T.hax, T.hay, T.hdinv, T.hx, T.w, T.h, C.hb, C.w, C.h);
         vcycle_h(S, l + 1, s);
         if (z32) {
-            lsb_launched(), vc_up_h_kernel<BT, float><<<g2(T.w, T.h), B2, 0, s>>>(T.hx, C.hx, C.w, b, T.hwd, T.hax, T.hay, T.hdinv, z32, T.w, T.h);
+            lsb_launched(), vc_up_h_kernel<BT, float, true><<<red_grid(T.w, T.h), B2, 0, s>>>(T.hx, C.hx, C.w, b, T.hwd, T.hax, T.hay, T.hdinv, z32,
+                                                                                             T.w, T.h, cg_ref(S));
         } else {
-            lsb_launched(), vc_up_h_kernel<BT, uint16_t><<<g2(T.w, T.h), B2, 0, s>>>(T.hx, C.hx, C.w, b, T.hwd, T.hax, T.hay, T.hdinv, T.hr, T.w,
-                                                                                    T.h);
+            lsb_launched(), vc_up_h_kernel<BT, uint16_t, false><<<((T.w + 31) / 32) * ((T.h + 7) / 8), B2, 0, s>>>(
+                T.hx, C.hx, C.w, b, T.hwd, T.hax, T.hay, T.hdinv, T.hr, T.w, T.h, cg_ref(S));
             std::swap(T.hx, T.hr);
         }
     };
     if (b32) down_up(b32);
     else down_up((const uint16_t*)T.hb);
-}
-
-static void dot(WlsSolver* S, const float* a, const float* b, size_t n, int mode, cudaStream_t s) {
-    int nb = (int)std::min<size_t>(DOT_BLOCKS, (n + 255) / 256);
-    lsb_launched(), dot_partial_kernel<<<nb, 256, 0, s>>>(a, b, n, S->part);
-    lsb_launched(), dot_final_kernel<<<1, 256, 0, s>>>(S->part, nb, S->scal, S->alpha_beta, S->host_rel, mode);
 }
 
 cudaError_t wls_solve(WlsSolver* S, const float* d, int max_iters, float* u, float* rel_out, int* iters_out, cudaStream_t s,
@@ -1186,10 +1321,13 @@ cudaError_t wls_solve(WlsSolver* S, const float* d, int max_iters, float* u, flo
             from = u;
         }
     }
-    // b = W d, |b|, r = b - A u, z = M r, p = z
-    lsb_launched(), mul_kernel<<<g1(n), 256, 0, s>>>(L0.wd, d, S->f, n);
-    dot(S, S->f, S->f, n, 4, s);
-    lsb_launched(), stencil_kernel<<<g2(w, h), B2, 0, s>>>(u, S->f, L0.wd, L0.ax, L0.ay, L0.dinv, S->r, w, h, 1);
+    const CgRef C = cg_ref(S);
+    CgOut* host = (CgOut*)S->host_rel;
+    // b = W d, |b|, r = b - A u; the reductions' ticket starts at 0, and every reduction leaves it there
+    if (!S->ctl_zero) cudaMemsetAsync(S->ctl, 0, 4 * sizeof(int), s), S->ctl_zero = true;
+    lsb_launched(), cg_start_kernel<<<red_grid(w, h), B2, 0, s>>>(d, u, L0.wd, L0.ax, L0.ay, S->r, w, h, C);
+    const int nb1 = (int)std::min<size_t>(RED_BLOCKS, (n + 255) / 256);
+    // z = M r and r.z
     auto precond = [&]() {
         if (mode == 1) {
             if (std::min(S->lv.size(), (size_t)MG_H_LEVELS) > 1) {  // r in, z out, no conversion passes
@@ -1199,91 +1337,66 @@ cudaError_t wls_solve(WlsSolver* S, const float* d, int max_iters, float* u, flo
             lsb_launched(), to_bf16_kernel<<<g1(n), 256, 0, s>>>(S->r, L0.hb, n);
             vcycle_h(S, 0, s);
             lsb_launched(), from_bf16_kernel<<<g1(n), 256, 0, s>>>(S->lv[0].hx, S->z, n);
-            return;
+        } else {
+            if (!tail_level(S, 0)) {  // r in, z out: no copies
+                vcycle(S, 0, S->r, S->z, s);
+                return;
+            }
+            cudaMemcpyAsync(L0.b, S->r, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
+            vcycle(S, 0, nullptr, nullptr, s);
+            cudaMemcpyAsync(S->z, S->lv[0].x, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
         }
-        if (S->lv.size() > 1 && !tail_level(S, 0)) {  // r in, z out: no copies
-            vcycle_fused(S, 0, S->r, S->z, s);
-            return;
-        }
-        cudaMemcpyAsync(L0.b, S->r, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
-        vcycle(S, 0, s);
-        cudaMemcpyAsync(S->z, S->lv[0].x, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
+        lsb_launched(), cg_rz_kernel<<<nb1, 256, 0, s>>>(S->r, S->z, n, C);
     };
-    precond();
-    cudaMemcpyAsync(S->p, S->z, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
-    dot(S, S->r, S->z, n, 0, s);
-    dot(S, S->r, S->r, n, 3, s);
-    cudaError_t e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return e;
-    float rel = S->host_rel[0];
-    int iters = 0;
-    auto partA = [&]() {
-        lsb_launched(), stencil_kernel<<<g2(w, h), B2, 0, s>>>(S->p, S->f, L0.wd, L0.ax, L0.ay, L0.dinv, S->ap, w, h, 0);
-        dot(S, S->p, S->ap, n, 1, s);
-        lsb_launched(), axpy2_kernel<<<g1(n), 256, 0, s>>>(u, S->p, S->r, S->ap, S->alpha_beta, n);
-        dot(S, S->r, S->r, n, 3, s);
-    };
-    auto partB = [&]() {
+    auto iteration = [&]() {
         precond();
-        dot(S, S->r, S->z, n, 2, s);
-        lsb_launched(), pupd_kernel<<<g1(n), 256, 0, s>>>(S->p, S->z, S->alpha_beta, n);
+        lsb_launched(), cg_dir_kernel<<<red_grid(w, h), B2, 0, s>>>(S->z, S->p, S->p2, L0.wd, L0.ax, L0.ay, S->ap, w, h, C);
+        lsb_launched(), cg_step_kernel<<<nb1, 256, 0, s>>>(u, S->p, S->p2, S->r, S->ap, n, max_iters, C);
     };
     // Every V-cycle restarts each level from zero, so which of a level's two buffers holds x
-    // carries nothing from one cycle to the next: one captured cycle serves every iteration.
-    auto capture = [&](const std::function<void()>& part, cudaGraphExec_t* ex, long long* kcount) -> bool {
+    // carries nothing from one cycle to the next: one captured iteration serves them all.
+    bool graph = max_iters > 0;
+    if (graph && (!S->g || S->g_u != u || S->g_mode != mode || S->g_max != max_iters)) {
+        if (S->g) cudaGraphExecDestroy(S->g);
+        S->g = nullptr;
         cudaGraph_t g = nullptr;
         const uint64_t c0 = lsb_launched_now();
-        if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return false;
-        part();
-        const cudaError_t ec = cudaStreamEndCapture(s, &g);
-        *kcount = (long long)(lsb_launched_now() - c0);
-        lsb_launched_add(-*kcount);  // captured, not launched
-        bool ok = ec == cudaSuccess && g && cudaGraphInstantiate(ex, g, 0) == cudaSuccess;
-        if (g) cudaGraphDestroy(g);
-        return ok;
-    };
-    bool graphs = max_iters > 0;
-    if (graphs && (!S->gA || S->g_u != u || S->g_mode != mode)) {
-        if (S->gA) cudaGraphExecDestroy(S->gA);
-        if (S->gB) cudaGraphExecDestroy(S->gB);
-        S->gA = S->gB = nullptr;
-        graphs = capture(partA, &S->gA, &S->kA) && capture(partB, &S->gB, &S->kB);
-        if (!graphs) {  // launch directly instead
-            if (S->gA) cudaGraphExecDestroy(S->gA);
-            if (S->gB) cudaGraphExecDestroy(S->gB);
-            S->gA = S->gB = nullptr;
-            cudaGetLastError();
-        } else {
-            S->g_u = u;
-            S->g_mode = mode;
+        if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+            iteration();
+            const cudaError_t ec = cudaStreamEndCapture(s, &g);
+            S->g_kernels = (long long)(lsb_launched_now() - c0);
+            lsb_launched_add(-S->g_kernels);  // captured, not launched
+            if (ec != cudaSuccess || !g || cudaGraphInstantiate(&S->g, g, 0) != cudaSuccess) S->g = nullptr;
+            if (g) cudaGraphDestroy(g);
         }
+        if (S->g) S->g_u = u, S->g_mode = mode, S->g_max = max_iters;
+        else cudaGetLastError(), graph = false;  // launched directly instead
     }
+    // Iterations are queued one ahead of the result the host has seen: the GPU does not wait for the host between
+    // them (25 us each), and the one queued past the last does nothing (every kernel that changes the solution, the
+    // residual or the result sees the stop word; the solution is the one a wait per iteration gives).
+    cudaError_t e = cudaSuccess;
     for (int it = 0; it < max_iters; it++) {
-        if (rel < 1e-5f) break;
-        iters++;
-        if (graphs) {
-            e = cudaGraphLaunch(S->gA, s);
+        if (it >= 2) {
+            e = cudaEventSynchronize(S->done[it & 1]);  // iteration it - 2
             if (e != cudaSuccess) return e;
-            lsb_launched_add(S->kA);
-        } else {
-            partA();
+            if (*(volatile int*)&host->stop) break;
         }
-        e = cudaStreamSynchronize(s);
+        if (graph) {
+            e = cudaGraphLaunch(S->g, s);
+            lsb_launched_add(S->g_kernels);
+        } else {
+            iteration();
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(S->done[it & 1], s);
         if (e != cudaSuccess) return e;
-        if (S->host_rel[1] != 0.f) break;  // p.Ap <= 0: alpha was 0, u and r are unchanged (depth.rs:1060)
-        rel = S->host_rel[0];
-        if (rel < 1e-5f) break;
-        if (graphs) {
-            e = cudaGraphLaunch(S->gB, s);
-            if (e != cudaSuccess) return e;
-            lsb_launched_add(S->kB);
-        } else {
-            partB();
-        }
     }
-    *rel_out = rel;
-    *iters_out = iters;
-    if (rel64) *rel64 = ((double*)(S->host_rel + 4))[0];
+    e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
+    *rel_out = host->rel;
+    *iters_out = host->iters;
+    if (rel64) *rel64 = host->rel64;
     return cudaGetLastError();
 }
 
