@@ -6,6 +6,7 @@
 // a relative residual of 1e-5. The f32 stencil, smoother, restriction and
 // prolongation follow the reference's operation order; the CG dot products
 // are f64 sums in a fixed two-stage order.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -17,12 +18,13 @@
 #include "lsb_depth.h"
 
 namespace lsb {
+namespace cg = cooperative_groups;
 
 constexpr float MG_OMEGA = 0.8f;
 constexpr int MG_COARSE = 32, MG_MIN = 16;
 // the BF16 V-cycle: levels, and Jacobi sweeps before and after the coarse correction
 constexpr int MG_H_LEVELS = 6, MG_H_SWEEPS = 2;
-// blocks of a kernel that reduces (persistent: each takes every so many tiles): 8 of 256 threads an SM
+// blocks of the element-wise kernels that reduce: 8 of 256 threads an SM
 constexpr int RED_BLOCKS = 148 * 8;
 
 struct WlsSolver {
@@ -137,11 +139,6 @@ __device__ __forceinline__ float block_sum_at(const float* src, int w, int h, in
     }
     return o;
 }
-__global__ void block_sum_kernel(const float* __restrict__ src, int w, int h, float* __restrict__ dst, int cw, int ch) {
-    const int xx = blockIdx.x * blockDim.x + threadIdx.x, yy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (xx >= cw || yy >= ch) return;
-    dst[(size_t)yy * cw + xx] = block_sum_at(src, w, h, xx, yy);
-}
 // One coarse cell of the hierarchy: its edges (EDGES; else those that are there), weight and diagonal from the finer level F.
 template <bool EDGES>
 __device__ __forceinline__ void coarse_cell(const WlsLevel& F, const WlsLevel& C, const HOps& H, int xx, int yy) {
@@ -187,21 +184,31 @@ __global__ void __launch_bounds__(1024) coarse_tail_kernel(const MgSetup T) {
         __syncthreads();
     }
 }
-// depth.rs:786 `apply`: mode 0 out = A x; 1 out = b - A x; 2 out = x + w D^-1 (b - A x)
-__device__ __forceinline__ float stencil_at(const float* __restrict__ x, const float* __restrict__ b, const float* __restrict__ wd,
-                                            const float* __restrict__ ax, const float* __restrict__ ay, const float* __restrict__ dinv,
-                                            int w, int h, int i, int y, int mode) {
-    const size_t k = (size_t)y * w + i;
-    const float xk = x[k];
-    float v = __fmul_rn(wd[k], xk);
-    if (i > 0) v = __fadd_rn(v, __fmul_rn(ax[k - 1], __fsub_rn(xk, x[k - 1])));
-    if (i + 1 < w) v = __fadd_rn(v, __fmul_rn(ax[k], __fsub_rn(xk, x[k + 1])));
-    if (y > 0) v = __fadd_rn(v, __fmul_rn(ay[k - w], __fsub_rn(xk, x[k - w])));
-    if (y + 1 < h) v = __fadd_rn(v, __fmul_rn(ay[k], __fsub_rn(xk, x[k + w])));
-    if (mode == 0) return v;
-    if (mode == 1) return __fsub_rn(b[k], v);
-    return __fadd_rn(xk, __fmul_rn(__fmul_rn(MG_OMEGA, dinv[k]), __fsub_rn(b[k], v)));
+// The level kernels walk strips: a warp takes 32 columns, of which the outer HALO on each side are only there for their
+// neighbours (they belong to the warps beside it), and goes down `rows` rows, so that a cell's left and right neighbours
+// come by shuffles, the upper and lower ones stay in registers, and the next row's operands are loaded while this one is
+// worked on: every plane is read about once, no shared memory and no barrier. What bounds it: HBM and L2 on large
+// grids, the latency of a row (about 1200 cycles, its loads) times the rows on small ones, hence fewer rows a strip there:
+// on 2120 x 1416 the direction's pass takes 20 us with 16 rows (28 with 4, 26 with 32, 35 from shared-memory tiles).
+struct Strip {
+    int rows, nx, warps;  // rows a strip, strips side by side, strips in all
+};
+static Strip strip_of(int w, int h, int halo) {
+    Strip S;
+    S.nx = (w + 32 - 2 * halo - 1) / (32 - 2 * halo);
+    S.rows = 32;  // an even number; at least 6 warps an SM scheduler where the level is large enough for that
+    while (S.rows > 4 && S.nx * ((h + S.rows - 1) / S.rows) < 148 * 24) S.rows /= 2;
+    S.warps = S.nx * ((h + S.rows - 1) / S.rows);
+    return S;
 }
+static int strip_blocks(const Strip& S) { return (S.warps + 7) / 8; }
+__device__ __forceinline__ float from_left(float v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ float from_right(float v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+// One row's operands of a lane's column (0 outside the grid).
+struct RowOps {
+    float wd, ax, ay, dinv, b;
+};
+
 // Sums over the grid of the CG's dot products (depth.rs:1037 `dot`: f64 products, each exact), taken by the kernel
 // that has the factors in registers: each thread's sum, the block's in a fixed tree, its place in `part`; the last
 // block to arrive adds the blocks' parts in a fixed order (the same values every run). True in that block, whose
@@ -275,67 +282,83 @@ __device__ __forceinline__ void cg_rel(const CgRef& C, double rr, int iters, boo
 // depth.rs:1039: b = W d, r = b - A u, |b| and |r|.
 __global__ void __launch_bounds__(256) cg_start_kernel(const float* __restrict__ d, const float* __restrict__ u, const float* __restrict__ wd,
                                                        const float* __restrict__ ax, const float* __restrict__ ay, float* __restrict__ r, int w,
-                                                       int h, const CgRef C) {
-    const int tx = (w + 31) / 32, nt = tx * ((h + 7) / 8);
+                                                       int h, const Strip S, const CgRef C) {
+    const int lane = threadIdx.x & 31, wid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int gx = wid % S.nx * 30 + lane - 1, y0 = wid / S.nx * S.rows, y1 = wid < S.warps ? min(h, y0 + S.rows) : 0;
+    const bool inx = gx >= 0 && gx < w, own = lane >= 1 && lane <= 30 && gx < w;
+    auto U = [&](int y) { return inx && y >= 0 && y < h ? u[(size_t)y * w + gx] : 0.f; };
     double v[2] = {0.0, 0.0};
-    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int i = t % tx * 32 + threadIdx.x, y = t / tx * 8 + threadIdx.y;
-        if (i >= w || y >= h) continue;
-        const size_t k = (size_t)y * w + i;
-        const float bk = __fmul_rn(wd[k], d[k]);
-        const float rv = __fsub_rn(bk, stencil_at(u, nullptr, wd, ax, ay, nullptr, w, h, i, y, 0));
-        r[k] = rv;
-        v[0] += (double)bk * (double)bk;
-        v[1] += (double)rv * (double)rv;
+    if (y0 < y1) {
+        float um = U(y0 - 1), uc = U(y0), aym = inx && y0 > 0 ? ay[(size_t)(y0 - 1) * w + gx] : 0.f;
+#pragma unroll 2
+        for (int y = y0; y < y1; y++) {
+            const size_t k = (size_t)y * w + gx;
+            const float un = U(y + 1), wk = inx ? wd[k] : 0.f, axk = inx ? ax[k] : 0.f, ayk = inx ? ay[k] : 0.f, dk = inx ? d[k] : 0.f;
+            const float ul = from_left(uc), ur = from_right(uc), al = from_left(axk);
+            if (own) {
+                const float bk = __fmul_rn(wk, dk);
+                float a = __fmul_rn(wk, uc);
+                if (gx > 0) a = __fadd_rn(a, __fmul_rn(al, __fsub_rn(uc, ul)));
+                if (gx + 1 < w) a = __fadd_rn(a, __fmul_rn(axk, __fsub_rn(uc, ur)));
+                if (y > 0) a = __fadd_rn(a, __fmul_rn(aym, __fsub_rn(uc, um)));
+                if (y + 1 < h) a = __fadd_rn(a, __fmul_rn(ayk, __fsub_rn(uc, un)));
+                const float rv = __fsub_rn(bk, a);
+                r[k] = rv;
+                v[0] += (double)bk * (double)bk;
+                v[1] += (double)rv * (double)rv;
+            }
+            um = uc;
+            uc = un;
+            aym = ayk;
+        }
     }
-    if (reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0 && threadIdx.y == 0) {
+    if (reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0) {
         C.scal[1] = fmax(sqrt(v[0]), 1e-30);
         cg_rel(C, v[1], 0, false);
     }
 }
-// depth.rs:1074 p = z + beta p, then depth.rs:1056 A p and p.Ap -> alpha: the direction of a tile and its ring computed
-// into shared memory from z and the last direction, which stays in the other buffer (neighbours read it).
+// depth.rs:1074 p = z + beta p, then depth.rs:1056 A p and p.Ap -> alpha: the direction computed from z and the last one,
+// which stays in the other buffer (the strips beside read it).
 __global__ void __launch_bounds__(256) cg_dir_kernel(const float* __restrict__ z, float* p0, float* p1, const float* __restrict__ wd,
                                                      const float* __restrict__ ax, const float* __restrict__ ay, float* __restrict__ ap, int w,
-                                                     int h, const CgRef C) {
+                                                     int h, const Strip S, const CgRef C) {
     if (C.ctl[0]) return;
-    __shared__ float P[10][34];
-    const int it = C.ctl[1], tx = (w + 31) / 32, nt = tx * ((h + 7) / 8), tid = threadIdx.y * 32 + threadIdx.x;
+    const int it = C.ctl[1], lane = threadIdx.x & 31, wid = blockIdx.x * 8 + (threadIdx.x >> 5);
     const bool first = it == 0;
     const float beta = C.ab[1];
-    const float* old = it & 1 ? p1 : p0;
-    float* now = it & 1 ? p0 : p1;
+    const float* __restrict__ old = it & 1 ? p1 : p0;
+    float* __restrict__ now = it & 1 ? p0 : p1;
+    const int gx = wid % S.nx * 30 + lane - 1, y0 = wid / S.nx * S.rows, y1 = wid < S.warps ? min(h, y0 + S.rows) : 0;
+    const bool inx = gx >= 0 && gx < w, own = lane >= 1 && lane <= 30 && gx < w;
+    auto P = [&](int y) {
+        if (!inx || y < 0 || y >= h) return 0.f;
+        const size_t k = (size_t)y * w + gx;
+        return first ? z[k] : __fadd_rn(z[k], __fmul_rn(beta, old[k]));
+    };
     double v[1] = {0.0};
-    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int x0 = t % tx * 32, y0 = t / tx * 8;
-        const int i = x0 + threadIdx.x, y = y0 + threadIdx.y;
-        const bool in = i < w && y < h;
-        const size_t k = in ? (size_t)y * w + i : 0;
-        const float wk = wd[k], ar = ax[k], al = k > 0 ? ax[k - 1] : 0.f, ab = ay[k], at = k >= (size_t)w ? ay[k - w] : 0.f;
-        __syncthreads();  // the tile before is done with P
-        for (int e = tid; e < 10 * 34; e += 256) {
-            const int rr = e / 34, c = e - rr * 34, gx = x0 - 1 + c, gy = y0 - 1 + rr;
-            float pv = 0.f;
-            if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-                const size_t q = (size_t)gy * w + gx;
-                pv = first ? z[q] : __fadd_rn(z[q], __fmul_rn(beta, old[q]));
+    if (y0 < y1) {
+        float pm = P(y0 - 1), pc = P(y0), aym = inx && y0 > 0 ? ay[(size_t)(y0 - 1) * w + gx] : 0.f;
+#pragma unroll 2
+        for (int y = y0; y < y1; y++) {
+            const size_t k = (size_t)y * w + gx;
+            const float pn = P(y + 1), wk = inx ? wd[k] : 0.f, axk = inx ? ax[k] : 0.f, ayk = inx ? ay[k] : 0.f;
+            const float pl = from_left(pc), pr = from_right(pc), al = from_left(axk);
+            if (own) {
+                float a = __fmul_rn(wk, pc);
+                if (gx > 0) a = __fadd_rn(a, __fmul_rn(al, __fsub_rn(pc, pl)));
+                if (gx + 1 < w) a = __fadd_rn(a, __fmul_rn(axk, __fsub_rn(pc, pr)));
+                if (y > 0) a = __fadd_rn(a, __fmul_rn(aym, __fsub_rn(pc, pm)));
+                if (y + 1 < h) a = __fadd_rn(a, __fmul_rn(ayk, __fsub_rn(pc, pn)));
+                now[k] = pc;
+                ap[k] = a;
+                v[0] += (double)pc * (double)a;
             }
-            P[rr][c] = pv;
+            pm = pc;
+            pc = pn;
+            aym = ayk;
         }
-        __syncthreads();
-        if (!in) continue;
-        const int r = threadIdx.y + 1, c = threadIdx.x + 1;
-        const float xk = P[r][c];
-        float a = __fmul_rn(wk, xk);
-        if (i > 0) a = __fadd_rn(a, __fmul_rn(al, __fsub_rn(xk, P[r][c - 1])));
-        if (i + 1 < w) a = __fadd_rn(a, __fmul_rn(ar, __fsub_rn(xk, P[r][c + 1])));
-        if (y > 0) a = __fadd_rn(a, __fmul_rn(at, __fsub_rn(xk, P[r - 1][c])));
-        if (y + 1 < h) a = __fadd_rn(a, __fmul_rn(ab, __fsub_rn(xk, P[r + 1][c])));
-        now[k] = xk;
-        ap[k] = a;
-        v[0] += (double)xk * (double)a;
     }
-    if (reduce_last(v, C.part, C.ctl + 2) && tid == 0) {
+    if (reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0) {
         // p.Ap <= 0: alpha 0, u and r stay as they are and the iteration ends (depth.rs:1060)
         C.ab[0] = v[0] <= 0.0 ? 0.f : (float)(C.scal[0] / v[0]);
         C.ctl[3] = v[0] <= 0.0;
@@ -380,136 +403,257 @@ __global__ void __launch_bounds__(256) cg_rz_kernel(const float* __restrict__ r,
     if (reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0) cg_rz(C, v[0]);
 }
 
-// One fine level's way down the V-cycle in one pass (depth.rs:924-930): the zero-start Jacobi sweep
-// x = w D^-1 b (depth.rs:840), the residual b - A x (depth.rs:786) and its restriction to the coarse
-// right-hand side (depth.rs:911), one thread per coarse cell and its 2x2 fine cells; the neighbours'
-// x are recomputed from b and D^-1 by the same product, so every value is the separate kernels' own.
-__device__ __forceinline__ float jac0_at(const float* __restrict__ b, const float* __restrict__ dinv, size_t k) {
-    return __fmul_rn(__fmul_rn(MG_OMEGA, dinv[k]), b[k]);
-}
-// A 32 x 8 block of coarse cells covers 64 x 16 fine cells: their x and a one-cell ring are
-// computed once into shared memory, and every fine cell's residual reads its neighbours there.
-constexpr int VC_FW = 2 * 32 + 2, VC_FH = 2 * 8 + 2;
+// One fine level's way down the V-cycle in one pass (depth.rs:924-930): the zero-start Jacobi sweep x = w D^-1 b
+// (depth.rs:840), the residual b - A x (depth.rs:786) and its restriction to the coarse right-hand side (depth.rs:911).
+// A lane's pair of columns (even, odd) belongs to one coarse cell: the odd one's residual comes by a shuffle.
 __global__ void __launch_bounds__(256) vc_down_kernel(const float* __restrict__ b, const float* __restrict__ wd, const float* __restrict__ ax,
                                                       const float* __restrict__ ay, const float* __restrict__ dinv, float* __restrict__ x,
-                                                      int w, int h, float* __restrict__ cb, int cw, int ch) {
-    __shared__ float J[VC_FH][VC_FW];
-    const int fx0 = 2 * blockIdx.x * blockDim.x - 1, fy0 = 2 * blockIdx.y * blockDim.y - 1;
-    for (int e = threadIdx.y * blockDim.x + threadIdx.x; e < VC_FW * VC_FH; e += blockDim.x * blockDim.y) {
-        const int r = e / VC_FW, c = e - r * VC_FW, gx = fx0 + c, gy = fy0 + r;
-        J[r][c] = gx >= 0 && gx < w && gy >= 0 && gy < h ? jac0_at(b, dinv, (size_t)gy * w + gx) : 0.f;
-    }
-    __syncthreads();
-    const int xx = blockIdx.x * blockDim.x + threadIdx.x, yy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (xx >= cw || yy >= ch) return;
-    float o = 0.f;
-    for (int y = 2 * yy; y < min(2 * yy + 2, h); y++) {
-        float rs = 0.f;
-        const int jr = y - fy0;
-        for (int i = 2 * xx; i < min(2 * xx + 2, w); i++) {
-            const size_t k = (size_t)y * w + i;
-            const int jc = i - fx0;
-            const float xk = J[jr][jc];
-            x[k] = xk;
-            float v = __fmul_rn(wd[k], xk);
-            if (i > 0) v = __fadd_rn(v, __fmul_rn(ax[k - 1], __fsub_rn(xk, J[jr][jc - 1])));
-            if (i + 1 < w) v = __fadd_rn(v, __fmul_rn(ax[k], __fsub_rn(xk, J[jr][jc + 1])));
-            if (y > 0) v = __fadd_rn(v, __fmul_rn(ay[k - w], __fsub_rn(xk, J[jr - 1][jc])));
-            if (y + 1 < h) v = __fadd_rn(v, __fmul_rn(ay[k], __fsub_rn(xk, J[jr + 1][jc])));
-            rs = __fadd_rn(rs, __fsub_rn(b[k], v));
+                                                      int w, int h, float* __restrict__ cb, int cw, const Strip S) {
+    const int lane = threadIdx.x & 31, wid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (wid >= S.warps) return;
+    const int gx = wid % S.nx * 30 + lane - 1, y0 = wid / S.nx * S.rows, y1 = min(h, y0 + S.rows);
+    const bool inx = gx >= 0 && gx < w, own = lane >= 1 && lane <= 30 && gx < w;
+    float bc = 0.f, bn = 0.f;  // b of this row and the next
+    auto J = [&](int y, float& bv) {
+        bv = 0.f;
+        if (!inx || y < 0 || y >= h) return 0.f;
+        const size_t k = (size_t)y * w + gx;
+        bv = b[k];
+        return __fmul_rn(__fmul_rn(MG_OMEGA, dinv[k]), bv);
+    };
+    float xm = J(y0 - 1, bc), xc = J(y0, bc), aym = inx && y0 > 0 ? ay[(size_t)(y0 - 1) * w + gx] : 0.f, o = 0.f;
+#pragma unroll 2
+    for (int y = y0; y < y1; y++) {
+        const size_t k = (size_t)y * w + gx;
+        const float xn = J(y + 1, bn), wk = inx ? wd[k] : 0.f, axk = inx ? ax[k] : 0.f, ayk = inx ? ay[k] : 0.f;
+        const float xl = from_left(xc), xr = from_right(xc), al = from_left(axk);
+        float r = 0.f;
+        if (own) {
+            float v = __fmul_rn(wk, xc);
+            if (gx > 0) v = __fadd_rn(v, __fmul_rn(al, __fsub_rn(xc, xl)));
+            if (gx + 1 < w) v = __fadd_rn(v, __fmul_rn(axk, __fsub_rn(xc, xr)));
+            if (y > 0) v = __fadd_rn(v, __fmul_rn(aym, __fsub_rn(xc, xm)));
+            if (y + 1 < h) v = __fadd_rn(v, __fmul_rn(ayk, __fsub_rn(xc, xn)));
+            r = __fsub_rn(bc, v);
+            x[k] = xc;
         }
-        o = __fadd_rn(o, rs);
+        const float r1 = from_right(r);  // strips start at even columns and rows
+        float rs = __fadd_rn(0.f, r);
+        if (gx + 1 < w) rs = __fadd_rn(rs, r1);
+        o = __fadd_rn(y & 1 ? o : 0.f, rs);
+        if (own && !(gx & 1) && ((y & 1) || y + 1 == h)) cb[(size_t)(y >> 1) * cw + (gx >> 1)] = o;
+        xm = xc;
+        xc = xn;
+        bc = bn;
+        aym = ayk;
     }
-    cb[(size_t)yy * cw + xx] = o;
 }
-// ... and its way up in one pass (depth.rs:932-946): the prolongation x += P x_c (depth.rs:901) and the
-// damped Jacobi sweep (depth.rs:837) on the corrected x, the neighbours' corrected x recomputed by the
-// same addition; into out (another buffer than x).
-__device__ __forceinline__ float prolonged_at(const float* __restrict__ x, const float* __restrict__ xc, int w, int cw, int i, int y) {
-    return __fadd_rn(x[(size_t)y * w + i], xc[(size_t)(y >> 1) * cw + (i >> 1)]);
-}
-// The block's 32 x 8 corrected x and a one-cell ring are computed once into shared memory, the cell's own operands
-// loaded before. DOT (level 0): persistent over the tiles, r.z taken on the way (b is the CG's r).
+// ... and its way up in one pass (depth.rs:932-946): the prolongation x += P x_c (depth.rs:901) and the damped Jacobi
+// sweep (depth.rs:837) on the corrected x, into out (another buffer than x). DOT (level 0): r.z taken on the way (b is
+// the CG's r).
 template <bool DOT>
-__global__ void __launch_bounds__(256) vc_up_kernel(const float* __restrict__ x, const float* __restrict__ xc, int cw,
+__global__ void __launch_bounds__(256) vc_up_kernel(const float* __restrict__ x, const float* __restrict__ xc_, int cw,
                                                     const float* __restrict__ b, const float* __restrict__ wd,
                                                     const float* __restrict__ ax, const float* __restrict__ ay,
-                                                    const float* __restrict__ dinv, float* __restrict__ out, int w, int h, const CgRef C) {
+                                                    const float* __restrict__ dinv, float* __restrict__ out, int w, int h, const Strip S,
+                                                    const CgRef C) {
     if (DOT && C.ctl[0]) return;
-    __shared__ float X[8 + 2][32 + 2];
-    const int tx = (w + 31) / 32, nt = tx * ((h + 7) / 8), tid = threadIdx.y * 32 + threadIdx.x;
+    const int lane = threadIdx.x & 31, wid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int gx = wid % S.nx * 30 + lane - 1, y0 = wid / S.nx * S.rows, y1 = wid < S.warps ? min(h, y0 + S.rows) : 0;
+    const bool inx = gx >= 0 && gx < w, own = lane >= 1 && lane <= 30 && gx < w;
+    auto X = [&](int y) { return inx && y >= 0 && y < h ? __fadd_rn(x[(size_t)y * w + gx], xc_[(size_t)(y >> 1) * cw + (gx >> 1)]) : 0.f; };
     double v[1] = {0.0};
-    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int x0 = t % tx * 32, y0 = t / tx * 8, i = x0 + threadIdx.x, y = y0 + threadIdx.y;
-        const bool in = i < w && y < h;
-        const size_t k = in ? (size_t)y * w + i : 0;
-        const float bk = b[k], wk = wd[k], dk = dinv[k], ar = ax[k], al = k > 0 ? ax[k - 1] : 0.f, ab = ay[k], at = k >= (size_t)w ? ay[k - w] : 0.f;
-        if (DOT) __syncthreads();  // the tile before is done with X
-        for (int e = tid; e < 10 * 34; e += 256) {
-            const int r = e / 34, c = e - r * 34, gx = x0 - 1 + c, gy = y0 - 1 + r;
-            X[r][c] = gx >= 0 && gx < w && gy >= 0 && gy < h ? prolonged_at(x, xc, w, cw, gx, gy) : 0.f;
+    if (y0 < y1) {
+        float xm = X(y0 - 1), xc = X(y0), aym = inx && y0 > 0 ? ay[(size_t)(y0 - 1) * w + gx] : 0.f;
+#pragma unroll 2
+        for (int y = y0; y < y1; y++) {
+            const size_t k = (size_t)y * w + gx;
+            const float xn = X(y + 1), wk = inx ? wd[k] : 0.f, axk = inx ? ax[k] : 0.f, ayk = inx ? ay[k] : 0.f, bk = inx ? b[k] : 0.f,
+                        dk = inx ? dinv[k] : 0.f;
+            const float xl = from_left(xc), xr = from_right(xc), al = from_left(axk);
+            if (own) {
+                float a = __fmul_rn(wk, xc);
+                if (gx > 0) a = __fadd_rn(a, __fmul_rn(al, __fsub_rn(xc, xl)));
+                if (gx + 1 < w) a = __fadd_rn(a, __fmul_rn(axk, __fsub_rn(xc, xr)));
+                if (y > 0) a = __fadd_rn(a, __fmul_rn(aym, __fsub_rn(xc, xm)));
+                if (y + 1 < h) a = __fadd_rn(a, __fmul_rn(ayk, __fsub_rn(xc, xn)));
+                const float o = __fadd_rn(xc, __fmul_rn(__fmul_rn(MG_OMEGA, dk), __fsub_rn(bk, a)));
+                out[k] = o;
+                if (DOT) v[0] += (double)bk * (double)o;
+            }
+            xm = xc;
+            xc = xn;
+            aym = ayk;
         }
-        __syncthreads();
-        if (!in) continue;
-        const int r = threadIdx.y + 1, c = threadIdx.x + 1;
-        const float xk = X[r][c];
-        float a = __fmul_rn(wk, xk);
-        if (i > 0) a = __fadd_rn(a, __fmul_rn(al, __fsub_rn(xk, X[r][c - 1])));
-        if (i + 1 < w) a = __fadd_rn(a, __fmul_rn(ar, __fsub_rn(xk, X[r][c + 1])));
-        if (y > 0) a = __fadd_rn(a, __fmul_rn(at, __fsub_rn(xk, X[r - 1][c])));
-        if (y + 1 < h) a = __fadd_rn(a, __fmul_rn(ab, __fsub_rn(xk, X[r + 1][c])));
-        const float o = __fadd_rn(xk, __fmul_rn(__fmul_rn(MG_OMEGA, dk), __fsub_rn(bk, a)));
-        out[k] = o;
-        if (DOT) v[0] += (double)bk * (double)o;
     }
-    if (DOT && reduce_last(v, C.part, C.ctl + 2) && tid == 0) cg_rz(C, v[0]);
+    if (DOT && reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0) cg_rz(C, v[0]);
 }
 
-// The coarse end of the V-cycle (depth.rs:924 `vcycle` from level 0 of `T`
-// down) in ONE CTA: each level's zero-start Jacobi, residual, restriction,
-// the coarsest level's MG_COARSE sweeps, then prolongation and the smoothing
-// sweep back up; __syncthreads between steps. The per-element arithmetic is
-// the separate kernels'. Each level's solution ends in its lv[].x (a sweep
-// writes r, then copies back), as the host-driven levels above expect.
+__device__ __forceinline__ void cp_async4f(float* smem, const float* gmem) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem));
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+// The coarse end of the V-cycle (depth.rs:924 `vcycle` from level 0 of `T` down) in ONE CTA: each level's zero-start
+// Jacobi, residual and restriction, the coarsest level's MG_COARSE sweeps, then prolongation and the smoothing sweep
+// back up. The per-element arithmetic is the separate kernels'. The levels' x and b live in shared memory, and below
+// the first level their operators too (copied while the first level is worked on); the coarsest level (at most 256
+// cells) is one cell per thread with its operators in registers and x in two shared buffers, one barrier a sweep.
+// What bounds it: latency, barrier by barrier (MG_COARSE of its about 45 are the sweeps'). With everything in global
+// memory and two barriers a sweep it took 22 to 27 us of an iteration, 14 to 20 here (one SM's instruction rate).
 struct MgTail {
     WlsLevel lv[MG_TAIL_MAX];
     int n;
 };
-__device__ __forceinline__ void tail_sweep(const WlsLevel& L, bool zero) {
-    const int n = L.w * L.h;
-    if (zero) {
-        for (int k = threadIdx.x; k < n; k += blockDim.x) L.x[k] = __fmul_rn(__fmul_rn(MG_OMEGA, L.dinv[k]), L.b[k]);
-        __syncthreads();
-        return;
-    }
-    for (int k = threadIdx.x; k < n; k += blockDim.x) L.r[k] = stencil_at(L.x, L.b, L.wd, L.ax, L.ay, L.dinv, L.w, L.h, k % L.w, k / L.w, 2);
-    __syncthreads();
-    for (int k = threadIdx.x; k < n; k += blockDim.x) L.x[k] = L.r[k];
-    __syncthreads();
+constexpr int TAIL_THREADS = 1024, TAIL_PER = MG_TAIL_CELLS / TAIL_THREADS;
+// floats of shared memory: x and b of every level, the operators (wd, ax, ay, dinv) below the first, a spare x for the coarsest
+static size_t tail_floats(const WlsSolver* S, size_t l) {
+    size_t f = 256;
+    for (size_t q = l; q < S->lv.size(); q++) f += (size_t)S->lv[q].w * S->lv[q].h * (q == l ? 2 : 6);
+    return f;
 }
-// depth.rs:924 `vcycle` from the first level small enough for one CTA down to the coarsest.
-__global__ void __launch_bounds__(1024) vcycle_tail_kernel(const MgTail T) {
+constexpr size_t TAIL_MAX_SMEM = 220 * 1024;
+struct TailOps {  // a level's operators and vectors as the tail reads them
+    const float *wd, *ax, *ay, *dinv;
+    float *x, *b;
+    int w, h;
+};
+// A x of one cell: the neighbours from x, in the order left, right, up, down (depth.rs:786)
+__device__ __forceinline__ float tail_apply(const TailOps& L, int k, int i, int y) {
+    const float xk = L.x[k];
+    float v = __fmul_rn(L.wd[k], xk);
+    if (i > 0) v = __fadd_rn(v, __fmul_rn(L.ax[k - 1], __fsub_rn(xk, L.x[k - 1])));
+    if (i + 1 < L.w) v = __fadd_rn(v, __fmul_rn(L.ax[k], __fsub_rn(xk, L.x[k + 1])));
+    if (y > 0) v = __fadd_rn(v, __fmul_rn(L.ay[k - L.w], __fsub_rn(xk, L.x[k - L.w])));
+    if (y + 1 < L.h) v = __fadd_rn(v, __fmul_rn(L.ay[k], __fsub_rn(xk, L.x[k + L.w])));
+    return v;
+}
+__global__ void __launch_bounds__(TAIL_THREADS) vcycle_tail_kernel(const MgTail T) {
+    extern __shared__ float tail_sm[];
+    const int tid = threadIdx.x;
+    // where level l lies (the few levels are walked again by every thread: no table to wait for)
+    auto level = [&](int l) {
+        float* at = tail_sm + 256;
+        TailOps L{};
+        for (int q = 0; q <= l; q++) {
+            const WlsLevel& G = T.lv[q];
+            const int n = G.w * G.h;
+            L.w = G.w;
+            L.h = G.h;
+            L.x = at;
+            L.b = at + n;
+            if (q == 0) {
+                L.wd = G.wd, L.ax = G.ax, L.ay = G.ay, L.dinv = G.dinv;
+                at += 2 * n;
+            } else {
+                L.wd = at + 2 * n, L.ax = at + 3 * n, L.ay = at + 4 * n, L.dinv = at + 5 * n;
+                at += 6 * n;
+            }
+        }
+        return L;
+    };
+    // the operators below the first level, on their way while it is worked on
+    for (int l = 1; l < T.n; l++) {
+        const WlsLevel& G = T.lv[l];
+        const TailOps L = level(l);
+        const int n = G.w * G.h;
+        for (int k = tid; k < n; k += TAIL_THREADS) {
+            cp_async4f(const_cast<float*>(L.wd) + k, G.wd + k);
+            cp_async4f(const_cast<float*>(L.ax) + k, G.ax + k);
+            cp_async4f(const_cast<float*>(L.ay) + k, G.ay + k);
+            cp_async4f(const_cast<float*>(L.dinv) + k, G.dinv + k);
+        }
+    }
+    cp_commit();
     for (int l = 0; l + 1 < T.n; l++) {
-        const WlsLevel &L = T.lv[l], &C = T.lv[l + 1];
-        tail_sweep(L, true);
-        for (int k = threadIdx.x; k < L.w * L.h; k += blockDim.x)
-            L.r[k] = stencil_at(L.x, L.b, L.wd, L.ax, L.ay, L.dinv, L.w, L.h, k % L.w, k / L.w, 1);
+        const TailOps L = level(l), C = level(l + 1);
+        const int n = L.w * L.h;
+        if (l == 0)
+            for (int k = tid; k < n; k += TAIL_THREADS) L.b[k] = T.lv[0].b[k];
+        for (int k = tid; k < n; k += TAIL_THREADS) L.x[k] = __fmul_rn(__fmul_rn(MG_OMEGA, L.dinv[k]), L.b[k]);
         __syncthreads();
-        for (int k = threadIdx.x; k < C.w * C.h; k += blockDim.x) C.b[k] = block_sum_at(L.r, L.w, L.h, k % C.w, k / C.w);
+        // the residual's 2x2 block sums, a coarse cell per thread
+        for (int k = tid; k < C.w * C.h; k += TAIL_THREADS) {
+            const int xx = k % C.w, yy = k / C.w;
+            float o = 0.f;
+            for (int y = 2 * yy; y < min(2 * yy + 2, L.h); y++) {
+                float rs = 0.f;
+                for (int x = 2 * xx; x < min(2 * xx + 2, L.w); x++) {
+                    const int q = y * L.w + x;
+                    rs = __fadd_rn(rs, __fsub_rn(L.b[q], tail_apply(L, q, x, y)));
+                }
+                o = __fadd_rn(o, rs);
+            }
+            C.b[k] = o;
+        }
+        if (l == 0) cp_wait<0>();
         __syncthreads();
     }
-    const WlsLevel& Z = T.lv[T.n - 1];
-    for (int it = 0; it < MG_COARSE; it++) tail_sweep(Z, it == 0);
-    for (int l = T.n - 2; l >= 0; l--) {
-        const WlsLevel &L = T.lv[l], &C = T.lv[l + 1];
-        for (int k = threadIdx.x; k < L.w * L.h; k += blockDim.x) {
-            const int i = k % L.w, y = k / L.w;
-            L.x[k] = __fadd_rn(L.x[k], C.x[(size_t)(y / 2) * C.w + i / 2]);
+    {
+        const TailOps Z = level(T.n - 1);
+        const int n = Z.w * Z.h;
+        if (T.n == 1) {
+            for (int k = tid; k < n; k += TAIL_THREADS) Z.b[k] = T.lv[0].b[k];
+            __syncthreads();
+        }
+        const bool mine = tid < n;  // the coarsest level: at most MG_MIN x MG_MIN = 256 cells
+        const int i = tid % Z.w, y = tid / Z.w;
+        const bool l = mine && i > 0, r = mine && i + 1 < Z.w, t = mine && y > 0, b = mine && y + 1 < Z.h;
+        const float wk = mine ? Z.wd[tid] : 0.f, od = mine ? __fmul_rn(MG_OMEGA, Z.dinv[tid]) : 0.f, bk = mine ? Z.b[tid] : 0.f;
+        const float al = l ? Z.ax[tid - 1] : 0.f, ar = r ? Z.ax[tid] : 0.f, at = t ? Z.ay[tid - Z.w] : 0.f, ab = b ? Z.ay[tid] : 0.f;
+        float *src = tail_sm, *dst = Z.x;  // MG_COARSE even: the last sweep writes Z.x
+        float xk = __fmul_rn(od, bk);
+        if (mine) src[tid] = xk;
+        if (tid < 256) {
+            for (int it = 1; it < MG_COARSE; it++) {
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                if (mine) {
+                    float v = __fmul_rn(wk, xk);
+                    if (l) v = __fadd_rn(v, __fmul_rn(al, __fsub_rn(xk, src[tid - 1])));
+                    if (r) v = __fadd_rn(v, __fmul_rn(ar, __fsub_rn(xk, src[tid + 1])));
+                    if (t) v = __fadd_rn(v, __fmul_rn(at, __fsub_rn(xk, src[tid - Z.w])));
+                    if (b) v = __fadd_rn(v, __fmul_rn(ab, __fsub_rn(xk, src[tid + Z.w])));
+                    xk = __fadd_rn(xk, __fmul_rn(od, __fsub_rn(bk, v)));
+                    dst[tid] = xk;
+                }
+                float* q = src;
+                src = dst;
+                dst = q;
+            }
         }
         __syncthreads();
-        tail_sweep(L, false);
+    }
+    static_assert(MG_COARSE % 2 == 0, "the last sweep is written to Z.x");
+    for (int l = T.n - 2; l >= 0; l--) {
+        const TailOps L = level(l), C = level(l + 1);
+        const int n = L.w * L.h;
+        for (int k = tid; k < n; k += TAIL_THREADS) {
+            const int i = k % L.w, y = k / L.w;
+            L.x[k] = __fadd_rn(L.x[k], C.x[(y / 2) * C.w + i / 2]);
+        }
+        __syncthreads();
+        float nv[TAIL_PER];
+#pragma unroll
+        for (int q = 0; q < TAIL_PER; q++) {
+            const int k = tid + q * TAIL_THREADS;
+            if (k < n) nv[q] = __fadd_rn(L.x[k], __fmul_rn(__fmul_rn(MG_OMEGA, L.dinv[k]), __fsub_rn(L.b[k], tail_apply(L, k, k % L.w, k / L.w))));
+        }
+        if (l > 0) __syncthreads();
+        float* out = l > 0 ? L.x : T.lv[0].x;
+#pragma unroll
+        for (int q = 0; q < TAIL_PER; q++)
+            if (tid + q * TAIL_THREADS < n) out[tid + q * TAIL_THREADS] = nv[q];
+        __syncthreads();
+    }
+    if (T.n == 1) {
+        const TailOps Z = level(0);
+        for (int k = tid; k < Z.w * Z.h; k += TAIL_THREADS) T.lv[0].x[k] = Z.x[k];
     }
 }
+
 // depth.rs:677 `solve_rows` / :707 `solve_cols`: the Thomas algorithm along
 // every line, one thread per line, 32 lines per warp. The warp stages 32x32
 // tiles of the coefficients through shared memory with coalesced row-segment
@@ -521,14 +665,6 @@ template <bool ROWS>
 __device__ __forceinline__ float& tl(float (*t)[TT + 1], int line, int e) {
     return ROWS ? t[line][e] : t[e][line];
 }
-__device__ __forceinline__ void cp_async4f(float* smem, const float* gmem) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem));
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-
 // The 32 lines' elements e0 .. e0+31 of `src` into tile t (cp.async; `fill` where out of range).
 template <bool ROWS>
 __device__ __forceinline__ void tile_load(float (*t)[TT + 1], const float* __restrict__ src, int l0, int e0, int nlines, int len, int w,
@@ -983,139 +1119,204 @@ __global__ void jac0_h_kernel(const BT* __restrict__ b, const uint16_t* __restri
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
         sth(x, k, MG_OMEGA * ldh(dinv, k) * ldv(b, k));
 }
-// A fine level's way down and way up in one pass each, on tiles in shared memory: the same values
-// as the separate kernels (every sweep's output rounded to BF16 where they store it), the
-// neighbours' values computed once per block over a ring around the tile.
+// A fine level's way down and way up in one pass each, the values the separate sweeps would store (each rounded to
+// BF16): two sweeps deep, so two halo columns a side, and each step of the walk works on three rows -- the sweep's
+// start on row t, one sweep on row t - 1, the next (or the residual) on row t - 2.
 __device__ __forceinline__ float rbf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-// stencil_h_at with x read from a shared tile: (r, c) the cell's place in the tile
-template <int PITCH>
-__device__ __forceinline__ float sweep_tile(const float* X, int r, int c, float bk, const uint16_t* __restrict__ wd,
-                                            const uint16_t* __restrict__ ax, const uint16_t* __restrict__ ay,
-                                            const uint16_t* __restrict__ dinv, int w, int h, int i, int y, int mode) {
-    const size_t k = (size_t)y * w + i;
-    const float xk = X[r * PITCH + c];
-    float v = ldh(wd, k) * xk;
-    if (i > 0) v += ldh(ax, k - 1) * (xk - X[r * PITCH + c - 1]);
-    if (i + 1 < w) v += ldh(ax, k) * (xk - X[r * PITCH + c + 1]);
-    if (y > 0) v += ldh(ay, k - w) * (xk - X[(r - 1) * PITCH + c]);
-    if (y + 1 < h) v += ldh(ay, k) * (xk - X[(r + 1) * PITCH + c]);
-    const float rr = bk - v;
-    return mode == 1 ? rr : xk + MG_OMEGA * ldh(dinv, k) * rr;
+template <class BT>
+__device__ __forceinline__ RowOps row_ops(const BT* __restrict__ b, const uint16_t* __restrict__ wd, const uint16_t* __restrict__ ax,
+                                          const uint16_t* __restrict__ ay, const uint16_t* __restrict__ dinv, bool in, size_t k) {
+    if (!in) return RowOps{0.f, 0.f, 0.f, 0.f, 0.f};
+    return RowOps{ldh(wd, k), ldh(ax, k), ldh(ay, k), ldh(dinv, k), ldv(b, k)};
+}
+// b - A x of a cell (its left edge al, its upper edge at; neighbours outside the grid left out)
+__device__ __forceinline__ float resid_h(const RowOps& q, float al, float at, float xc, float xl, float xr, float xm, float xn, int gx, int y, int w,
+                                         int h) {
+    float v = q.wd * xc;
+    if (gx > 0) v += al * (xc - xl);
+    if (gx + 1 < w) v += q.ax * (xc - xr);
+    if (y > 0) v += at * (xc - xm);
+    if (y + 1 < h) v += q.ay * (xc - xn);
+    return q.b - v;
 }
 // Down: x0 = w D^-1 b, x1 = one sweep, r = b - A x1, its 2x2 block sums; x1 -> x, the sums -> cb.
-// A 32 x 8 block of coarse cells: x0 over its 64 x 16 fine cells and a 2-cell ring, x1 with a 1-cell ring.
-constexpr int VH_D0W = 64 + 4, VH_D0H = 16 + 4, VH_D1W = 64 + 2, VH_D1H = 16 + 2;
 template <class BT>
 __global__ void __launch_bounds__(256) vc_down_h_kernel(const BT* __restrict__ b, const uint16_t* __restrict__ wd,
                                                         const uint16_t* __restrict__ ax, const uint16_t* __restrict__ ay,
                                                         const uint16_t* __restrict__ dinv, uint16_t* __restrict__ x, int w, int h,
-                                                        uint16_t* __restrict__ cb, int cw, int ch) {
-    __shared__ float X0[VH_D0H * VH_D0W], X1[VH_D1H * VH_D1W];
-    const int tid = threadIdx.y * 32 + threadIdx.x, fx = 64 * blockIdx.x, fy = 16 * blockIdx.y;
-    for (int e = tid; e < VH_D0W * VH_D0H; e += 256) {
-        const int r = e / VH_D0W, c = e - r * VH_D0W, gx = fx - 2 + c, gy = fy - 2 + r;
-        X0[e] = gx >= 0 && gx < w && gy >= 0 && gy < h ? rbf(MG_OMEGA * ldh(dinv, (size_t)gy * w + gx) * ldv(b, (size_t)gy * w + gx)) : 0.f;
-    }
-    __syncthreads();
-    for (int e = tid; e < VH_D1W * VH_D1H; e += 256) {
-        const int r = e / VH_D1W, c = e - r * VH_D1W, gx = fx - 1 + c, gy = fy - 1 + r;
-        X1[e] = gx >= 0 && gx < w && gy >= 0 && gy < h
-                    ? rbf(sweep_tile<VH_D0W>(X0, r + 1, c + 1, ldv(b, (size_t)gy * w + gx), wd, ax, ay, dinv, w, h, gx, gy, 2))
-                    : 0.f;
-    }
-    __syncthreads();
-    const int xx = blockIdx.x * 32 + threadIdx.x, yy = blockIdx.y * 8 + threadIdx.y;
-    if (xx >= cw || yy >= ch) return;
-    float o = 0.f;
-    for (int y = 2 * yy; y < min(2 * yy + 2, h); y++)
-        for (int i = 2 * xx; i < min(2 * xx + 2, w); i++) {
-            const size_t k = (size_t)y * w + i;
-            const int r = y - fy + 1, c = i - fx + 1;
-            sth(x, k, X1[r * VH_D1W + c]);
-            o += rbf(sweep_tile<VH_D1W>(X1, r, c, ldv(b, k), wd, ax, ay, dinv, w, h, i, y, 1));
+                                                        uint16_t* __restrict__ cb, int cw, const Strip S) {
+    const int lane = threadIdx.x & 31, wid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (wid >= S.warps) return;
+    const int gx = wid % S.nx * 28 + lane - 2, y0 = wid / S.nx * S.rows, y1 = min(h, y0 + S.rows);
+    const bool inx = gx >= 0 && gx < w, own = lane >= 2 && lane <= 29 && gx < w;
+    auto load = [&](int y) { return row_ops(b, wd, ax, ay, dinv, inx && y >= 0 && y < h, (size_t)y * w + gx); };
+    // rows t, t-1, t-2 of the operands and of x0; t-1, t-2, t-3 of x1
+    RowOps q2{}, q1 = load(y0 - 2), q0 = load(y0 - 1), qn;
+    float a2 = 0.f;                                                // x0 of row t-2
+    float a1 = rbf(MG_OMEGA * q1.dinv * q1.b), s2 = 0.f, s3 = 0.f, o3ay = 0.f, o = 0.f;  // x0 of t-1; x1 of t-2 and t-3
+    for (int t = y0 - 1; t < y1 + 2; t++) {
+        // q0 is row t; its successor on the way
+        qn = load(t + 1);
+        const float a0 = rbf(MG_OMEGA * q0.dinv * q0.b);
+        // x1 of row t-1
+        const float al1 = from_left(q1.ax), xl = from_left(a1), xr = from_right(a1);
+        float s1 = 0.f;
+        {
+            const int y = t - 1;
+            if (inx && y >= 0 && y < h) s1 = rbf(a1 + MG_OMEGA * q1.dinv * resid_h(q1, al1, q2.ay, a1, xl, xr, a2, a0, gx, y, w, h));
         }
-    sth(cb, (size_t)yy * cw + xx, o);
+        // the residual of row t-2
+        const int y = t - 2;
+        const float al2 = from_left(q2.ax), sl = from_left(s2), sr = from_right(s2);
+        float r = 0.f;
+        const bool row = y >= y0 && y < y1;
+        if (own && row) {
+            sth(x, (size_t)y * w + gx, s2);
+            r = rbf(resid_h(q2, al2, o3ay, s2, sl, sr, s3, s1, gx, y, w, h));
+        }
+        const float r1 = from_right(r);
+        if (row) {
+            if (!(y & 1)) o = 0.f;
+            o += r;
+            if (gx + 1 < w) o += r1;
+            if (own && !(gx & 1) && ((y & 1) || y + 1 == h)) sth(cb, (size_t)(y >> 1) * cw + (gx >> 1), o);
+        }
+        o3ay = q2.ay;
+        s3 = s2;
+        s2 = s1;
+        a2 = a1;
+        a1 = a0;
+        q2 = q1;
+        q1 = q0;
+        q0 = qn;
+    }
 }
-// Up: x2 = x1 + P x_c, then two sweeps; the result -> out (BF16, or level 0's FP32 z).
-// A 32 x 8 block of fine cells: x2 with a 2-cell ring, the first sweep with a 1-cell ring.
-constexpr int VH_U2W = 32 + 4, VH_U2H = 8 + 4, VH_U3W = 32 + 2, VH_U3H = 8 + 2;
+// Up: x2 = x1 + P x_c, then two sweeps; the result -> out (BF16, or level 0's FP32 z with r.z: DOT, b is the CG's r).
 template <class BT, class OT, bool DOT>
 __global__ void __launch_bounds__(256) vc_up_h_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ xc, int cw,
                                                       const BT* __restrict__ b, const uint16_t* __restrict__ wd,
                                                       const uint16_t* __restrict__ ax, const uint16_t* __restrict__ ay,
-                                                      const uint16_t* __restrict__ dinv, OT* __restrict__ out, int w, int h, const CgRef C) {
+                                                      const uint16_t* __restrict__ dinv, OT* __restrict__ out, int w, int h, const Strip S,
+                                                      const CgRef C) {
     if (DOT && C.ctl[0]) return;
-    __shared__ float X2[VH_U2H * VH_U2W], X3[VH_U3H * VH_U3W];
-    const int tx = (w + 31) / 32, nt = tx * ((h + 7) / 8), tid = threadIdx.y * 32 + threadIdx.x;
+    const int lane = threadIdx.x & 31, wid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int gx = wid % S.nx * 28 + lane - 2, y0 = wid / S.nx * S.rows, y1 = wid < S.warps ? min(h, y0 + S.rows) : 0;
+    const bool inx = gx >= 0 && gx < w, own = lane >= 2 && lane <= 29 && gx < w;
+    auto load = [&](int y) { return row_ops(b, wd, ax, ay, dinv, inx && y >= 0 && y < h, (size_t)y * w + gx); };
+    auto X = [&](int y) { return inx && y >= 0 && y < h ? rbf(ldh(x, (size_t)y * w + gx) + ldh(xc, (size_t)(y >> 1) * cw + (gx >> 1))) : 0.f; };
     double v[1] = {0.0};
-    for (int t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int fx = t % tx * 32, fy = t / tx * 8;
-        if (DOT) __syncthreads();  // the tile before is done with X2 and X3
-        for (int e = tid; e < VH_U2W * VH_U2H; e += 256) {
-            const int r = e / VH_U2W, c = e - r * VH_U2W, gx = fx - 2 + c, gy = fy - 2 + r;
-            X2[e] = gx >= 0 && gx < w && gy >= 0 && gy < h ? rbf(ldh(x, (size_t)gy * w + gx) + ldh(xc, (size_t)(gy / 2) * cw + gx / 2)) : 0.f;
+    if (y0 < y1) {
+        RowOps q2{}, q1 = load(y0 - 2), q0 = load(y0 - 1), qn;
+        float a2 = 0.f, a1 = X(y0 - 2), a0 = X(y0 - 1), s2 = 0.f, s3 = 0.f, o3ay = 0.f;
+        for (int t = y0 - 1; t < y1 + 2; t++) {
+            qn = load(t + 1);
+            const float an = X(t + 1);
+            // the first sweep of row t-1
+            const float al1 = from_left(q1.ax), xl = from_left(a1), xr = from_right(a1);
+            float s1 = 0.f;
+            {
+                const int y = t - 1;
+                if (inx && y >= 0 && y < h) s1 = rbf(a1 + MG_OMEGA * q1.dinv * resid_h(q1, al1, q2.ay, a1, xl, xr, a2, a0, gx, y, w, h));
+            }
+            // the second of row t-2
+            const int y = t - 2;
+            const float al2 = from_left(q2.ax), sl = from_left(s2), sr = from_right(s2);
+            if (own && y >= y0 && y < y1) {
+                const float o = s2 + MG_OMEGA * q2.dinv * resid_h(q2, al2, o3ay, s2, sl, sr, s3, s1, gx, y, w, h);
+                stv(out, (size_t)y * w + gx, o);
+                if (DOT) v[0] += (double)q2.b * (double)o;
+            }
+            o3ay = q2.ay;
+            s3 = s2;
+            s2 = s1;
+            a2 = a1;
+            a1 = a0;
+            a0 = an;
+            q2 = q1;
+            q1 = q0;
+            q0 = qn;
         }
-        __syncthreads();
-        for (int e = tid; e < VH_U3W * VH_U3H; e += 256) {
-            const int r = e / VH_U3W, c = e - r * VH_U3W, gx = fx - 1 + c, gy = fy - 1 + r;
-            X3[e] = gx >= 0 && gx < w && gy >= 0 && gy < h
-                        ? rbf(sweep_tile<VH_U2W>(X2, r + 1, c + 1, ldv(b, (size_t)gy * w + gx), wd, ax, ay, dinv, w, h, gx, gy, 2))
-                        : 0.f;
-        }
-        __syncthreads();
-        const int i = fx + threadIdx.x, y = fy + threadIdx.y;
-        if (i >= w || y >= h) continue;
-        const size_t k = (size_t)y * w + i;
-        const float bk = ldv(b, k), o = sweep_tile<VH_U3W>(X3, threadIdx.y + 1, threadIdx.x + 1, bk, wd, ax, ay, dinv, w, h, i, y, 2);
-        stv(out, k, o);
-        if (DOT) v[0] += (double)bk * (double)o;
     }
-    if (DOT && reduce_last(v, C.part, C.ctl + 2) && tid == 0) cg_rz(C, v[0]);
+    if (DOT && reduce_last(v, C.part, C.ctl + 2) && threadIdx.x == 0) cg_rz(C, v[0]);
 }
 
-// The coarsest level's sweeps in one CTA of 32 x 32 threads with the level's planes in shared memory:
-// the zero-start sweep, then sweeps - 1 damped Jacobi sweeps between two buffers, __syncthreads
-// between them; the result is written to x.
-constexpr int COARSE_H_PLANES = 7;
-__global__ void __launch_bounds__(1024) coarse_h_kernel(uint16_t* __restrict__ x, const uint16_t* __restrict__ b,
-                                                        const uint16_t* __restrict__ wd, const uint16_t* __restrict__ ax,
-                                                        const uint16_t* __restrict__ ay, const uint16_t* __restrict__ dinv, int w,
-                                                        int h, int sweeps) {
-    extern __shared__ uint16_t csm[];
-    const int n = w * h, tid = threadIdx.y * 32 + threadIdx.x;
-    uint16_t *sb = csm, *swd = sb + n, *sax = swd + n, *say = sax + n, *sdi = say + n, *s0 = sdi + n, *s1 = s0 + n;
-    for (int k = tid; k < n; k += 1024) {
-        sb[k] = b[k];
-        swd[k] = wd[k];
-        sax[k] = ax[k];
-        say[k] = ay[k];
-        sdi[k] = dinv[k];
-    }
-    __syncthreads();
-    for (int k = tid; k < n; k += 1024) sth(s0, k, MG_OMEGA * ldh(sdi, k) * ldh(sb, k));
-    uint16_t *src = s0, *dst = s1;
-    for (int sw = 1; sw < sweeps; sw++) {
-        __syncthreads();
-        for (int y = threadIdx.y; y < h; y += 32)
-            for (int i = threadIdx.x; i < w; i += 32) {
-                const size_t k = (size_t)y * w + i;
-                sth(dst, k, stencil_h_at(src, ldh(sb, k), swd, sax, say, sdi, w, h, i, y, 2));
-            }
-        uint16_t* t = src;
-        src = dst;
-        dst = t;
-    }
-    __syncthreads();
-    for (int k = tid; k < n; k += 1024) x[k] = src[k];
+// The coarsest level's sweeps in one cluster of 8 CTAs: each holds a band of rows, operators and both x buffers in
+// shared memory, a warp per row; a sweep writes its band's first and last row into the neighbours' halo rows too
+// (distributed shared memory) and ends in a cluster barrier. The zero-start sweep, then sweeps - 1 damped Jacobi ones,
+// the result to x. What bounds it: the barrier and one pass over a few rows per warp (133 x 89 cells: 153 us in one
+// CTA, 48 here); the bands hold levels of up to about 90 k cells, which fell to a launch per sweep before.
+constexpr int CH_CTAS = 8, CH_THREADS = 512;
+constexpr size_t CH_MAX_SMEM = 220 * 1024;
+static size_t coarse_h_smem(const WlsLevel& L) {
+    const size_t rows = (L.h + CH_CTAS - 1) / CH_CTAS;
+    return sizeof(uint16_t) * L.w * (rows * 4 + (rows + 1) + 2 * (rows + 2));
 }
+static bool coarse_h_fits(const WlsLevel& L) { return coarse_h_smem(L) <= CH_MAX_SMEM; }
+__global__ void __launch_bounds__(CH_THREADS) coarse_h_kernel(uint16_t* __restrict__ x, const uint16_t* __restrict__ b,
+                                                              const uint16_t* __restrict__ wd, const uint16_t* __restrict__ ax,
+                                                              const uint16_t* __restrict__ ay, const uint16_t* __restrict__ dinv, int w, int h,
+                                                              int sweeps) {
+    extern __shared__ uint16_t csm[];
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), rows = (h + CH_CTAS - 1) / CH_CTAS, r0 = rank * rows, nr = max(0, min(rows, h - r0));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint16_t *sb = csm, *swd = sb + rows * w, *sax = swd + rows * w, *sdi = sax + rows * w;
+    uint16_t* say = sdi + rows * w;              // from the row above the band on
+    uint16_t* xb[2] = {say + (rows + 1) * w, say + (rows + 1) * w + (rows + 2) * w};  // from the row above to the row below
+    for (int k = tid; k < nr * w; k += CH_THREADS) {
+        const size_t q = (size_t)r0 * w + k;
+        sb[k] = b[q];
+        swd[k] = wd[q];
+        sax[k] = ax[q];
+        sdi[k] = dinv[q];
+        say[w + k] = ay[q];
+    }
+    if (r0 > 0 && nr > 0)
+        for (int k = tid; k < w; k += CH_THREADS) say[k] = ay[(size_t)(r0 - 1) * w + k];
+    uint16_t* up[2] = {nullptr, nullptr};    // the band above's lower halo row, the band below's upper one
+    uint16_t* down[2] = {nullptr, nullptr};
+    for (int q = 0; q < 2; q++) {
+        if (rank > 0) up[q] = cl.map_shared_rank(xb[q], rank - 1) + (rows + 1) * w;  // every band above a band is whole
+        if (rank + 1 < CH_CTAS) down[q] = cl.map_shared_rank(xb[q], rank + 1);
+    }
+    auto put = [&](int q, int r, int i, float v) {
+        const bf e = __float2bfloat16_rn(v);
+        const uint16_t u = *(const uint16_t*)&e;
+        xb[q][(r + 1) * w + i] = u;
+        if (r == 0 && up[q]) up[q][i] = u;
+        if (r == nr - 1 && down[q]) down[q][i] = u;
+    };
+    __syncthreads();
+    for (int r = warp; r < nr; r += CH_THREADS / 32)
+        for (int i = lane; i < w; i += 32) put(0, r, i, MG_OMEGA * ldh(sdi, r * w + i) * ldh(sb, r * w + i));
+    cl.sync();
+    for (int sw = 1; sw < sweeps; sw++) {
+        const uint16_t* src = xb[(sw - 1) & 1];
+        for (int r = warp; r < nr; r += CH_THREADS / 32) {
+            const bool top = r0 + r > 0, bot = r0 + r + 1 < h;
+            for (int i = lane; i < w; i += 32) {
+                const int k = r * w + i, c = k + w;  // c: the cell in the x buffers and in say
+                const float xk = ldh(src, c);
+                float v = ldh(swd, k) * xk;
+                if (i > 0) v += ldh(sax, k - 1) * (xk - ldh(src, c - 1));
+                if (i + 1 < w) v += ldh(sax, k) * (xk - ldh(src, c + 1));
+                if (top) v += ldh(say, c - w) * (xk - ldh(src, c - w));
+                if (bot) v += ldh(say, c) * (xk - ldh(src, c + w));
+                put(sw & 1, r, i, xk + MG_OMEGA * ldh(sdi, k) * (ldh(sb, k) - v));
+            }
+        }
+        cl.sync();
+    }
+    const uint16_t* res = xb[(sweeps - 1) & 1] + w;
+    for (int k = tid; k < nr * w; k += CH_THREADS) x[(size_t)r0 * w + k] = res[k];
+}
+
 WlsSolver* wls_alloc(int w, int h, cudaError_t* err) {
     *err = cudaSuccess;
     // set here, outside the graph captures of the CG iteration that launch it
-    static const cudaError_t coarse_attr = cudaFuncSetAttribute(coarse_h_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (coarse_attr != cudaSuccess) {
-        *err = coarse_attr;
-        return nullptr;
-    }
+    *err = cudaFuncSetAttribute(coarse_h_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_MAX_SMEM);
+    if (*err == cudaSuccess) *err = cudaFuncSetAttribute(vcycle_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_MAX_SMEM);
+    if (*err != cudaSuccess) return nullptr;
     WlsSolver* S = new WlsSolver();
     S->w = w;
     S->h = h;
@@ -1141,7 +1342,7 @@ WlsSolver* wls_alloc(int w, int h, cudaError_t* err) {
             for (uint16_t** q : {&L.hwd, &L.hax, &L.hay, &L.hdinv, &L.hx, &L.hb, &L.hr}) put(q, m);
         }
         for (float** q : {&S->ex, &S->ey, &S->cp, &S->dp, &S->f, &S->r, &S->z, &S->p, &S->p2, &S->ap}) put(q, n);
-        put(&S->part, (size_t)2 * RED_BLOCKS);
+        put(&S->part, (size_t)2 * std::max(RED_BLOCKS, std::max(strip_blocks(strip_of(w, h, 1)), strip_blocks(strip_of(w, h, 2)))));
         put(&S->scal, 4);
         put(&S->alpha_beta, 4);
         put(&S->ctl, 4);
@@ -1183,7 +1384,8 @@ void wls_destroy(WlsSolver* s) {
 int wls_levels(const WlsSolver* s) { return (int)s->lv.size(); }
 
 static bool tail_level(const WlsSolver* S, size_t l) {
-    return (size_t)S->lv[l].w * S->lv[l].h <= (size_t)MG_TAIL_CELLS && S->lv.size() - l <= (size_t)MG_TAIL_MAX;
+    return (size_t)S->lv[l].w * S->lv[l].h <= (size_t)MG_TAIL_CELLS && S->lv.size() - l <= (size_t)MG_TAIL_MAX &&
+           tail_floats(S, l) * sizeof(float) <= TAIL_MAX_SMEM;  // a long thin grid's levels only halve
 }
 static CgRef cg_ref(const WlsSolver* S) { return CgRef{S->part, S->scal, S->alpha_beta, S->ctl, (CgOut*)S->host_rel}; }
 
@@ -1220,8 +1422,6 @@ cudaError_t wls_set_weights(WlsSolver* S, const float* conf, int mode, cudaStrea
     return cudaGetLastError();
 }
 
-static int red_grid(int w, int h) { return std::min(RED_BLOCKS, ((w + 31) / 32) * ((h + 7) / 8)); }
-
 // depth.rs:924 `vcycle` (MG_PRE = MG_POST = 1): a level's way down and its way up in one pass each, the small levels in
 // one CTA (every chain of levels ends in them: the coarsest has at most 16 x 16 cells). The right-hand side is bin
 // (null: the level's b); the result lands in xout (null: the level's x, through its r buffer), with r.z at level 0.
@@ -1231,19 +1431,19 @@ static void vcycle(WlsSolver* S, size_t l, const float* bin, float* xout, cudaSt
         MgTail tl;
         tl.n = (int)(S->lv.size() - l);
         for (int q = 0; q < tl.n; q++) tl.lv[q] = S->lv[l + q];
-        lsb_launched(), vcycle_tail_kernel<<<1, 1024, 0, s>>>(tl);
+        lsb_launched(), vcycle_tail_kernel<<<1, TAIL_THREADS, tail_floats(S, l) * sizeof(float), s>>>(tl);
         return;
     }
     WlsLevel& C = S->lv[l + 1];
     const float* b = bin ? bin : T.b;
-    lsb_launched(), vc_down_kernel<<<g2(C.w, C.h), B2, 0, s>>>(b, T.wd, T.ax, T.ay, T.dinv, T.x, T.w, T.h, C.b, C.w, C.h);
+    const Strip st = strip_of(T.w, T.h, 1);
+    lsb_launched(), vc_down_kernel<<<strip_blocks(st), 256, 0, s>>>(b, T.wd, T.ax, T.ay, T.dinv, T.x, T.w, T.h, C.b, C.w, st);
     vcycle(S, l + 1, nullptr, nullptr, s);
     if (xout) {
-        lsb_launched(), vc_up_kernel<true><<<red_grid(T.w, T.h), B2, 0, s>>>(T.x, C.x, C.w, b, T.wd, T.ax, T.ay, T.dinv, xout, T.w, T.h, cg_ref(S));
+        lsb_launched(), vc_up_kernel<true><<<strip_blocks(st), 256, 0, s>>>(T.x, C.x, C.w, b, T.wd, T.ax, T.ay, T.dinv, xout, T.w, T.h, st, cg_ref(S));
         return;
     }
-    const int nt = ((T.w + 31) / 32) * ((T.h + 7) / 8);
-    lsb_launched(), vc_up_kernel<false><<<nt, B2, 0, s>>>(T.x, C.x, C.w, b, T.wd, T.ax, T.ay, T.dinv, T.r, T.w, T.h, cg_ref(S));
+    lsb_launched(), vc_up_kernel<false><<<strip_blocks(st), 256, 0, s>>>(T.x, C.x, C.w, b, T.wd, T.ax, T.ay, T.dinv, T.r, T.w, T.h, st, cg_ref(S));
     std::swap(T.x, T.r);
 }
 
@@ -1258,18 +1458,28 @@ static void jacobi_h(WlsLevel& L, bool zero, cudaStream_t s) {
                                                                                    L.h, 2);
     std::swap(L.hx, L.hr);
 }
-static size_t coarse_h_smem(const WlsLevel& L) { return sizeof(uint16_t) * COARSE_H_PLANES * (size_t)L.w * L.h; }
-static bool coarse_h_fits(const WlsLevel& L) { return coarse_h_smem(L) <= 227 * 1024; }
 // the mixed-precision V-cycle: MG_H_SWEEPS pre/post sweeps, MG_H_LEVELS levels, MG_COARSE sweeps on
-// the coarsest (one CTA). b32 / z32: level 0 takes the CG's FP32 residual as its right-hand side and
+// the coarsest (one cluster). b32 / z32: level 0 takes the CG's FP32 residual as its right-hand side and
 // its last sweep writes the FP32 z (no conversion passes).
 static void vcycle_h(WlsSolver* S, size_t l, cudaStream_t s, const float* b32 = nullptr, float* z32 = nullptr) {
     WlsLevel& T = S->lv[l];
     const size_t last = std::min(S->lv.size(), (size_t)MG_H_LEVELS) - 1;
     if (l == last) {
         if (coarse_h_fits(T)) {
-            const size_t smem = coarse_h_smem(T);  // at most 227 KB (wls_alloc raised the kernel's limit)
-            lsb_launched(), coarse_h_kernel<<<1, dim3(32, 32), smem, s>>>(T.hx, T.hb, T.hwd, T.hax, T.hay, T.hdinv, T.w, T.h, MG_COARSE);
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(CH_CTAS);
+            cfg.blockDim = dim3(CH_THREADS);
+            cfg.dynamicSmemBytes = coarse_h_smem(T);  // wls_alloc raised the kernel's limit
+            cfg.stream = s;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = CH_CTAS;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            lsb_launched();
+            cudaLaunchKernelEx(&cfg, coarse_h_kernel, T.hx, (const uint16_t*)T.hb, (const uint16_t*)T.hwd, (const uint16_t*)T.hax,
+                               (const uint16_t*)T.hay, (const uint16_t*)T.hdinv, T.w, T.h, MG_COARSE);
         } else {
             for (int k = 0; k < MG_COARSE; k++) jacobi_h(T, k == 0, s);
         }
@@ -1279,14 +1489,15 @@ static void vcycle_h(WlsSolver* S, size_t l, cudaStream_t s, const float* b32 = 
     auto down_up = [&](auto* b) {  // the way down and the way up in one pass each
         using BT = std::remove_cv_t<std::remove_pointer_t<decltype(b)>>;
         WlsLevel& C = S->lv[l + 1];
-        lsb_launched(), vc_down_h_kernel<BT><<<g2(C.w, C.h), B2, 0, s>>>(b, T.hwd, T.hax, T.hay, T.hdinv, T.hx, T.w, T.h, C.hb, C.w, C.h);
+        const Strip st = strip_of(T.w, T.h, 2);
+        lsb_launched(), vc_down_h_kernel<BT><<<strip_blocks(st), 256, 0, s>>>(b, T.hwd, T.hax, T.hay, T.hdinv, T.hx, T.w, T.h, C.hb, C.w, st);
         vcycle_h(S, l + 1, s);
         if (z32) {
-            lsb_launched(), vc_up_h_kernel<BT, float, true><<<red_grid(T.w, T.h), B2, 0, s>>>(T.hx, C.hx, C.w, b, T.hwd, T.hax, T.hay, T.hdinv, z32,
-                                                                                             T.w, T.h, cg_ref(S));
+            lsb_launched(), vc_up_h_kernel<BT, float, true><<<strip_blocks(st), 256, 0, s>>>(T.hx, C.hx, C.w, b, T.hwd, T.hax, T.hay, T.hdinv, z32, T.w,
+                                                                                          T.h, st, cg_ref(S));
         } else {
-            lsb_launched(), vc_up_h_kernel<BT, uint16_t, false><<<((T.w + 31) / 32) * ((T.h + 7) / 8), B2, 0, s>>>(
-                T.hx, C.hx, C.w, b, T.hwd, T.hax, T.hay, T.hdinv, T.hr, T.w, T.h, cg_ref(S));
+            lsb_launched(), vc_up_h_kernel<BT, uint16_t, false><<<strip_blocks(st), 256, 0, s>>>(T.hx, C.hx, C.w, b, T.hwd, T.hax, T.hay, T.hdinv,
+                                                                                              T.hr, T.w, T.h, st, cg_ref(S));
             std::swap(T.hx, T.hr);
         }
     };
@@ -1323,9 +1534,10 @@ cudaError_t wls_solve(WlsSolver* S, const float* d, int max_iters, float* u, flo
     }
     const CgRef C = cg_ref(S);
     CgOut* host = (CgOut*)S->host_rel;
+    const Strip st = strip_of(w, h, 1);
     // b = W d, |b|, r = b - A u; the reductions' ticket starts at 0, and every reduction leaves it there
     if (!S->ctl_zero) cudaMemsetAsync(S->ctl, 0, 4 * sizeof(int), s), S->ctl_zero = true;
-    lsb_launched(), cg_start_kernel<<<red_grid(w, h), B2, 0, s>>>(d, u, L0.wd, L0.ax, L0.ay, S->r, w, h, C);
+    lsb_launched(), cg_start_kernel<<<strip_blocks(st), 256, 0, s>>>(d, u, L0.wd, L0.ax, L0.ay, S->r, w, h, st, C);
     const int nb1 = (int)std::min<size_t>(RED_BLOCKS, (n + 255) / 256);
     // z = M r and r.z
     auto precond = [&]() {
@@ -1350,7 +1562,7 @@ cudaError_t wls_solve(WlsSolver* S, const float* d, int max_iters, float* u, flo
     };
     auto iteration = [&]() {
         precond();
-        lsb_launched(), cg_dir_kernel<<<red_grid(w, h), B2, 0, s>>>(S->z, S->p, S->p2, L0.wd, L0.ax, L0.ay, S->ap, w, h, C);
+        lsb_launched(), cg_dir_kernel<<<strip_blocks(st), 256, 0, s>>>(S->z, S->p, S->p2, L0.wd, L0.ax, L0.ay, S->ap, w, h, st, C);
         lsb_launched(), cg_step_kernel<<<nb1, 256, 0, s>>>(u, S->p, S->p2, S->r, S->ap, n, max_iters, C);
     };
     // Every V-cycle restarts each level from zero, so which of a level's two buffers holds x
