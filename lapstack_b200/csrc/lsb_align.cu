@@ -806,6 +806,8 @@ struct NmJob {
     double* out;    // the transform found [8]
     // chained searches (no host round trip between frames):
     const double* init_dev;        // if set, the initial transform (the previous frame's result) instead of init
+    double* mid;                   // [0..7] the transform after the cluster's levels, [8] their evaluations
+    int nlv_cluster;               // the first levels, searched by nm_cluster_kernel before the grid takes the rest
     double* warp_dev;              // if set, the full-resolution warp of the result: inverse [9], affine, identity
     unsigned long long* evals_dev; // if set, evaluations are added here
     long long spin_limit;          // polls of the hand-off's wait before it gives up
@@ -813,11 +815,12 @@ struct NmJob {
 
 __device__ void dev_sim_matrix(const double* v, int w, int h, double m[9]) {
     const double cx = (double)w / 2.0, cy = (double)h / 2.0;
-    const double c = cos(v[3]), sn = sin(v[3]);
+    double c, sn;
+    sincos(v[3], &sn, &c);
     const double sc = v[2], shear = v[5], aspect = v[4];
     const double a = __dmul_rn(sc, c), b = __dmul_rn(sc, __dsub_rn(__dmul_rn(c, shear), __dmul_rn(sn, aspect)));
     const double d = __dmul_rn(sc, sn), e = __dmul_rn(sc, __dadd_rn(__dmul_rn(sn, shear), __dmul_rn(c, aspect)));
-    const double gx = __ddiv_rn(v[6], (double)w), gy = __ddiv_rn(v[7], (double)h);
+    const double gx = v[6] == 0.0 ? v[6] : __ddiv_rn(v[6], (double)w), gy = v[7] == 0.0 ? v[7] : __ddiv_rn(v[7], (double)h);
     const double a2 = __dadd_rn(a, __dmul_rn(cx, gx)), b2 = __dadd_rn(b, __dmul_rn(cx, gy));
     const double d2 = __dadd_rn(d, __dmul_rn(cy, gx)), e2 = __dadd_rn(e, __dmul_rn(cy, gy));
     m[0] = a2;
@@ -1029,6 +1032,25 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// The search's end: the transform, the evaluations and the full-resolution warp.
+__device__ void nm_publish(const NmJob& J, const double* cur, int evals) {
+    for (int q = 0; q < 8; q++) J.out[q] = cur[q];
+    J.ctl[1] = evals;
+    if (J.evals_dev) atomicAdd(J.evals_dev, (unsigned long long)evals);
+    if (J.warp_dev) {
+        // align.rs:258: the inverse of the frame's matrix, as the warp of the next reference reads it
+        const double id[8] = {0.0, 0.0, 1.0, 0.0, 1.0, 0.0, 0.0, 0.0};
+        bool ident = true;
+        for (int q = 0; q < 8; q++) ident = ident && cur[q] == id[q];
+        double m[9], inv[9];
+        dev_sim_matrix(cur, J.W, J.H, m);
+        dev_mat_inverse(m, inv);
+        for (int q = 0; q < 9; q++) J.warp_dev[q] = inv[q];
+        J.warp_dev[9] = inv[6] == 0.0 && inv[7] == 0.0 && inv[8] == 1.0 ? 1.0 : 0.0;
+        J.warp_dev[10] = ident ? 1.0 : 0.0;
+    }
+}
+
 constexpr int NM_THREADS = 256, NM_WARPS = NM_THREADS / 32;
 // align.rs:896 `multiscale_align` of one frame: the NmJob's whole coarse-to-fine search.
 __global__ void __launch_bounds__(NM_THREADS) nm_search_kernel(const NmJob J) {
@@ -1047,11 +1069,15 @@ __global__ void __launch_bounds__(NM_THREADS) nm_search_kernel(const NmJob J) {
             S.hi[q] = __dadd_rn(S.cur[J.free_idx[q]], c_span[J.free_idx[q]]);
         }
         S.evals = 0;
+        if (J.nlv_cluster > 0) {  // the cluster's levels are done: on from their result, in the box of the start
+            for (int q = 0; q < 8; q++) S.cur[q] = J.mid[q];
+            S.evals = (int)J.mid[8];
+        }
     }
     int batch = 0;
     unsigned arrived = 0;  // the counter's value once this batch's arrivals are in
     const unsigned stride = gridDim.x * NM_THREADS;
-    for (int L = 0; L < J.nlv; L++) {
+    for (int L = J.nlv_cluster; L < J.nlv; L++) {
         const NmLevel lv = J.lv[L];
         __syncthreads();
         if (tid == 0) pending = J.nfree > 0 ? nm_level_start(J, S, L) : 0;
@@ -1229,23 +1255,382 @@ __global__ void __launch_bounds__(NM_THREADS) nm_search_kernel(const NmJob J) {
             __syncthreads();
         }
     }
-    if (blockIdx.x == 0 && tid == 0) {
-        for (int q = 0; q < 8; q++) J.out[q] = S.cur[q];
-        J.ctl[1] = S.evals;
-        if (J.evals_dev) atomicAdd(J.evals_dev, (unsigned long long)S.evals);
-        if (J.warp_dev) {
-            // align.rs:258: the inverse of the frame's matrix, as the warp of the next reference reads it
-            const double id[8] = {0.0, 0.0, 1.0, 0.0, 1.0, 0.0, 0.0, 0.0};
-            bool ident = true;
-            for (int q = 0; q < 8; q++) ident = ident && S.cur[q] == id[q];
-            double m[9], inv[9];
-            dev_sim_matrix(S.cur, J.W, J.H, m);
-            dev_mat_inverse(m, inv);
-            for (int q = 0; q < 9; q++) J.warp_dev[q] = inv[q];
-            J.warp_dev[9] = inv[6] == 0.0 && inv[7] == 0.0 && inv[8] == 1.0 ? 1.0 : 0.0;
-            J.warp_dev[10] = ident ? 1.0 : 0.0;
+    if (blockIdx.x == 0 && tid == 0) nm_publish(J, S.cur, S.evals);
+}
+
+// How a level is shared out: strips of 32 columns x `rows` rows, one warp at a time.
+struct NmStrips {
+    int nx, rows, n;
+};
+constexpr int NM_ROWS = 16;
+// One strip per warp where the level is that small (as few rows as that takes), else strips of at most NM_ROWS rows.
+__device__ __forceinline__ NmStrips nm_strips(const NmLevel& lv, int warps) {
+    NmStrips S;
+    S.nx = (lv.w + 31) / 32;
+    const int ny = max(1, warps / S.nx);
+    S.rows = min(NM_ROWS, (lv.h + ny - 1) / ny);
+    S.n = S.nx * ((lv.h + S.rows - 1) / S.rows);
+    return S;
+}
+// A sample of the target at (sx, sy) = (xa + fx, ya + fy): align.rs:581's Spline4x4 taps, clamped at the border.
+__device__ __forceinline__ float nm_sample(const NmLevel& lv, int xa, int ya, float fx, float fy) {
+    float wx[4], wy[4];
+    spline4f(fx, wx);
+    spline4f(fy, wy);
+    float acc = 0.f;
+    if (xa >= 1 && xa + 2 < lv.w && ya >= 1 && ya + 2 < lv.h) {
+        // the 4x4 footprint inside the plane: no clamps
+        const float* row = lv.tg + (size_t)(ya - 1) * lv.w + (xa - 1);
+#pragma unroll
+        for (int j = 0; j < 4; j++, row += lv.w) {
+            float r = 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; u++) r = __fadd_rn(r, __fmul_rn(wx[u], __ldg(row + u)));
+            acc = __fadd_rn(acc, __fmul_rn(wy[j], r));
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float* row = lv.tg + (size_t)min(max(ya + j - 1, 0), lv.h - 1) * lv.w;
+            float r = 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; u++) r = __fadd_rn(r, __fmul_rn(wx[u], __ldg(row + min(max(xa + u - 1, 0), lv.w - 1))));
+            acc = __fadd_rn(acc, __fmul_rn(wy[j], r));
         }
     }
+    return acc;
+}
+// floor(v) as an integer, and v - floor(v) as f64, for 0 <= v < 2^31 (-0 too): v + 1.5 2^52 rounded down has the floor in
+// its low word, so no conversion instruction is spent on it. False outside that range (NaN too).
+__device__ __forceinline__ bool nm_split(double v, int& i, double& frac) {
+    constexpr double M = 6755399441055744.0;
+    const unsigned hi = (unsigned)__double2hiint(v);
+    const double t = __dadd_rd(v, M);
+    i = __double2loint(t);
+    frac = __dsub_rn(v, __dsub_rn(t, M));
+    return hi < 0x41E00000u || hi == 0x80000000u;
+}
+// Three candidates (k0 .. k0 + kn - 1) over this warp's strips of a level: align.rs:581's sums of d, d^2 and the count.
+// What bounds it: instructions issued (about half of the SM's slots over the whole kernel, 8 % of the f64 unit), f64 and
+// conversions the dearest. The affine source point is (m1 y + m2) + m0 x in that order (align.rs:485), so the row's
+// part comes from a table the warp makes per strip and the column's is the thread's own for the strip: 2 f64 additions
+// a sample instead of 8 operations, and 11 f64 operations and 3 conversions in all instead of 17 and 7. 128 registers:
+// nm_search_kernel, whose CTAs share their SMs with the fold's, keeps the plain loop in 64 (with this one 8256 x 5504
+// is 80.2 -> 83.2 ms). rt: the warp's table, [rows][3 candidates x 2 axes].
+__device__ __forceinline__ void nm_eval(const NmLevel& lv, const double (*cand)[9], int k0, int kn, const NmStrips& S, int gw, int warps,
+                                        double (*rt)[6], double (&sd)[3], double (&sd2)[3], int (&cnt)[3]) {
+    const int lane = threadIdx.x & 31;
+    bool aff = true;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        sd[c] = sd2[c] = 0.0, cnt[c] = 0;
+        const double* m = cand[k0 + min(c, kn - 1)];
+        aff = aff && m[6] == 0.0 && m[7] == 0.0 && m[8] == 1.0;
+    }
+    auto add = [&](int c, float rv, float v) {
+        const double d = (double)__fsub_rn(rv, v);
+        sd[c] += d;
+        sd2[c] += d * d;
+        cnt[c]++;
+    };
+    for (int s = gw; s < S.n; s += warps) {
+        const int sy_ = s / S.nx, x = (s - sy_ * S.nx) * 32 + lane, y0 = sy_ * S.rows, ny = min(S.rows, lv.h - y0);
+        if (!aff) {
+            const double xmax = (double)(lv.w - 1), ymax = (double)(lv.h - 1);
+            for (int r = 0; r < ny && x < lv.w; r++) {
+                const float rv = lv.rf[(size_t)(y0 + r) * lv.w + x];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    if (c >= kn) break;
+                    const double* m = cand[k0 + c];
+                    double sx, sy;
+                    src_point(m, m[6] == 0.0 && m[7] == 0.0 && m[8] == 1.0, (double)x, (double)(y0 + r), sx, sy);
+                    if (!(sx >= 0.0 && sx <= xmax && sy >= 0.0 && sy <= ymax)) continue;
+                    const double fx = floor(sx), fy = floor(sy);
+                    add(c, rv, nm_sample(lv, (int)fx, (int)fy, (float)__dsub_rn(sx, fx), (float)__dsub_rn(sy, fy)));
+                }
+            }
+            continue;
+        }
+        __syncwarp();
+        for (int e = lane; e < ny * 6; e += 32) {
+            const int r = e / 6, q = e - r * 6, axis = q & 1;
+            const double* m = cand[k0 + min(q >> 1, kn - 1)] + 3 * axis;
+            rt[r][q] = __dadd_rn(__dmul_rn(m[1], (double)(y0 + r)), m[2]);
+        }
+        __syncwarp();
+        if (x >= lv.w) continue;
+        double cx[3], cy[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const double* m = cand[k0 + min(c, kn - 1)];
+            cx[c] = __dmul_rn(m[0], (double)x);
+            cy[c] = __dmul_rn(m[3], (double)x);
+        }
+        const float* rf = lv.rf + (size_t)y0 * lv.w + x;
+        for (int r = 0; r < ny; r++, rf += lv.w) {
+            const float rv = *rf;
+            // the three candidates side by side, without branches (a sample outside reads the corner and counts
+            // for nothing): their chains of about 400 cycles overlap
+            int xa[3], ya[3];
+            bool ok[3];
+            float wx[3][4], wy[3][4], acc[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                double fx, fy;
+                const bool okx = nm_split(__dadd_rn(rt[r][2 * c], cx[c]), xa[c], fx);
+                const bool oky = nm_split(__dadd_rn(rt[r][2 * c + 1], cy[c]), ya[c], fy);
+                // 0 <= sx <= w - 1 and 0 <= sy <= h - 1
+                ok[c] = okx && oky && (unsigned)xa[c] < (unsigned)lv.w && (unsigned)ya[c] < (unsigned)lv.h && (xa[c] < lv.w - 1 || fx == 0.0) &&
+                        (ya[c] < lv.h - 1 || fy == 0.0) && c < kn;
+                if (!ok[c]) xa[c] = ya[c] = 0;
+                spline4f((float)fx, wx[c]);
+                spline4f((float)fy, wy[c]);
+                acc[c] = 0.f;
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                int xo[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) xo[u] = min(max(xa[c] + u - 1, 0), lv.w - 1);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float* row = lv.tg + (size_t)min(max(ya[c] + j - 1, 0), lv.h - 1) * lv.w;
+                    float t = 0.f;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) t = __fadd_rn(t, __fmul_rn(wx[c][u], __ldg(row + xo[u])));
+                    acc[c] = __fadd_rn(acc[c], __fmul_rn(wy[c][j], t));
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const double d = ok[c] ? (double)__fsub_rn(rv, acc[c]) : 0.0;
+                sd[c] += d;
+                sd2[c] += d * d;
+                cnt[c] += ok[c];
+            }
+        }
+    }
+}
+
+// The levels of up to NM_CLUSTER_PX pixels, coarsest first, in ONE cluster of 16 CTAs before the grid-wide kernel takes
+// the finer ones. What bounds a batch there is latency, and most of it was the hand-off between 296 CTAs through
+// global memory (4 us), their partial sums (2.5) and the Nelder-Mead step in shared memory (2.5): here every CTA's
+// sums go straight into every other's shared memory, one cluster barrier hands them over, and warp 0 of each CTA keeps
+// the sorted simplex in registers (lane q: parameter q of every vertex; the costs in every lane). N: the number of
+// free parameters. The search is align.rs:796's, step for step, as in nm_search_kernel; the f64 sums are added in
+// another order. A batch of the coarsest levels of 2048 x 1536: 14 us there, 6 here.
+// Where the line lies: 16 SMs evaluate a larger level more slowly than the grid does, and the grid pays its hand-off
+// only once per batch. A 516 x 344 pair, a 2048 x 1536 stack of 16 and an 8256 x 5504 one of 10, ms: no cluster 1.24 /
+// 22.7 / 80.2, levels of up to 4096 pixels 1.13 / 20.0 / -, 16384 1.11 / 18.4 / 77.9, 65536 1.37 / 20.7 / 78.1.
+constexpr int NMC_THREADS = 512, NMC_WARPS = NMC_THREADS / 32, NMC_MAX = 16;
+constexpr unsigned NM_CLUSTER_PX = 16 * 1024;
+template <int N>
+__global__ void __launch_bounds__(NMC_THREADS) nm_cluster_kernel(const NmJob J) {
+    __shared__ double cand[MAX_CAND][9];
+    __shared__ double wred[MAX_CAND * 3][NMC_WARPS];
+    __shared__ double slot[2][MAX_CAND * 3][NMC_MAX];  // every CTA's sums of a batch, two batches in turn
+    __shared__ double rt[NMC_WARPS][NM_ROWS][6];
+    __shared__ double pts[MAX_CAND][8];  // the pending candidates, all 8 parameters
+    __shared__ double cur[8];
+    __shared__ int pending;
+    cg::cluster_group cl = cg::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, rank = (int)cl.block_rank(), nb = (int)cl.num_blocks();
+    const bool lq = lane < N;
+    // warp 0's copy of the search: this lane's parameter of the vertices (sorted by cost), its box, step and tolerance
+    double col[N + 1], f[N + 1], lo = 0.0, hi = 0.0, tol = 0.0, xr = 0.0, xe = 0.0, xc = 0.0;
+    int it = 0, phase = NM_INIT, evals = 0, passes = 0;
+    if (tid < 8) cur[tid] = J.init_dev ? J.init_dev[tid] : J.init[tid];
+    __syncthreads();
+    int fi = 0;
+#pragma unroll
+    for (int q = 0; q < N; q++)
+        if (lane == q) fi = J.free_idx[q];
+    if (lq) {
+        lo = __dsub_rn(cur[fi], c_span[fi]);
+        hi = __dadd_rn(cur[fi], c_span[fi]);
+    }
+    auto clampq = [&](double v) { return fmin(fmax(v, lo), hi); };
+    auto put = [&](int k, double v) {
+        if (lq) pts[k][fi] = v;
+    };
+    // align.rs:815's loop from its top: stable sort, convergence, the next candidates. Returns how many are pending.
+    auto iterate = [&]() -> int {
+        bool done = it >= 200;
+        // insertion from the back; strictly smaller moves forward, so equal costs keep their order
+#pragma unroll
+        for (int i = 1; i <= N; i++)
+#pragma unroll
+            for (int j = i; j > 0; j--)
+                if (f[j] < f[j - 1]) {
+                    const double tf = f[j], tc = col[j];
+                    f[j] = f[j - 1], col[j] = col[j - 1];
+                    f[j - 1] = tf, col[j - 1] = tc;
+                }
+        if (!done) {
+            it++;
+            // align.rs:888 `converged`
+            const bool conv = fabs(__dsub_rn(f[N], f[0])) <= __dmul_rn(1e-4, __dadd_rn(1.0, fabs(f[0])));
+            bool mine = true;
+            if (lq)
+#pragma unroll
+                for (int i = 1; i <= N; i++) mine = mine && fabs(__dsub_rn(col[i], col[0])) <= tol;
+            done = conv && __all_sync(0xffffffffu, mine);
+        }
+        if (done) {
+            if (lq) cur[fi] = col[0];
+            return 0;
+        }
+        double c = 0.0;
+#pragma unroll
+        for (int i = 0; i < N; i++) c = __dadd_rn(c, col[i]);
+        c = __ddiv_rn(c, (double)N);
+        xr = clampq(__dadd_rn(c, __dmul_rn(1.0, __dsub_rn(c, col[N]))));
+        xe = clampq(__dadd_rn(c, __dmul_rn(2.0, __dsub_rn(xr, c))));
+        xc = clampq(__dadd_rn(c, __dmul_rn(0.5, __dsub_rn(col[N], c))));
+        put(0, xr);
+        put(1, xe);
+        put(2, xc);
+        phase = NM_RXC;
+        return 3;
+    };
+    int batch = 0;
+    for (int L = 0; L < J.nlv_cluster; L++) {
+        const NmLevel lv = J.lv[L];
+        const NmStrips S_ = nm_strips(lv, nb * NMC_WARPS);
+        // the pending candidates' matrices, by warp 0 (their parameters that are not free: the level's start)
+        auto matrices = [&](int nc) {
+            __syncwarp();
+            if (lane < nc) {
+                double v[8], m[9];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[q] = pts[lane][q];
+                dev_sim_matrix(v, lv.w, lv.h, m);
+                dev_mat_inverse(m, cand[lane]);
+            }
+            if (lane == 0) pending = nc;
+        };
+        if (wid == 0) {  // align.rs:784 `level_steps`, align.rs:806-813 the first simplex
+            double step = 0.0;
+            if (lq) {
+                const double wf = J.W, hf = J.H, r = fmax(wf, hf) / 2.0;
+                const double gain[8] = {wf, hf, r, r, hf / 2.0, hf / 2.0, wf / 4.0, hf / 4.0};
+                const double px = (double)(1ull << lv.lvl);
+                double g = 1.0;
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    if (q == fi) g = gain[q];
+                step = __ddiv_rn(__dmul_rn(1.0, px), g);
+                tol = __ddiv_rn(__dmul_rn(0.1, px), g);
+            }
+            const double x0 = lq ? cur[fi] : 0.0;
+            for (int e = lane; e < MAX_CAND * 8; e += 32) pts[e / 8][e % 8] = cur[e % 8];
+            __syncwarp();
+            col[0] = x0;
+#pragma unroll
+            for (int k = 0; k < N; k++) col[k + 1] = clampq(k == lane ? __dadd_rn(x0, step) : x0);
+#pragma unroll
+            for (int k = 0; k <= N; k++) put(k, col[k]);
+            phase = NM_INIT;
+            it = 0;
+            passes = 0;
+            matrices(N + 1);
+        }
+        __syncthreads();
+        while (pending > 0) {
+            const int nc = pending;
+            for (int k0 = 0; k0 < nc; k0 += 3) {
+                const int kn = min(3, nc - k0);
+                double sd[3], sd2[3];
+                int cnt[3];
+                nm_eval(lv, cand, k0, kn, S_, rank * NMC_WARPS + wid, nb * NMC_WARPS, rt[wid], sd, sd2, cnt);
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    if (c >= kn) break;
+                    const double a = warp_sum(sd[c]), b = warp_sum(sd2[c]), n1 = warp_sum((double)cnt[c]);
+                    if (lane == 0) {
+                        wred[3 * (k0 + c)][wid] = a;
+                        wred[3 * (k0 + c) + 1][wid] = b;
+                        wred[3 * (k0 + c) + 2][wid] = n1;
+                    }
+                }
+            }
+            __syncthreads();
+            // this CTA's sums (the warps in order) into every CTA's slots
+            const int par = batch & 1;
+            for (int e = tid; e < 3 * nc * nb; e += NMC_THREADS) {
+                const int q = e / nb, to = e - q * nb;
+                double t = 0.0;
+#pragma unroll
+                for (int i = 0; i < NMC_WARPS; i++) t += wred[q][i];
+                *cl.map_shared_rank(&slot[par][q][rank], to) = t;
+            }
+            cl.sync();
+            if (wid == 0) {
+                double t = 0.0;
+                if (lane < 3 * nc)
+                    for (int i = 0; i < nb; i++) t += slot[par][lane][i];
+                const int src = min(3 * lane, 29);
+                const double sdv = __shfl_sync(0xffffffffu, t, src), sd2v = __shfl_sync(0xffffffffu, t, src + 1), cn = __shfl_sync(0xffffffffu, t, src + 2);
+                const double cost = cn < 16.0 ? 1e9 : sqrt(fmax(__ddiv_rn(__dsub_rn(sd2v, __ddiv_rn(__dmul_rn(sdv, sdv), cn)), cn), 0.0));
+                int nx;
+                if (phase == NM_INIT) {
+#pragma unroll
+                    for (int k = 0; k <= N; k++) f[k] = __shfl_sync(0xffffffffu, cost, k);
+                    evals += N + 1;
+                    nx = iterate();
+                } else if (phase == NM_SHRINK) {
+#pragma unroll
+                    for (int k = 1; k <= N; k++) f[k] = __shfl_sync(0xffffffffu, cost, k - 1);
+                    evals += N;
+                    nx = iterate();
+                } else {
+                    const double fr = __shfl_sync(0xffffffffu, cost, 0), fe = __shfl_sync(0xffffffffu, cost, 1), fc = __shfl_sync(0xffffffffu, cost, 2);
+                    evals++;
+                    int take;  // 0 xr, 1 xe, 2 xc, 3 shrink
+                    if (fr < f[0]) {
+                        evals++;
+                        take = fe < fr ? 1 : 0;
+                    } else if (fr < f[N - 1]) {
+                        take = 0;
+                    } else {
+                        evals++;
+                        take = fc < f[N] ? 2 : 3;
+                    }
+                    if (take < 3) {
+                        col[N] = take == 0 ? xr : take == 1 ? xe : xc;
+                        f[N] = take == 0 ? fr : take == 1 ? fe : fc;
+                        nx = iterate();
+                    } else {
+#pragma unroll
+                        for (int i = 1; i <= N; i++) {
+                            col[i] = clampq(__dadd_rn(col[0], __dmul_rn(0.5, __dsub_rn(col[i], col[0]))));
+                            put(i - 1, col[i]);
+                        }
+                        phase = NM_SHRINK;
+                        nx = N;
+                    }
+                }
+                // <= 200 iterations of at most two batches each, plus the first simplex
+                if (++passes > 402 && nx > 0) {
+                    nx = 0;
+                    if (rank == 0 && lane == 0) atomicCAS(J.ctl, 0, 2);
+                }
+                matrices(nx);
+            }
+            batch++;
+            __syncthreads();
+        }
+    }
+    if (rank == 0 && tid == 0) {
+        if (J.nlv_cluster == J.nlv) {
+            nm_publish(J, cur, evals);
+        } else {
+            for (int q = 0; q < 8; q++) J.mid[q] = cur[q];
+            J.mid[8] = (double)evals;
+        }
+    }
+    cl.sync();
 }
 
 static std::atomic<int> g_nm_blocks{0};  // the search's grid on this device (set once, by any thread)
@@ -1287,11 +1672,77 @@ static cudaError_t nm_job(AlignCtx& C, const float* rf, const std::vector<float*
     J.bar = (unsigned*)C.nm_ctl + 2;
     J.ctl = C.nm_ctl;
     J.out = C.nm_out;
+    J.mid = C.nm_mid;
     return cudaSuccess;
+}
+// The largest cluster (16 CTAs, or the portable 8) this device can run nm_cluster_kernel<N> in, 0 if none: asked once.
+template <int N>
+static int nm_cluster_size() {
+    static const int size = [] {
+        if (cudaFuncSetAttribute(nm_cluster_kernel<N>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
+        for (int n : {NMC_MAX, 8}) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(n);
+            cfg.blockDim = dim3(NMC_THREADS);
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = n;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            int fit = 0;
+            if (cudaOccupancyMaxActiveClusters(&fit, nm_cluster_kernel<N>, &cfg) == cudaSuccess && fit > 0) return n;
+            cudaGetLastError();
+        }
+        return 0;
+    }();
+    return size;
+}
+template <int N>
+static cudaError_t nm_cluster_launch(AlignCtx& C, NmJob& J, int limit) {
+    int n = nm_cluster_size<N>();
+    if (limit > 0 && n > limit) n = limit >= 8 && n > 8 ? 8 : 0;
+    if (n == 0) {
+        J.nlv_cluster = 0;
+        return cudaSuccess;
+    }
+    cudaFuncSetAttribute(nm_cluster_kernel<N>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);  // on every device
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(n);
+    cfg.blockDim = dim3(NMC_THREADS);
+    cfg.stream = C.s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = n;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    lsb_launched();
+    return cudaLaunchKernelEx(&cfg, nm_cluster_kernel<N>, J);
 }
 static cudaError_t nm_launch(AlignCtx& C, NmJob& J) {
     cudaError_t e = cudaMemsetAsync(C.nm_ctl + 2, 0, sizeof(int) * 2, C.s);  // the barrier; the error word stays sticky
     if (e != cudaSuccess) return e;
+    // the small levels first, in one cluster (not with the spin limit overridden: that is for the grid-wide hand-off's
+    // wait, which a cluster barrier does not have)
+    J.nlv_cluster = 0;
+    if (!getenv("LSB_NM_SPIN_LIMIT"))
+        while (J.nlv_cluster < J.nlv && (unsigned)J.lv[J.nlv_cluster].w * J.lv[J.nlv_cluster].h <= NM_CLUSTER_PX) J.nlv_cluster++;
+    if (J.nlv_cluster > 0) {
+        switch (J.nfree) {
+            case 1: e = nm_cluster_launch<1>(C, J, C.max_blocks); break;
+            case 2: e = nm_cluster_launch<2>(C, J, C.max_blocks); break;
+            case 3: e = nm_cluster_launch<3>(C, J, C.max_blocks); break;
+            case 4: e = nm_cluster_launch<4>(C, J, C.max_blocks); break;
+            case 5: e = nm_cluster_launch<5>(C, J, C.max_blocks); break;
+            case 6: e = nm_cluster_launch<6>(C, J, C.max_blocks); break;
+            case 7: e = nm_cluster_launch<7>(C, J, C.max_blocks); break;
+            case 8: e = nm_cluster_launch<8>(C, J, C.max_blocks); break;
+            default: J.nlv_cluster = 0; break;  // nothing to search
+        }
+        if (e != cudaSuccess) return e;
+        if (J.nlv_cluster == J.nlv) return cudaSuccess;
+    }
     void* args[] = {(void*)&J};
     lsb_launched();
     const int blocks = C.max_blocks > 0 ? std::min(g_nm_blocks.load(), C.max_blocks) : g_nm_blocks.load();

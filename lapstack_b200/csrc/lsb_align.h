@@ -34,6 +34,7 @@ struct AlignCtx {
     double* nm_part;   // device, 2 * MAX_CAND * NM_MAX_BLOCKS * 3
     int* nm_ctl;       // device, 4: error, evaluations, barrier arrivals, spare
     double* nm_out;    // device, 8: the transform
+    double* nm_mid;    // device, 9: the transform and evaluations after the small levels
     int device_search = 1;  // 0: the host drives the search, one launch per simplex step
     int max_blocks = 0;     // CTAs of the device search at most (0: two per SM); the engine's grid limit
     size_t evals = 0, launches = 0;

@@ -490,6 +490,7 @@ static char* engine_init(lsb_engine* e) {
     TRY(e->pool.get(&e->actx.nm_part, (size_t)2 * MAX_CAND * NM_MAX_BLOCKS * 3));
     TRY(e->pool.get(&e->actx.nm_ctl, 4));
     TRY(e->pool.get(&e->actx.nm_out, 8));
+    TRY(e->pool.get(&e->actx.nm_mid, 9));
     {
         int coop = 0;
         TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->cfg.device));

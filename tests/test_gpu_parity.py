@@ -307,6 +307,26 @@ def test_device_search_matches_host_search(model):
     assert np.max(np.abs(outs[0].align - ref.sims)) < 1e-9
 
 
+# 128 x 128 is the largest level the cluster takes; a level of 33 x 31 is one strip and a column; 6 x 5 is smaller than a
+# sample's footprint and has the search's 16 samples only near the identity
+@pytest.mark.parametrize("w,h", [(128, 128), (129, 128), (127, 65), (33, 31), (6, 5), (301, 17)])
+@pytest.mark.parametrize("free", [(0,), (0, 1), (0, 1, 3), (0, 1, 2, 3), (0, 1, 2, 3, 4), (0, 1, 2, 3, 4, 5), (0, 1, 2, 3, 4, 6, 7), tuple(range(8))])
+def test_search_of_small_levels_takes_the_host_loops_steps(w, h, free):
+    """Levels of up to 16384 pixels are searched by one cluster, with the
+    simplex in registers and one instance per number of free parameters: the
+    same evaluations as the host-side loop of the oracle, and its transform to
+    the summation order of the f64 costs."""
+    rng = np.random.default_rng(100 * w + h)
+    rf = O.window_sum(rng.random((h + 8, w + 8), np.float32), np.array([1, 4, 6, 4, 1], np.float32) / np.float32(16))
+    tg = np.ascontiguousarray(rf[3 : 3 + h, 5 : 5 + w]) * np.float32(0.97)
+    rf = np.ascontiguousarray(rf[4 : 4 + h, 4 : 4 + w])
+    mask = [q in free for q in range(8)]
+    want, ev = O.multiscale_align(rf, tg, free=mask)
+    got, ev2 = L.multiscale_align(rf, tg, free=mask)
+    assert ev2 == ev, (got, want)
+    assert np.max(np.abs(got - want)) < 1e-9, (got, want)
+
+
 def test_search_wait_running_out_falls_back_to_the_host_search(monkeypatch):
     """The device search's hand-off wait is bounded. When it runs out (here
     after one poll) the kernel returns, the stack is registered again by the
