@@ -759,7 +759,7 @@ cudaError_t aggregate_peaks(AggArgs a, bool slice_fp16, cudaStream_t s, int grid
 
 // ------------------------------------------------------------- k-th value
 // depth.rs:580 and :618 `select_nth_unstable_by(total_cmp)` (the noise floor's median, p90):
-// the k-th value by a two-pass 16-bit radix histogram of total-order keys.
+// the k-th value by radix histograms of total-order keys, 11, 11 and 10 bits.
 // The key of a float in the total order (total_cmp): monotone as u32.
 __device__ __forceinline__ unsigned fkey(float f) {
     unsigned b = __float_as_uint(f);
@@ -768,46 +768,69 @@ __device__ __forceinline__ unsigned fkey(float f) {
 __device__ __forceinline__ float fkey_inv(unsigned k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
-__global__ void hist_kernel(const float* __restrict__ v, size_t cnt, int stride, unsigned* hist, const unsigned* sel, int pass) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cnt; i += (size_t)gridDim.x * blockDim.x) {
-        const unsigned k = fkey(v[i * stride]);
-        if (pass == 0) atomicAdd(&hist[k >> 16], 1u);
-        else if ((k >> 16) == sel[0]) atomicAdd(&hist[k & 0xffffu], 1u);
-    }
-}
-// One block: find the bin holding rank sel[1] (pass 0) / sel[2] (pass 1).
-__global__ void scan_kernel(const unsigned* hist, unsigned* sel, int pass, float* out) {
-    __shared__ unsigned part[1024];
-    const int t = threadIdx.x;
-    unsigned s = 0;
-    for (int b = t * 64; b < t * 64 + 64; b++) s += hist[b];
-    part[t] = s;
+// One pass over the keys' next bits: the histogram of the keys that share the prefix found so far, and, in the CTA that
+// ends last, the bin that holds the rank. sel: [0] the prefix, [1] the rank within it. What bounds it: the read of
+// every 7th float (a 32-byte sector each), if the counting does not: 65536 bins in global memory, most keys in a few of
+// them, and a one-CTA kernel over all of them took 0.14 ms a pass at 860 k keys and 0.05 at 6 k. Here the bins are in
+// shared memory, a CTA adds those it has hit to the global ones, and the scan reads 2048: 10 us a pass at 860 k keys, 5 at 6 k.
+constexpr int KTH_T = 512, KTH_BINS = 2048;
+template <int PASS>
+__global__ void __launch_bounds__(KTH_T) kth_pass_kernel(const float* __restrict__ v, unsigned cnt, int stride, unsigned rank, unsigned* hist,
+                                                         unsigned* done, unsigned* sel, float* out) {
+    constexpr int BITS = PASS == 2 ? 10 : 11, SHIFT = PASS == 0 ? 21 : PASS == 1 ? 10 : 0, NB = 1 << BITS, PER = NB / KTH_T;
+    __shared__ unsigned bins[NB];
+    __shared__ unsigned wsum[KTH_T / 32];
+    __shared__ bool last;
+    const int t = threadIdx.x, lane = t & 31;
+    for (int b = t; b < NB; b += KTH_T) bins[b] = 0;
+    const unsigned prefix = PASS > 0 ? sel[0] : 0, want = PASS > 0 ? sel[1] : rank;
     __syncthreads();
-    if (t == 0) {
-        unsigned want = pass == 0 ? sel[1] : sel[2], acc = 0;
-        int chunk = 0;
-        while (chunk < 1023 && acc + part[chunk] <= want) acc += part[chunk++];
-        int b = chunk * 64;
-        while (b < chunk * 64 + 63 && acc + hist[b] <= want) acc += hist[b++];
-        if (pass == 0) {
-            sel[0] = (unsigned)b;
-            sel[2] = want - acc;
-        } else {
-            *out = fkey_inv((sel[0] << 16) | (unsigned)b);
-        }
+    for (unsigned i = blockIdx.x * KTH_T + t; i < cnt; i += gridDim.x * KTH_T) {
+        const unsigned k = fkey(v[(size_t)i * stride]);
+        if (PASS == 0 || (unsigned)((unsigned long long)k >> (SHIFT + BITS)) == prefix) atomicAdd(&bins[(k >> SHIFT) & (NB - 1)], 1u);
+    }
+    __syncthreads();
+    for (int b = t; b < NB; b += KTH_T)
+        if (bins[b]) atomicAdd(&hist[b], bins[b]);
+    __threadfence();
+    __syncthreads();
+    if (t == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // thread t: bins t PER .. ; the exclusive sums before them
+    unsigned c[PER], mine = 0;
+#pragma unroll
+    for (int q = 0; q < PER; q++) mine += c[q] = __ldcg(&hist[t * PER + q]);
+    unsigned inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    if (lane == 31) wsum[t >> 5] = inc;
+    __syncthreads();
+    unsigned acc = inc - mine;
+    for (int w = 0; w < t >> 5; w++) acc += wsum[w];
+    if (acc <= want && want < acc + mine) {  // one thread: rank < cnt
+        int q = 0;
+        while (acc + c[q] <= want) acc += c[q++];
+        const unsigned key = (prefix << BITS) | (unsigned)(t * PER + q);
+        if (PASS == 2) *out = fkey_inv(key);
+        else sel[0] = key, sel[1] = want - acc;
     }
 }
-__global__ void set_rank_kernel(unsigned* sel, unsigned rank) { sel[1] = rank; }
 
 cudaError_t select_kth(const float* v, size_t cnt, int stride, size_t rank, unsigned* hist, unsigned* sel, float* out,
                        cudaStream_t s) {
-    cudaMemsetAsync(hist, 0, sizeof(unsigned) * 65536, s);
-    lsb_launched(), set_rank_kernel<<<1, 1, 0, s>>>(sel, (unsigned)rank);
-    lsb_launched(), hist_kernel<<<grid1(cnt), 256, 0, s>>>(v, cnt, stride, hist, sel, 0);
-    lsb_launched(), scan_kernel<<<1, 1024, 0, s>>>(hist, sel, 0, out);
-    cudaMemsetAsync(hist, 0, sizeof(unsigned) * 65536, s);
-    lsb_launched(), hist_kernel<<<grid1(cnt), 256, 0, s>>>(v, cnt, stride, hist, sel, 1);
-    lsb_launched(), scan_kernel<<<1, 1024, 0, s>>>(hist, sel, 1, out);
+    // three histograms, then the three passes' counters of CTAs done
+    unsigned* done = hist + 3 * KTH_BINS;
+    cudaMemsetAsync(hist, 0, sizeof(unsigned) * (3 * KTH_BINS + 3), s);
+    // 2 CTAs an SM at most, 4 keys a thread at least: more CTAs add their bins more often
+    const int g = (int)std::max<size_t>(1, std::min<size_t>((cnt + 4 * KTH_T - 1) / (4 * KTH_T), 148 * 2));
+    lsb_launched(), kth_pass_kernel<0><<<g, KTH_T, 0, s>>>(v, (unsigned)cnt, stride, (unsigned)rank, hist, done, sel, out);
+    lsb_launched(), kth_pass_kernel<1><<<g, KTH_T, 0, s>>>(v, (unsigned)cnt, stride, 0, hist + KTH_BINS, done + 1, sel, out);
+    lsb_launched(), kth_pass_kernel<2><<<g, KTH_T, 0, s>>>(v, (unsigned)cnt, stride, 0, hist + 2 * KTH_BINS, done + 2, sel, out);
     return cudaGetLastError();
 }
 

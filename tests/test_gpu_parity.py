@@ -361,6 +361,35 @@ def test_search_wait_running_out_falls_back_to_the_host_search(monkeypatch):
         assert_same(out.depth.depth, normal.depth.depth, "depth")
 
 
+@pytest.mark.parametrize("n", [3, 1100])
+def test_winner_shares_count_every_frame(n):
+    """Frames on both sides of the CTA's own table of 1024 winners (one 17 x
+    15 frame after another, the last ones the sharpest somewhere)."""
+    rng = np.random.default_rng(n)
+    frames = [rng.random((3, 15, 17), np.float32) * np.float32(0.2 + 0.8 * (k % 97) / 97) for k in range(n)]
+    params = L.FuseParams(levels=1, depth_level=0)
+    ref = O.Fuser(17, 15, O.FuseParams(**vars(params)))
+    dev = L.GpuFuser(17, 15, params, n_max=n)
+    for f in frames:
+        ref.push(f)
+        dev.push(f)
+    rs, ds = ref.shares(), dev.shares()
+    assert n < 1024 or np.any(rs[1024:] > 0)
+    assert_same(rs, ds, "shares")
+
+
+# one key; a CTA's share and one more; more keys than two CTAs an SM take in one go; keys that differ in the last bits
+@pytest.mark.parametrize("w,h,spread", [(2, 3, 20.0), (113, 127, 20.0), (120, 120, 0.0), (2101, 2053, 20.0), (2101, 2053, 0.0)])
+def test_noise_floor_is_the_middle_value(w, h, spread):
+    rng = np.random.default_rng(w)
+    sl = (np.float32(10) ** rng.uniform(-spread, spread, (2, h, w))).astype(np.float32)
+    if spread == 0.0:
+        sl = (sl.view(np.uint32) + rng.integers(0, 1 << 12, sl.shape, dtype=np.uint32)).view(np.float32)
+    dm = L.depth_from_slices(sl, rng.random((3, h, w), np.float32), L.DepthParams(scale=1, agg_radius=0, lam=0.0))
+    keys = np.sort(dm.floor.reshape(-1)[::7])
+    assert dm.floor_value == keys[keys.size // 2]
+
+
 # ---------------------------------------------------------------- precision
 def _errors(img, ref):
     e = np.abs(img.astype(np.float64) - ref.astype(np.float64)) * 65535
