@@ -204,8 +204,6 @@ struct lsb_stack {
     double rel64 = 0.0;
     int iters = 0, iters_first = 0;
     uint32_t crop_rect[4] = {0, 0, 0, 0};  // the common area of the last run (x, y, w, h)
-    float* gsel = nullptr;  // the frame groups' selection states of the small levels
-    size_t gsel_floats = 0;
     double ms[12] = {0};
     // registration chained on the device: per-frame transforms, the last warp, evaluations
     double* sims_dev = nullptr;  // n*8
@@ -603,8 +601,6 @@ static char* stack_alloc(lsb_stack* s, bool depth_only) {
     TRY(P.get(&s->mpart, N * 64 * 3));
     TRY(P.get(&s->means, N * 3));
     TRY(P.get(&s->status, 4));
-    s->gsel_floats = (size_t)16 << 20;  // 64 MB: the small levels' frame-group states
-    TRY(P.get(&s->gsel, s->gsel_floats));
     TRY(P.get(&s->xf_dev, N));
     }
     if (s->dp.enabled) {
@@ -1117,9 +1113,6 @@ static FoldArgs level_args(const lsb_stack* s, int l, bool warped, bool depth_on
     a.H = s->lh[l];
     a.W1 = s->lw[l + 1];
     a.H1 = s->lh[l + 1];
-    a.tiles_x = (a.W + 63) / 64;
-    a.tiles_y = (a.H + 31) / 32;
-    a.ntiles = a.tiles_x * a.tiles_y;
     a.src_u16 = warped && s->storage != STORE_F32 ? (const uint16_t*)s->warped : s->frames;
     a.src_f32 = warped && s->storage == STORE_F32 ? (const float*)s->warped : s->frames_f32;
     a.xf = s->xf_dev;
@@ -1145,24 +1138,6 @@ static FoldArgs level_args(const lsb_stack* s, int l, bool warped, bool depth_on
     }
     *src = l > 0 ? SRC_G : ((s->f32src || (warped && s->storage == STORE_F32)) ? SRC_F32 : SRC_U16);
     return a;
-}
-
-// Levels with too few tiles to fill the GPU: the frames of the selection
-// split into groups selected side by side, then merged in order (about 1.5
-// work items per block, each group at least 2 frames; the first group resumes
-// the state of the frames before, if any).
-static void set_groups(const lsb_stack* s, FoldArgs& a) {
-    const lsb_engine* e = s->e;
-    const int gl = e->grid_select > 0 ? e->grid_select : e->grid;
-    const size_t np = (size_t)a.W * a.H;
-    int G = std::min((3 * gl / 2 + a.ntiles - 1) / std::max(a.ntiles, 1), std::max(1, (a.sel_k1 - a.sel_k0) / 2));
-    while (G > 1 && (size_t)G * 5 * np > s->gsel_floats) G--;
-    if (G > 1) {
-        a.sel_groups = G;
-        a.gacc = s->gsel;
-        a.gbest = s->gsel + (size_t)G * 3 * np;
-        a.gwin = (int*)(s->gsel + (size_t)G * 4 * np);
-    }
 }
 
 // Each frame's warp (align.rs:489, stack.rs:662-679) and brightness sums
@@ -1238,6 +1213,7 @@ static char* stream_warps(lsb_stack* s, bool pushed, bool reduce, bool select) {
             // the last chunk, after the chain, on the whole GPU
             const int ch = s->chunks;
             const bool last = i + 1 == n;
+            std::vector<FoldArgs> later;  // the levels above 0: every REDUCE, then one selection of them all
             for (int l = 0; l < s->levels; l++) {
                 bool focus = false;
                 int src = 0;
@@ -1247,15 +1223,16 @@ static char* stream_warps(lsb_stack* s, bool pushed, bool reduce, bool select) {
                 a.sel_k0 = sel_from;
                 a.sel_k1 = i + 1;
                 a.beside = last ? 0 : 1;
-                set_groups(s, a);
                 if (l == 0) {  // the level-0 fold of the chunk, timed: [start, after the fused kernel, end]
                     TRY(cudaEventRecord(s->chunk_ev[3 * ch], e->ws));
                     TRY(cudaEventRecord(s->chunk_ev[3 * ch + 1], e->ws));
                     a.after_fused = s->chunk_ev[3 * ch + 1];
                 }
+                if (l > 0) later.push_back(a), a.select = 0;
                 TRY(fold_level(a, src, s->storage, (int)s->fp.energy_radius, focus, e->ws, last ? e->grid : e->sms));
                 if (l == 0) TRY(cudaEventRecord(s->chunk_ev[3 * ch + 2], e->ws));
             }
+            TRY(fold_select(later.data(), (int)later.size(), s->storage, (int)s->fp.energy_radius, e->ws));
             s->chunks = ch + 1;
             sel_from = i + 1;
         }
@@ -1479,7 +1456,7 @@ static char* run_pipeline_once(lsb_stack* s) {
     }
     // Once its level is folded the winner map goes back on rs, and the shares are counted: what bounds a large stack's
     // end is the 31 bytes a pixel of results at 55 GB/s, so the link starts on them before the coarser levels and the
-    // collapse (8256 x 5504, 10 frames: 76.6 -> 71.6 ms).
+    // collapse (8256 x 5504, 10 frames: 76.6 -> 72 ms).
     bool winner_sent = false;
     auto send_winner = [&]() -> char* {
         lsb_result* r = s->early;
@@ -1495,6 +1472,9 @@ static char* run_pipeline_once(lsb_stack* s) {
         TRY(winner_counts(s->winner, s->best[dl], s->lw[dl] * s->lh[dl], n, s->counts, s->mx, st));
         return nullptr;
     };
+    // without halo control (whose weights go down the levels one by one) the levels above 0: every REDUCE, then one
+    // selection of them all
+    std::vector<FoldArgs> later;
     if (sel_streamed)  // the level-0 timings of a fold that ran on ws: none here
         for (int q : {8, 10, 9}) TRY(cudaEventRecord(ev[q], st));
     for (int l = 0; l < s->levels && !sel_streamed; l++) {
@@ -1502,7 +1482,6 @@ static char* run_pipeline_once(lsb_stack* s) {
         int src = 0;
         FoldArgs a = level_args(s, l, warped, depth_on, &focus, &src);
         if (streamed && pushed) a.red_n = 0;  // stream_warps has REDUCEd every frame
-        if (!(halo && l >= guide)) set_groups(s, a);
         if (halo && l >= guide) {
             a.halo_mode = l == guide ? 1 : 2;
             a.halo_p = std::min(s->fp.halo, 8.0f);
@@ -1510,12 +1489,14 @@ static char* run_pipeline_once(lsb_stack* s) {
             if (l > guide) TRY(reduce_weights(s->halo_w[l - 1], s->lw[l - 1], s->lh[l - 1], n, s->halo_w[l], s->lw[l], s->lh[l], st));
         }
         a.between = l == 0 ? ev[10] : nullptr;
+        if (l > 0 && !halo) later.push_back(a), a.select = 0;
         if (l == 0) TRY(cudaEventRecord(ev[8], st));
         TRY(fold_level(a, src, s->storage, (int)s->fp.energy_radius, focus, st, e->grid_select > 0 ? e->grid_select : e->grid));
         if (l == 0) TRY(cudaEventRecord(ev[9], st));
-        if (l == (int)s->depth_level)
+        if (l == (int)s->depth_level && a.select)
             if (char* err = send_winner()) return err;
     }
+    TRY(fold_select(later.data(), (int)later.size(), s->storage, (int)s->fp.energy_radius, st));
     if (char* err = send_winner()) return err;
     TRY(cudaEventRecord(ev[3], st));
     // ---- residual, collapse
@@ -2178,6 +2159,7 @@ static char* slab_fold(lsb_stack* s, int lo, int hi) {
     const int guide = std::min((int)s->fp.depth_level, L - 1);
     auto frame_g = [&](int l) { return (size_t)lo * 3 * s->lw[l] * s->lh[l] * gsb; };
     auto frame_w = [&](int l) { return (size_t)lo * s->lw[l] * s->lh[l]; };
+    std::vector<FoldArgs> later;  // the levels above 0, selected in one launch
     TRY(cudaMemsetAsync(s->status, 0, sizeof(int), st));
     for (int l = 0; l < L; l++) {
         bool focus = false;
@@ -2205,11 +2187,11 @@ static char* slab_fold(lsb_stack* s, int lo, int hi) {
             a.halo_w = s->halo_w[l] + frame_w(l);
             if (l > guide)
                 TRY(reduce_weights(s->halo_w[l - 1] + frame_w(l - 1), s->lw[l - 1], s->lh[l - 1], n, a.halo_w, s->lw[l], s->lh[l], st));
-        } else {
-            set_groups(s, a);
         }
+        if (l > 0 && !halo) later.push_back(a), a.select = 0;
         TRY(fold_level(a, src, s->storage, (int)s->fp.energy_radius, false, st, e->grid_select > 0 ? e->grid_select : e->grid));
     }
+    TRY(fold_select(later.data(), (int)later.size(), s->storage, (int)s->fp.energy_radius, st));
     const int wt = s->lw[L], ht = s->lh[L];
     const void* tops = (const char*)s->g[L] + frame_g(L);
     if (halo) {

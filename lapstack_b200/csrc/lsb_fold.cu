@@ -35,8 +35,8 @@ namespace lsb {
 
 #include "lsb_level.cuh"
 #include "lsb_fold0.cuh"
+#include "lsb_select.cuh"
 
-size_t fold_smem_bytes(int, bool) { return (size_t)SEL_FLOATS * sizeof(float); }
 
 // The taps live in constant memory, one copy per device for every engine on it: they are written
 // (stream-ordered on s) only when they change, and an engine that finds them already requested
@@ -78,33 +78,9 @@ static cudaError_t with_smem(K k, size_t smem) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
-// fuse.rs:429 strict `>` across frame groups: the groups' selection states merged in group order: the first group
-// holding the largest energy wins, and within it its first frame did.
-__global__ void select_merge_kernel(const FoldArgs a, int G) {
-    const size_t np = (size_t)a.W * a.H;
-    for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < np; o += (size_t)gridDim.x * blockDim.x) {
-        int bg = 0;
-        float best = a.gbest[o];
-        for (int g = 1; g < G; g++) {
-            const float b = a.gbest[(size_t)g * np + o];
-            if (b > best) {
-                best = b;
-                bg = g;
-            }
-        }
-        const float* ga = a.gacc + (size_t)bg * 3 * np;
-        a.acc[o] = ga[o];
-        a.acc[np + o] = ga[np + o];
-        a.acc[2 * np + o] = ga[2 * np + o];
-        a.best[o] = best;
-        if (a.winner) a.winner[o] = (uint16_t)a.gwin[(size_t)bg * np + o];
-    }
-}
-
 // The fused level-0 kernel applies: 16-bit frames, one call doing the REDUCE and the selection of the
 // same frames, no halo control, no focus slice or the default one (ring difference filter r 1..3 on
-// 2x2 blocks), and a frame with interior tiles. It walks all the frames per tile, so the level is then
-// selected without frame groups.
+// 2x2 blocks), and a frame with interior tiles.
 static bool fold0_applies(const FoldArgs& a, int src, bool focus, int R) {
     if (src != SRC_U16 || a.level != 0 || a.halo_mode != 0 || !a.select || a.red_n <= 0) return false;
     if (a.red_k0 != a.sel_k0 || a.red_n != a.sel_k1 - a.sel_k0) return false;
@@ -112,21 +88,81 @@ static bool fold0_applies(const FoldArgs& a, int src, bool focus, int R) {
     return fold0_count(fold0_range(a.W, a.H, R)) > 0;
 }
 
+// The level-0 tiles the fused kernel leaves, as rectangles: the rows above and below its tiles, the columns beside them.
+static void fold0_border_rects(int W, int H, const Fold0Range& rg, SelBatch& T) {
+    const int ya = 32, yb = std::min(H, 32 * rg.iy1), xa = 64, xb = std::min(W, 64 * rg.ix1);
+    const int r[4][4] = {{0, 0, W, std::min(ya, H)}, {0, ya, std::min(xa, W), yb}, {xb, ya, W, yb}, {0, yb, W, H}};
+    T.n = 0;
+    for (const auto& q : r)
+        if (q[2] > q[0] && q[3] > q[1]) T.r[T.n++] = {0, q[0], q[1], q[2], q[3]};
+}
+// The selection of T's rectangles. Where a level's tiles are too few for the GPU's warps, 2, 3 or all 6 warps of a CTA
+// take a share of the frames each of one tile (not with halo control, which adds the frames up in order).
+template <int SRC, class GS, int R>
+static cudaError_t launch_select(SelBatch& T, cudaStream_t s) {
+    auto k = select_strip_kernel<SRC, GS, R>;
+    auto tiles = [](const SelBatch::Rect& r) { return (long)((r.x1 - r.x0 + SS_W - 1) / SS_W) * ((r.y1 - r.y0 + SS_H - 1) / SS_H); };
+    constexpr long WANT = 148 * SS_CTAS * SS_WARPS;
+    int ctas = 0;
+    bool beside = false;
+    for (int i = 0; i < T.n; i++) {
+        auto& r = T.r[i];
+        const FoldArgs& a = T.a[r.lv];
+        long have = 0;
+        for (int q = 0; q < T.n; q++)
+            if (T.r[q].lv == r.lv) have += tiles(T.r[q]);
+        r.groups = 1;
+        if (a.halo_mode == 0)
+            for (int g : {2, 3, 6})
+                if (have * r.groups < WANT && g <= a.sel_k1 - a.sel_k0) r.groups = g;
+        const uintptr_t src = SRC == SRC_U16 ? 1 : SRC == SRC_F32 ? (uintptr_t)a.src_f32 : (uintptr_t)a.src_g;
+        r.vec = (a.W & 1) == 0 && src % (2 * (SRC == SRC_G ? sizeof(GS) : sizeof(float))) == 0;
+        const int per = SS_H * SS_WARPS / r.groups;
+        r.ntx = (r.x1 - r.x0 + SS_W - 1) / SS_W;
+        r.cta0 = ctas;
+        ctas += r.ntx * ((r.y1 - r.y0 + per - 1) / per);
+        beside = beside || a.beside;
+    }
+    const size_t smem = beside ? std::max(SS_SMEM, BESIDE_SMEM) : SS_SMEM;  // one CTA per SM beside the registration chain
+    cudaError_t e = with_smem(k, smem);
+    if (e != cudaSuccess) return e;
+    lsb_launched(), k<<<ctas, SS_WARPS * 32, smem, s>>>(T);
+    return cudaGetLastError();
+}
+template <class GS>
+static cudaError_t select_stored(SelBatch& T, int r, cudaStream_t s) {
+    return r == 0 ? launch_select<SRC_G, GS, 0>(T, s) : r == 1 ? launch_select<SRC_G, GS, 1>(T, s) : r == 2 ? launch_select<SRC_G, GS, 2>(T, s) : cudaErrorInvalidValue;
+}
+// The selection alone of n levels above level 0, in one launch: the small ones take 20 us each by themselves, most of
+// it the launch, cold instructions and one tile's latency.
+cudaError_t fold_select(const FoldArgs* lv, int n, int storage, int radius, cudaStream_t s) {
+    for (int i = 0; i < n;) {
+        SelBatch T{};
+        for (; i < n && T.n < SS_MAX; i++) {
+            T.a[T.n] = lv[i];
+            T.r[T.n] = {T.n, 0, 0, lv[i].W, lv[i].H};
+            T.n++;
+        }
+        const cudaError_t e = storage == STORE_UNORM16 ? select_stored<unorm16>(T, radius, s)
+                              : storage == STORE_F16   ? select_stored<__half>(T, radius, s) : select_stored<float>(T, radius, s);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 // One level: REDUCE the frames asked for (and take their focus slices at level 0), then select.
 // Level 0 of 16-bit frames: the fused kernel on the interior tiles, the two kernels on the others.
 template <int SRC, class GS, int R, bool FOCUS, class SS>
 static cudaError_t launch_level(const FoldArgs& a0, cudaStream_t s, int grid_limit) {
-    const size_t rsm = (size_t)RED_FLOATS * sizeof(float), ssm = Staging<SRC, GS, R>::SMEM;
+    const size_t rsm = (size_t)RED_FLOATS * sizeof(float);
     auto kr = reduce_level_kernel<SRC, GS, FOCUS, SS>;
-    auto ks = select_level_kernel<SRC, GS, R>;
     cudaError_t e = with_smem(kr, rsm);
-    if (e == cudaSuccess) e = with_smem(ks, ssm);
     if (e != cudaSuccess) return e;
     FoldArgs a = a0;
     int rtiles = ((a.W1 + RW - 1) / RW) * ((a.H1 + RH - 1) / RH);
-    // beside the registration chain: one persistent CTA per SM at most
-    const size_t ssm_run = a.beside ? std::max(ssm, BESIDE_SMEM) : ssm;
-    if (a.beside && (e = with_smem(ks, ssm_run)) != cudaSuccess) return e;
+    SelBatch T{};
+    T.n = 1;
+    T.r[0] = {0, 0, 0, a.W, a.H};
     if (SRC == SRC_U16 && !a0.no_fused && fold0_applies(a0, SRC, FOCUS, R)) {
         auto kf = fold0_kernel<GS, R, FOCUS, SS>;
         const size_t fsm = a.beside ? std::max((size_t)f0::SMEM, BESIDE_SMEM) : (size_t)f0::SMEM;
@@ -138,20 +174,18 @@ static cudaError_t launch_level(const FoldArgs& a0, cudaStream_t s, int grid_lim
         if (a.after_fused) cudaEventRecord(a.after_fused, s);
         if (a.between) cudaEventRecord(a.between, s);
         a.between = nullptr;
-        a.sel_groups = 1;  // the border tiles too: a group merge would run over the whole level
         a.fused0 = 1;
         a.f0r = R;
-        a.ntiles = fold0_border_count(a.tiles_x, a.tiles_y, rg);
-        rtiles = a.ntiles;  // the REDUCE's tiles are the level-0 tiles' G_1 blocks
-        if (a.ntiles <= 0) return cudaGetLastError();
+        // the REDUCE's tiles are the level-0 tiles' G_1 blocks
+        rtiles = fold0_border_count((a.W + 63) / 64, (a.H + 31) / 32, rg);
+        if (rtiles <= 0) return cudaGetLastError();
+        fold0_border_rects(a.W, a.H, rg, T);
     }
     if (a.red_n > 0) lsb_launched(), kr<<<dim3(rtiles, a.red_n), NT, rsm, s>>>(a);
     if (a.between) cudaEventRecord(a.between, s);
-    const int groups = std::max(a.sel_groups, 1);
-    if (a.select) lsb_launched(), ks<<<std::min(a.ntiles * groups, std::max(grid_limit, 1)), NT, ssm_run, s>>>(a);
-    if (a.select && groups > 1) {
-        const size_t np = (size_t)a.W * a.H;
-        lsb_launched(), select_merge_kernel<<<(unsigned)std::min<size_t>((np + 255) / 256, 148 * 8), 256, 0, s>>>(a, groups);
+    if (a.select) {
+        T.a[0] = a;
+        if ((e = launch_select<SRC, GS, R>(T, s)) != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }
@@ -219,11 +253,8 @@ cudaError_t wav_accumulate(const FoldArgs& a, int src_kind, const float* wts, in
 }
 
 cudaError_t fold_level(const FoldArgs& a0, int src_kind, int storage, int radius, bool focus, cudaStream_t s, int grid_limit) {
-    FoldArgs a = a0;  // the select kernel's tiling
-    a.tiles_x = (a.W + TW - 1) / TW;
-    a.tiles_y = (a.H + TH - 1) / TH;
-    a.ntiles = a.tiles_x * a.tiles_y;
-    if (a.ntiles <= 0) return cudaSuccess;
+    const FoldArgs& a = a0;
+    if (a.W <= 0 || a.H <= 0) return cudaSuccess;
     switch (storage) {
         case STORE_UNORM16: return pick_src<unorm16>(a, src_kind, radius, focus, s, grid_limit);
         case STORE_F16: return pick_src<__half>(a, src_kind, radius, focus, s, grid_limit);

@@ -28,7 +28,6 @@ enum SrcKind { SRC_U16 = 0, SRC_F32 = 1, SRC_G = 2 };
 struct FoldArgs {
     int level, nframes;
     int W, H, W1, H1;
-    int tiles_x, tiles_y, ntiles;
     // level-0 sources: interleaved u16 [n][H][W][3] or planar f32 [n][3][H][W]
     const uint16_t* src_u16;
     const float* src_f32;
@@ -61,14 +60,8 @@ struct FoldArgs {
     // (none if red_n is 0) and, if select is set, the selection over frames sel_k0 .. sel_k1 - 1
     // (from sel_k0 > 0 it resumes from the acc / best / winner the frames before it left)
     int red_k0, red_n, select, sel_k0, sel_k1;
-    // sel_groups > 1: the frames are split into that many groups selected side by side from a
-    // fresh state, each into its slice of gacc [g][3][H][W] / gbest [g][H][W] / gwin [g][H][W],
-    // then merged in group order (strict >, so the earliest frame with the largest energy wins)
-    int sel_groups;
-    float *gacc, *gbest;
-    int* gwin;
     // level 0 only: fused0 set, the interior tiles (fold0_range(W, H, f0r)) are the fused kernel's, and
-    // reduce_level_kernel / select_level_kernel walk the other ntiles tiles (fold0_border_tile)
+    // the two other kernels take the border's (fold0_border_tile, fold0_border_rects)
     int fused0, f0r;
     int no_fused;  // 1: level 0 runs the two kernels on every tile (the fused kernel's cross-check)
     // 1: the level runs beside the registration chain: its persistent kernels take at most one CTA per
@@ -84,6 +77,7 @@ enum Storage { STORE_F32 = 0, STORE_UNORM16 = 1, STORE_F16 = 2 };
 
 // Launchers (lsb_fold.cu).
 cudaError_t fold_level(const FoldArgs& a, int src_kind, int storage, int radius, bool focus, cudaStream_t s, int grid_limit);
+cudaError_t fold_select(const FoldArgs* lv, int n, int storage, int radius, cudaStream_t s);
 // The weighted average's accumulation (wav.rs:146-161): frames as level 0 of `a` reads them, weight planes
 // wts [n][dh][dw] (grid scale k), out [3][H][W].
 cudaError_t wav_accumulate(const FoldArgs& a, int src_kind, const float* wts, int n, int dw, int dh, int k, float* out, cudaStream_t s);
@@ -92,7 +86,6 @@ cudaError_t wav_accumulate(const FoldArgs& a, int src_kind, const float* wts, in
 cudaError_t warp_frames(const uint16_t* frames, const FrameXform* xf, int interp, int w, int h, int n, bool u16_out, void* out,
                         cudaStream_t s);
 cudaError_t set_focus_taps(const float* taps3, int ntaps, cudaStream_t s);
-size_t fold_smem_bytes(int radius, bool focus);
 
 // brightness.rs:93 `ratio` on the device for frame k: its gains from its
 // brightness partials (part as bright_sums writes them, nparts per frame,

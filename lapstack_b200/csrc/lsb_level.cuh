@@ -8,12 +8,7 @@
 //    (depth.rs:1097: luma -> ring difference filter -> block mean) from the
 //    same staged window. Parallel over frames, so even the coarse levels fill
 //    the GPU.
-//  * select_level_kernel, persistent over 64x32 tiles of level l: walks the
-//    frames in order, stages G_l over the tile +- R and G_{l+1} over what
-//    EXPAND needs, forms L = G - EXPAND(G_{l+1}) (pyramid.rs:143/209), the
-//    luma energy and its binomial window (fuse.rs:152/168) and keeps the
-//    strict-> selection (fuse.rs:429) in registers: thread (tx, ty) owns
-//    the tile pixels (tx + 32a, ty + 8b), a < 2, b < 4.
+//  * select_strip_kernel (lsb_select.cuh) selects from G_l and G_{l+1}.
 // Tiles whose windows never reach the border index without reflect-101
 // (IN = true); border tiles reflect as pyramid.rs:51 does. Every float op is
 // an explicit round-to-nearest intrinsic in the reference's order.
@@ -21,26 +16,9 @@
 
 constexpr int NT = 256;
 // resident CTAs per SM the compiler keeps the register budget for
-#ifndef LSB_SEL_MINB
-#define LSB_SEL_MINB 2
-#endif
 #ifndef LSB_RED_MINB
 #define LSB_RED_MINB 3
 #endif
-// select: tile, own pixels per thread, windows
-#ifndef LSB_TH
-#define LSB_TH 32
-#endif
-constexpr int TW = 64, TH = LSB_TH, PPT = (TW * TH) / NT;
-static_assert(TH % 16 == 0 && PPT % 2 == 0, "thread (tx, ty) owns (tx + 32a, ty + 8b)");
-constexpr int RMAX = 2;
-constexpr int LW_MAX = TW + 2 * RMAX, LH_MAX = TH + 2 * RMAX;
-constexpr int AW_MAX = LW_MAX / 2 + 5, AH_MAX = LH_MAX / 2 + 5;
-constexpr int SEL_GL = LW_MAX * LH_MAX;  // per channel
-constexpr int SEL_G1 = AW_MAX * AH_MAX;
-constexpr int SEL_EXP = AH_MAX * LW_MAX;
-constexpr int SEL_FLOATS = 3 * (SEL_GL + SEL_G1 + SEL_EXP) + LW_MAX * LH_MAX;
-static_assert(LH_MAX * TW <= 3 * SEL_EXP, "the window rows fit the EXPAND scratch");
 // reduce: tile of G_{l+1}, G_l window with the focus halo
 constexpr int RW = 32, RH = 16, FOC_R = 3;
 constexpr int RGW = 2 * RW + 2 * FOC_R, RGH = 2 * RH + 2 * FOC_R;  // 70 x 38
@@ -334,379 +312,6 @@ __global__ void __launch_bounds__(NT, LSB_RED_MINB) reduce_level_kernel(const Fo
                           2 * gy0 + 2 * RH + FOC_R <= a.H;
     if (interior) reduce_tile<SRC, GS, FOCUS, SS, true>(a, sm, k, gx0, gy0);
     else reduce_tile<SRC, GS, FOCUS, SS, false>(a, sm, k, gx0, gy0);
-}
-
-// ------------------------------------------------------------------ select
-template <int R>
-struct InTile {  // interior-tile window sizes (x0, y0 multiples of TW, TH)
-    static constexpr int LW = TW + 2 * R, LH = TH + 2 * R;
-    static constexpr int AW = ((TW + R - 1) >> 1) + ((R + 1) >> 1) + 3;
-    static constexpr int AH = ((TH + R - 1) >> 1) + ((R + 1) >> 1) + 3;
-};
-struct TileWin {
-    int x0, y0, xL0, xL1, yL0, yL1, xA0, xA1, yA0, yA1, lw, lh, aw, ah, ox1, oy1;
-};
-
-template <int SRC, class GS, int R, bool IN, bool STAGED = false>
-__device__ __forceinline__ void select_frame(const FoldArgs& a, float* __restrict__ sm, int k, const TileWin& t,
-                                             float (&best)[PPT], float (&acc)[PPT][3], int (&win)[PPT]) {
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int W = a.W, H = a.H, W1 = a.W1, H1 = a.H1;
-#define RX(i) (IN ? (i) : lsb_reflect((i), W))
-#define RY(i) (IN ? (i) : lsb_reflect((i), H))
-#define RX1(i) (IN ? (i) : lsb_reflect((i), W1))
-#define RY1(i) (IN ? (i) : lsb_reflect((i), H1))
-    float* gl = sm;                      // [3][lh][lw]   G_l over the tile +- R
-    float* g1 = gl + 3 * SEL_GL;         // [3][ah][aw]   G_{l+1} as stored
-    float* exph = g1 + 3 * SEL_G1;       // [3][ah][lw]   EXPAND along rows
-    float* yb = exph + 3 * SEL_EXP;      // [lh][lw]      node energy
-    // staged tiles are interior: their window sizes and extents are the compile-time ones
-    const int lw = STAGED ? InTile<R>::LW : t.lw, lh = STAGED ? InTile<R>::LH : t.lh;
-    const int aw = STAGED ? InTile<R>::AW : t.aw, ah = STAGED ? InTile<R>::AH : t.ah;
-    const int ox1 = STAGED ? TW : t.ox1, oy1 = STAGED ? TH : t.oy1;
-    const float2 sc = make_float2(a.xf[k].gscale, a.xf[k].ginv);
-
-    // ---- 1: stage G_l and G_{l+1} (STAGED: already in gl / g1 from the async copies)
-    if (!STAGED) {
-    for (int r = ty; r < lh; r += 8)
-        for (int c = tx; c < lw; c += 32) {
-            float v[3];
-            level_px<SRC, GS>(a, k, t.xL0 + c, t.yL0 + r, v);
-            const int i = r * lw + c;
-            gl[i] = v[0];
-            gl[SEL_GL + i] = v[1];
-            gl[2 * SEL_GL + i] = v[2];
-        }
-    {
-        const GS* f = (const GS*)a.dst_g + (size_t)k * 3 * W1 * H1;
-        for (int c = 0; c < 3; c++)
-            for (int r = ty; r < ah; r += 8) {
-                const GS* row = f + ((size_t)c * H1 + t.yA0 + r) * W1 + t.xA0;
-                for (int x = tx; x < aw; x += 32) g1[c * SEL_G1 + r * aw + x] = Store<GS>::ld(row + x, sc);
-            }
-    }
-    __syncthreads();
-    }
-
-    // ---- 2: EXPAND along rows (pyramid.rs:147), the ah x lw outputs spread over all threads
-    for (int m = threadIdx.x; m < ah * lw; m += NT) {
-        const int i = m / lw, xi = m - i * lw;
-        {
-            const int x = t.xL0 + xi, cx = x >> 1;
-            const bool even = (x & 1) == 0;
-            const int ja = RX1(cx - 1) - t.xA0, jb = RX1(cx) - t.xA0, jc = RX1(cx + 1) - t.xA0;
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const float* row = g1 + c * SEL_G1 + i * aw;
-                exph[c * SEL_EXP + i * lw + xi] = even ? lsb_exp_even(row[ja], row[jb], row[jc]) : lsb_exp_odd(row[jb], row[jc]);
-            }
-        }
-    }
-    __syncthreads();
-
-    // ---- 3: EXPAND along columns, L = G - EXPAND(G_{l+1}), node energy (fuse.rs:152)
-    auto lpoint = [&](int x, int y, float L[3]) -> float {
-        const int xi = x - t.xL0, cy = y >> 1;
-        const bool even = (y & 1) == 0;
-        const int ra = (RY1(cy - 1) - t.yA0) * lw, rb = (RY1(cy) - t.yA0) * lw, rc = (RY1(cy + 1) - t.yA0) * lw;
-        const int gi = (y - t.yL0) * lw + xi;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const float* col = exph + c * SEL_EXP + xi;
-            const float up = even ? lsb_exp_even(col[ra], col[rb], col[rc]) : lsb_exp_odd(col[rb], col[rc]);
-            L[c] = __fsub_rn(gl[c * SEL_GL + gi], up);
-        }
-        if (a.use_chroma) return __fadd_rn(__fadd_rn(__fmul_rn(L[0], L[0]), __fmul_rn(L[1], L[1])), __fmul_rn(L[2], L[2]));
-        const float Y = lsb_luma(L[0], L[1], L[2]);
-        return __fmul_rn(Y, Y);
-    };
-    float Lr[PPT][3];
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const int px = tx + 32 * (j & 1), py = ty + 8 * (j >> 1);
-        Lr[j][0] = Lr[j][1] = Lr[j][2] = 0.f;
-        if (px < ox1 && py < oy1) {
-            const int x = t.x0 + px, y = t.y0 + py;
-            yb[(y - t.yL0) * lw + x - t.xL0] = lpoint(x, y, Lr[j]);
-        }
-    }
-    if (R > 0 && a.halo_mode != 2) {
-        // the window's halo ring around the tile, energy only, spread over all threads:
-        // the full-width rows above and below the tile, then the columns beside its rows
-        const int left = t.x0 - t.xL0, right = t.xL1 - (t.x0 + ox1), side = left + right;
-        const int top = t.y0 - t.yL0, bot = lh - top - oy1;
-        for (int m = threadIdx.x; m < (top + bot) * lw; m += NT) {
-            const int rr = m / lw, xi = m - rr * lw;
-            const int yi = rr < top ? rr : oy1 + rr;
-            float L[3];
-            yb[yi * lw + xi] = lpoint(t.xL0 + xi, t.yL0 + yi, L);
-        }
-        for (int m = threadIdx.x; m < oy1 * side; m += NT) {
-            const int rr = m / side, c = m - rr * side;
-            const int xi = c < left ? c : (lw - right) + (c - left);
-            float L[3];
-            yb[(top + rr) * lw + xi] = lpoint(t.xL0 + xi, t.yL0 + top + rr, L);
-        }
-    }
-    __syncthreads();
-
-    // ---- 4: the binomial window (fuse.rs:168) along rows, then columns + the selection
-    if (a.halo_mode == 2) {
-        // halo control below the guide (fuse.rs:466-470): acc = L * w for the first frame,
-        // then acc += w * L; best = the sum of the weights
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            const int px = tx + 32 * (j & 1), py = ty + 8 * (j >> 1);
-            if (px >= ox1 || py >= oy1) continue;
-            const float wv = a.halo_w[((size_t)k * H + t.y0 + py) * W + t.x0 + px];
-#pragma unroll
-            for (int c = 0; c < 3; c++) acc[j][c] = k == 0 ? __fmul_rn(Lr[j][c], wv) : __fadd_rn(acc[j][c], __fmul_rn(wv, Lr[j][c]));
-            best[j] = k == 0 ? wv : __fadd_rn(best[j], wv);
-        }
-        __syncthreads();
-        return;
-    }
-    float* eh = exph;
-    if (R > 0) {
-        for (int m = threadIdx.x; m < lh * ox1; m += NT) {  // the lh x ox1 row sums over all threads
-            const int r = m / ox1, xo = m - r * ox1;
-            {
-                const float* row = yb + r * lw - t.xL0;
-                float s = 0.f;
-#pragma unroll
-                for (int q = 0; q <= 2 * R; q++) s = __fadd_rn(s, __fmul_rn(binw<R>(q), row[RX(t.x0 + xo + q - R)]));
-                eh[r * TW + xo] = s;
-            }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const int px = tx + 32 * (j & 1), py = ty + 8 * (j >> 1);
-        if (px >= ox1 || py >= oy1) continue;
-        float e;
-        if (R > 0) {
-            e = 0.f;
-#pragma unroll
-            for (int q = 0; q <= 2 * R; q++) e = __fadd_rn(e, __fmul_rn(binw<R>(q), eh[(RY(t.y0 + py + q - R) - t.yL0) * TW + px]));
-        } else {
-            e = yb[(py + t.y0 - t.yL0) * lw + px + t.x0 - t.xL0];
-        }
-        if (a.halo_mode == 1) a.halo_w[((size_t)k * H + t.y0 + py) * W + t.x0 + px] = halo_weight(e, a.halo_p);
-        if (e > best[j]) {
-            best[j] = e;
-            acc[j][0] = Lr[j][0];
-            acc[j][1] = Lr[j][1];
-            acc[j][2] = Lr[j][2];
-            win[j] = k;
-        }
-    }
-    __syncthreads();  // the next frame restages gl / g1 / exph
-#undef RX
-#undef RY
-#undef RX1
-#undef RY1
-}
-
-// ------------------------------------------------------- async tile staging
-// For interior tiles the next frame's window rows (G_l over the tile +- R, and
-// G_{l+1} over what EXPAND reads) are copied global -> shared with cp.async
-// while the current frame computes, so the loads' latency is off the critical
-// path. Rows are copied as 4-byte words from the word boundary at or before
-// the row's first byte (`mis` bytes of slack in front); every fold input is
-// allocated with 64 bytes of tail padding for the word after a row's end.
-template <int SRC, class GS, int R>
-struct Staging {
-    static constexpr bool INTERLEAVED = SRC == SRC_U16;
-    static constexpr int G0_EB = SRC == SRC_U16 ? 6 : (SRC == SRC_F32 ? 4 : (int)sizeof(GS));  // bytes per px in a row
-    static constexpr int G0_ROWS = INTERLEAVED ? InTile<R>::LH : 3 * InTile<R>::LH;
-    static constexpr int G0_WPR = (InTile<R>::LW * G0_EB + 2 + 3) / 4;  // words per row, with 2 bytes of slack
-    static constexpr int G1_ROWS = 3 * InTile<R>::AH;
-    static constexpr int G1_WPR = (InTile<R>::AW * (int)sizeof(GS) + 2 + 3) / 4;
-    static constexpr int WORDS = G0_ROWS * G0_WPR + G1_ROWS * G1_WPR;  // one stage
-    // two stages beside the compute buffers, if two CTAs still fit an SM
-    static constexpr bool ON = SRC != SRC_F32 && sizeof(GS) == 2 && (2 * WORDS + SEL_FLOATS) * 4 <= 110 * 1024;
-    static constexpr size_t SMEM = (size_t)(SEL_FLOATS + (ON ? 2 * WORDS : 0)) * 4;
-};
-
-
-// Issue the copies of frame k's interior window into `raw` (one stage).
-template <int SRC, class GS, int R>
-__device__ __forceinline__ void stage_issue(const FoldArgs& a, int k, const TileWin& t, uint32_t* raw) {
-    using S = Staging<SRC, GS, R>;
-    const int W = a.W, H = a.H, W1 = a.W1, H1 = a.H1;
-    const size_t np = (size_t)W * H, np1 = (size_t)W1 * H1;
-    for (int i = threadIdx.x; i < S::G0_ROWS * S::G0_WPR; i += NT) {
-        const int row = i / S::G0_WPR, wd = i - row * S::G0_WPR;
-        size_t byte;
-        if (SRC == SRC_U16) {
-            byte = (((size_t)k * np + (size_t)(t.yL0 + row) * W + t.xL0) * 3) * 2;
-        } else {
-            const int c = row / InTile<R>::LH, r = row - c * InTile<R>::LH;
-            byte = ((((size_t)k * 3 + c) * H + t.yL0 + r) * W + t.xL0) * sizeof(GS);
-        }
-        const unsigned char* base = SRC == SRC_U16 ? (const unsigned char*)a.src_u16 : (const unsigned char*)a.src_g;
-        cp_async4(raw + i, base + (byte & ~(size_t)3) + 4 * wd);
-    }
-    uint32_t* raw1 = raw + S::G0_ROWS * S::G0_WPR;
-    for (int i = threadIdx.x; i < S::G1_ROWS * S::G1_WPR; i += NT) {
-        const int row = i / S::G1_WPR, wd = i - row * S::G1_WPR;
-        const int c = row / InTile<R>::AH, r = row - c * InTile<R>::AH;
-        const size_t byte = ((((size_t)k * 3 + c) * H1 + t.yA0 + r) * W1 + t.xA0) * sizeof(GS);
-        cp_async4(raw1 + i, (const unsigned char*)a.dst_g + (byte & ~(size_t)3) + 4 * wd);
-    }
-    (void)np1;
-}
-// The staged words of frame k -> the f32 windows gl / g1 select_frame reads
-// (level_px's conversion and gains, Store<GS>::ld for the stored levels).
-template <int SRC, class GS, int R>
-__device__ __forceinline__ void stage_convert(const FoldArgs& a, int k, const TileWin& t, const uint32_t* raw, float* sm) {
-    using S = Staging<SRC, GS, R>;
-    using T = InTile<R>;
-    const int W = a.W, H = a.H, W1 = a.W1, H1 = a.H1;
-    const size_t np = (size_t)W * H;
-    float* gl = sm;
-    float* g1 = gl + 3 * SEL_GL;
-    const float2 sc = make_float2(a.xf[k].gscale, a.xf[k].ginv);
-    int gon = 0;
-    float gain[3] = {1.f, 1.f, 1.f};
-    if (SRC == SRC_U16) {
-        gon = a.xf[k].gain_on;
-        for (int c = 0; c < 3; c++) gain[c] = a.xf[k].gain[c];
-    }
-    for (int i = threadIdx.x; i < T::LH * T::LW; i += NT) {
-        const int r = i / T::LW, x = i - r * T::LW;
-        float v[3];
-        if (SRC == SRC_U16) {
-            const size_t byte = (((size_t)k * np + (size_t)(t.yL0 + r) * W + t.xL0) * 3) * 2;
-            const uint16_t* p = (const uint16_t*)((const unsigned char*)(raw + r * S::G0_WPR) + (byte & 3)) + 3 * x;
-            for (int c = 0; c < 3; c++) {
-                v[c] = __fmul_rn((float)p[c], LSB_INV16);
-                if (gon & (1 << c)) v[c] = __fmul_rn(v[c], gain[c]);
-            }
-        } else {
-            for (int c = 0; c < 3; c++) {
-                const size_t byte = ((((size_t)k * 3 + c) * H + t.yL0 + r) * W + t.xL0) * sizeof(GS);
-                const GS* p = (const GS*)((const unsigned char*)(raw + (c * T::LH + r) * S::G0_WPR) + (byte & 3)) + x;
-                v[c] = Store<GS>::ld(p, sc);
-            }
-        }
-        const int o = r * T::LW + x;
-        gl[o] = v[0];
-        gl[SEL_GL + o] = v[1];
-        gl[2 * SEL_GL + o] = v[2];
-    }
-    const uint32_t* raw1 = raw + S::G0_ROWS * S::G0_WPR;
-    for (int i = threadIdx.x; i < 3 * T::AH * T::AW; i += NT) {
-        const int c = i / (T::AH * T::AW), rem = i - c * (T::AH * T::AW), r = rem / T::AW, x = rem - r * T::AW;
-        const size_t byte = ((((size_t)k * 3 + c) * H1 + t.yA0 + r) * W1 + t.xA0) * sizeof(GS);
-        const GS* p = (const GS*)((const unsigned char*)(raw1 + (c * T::AH + r) * S::G1_WPR) + (byte & 3)) + x;
-        g1[c * SEL_G1 + r * T::AW + x] = Store<GS>::ld(p, sc);
-    }
-}
-
-template <int SRC, class GS, int R>
-__global__ void __launch_bounds__(NT, LSB_SEL_MINB) select_level_kernel(const FoldArgs a) {
-    extern __shared__ float sm[];
-    const int W = a.W, H = a.H, W1 = a.W1, H1 = a.H1;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int G = a.sel_groups > 1 ? a.sel_groups : 1;
-    for (int wi = blockIdx.x; wi < a.ntiles * G; wi += gridDim.x) {
-        const int tile = a.fused0 ? fold0_border_tile(wi % a.ntiles, a.tiles_x, fold0_range(W, H, a.f0r)) : wi % a.ntiles;
-        const int g = wi / a.ntiles;
-        const int k0 = G > 1 ? a.sel_k0 + (a.sel_k1 - a.sel_k0) * g / G : a.sel_k0;
-        const int k1 = G > 1 ? a.sel_k0 + (a.sel_k1 - a.sel_k0) * (g + 1) / G : a.sel_k1;
-        TileWin t;
-        t.x0 = (tile % a.tiles_x) * TW;
-        t.y0 = (tile / a.tiles_x) * TH;
-        const int uxL0 = t.x0 - R, uxL1 = t.x0 + TW + R, uyL0 = t.y0 - R, uyL1 = t.y0 + TH + R;
-        const bool interior = ((uxL0 >> 1) - 1) >= 0 && uxL1 <= W && ((uxL1 - 1) >> 1) + 2 <= W1 && ((uyL0 >> 1) - 1) >= 0 &&
-                              uyL1 <= H && ((uyL1 - 1) >> 1) + 2 <= H1;
-        t.xL0 = max(0, uxL0);
-        t.xL1 = min(W, uxL1);
-        t.yL0 = max(0, uyL0);
-        t.yL1 = min(H, uyL1);
-        t.xA0 = max(0, (t.xL0 >> 1) - 1);
-        t.xA1 = min(W1, ((t.xL1 - 1) >> 1) + 2);
-        t.yA0 = max(0, (t.yL0 >> 1) - 1);
-        t.yA1 = min(H1, ((t.yL1 - 1) >> 1) + 2);
-        t.lw = t.xL1 - t.xL0;
-        t.lh = t.yL1 - t.yL0;
-        t.aw = t.xA1 - t.xA0;
-        t.ah = t.yA1 - t.yA0;
-        t.ox1 = min(TW, W - t.x0);
-        t.oy1 = min(TH, H - t.y0);
-        if (t.lw > LW_MAX || t.lh > LH_MAX || t.aw > AW_MAX || t.ah > AH_MAX) {
-            if (threadIdx.x == 0) atomicOr(a.status, LSB_ERR_SHAPE);
-            return;
-        }
-        float best[PPT], acc[PPT][3];
-        int win[PPT];
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            best[j] = -1.f;  // any energy (>= 0) beats it: frame 0 fills the accumulator (fuse.rs:409-412)
-            acc[j][0] = acc[j][1] = acc[j][2] = 0.f;
-            win[j] = 0;
-            const int px = tx + 32 * (j & 1), py = ty + 8 * (j >> 1);
-            if (g == 0 && a.sel_k0 > 0 && px < t.ox1 && py < t.oy1) {  // resume: the state the frames before left
-                const size_t o = (size_t)(t.y0 + py) * W + t.x0 + px;
-                acc[j][0] = a.acc[o];
-                acc[j][1] = a.acc[(size_t)W * H + o];
-                acc[j][2] = a.acc[2 * (size_t)W * H + o];
-                best[j] = a.best[o];
-                if (a.winner) win[j] = a.winner[o];
-            }
-        }
-        using S = Staging<SRC, GS, R>;
-        if (S::ON && interior) {
-            if (t.lw != InTile<R>::LW || t.lh != InTile<R>::LH || t.aw != InTile<R>::AW || t.ah != InTile<R>::AH) {
-                if (threadIdx.x == 0) atomicOr(a.status, LSB_ERR_SHAPE);
-                return;
-            }
-            uint32_t* raw = (uint32_t*)(sm + SEL_FLOATS);
-            stage_issue<SRC, GS, R>(a, k0, t, raw);
-            cp_async_commit();
-            for (int k = k0; k < k1; k++) {
-                uint32_t* cur = raw + ((k - k0) & 1) * S::WORDS;
-                if (k + 1 < k1) {
-                    stage_issue<SRC, GS, R>(a, k + 1, t, raw + ((k + 1 - k0) & 1) * S::WORDS);
-                    cp_async_commit();
-                    cp_async_wait<1>();
-                } else {
-                    cp_async_wait<0>();
-                }
-                __syncthreads();
-                stage_convert<SRC, GS, R>(a, k, t, cur, sm);
-                __syncthreads();
-                select_frame<SRC, GS, R, true, true>(a, sm, k, t, best, acc, win);
-            }
-        } else {
-            for (int k = k0; k < k1; k++) {
-                if (interior) select_frame<SRC, GS, R, true>(a, sm, k, t, best, acc, win);
-                else select_frame<SRC, GS, R, false>(a, sm, k, t, best, acc, win);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < PPT; j++) {
-            const int px = tx + 32 * (j & 1), py = ty + 8 * (j >> 1);
-            if (px >= t.ox1 || py >= t.oy1) continue;
-            const size_t o = (size_t)(t.y0 + py) * W + t.x0 + px, np = (size_t)W * H;
-            if (G > 1) {  // this group's state, merged by select_merge_kernel
-                float* ga = a.gacc + (size_t)g * 3 * np;
-                ga[o] = acc[j][0];
-                ga[np + o] = acc[j][1];
-                ga[2 * np + o] = acc[j][2];
-                a.gbest[(size_t)g * np + o] = best[j];
-                a.gwin[(size_t)g * np + o] = win[j];
-                continue;
-            }
-            a.acc[o] = acc[j][0];
-            a.acc[np + o] = acc[j][1];
-            a.acc[2 * np + o] = acc[j][2];
-            a.best[o] = best[j];
-            if (a.winner) a.winner[o] = (uint16_t)win[j];
-        }
-    }
 }
 
 // --------------------------------------------------------------------- warp
