@@ -154,10 +154,7 @@ cudaError_t fold_select(const FoldArgs* lv, int n, int storage, int radius, cuda
 // Level 0 of 16-bit frames: the fused kernel on the interior tiles, the two kernels on the others.
 template <int SRC, class GS, int R, bool FOCUS, class SS>
 static cudaError_t launch_level(const FoldArgs& a0, cudaStream_t s, int grid_limit) {
-    const size_t rsm = (size_t)RED_FLOATS * sizeof(float);
-    auto kr = reduce_level_kernel<SRC, GS, FOCUS, SS>;
-    cudaError_t e = with_smem(kr, rsm);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     FoldArgs a = a0;
     int rtiles = ((a.W1 + RW - 1) / RW) * ((a.H1 + RH - 1) / RH);
     SelBatch T{};
@@ -181,7 +178,20 @@ static cudaError_t launch_level(const FoldArgs& a0, cudaStream_t s, int grid_lim
         if (rtiles <= 0) return cudaGetLastError();
         fold0_border_rects(a.W, a.H, rg, T);
     }
-    if (a.red_n > 0) lsb_launched(), kr<<<dim3(rtiles, a.red_n), NT, rsm, s>>>(a);
+    if (a.red_n > 0) {
+        if constexpr (SRC != SRC_U16 && !FOCUS) {
+            const uintptr_t from = SRC == SRC_F32 ? (uintptr_t)a.src_f32 : (uintptr_t)a.src_g;
+            const int vec = (a.W & 1) == 0 && from % (2 * (SRC == SRC_G ? sizeof(GS) : sizeof(float))) == 0;
+            const int ntx = (a.W1 + RS_W - 1) / RS_W, nty = (a.H1 + RS_H * RS_WARPS - 1) / (RS_H * RS_WARPS);
+            lsb_launched(), reduce_strip_kernel<SRC, GS><<<dim3(ntx * nty, a.red_n, 3), RS_WARPS * 32, 0, s>>>(a, ntx, vec);
+        } else {
+            auto kr = reduce_level_kernel<SRC, GS, FOCUS, SS>;
+            const size_t rsm = (size_t)RED_FLOATS * sizeof(float);
+            cudaError_t e = with_smem(kr, rsm);
+            if (e != cudaSuccess) return e;
+            lsb_launched(), kr<<<dim3(rtiles, a.red_n), NT, rsm, s>>>(a);
+        }
+    }
     if (a.between) cudaEventRecord(a.between, s);
     if (a.select) {
         T.a[0] = a;
@@ -437,32 +447,88 @@ cudaError_t halo_divide(float* acc, const float* best, int w, int h, cudaStream_
 // pyramid.rs:219: G_l = L_l + EXPAND(G_{l+1}), EXPAND horizontal then
 // vertical (pyramid.rs:143) evaluated per output pixel with the same taps;
 // at level 0 also fuse.rs:516 clamp and io.rs:287 u16 packing.
-__device__ __forceinline__ float exp_row(const float* row, int cw, int x) {
-    const int cx = x >> 1;
-    return (x & 1) == 0 ? lsb_exp_even(row[lsb_reflect(cx - 1, cw)], row[lsb_reflect(cx, cw)], row[lsb_reflect(cx + 1, cw)])
-                        : lsb_exp_odd(row[lsb_reflect(cx, cw)], row[lsb_reflect(cx + 1, cw)]);
-}
-
-__global__ void collapse_kernel(const float* __restrict__ acc, const float* __restrict__ coarse, float* __restrict__ out,
-                                int w, int h, int cw, int ch, int last, uint16_t* __restrict__ rgb) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= w || y >= h) return;
-    const int cy = y >> 1;
-    for (int c = 0; c < 3; c++) {
-        const float* C = coarse + (size_t)c * cw * ch;
-        float up;
-        if ((y & 1) == 0)
-            up = lsb_exp_even(exp_row(C + (size_t)lsb_reflect(cy - 1, ch) * cw, cw, x), exp_row(C + (size_t)lsb_reflect(cy, ch) * cw, cw, x),
-                              exp_row(C + (size_t)lsb_reflect(cy + 1, ch) * cw, cw, x));
-        else
-            up = lsb_exp_odd(exp_row(C + (size_t)lsb_reflect(cy, ch) * cw, cw, x), exp_row(C + (size_t)lsb_reflect(cy + 1, ch) * cw, cw, x));
-        const size_t o = (size_t)c * w * h + (size_t)y * w + x;
-        float v = __fadd_rn(acc[o], up);
-        if (last) {
-            v = fminf(fmaxf(v, 0.f), 1.f);
-            if (rgb) rgb[((size_t)y * w + x) * 3 + c] = (uint16_t)__fadd_rn(__fmul_rn(v, 65535.f), 0.5f);
+// In register strips: a warp takes 60 x `rows` pixels, a lane the coarse column under its pixel pair; the row taps'
+// neighbours are shuffles, three expanded coarse rows stay in registers. What bounds it: its 33 bytes a pixel. One
+// pixel a thread, with its 9 coarse values of each channel read again, took 0.79 ms at 6000 x 4000 (0.12 of reads and
+// writes), 0.23 here; the five levels of 1024 x 768 68 us -> 27.
+constexpr int CS_W = 60, CS_WARPS = 4;
+template <bool LAST>
+__global__ void __launch_bounds__(CS_WARPS * 32) collapse_kernel(const float* __restrict__ acc, const float* __restrict__ coarse,
+                                                                 float* __restrict__ out, int w, int h, int cw, int ch, int ntx, int rows,
+                                                                 uint16_t* __restrict__ rgb) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int cx = (int)(blockIdx.x % ntx) * (CS_W / 2) - 1 + lane, x = 2 * cx;
+    const int y0 = ((int)(blockIdx.x / ntx) * CS_WARPS + wid) * rows;
+    if (y0 >= h) return;
+    const size_t np = (size_t)w * h, cp = (size_t)cw * ch;
+    const bool own0 = lane >= 1 && lane <= CS_W / 2 && x < w, own1 = own0 && x + 1 < w;
+    const bool vec = (w & 1) == 0;  // every row of pairs is aligned (the planes are the pool's own)
+    const float* cc = coarse + lsb_reflect(cx, cw);
+    auto load = [&](int cy, float v[3]) {
+        const float* p = cc + (size_t)lsb_reflect(cy, ch) * cw;
+#pragma unroll
+        for (int c = 0; c < 3; c++) v[c] = p[c * cp];
+    };
+    auto expand = [&](const float v[3], float2 e[3]) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const float l = __shfl_up_sync(ALL, v[c], 1), r = __shfl_down_sync(ALL, v[c], 1);
+            e[c] = make_float2(lsb_exp_even(l, v[c], r), lsb_exp_odd(v[c], r));
         }
-        out[o] = v;
+    };
+    float2 A[3], B[3], C[3];
+    float n[3];
+    {
+        float v0[3], v1[3];
+        load((y0 >> 1) - 1, v0);
+        load(y0 >> 1, v1);
+        load((y0 >> 1) + 1, n);
+        expand(v0, B);
+        expand(v1, C);
+    }
+#pragma unroll 2
+    for (int y = y0; y < y0 + rows && y < h; y += 2) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) A[c] = B[c], B[c] = C[c];
+        expand(n, C);
+        load((y >> 1) + 2, n);
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            if (y + s >= h) break;
+            const size_t o = (size_t)(y + s) * w + x;
+            float2 r[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const float* p = acc + c * np + o;
+                const float2 v = !own0 ? splat(0.f) : vec ? *(const float2*)p : make_float2(p[0], own1 ? p[1] : 0.f);
+                r[c] = add2(v, s ? exp_odd2(B[c], C[c]) : exp_even2(A[c], B[c], C[c]));
+                if (LAST) r[c] = make_float2(fminf(fmaxf(r[c].x, 0.f), 1.f), fminf(fmaxf(r[c].y, 0.f), 1.f));
+                float* q = out + c * np + o;
+                if (vec) {
+                    if (own0) *(float2*)q = r[c];
+                } else {
+                    if (own0) q[0] = r[c].x;
+                    if (own1) q[1] = r[c].y;
+                }
+            }
+            if (LAST && rgb) {
+                unsigned u[6];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    u[c] = (uint16_t)__fadd_rn(__fmul_rn(r[c].x, 65535.f), 0.5f);
+                    u[3 + c] = (uint16_t)__fadd_rn(__fmul_rn(r[c].y, 65535.f), 0.5f);
+                }
+                uint16_t* q = rgb + o * 3;
+                if (vec) {
+                    unsigned* q4 = (unsigned*)q;
+                    if (own0) q4[0] = u[0] | u[1] << 16, q4[1] = u[2] | u[3] << 16, q4[2] = u[4] | u[5] << 16;
+                } else {
+                    if (own0) q[0] = (uint16_t)u[0], q[1] = (uint16_t)u[1], q[2] = (uint16_t)u[2];
+                    if (own1) q[3] = (uint16_t)u[3], q[4] = (uint16_t)u[4], q[5] = (uint16_t)u[5];
+                }
+            }
+        }
     }
 }
 
@@ -480,8 +546,13 @@ cudaError_t upsample_index(const uint16_t* win, int dwl, int dhl, int scale, int
 
 cudaError_t collapse_level(const float* acc, const float* coarse, float* out, int w, int h, int cw, int ch, bool last,
                            uint16_t* rgb_out, cudaStream_t s) {
-    dim3 b(32, 8), g((w + 31) / 32, (h + 7) / 8);
-    lsb_launched(), collapse_kernel<<<g, b, 0, s>>>(acc, coarse, out, w, h, cw, ch, last ? 1 : 0, rgb_out);
+    // 16 rows a warp, fewer while the level has too few of them to fill the GPU: a row pair takes a round of latency
+    const int ntx = (w + CS_W - 1) / CS_W;
+    int rows = 16;
+    while (rows > 2 && (long)ntx * ((h + rows - 1) / rows) < 148 * 16) rows /= 2;
+    const int g = ntx * ((h + rows * CS_WARPS - 1) / (rows * CS_WARPS));
+    if (last) lsb_launched(), collapse_kernel<true><<<g, CS_WARPS * 32, 0, s>>>(acc, coarse, out, w, h, cw, ch, ntx, rows, rgb_out);
+    else lsb_launched(), collapse_kernel<false><<<g, CS_WARPS * 32, 0, s>>>(acc, coarse, out, w, h, cw, ch, ntx, rows, rgb_out);
     return cudaGetLastError();
 }
 
