@@ -858,165 +858,161 @@ __device__ void dev_mat_inverse(const double m[9], double inv[9]) {
     for (int i = 0; i < 9; i++) inv[i] = __ddiv_rn(inv[i], k);
 }
 
-// A block's copy of the search: the simplex, its costs, the box and steps of
-// the level, and the points of the batch in flight.
-struct NmState {
-    double cur[8], snap[8], simplex[9][8], fv[9], lo[8], hi[8], step[8], tol[8], xr[8], xe[8], xc[8];
-    double pts[MAX_CAND][8];  // the pending candidates (free coordinates)
-    int it, phase, evals;
-};
+// A warp's copy of the search (align.rs:796) over N free parameters, in registers: lane q holds parameter q of every
+// vertex (sorted by cost), its box, step and tolerance; the costs, the same in every lane. pts: the pending candidates,
+// all 8 parameters, and cur: the transform, in the CTA's shared memory.
 enum { NM_INIT = 0, NM_RXC = 1, NM_SHRINK = 2 };
-
-__device__ __forceinline__ void nm_put(NmState& S, int n, int k, const double* x) {
-    for (int q = 0; q < n; q++) S.pts[k][q] = x[q];
-}
-__device__ void nm_clamp(const NmState& S, int n, double* v) {
-    for (int q = 0; q < n; q++) v[q] = fmin(fmax(v[q], S.lo[q]), S.hi[q]);
-}
-// Start level L: the first simplex (align.rs:806-813). Returns the candidates pending.
-__device__ int nm_level_start(const NmJob& J, NmState& S, int L) {
-    const int n = J.nfree;
-    for (int q = 0; q < 8; q++) S.snap[q] = S.cur[q];
-    // align.rs:784 `level_steps`
-    const double wf = J.W, hf = J.H, r = fmax(wf, hf) / 2.0;
-    const double gain[8] = {wf, hf, r, r, hf / 2.0, hf / 2.0, wf / 4.0, hf / 4.0};
-    const double px = (double)(1ull << J.lv[L].lvl);
-    for (int q = 0; q < n; q++) {
-        S.step[q] = __ddiv_rn(__dmul_rn(1.0, px), gain[J.free_idx[q]]);
-        S.tol[q] = __ddiv_rn(__dmul_rn(0.1, px), gain[J.free_idx[q]]);
+template <int N>
+struct NmWarp {
+    double col[N + 1], f[N + 1], lo, hi, tol, xr, xe, xc;
+    int it, phase, evals, passes, fi, lane;
+    bool lq;
+    __device__ __forceinline__ double clampq(double v) const { return fmin(fmax(v, lo), hi); }
+    __device__ __forceinline__ void put(double (*pts)[8], int k, double v) const {
+        if (lq) pts[k][fi] = v;
     }
-    for (int q = 0; q < n; q++) S.simplex[0][q] = S.cur[J.free_idx[q]];
-    for (int k = 0; k < n; k++) {
-        for (int q = 0; q < n; q++) S.simplex[k + 1][q] = S.simplex[0][q];
-        S.simplex[k + 1][k] = __dadd_rn(S.simplex[k + 1][k], S.step[k]);
-        nm_clamp(S, n, S.simplex[k + 1]);
+    // the box around the start in cur
+    __device__ __forceinline__ void begin(const NmJob& J, const double* cur, int ln) {
+        lane = ln, lq = ln < N;
+        evals = 0, fi = 0;
+        lo = hi = tol = xr = xe = xc = 0.0;
+#pragma unroll
+        for (int q = 0; q < N; q++)
+            if (lane == q) fi = J.free_idx[q];
+        if (lq) {
+            lo = __dsub_rn(cur[fi], c_span[fi]);
+            hi = __dadd_rn(cur[fi], c_span[fi]);
+        }
     }
-    for (int k = 0; k <= n; k++) nm_put(S, n, k, S.simplex[k]);
-    S.phase = NM_INIT;
-    S.it = 0;
-    return n + 1;
-}
-// One step of align.rs:796's loop (the top of align.rs:815's loop and the branch on the
-// batch's costs), run by one warp: lane q owns free
-// parameter q of every vertex, so the per-parameter arithmetic (centroid,
-// reflection, expansion, contraction, shrink, clamps, the convergence test)
-// runs in parallel in the reference's per-parameter operation order; the
-// scalar decisions are taken identically by every lane. The stable sort by
-// cost places vertex i at #{j: f_j < f_i} + #{j < i: f_j == f_i}, the
-// position the insertion sort gives it.
-__device__ int nm_iterate_warp(const NmJob& J, NmState& S, int lane) {
-    const int n = J.nfree;
-    const bool lq = lane < n;
-    bool done = S.it >= 200;
-    if (!done) {
+    // align.rs:784 `level_steps`, align.rs:806-813 the first simplex, around cur: N + 1 pending
+    __device__ __forceinline__ int level(const NmJob& J, const NmLevel& lv, double (*pts)[8], const double* cur) {
+        double step = 0.0;
+        if (lq) {
+            const double wf = J.W, hf = J.H, r = fmax(wf, hf) / 2.0;
+            const double gain[8] = {wf, hf, r, r, hf / 2.0, hf / 2.0, wf / 4.0, hf / 4.0};
+            const double px = (double)(1ull << lv.lvl);
+            double g = 1.0;
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (q == fi) g = gain[q];
+            step = __ddiv_rn(__dmul_rn(1.0, px), g);
+            tol = __ddiv_rn(__dmul_rn(0.1, px), g);
+        }
+        const double x0 = lq ? cur[fi] : 0.0;
+        for (int e = lane; e < MAX_CAND * 8; e += 32) pts[e / 8][e % 8] = cur[e % 8];
         __syncwarp();
-        if (lane == 0) S.it++;
-        // stable sort: each lane i <= n moves its own vertex
-        double row[8], fi = 0.0;
-        int rank = 0;
-        if (lane <= n) {
-            fi = S.fv[lane];
-            for (int q = 0; q < n; q++) row[q] = S.simplex[lane][q];
-            for (int j = 0; j <= n; j++) {
-                const double fj = S.fv[j];
-                rank += (fj < fi) || (fj == fi && j < lane);
+        col[0] = x0;
+#pragma unroll
+        for (int k = 0; k < N; k++) col[k + 1] = clampq(k == lane ? __dadd_rn(x0, step) : x0);
+#pragma unroll
+        for (int k = 0; k <= N; k++) put(pts, k, col[k]);
+        phase = NM_INIT;
+        it = 0;
+        passes = 0;
+        return N + 1;
+    }
+    // align.rs:815's loop from its top: stable sort, convergence, the next candidates. Returns how many are pending.
+    __device__ __forceinline__ int iterate(double (*pts)[8], double* cur) {
+        bool done = it >= 200;
+        // insertion from the back; strictly smaller moves forward, so equal costs keep their order
+#pragma unroll
+        for (int i = 1; i <= N; i++)
+#pragma unroll
+            for (int j = i; j > 0; j--)
+                if (f[j] < f[j - 1]) {
+                    const double tf = f[j], tc = col[j];
+                    f[j] = f[j - 1], col[j] = col[j - 1];
+                    f[j - 1] = tf, col[j - 1] = tc;
+                }
+        if (!done) {
+            it++;
+            // align.rs:888 `converged`
+            const bool conv = fabs(__dsub_rn(f[N], f[0])) <= __dmul_rn(1e-4, __dadd_rn(1.0, fabs(f[0])));
+            bool mine = true;
+            if (lq)
+#pragma unroll
+                for (int i = 1; i <= N; i++) mine = mine && fabs(__dsub_rn(col[i], col[0])) <= tol;
+            done = conv && __all_sync(0xffffffffu, mine);
+        }
+        if (done) {
+            if (lq) cur[fi] = col[0];
+            return 0;
+        }
+        double c = 0.0;
+#pragma unroll
+        for (int i = 0; i < N; i++) c = __dadd_rn(c, col[i]);
+        c = __ddiv_rn(c, (double)N);
+        xr = clampq(__dadd_rn(c, __dmul_rn(1.0, __dsub_rn(c, col[N]))));
+        xe = clampq(__dadd_rn(c, __dmul_rn(2.0, __dsub_rn(xr, c))));
+        xc = clampq(__dadd_rn(c, __dmul_rn(0.5, __dsub_rn(col[N], c))));
+        put(pts, 0, xr);
+        put(pts, 1, xe);
+        put(pts, 2, xc);
+        phase = NM_RXC;
+        return 3;
+    }
+    // The pending candidates' costs (candidate k's in lane k) taken in; how many are pending next. ctl: set to 2 by
+    // the caller's `tell` copy past the limit of <= 200 iterations of at most two batches each, plus the first simplex.
+    __device__ __forceinline__ int advance(double cost, double (*pts)[8], double* cur, int* ctl, bool tell) {
+        int nx;
+        if (phase == NM_INIT) {
+#pragma unroll
+            for (int k = 0; k <= N; k++) f[k] = __shfl_sync(0xffffffffu, cost, k);
+            evals += N + 1;
+            nx = iterate(pts, cur);
+        } else if (phase == NM_SHRINK) {
+#pragma unroll
+            for (int k = 1; k <= N; k++) f[k] = __shfl_sync(0xffffffffu, cost, k - 1);
+            evals += N;
+            nx = iterate(pts, cur);
+        } else {
+            const double fr = __shfl_sync(0xffffffffu, cost, 0), fe = __shfl_sync(0xffffffffu, cost, 1), fc = __shfl_sync(0xffffffffu, cost, 2);
+            evals++;
+            int take;  // 0 xr, 1 xe, 2 xc, 3 shrink
+            if (fr < f[0]) {
+                evals++;
+                take = fe < fr ? 1 : 0;
+            } else if (fr < f[N - 1]) {
+                take = 0;
+            } else {
+                evals++;
+                take = fc < f[N] ? 2 : 3;
+            }
+            if (take < 3) {
+                col[N] = take == 0 ? xr : take == 1 ? xe : xc;
+                f[N] = take == 0 ? fr : take == 1 ? fe : fc;
+                nx = iterate(pts, cur);
+            } else {
+#pragma unroll
+                for (int i = 1; i <= N; i++) {
+                    col[i] = clampq(__dadd_rn(col[0], __dmul_rn(0.5, __dsub_rn(col[i], col[0]))));
+                    put(pts, i - 1, col[i]);
+                }
+                phase = NM_SHRINK;
+                nx = N;
             }
         }
-        __syncwarp();
-        if (lane <= n) {
-            S.fv[rank] = fi;
-            for (int q = 0; q < n; q++) S.simplex[rank][q] = row[q];
+        if (++passes > 402 && nx > 0) {
+            nx = 0;
+            if (tell && lane == 0) atomicCAS(ctl, 0, 2);
         }
+        return nx;
+    }
+    // the pending candidates' matrices
+    __device__ __forceinline__ void matrices(int nc, const NmLevel& lv, const double (*pts)[8], double (*cand)[9]) const {
         __syncwarp();
-        // align.rs:888 `converged`
-        bool conv = fabs(__dsub_rn(S.fv[n], S.fv[0])) <= __dmul_rn(1e-4, __dadd_rn(1.0, fabs(S.fv[0])));
-        bool mine = true;
-        if (lq)
-            for (int i = 1; i <= n; i++) mine = mine && fabs(__dsub_rn(S.simplex[i][lane], S.simplex[0][lane])) <= S.tol[lane];
-        done = conv && __all_sync(0xffffffffu, mine);
-    }
-    if (done) {
-        int best = 0;
-        for (int i = 1; i <= n; i++)
-            if (S.fv[i] < S.fv[best]) best = i;
-        __syncwarp();
-        if (lq) S.cur[J.free_idx[lane]] = S.simplex[best][lane];
-        __syncwarp();
-        return 0;
-    }
-    if (lq) {
-        const int q = lane;
-        double c = 0.0;
-        for (int i = 0; i < n; i++) c = __dadd_rn(c, S.simplex[i][q]);
-        c = __ddiv_rn(c, (double)n);
-        const double xn = S.simplex[n][q];
-        double xr = __dadd_rn(c, __dmul_rn(1.0, __dsub_rn(c, xn)));
-        xr = fmin(fmax(xr, S.lo[q]), S.hi[q]);
-        double xe = __dadd_rn(c, __dmul_rn(2.0, __dsub_rn(xr, c)));
-        xe = fmin(fmax(xe, S.lo[q]), S.hi[q]);
-        double xc = __dadd_rn(c, __dmul_rn(0.5, __dsub_rn(xn, c)));
-        xc = fmin(fmax(xc, S.lo[q]), S.hi[q]);
-        S.xr[q] = xr;
-        S.xe[q] = xe;
-        S.xc[q] = xc;
-        S.pts[0][q] = xr;
-        S.pts[1][q] = xe;
-        S.pts[2][q] = xc;
-    }
-    if (lane == 0) S.phase = NM_RXC;
-    __syncwarp();
-    return 3;
-}
-__device__ int nm_advance_warp(const NmJob& J, NmState& S, const double* cost, int lane) {
-    const int n = J.nfree;
-    const bool lq = lane < n;
-    const int phase = S.phase;
-    __syncwarp();
-    if (phase == NM_INIT) {
-        if (lane <= n) S.fv[lane] = cost[lane];
-        if (lane == 0) S.evals += n + 1;
-        __syncwarp();
-        return nm_iterate_warp(J, S, lane);
-    }
-    if (phase == NM_SHRINK) {
-        if (lane >= 1 && lane <= n) S.fv[lane] = cost[lane - 1];
-        if (lane == 0) S.evals += n;
-        __syncwarp();
-        return nm_iterate_warp(J, S, lane);
-    }
-    const double fr = cost[0], fe = cost[1], fc = cost[2];
-    int evals = 1;
-    int take = -1;  // 0 xr, 1 xe, 2 xc, 3 shrink
-    if (fr < S.fv[0]) {
-        evals += 1;
-        take = fe < fr ? 1 : 0;
-    } else if (fr < S.fv[n - 1]) {
-        take = 0;
-    } else {
-        evals += 1;
-        take = fc < S.fv[n] ? 2 : 3;
-    }
-    __syncwarp();
-    if (lane == 0) S.evals += evals;
-    if (take < 3) {
-        if (lq) S.simplex[n][lane] = take == 0 ? S.xr[lane] : (take == 1 ? S.xe[lane] : S.xc[lane]);
-        if (lane == 0) S.fv[n] = take == 0 ? fr : (take == 1 ? fe : fc);
-        __syncwarp();
-        return nm_iterate_warp(J, S, lane);
-    }
-    if (lq) {
-        const int q = lane;
-        const double s0 = S.simplex[0][q];
-        for (int i = 1; i <= n; i++) {
-            double v = __dadd_rn(s0, __dmul_rn(0.5, __dsub_rn(S.simplex[i][q], s0)));
-            v = fmin(fmax(v, S.lo[q]), S.hi[q]);
-            S.simplex[i][q] = v;
-            S.pts[i - 1][q] = v;
+        if (lane < nc) {
+            double v[8], m[9];
+#pragma unroll
+            for (int q = 0; q < 8; q++) v[q] = pts[lane][q];
+            dev_sim_matrix(v, lv.w, lv.h, m);
+            dev_mat_inverse(m, cand[lane]);
         }
     }
-    if (lane == 0) S.phase = NM_SHRINK;
-    __syncwarp();
-    return n;
+};
+// A candidate's cost from its sums of d, d^2 and the count
+__device__ __forceinline__ double nm_cost(double sd, double sd2, double cn) {
+    return cn < 16.0 ? 1e9 : sqrt(fmax(__ddiv_rn(__dsub_rn(sd2, __ddiv_rn(__dmul_rn(sd, sd), cn)), cn), 0.0));
 }
 
 // The bounded wait of the search's grid-wide hand-off (at least ~0.1 s of polling);
@@ -1053,25 +1049,28 @@ __device__ void nm_publish(const NmJob& J, const double* cur, int evals) {
 
 constexpr int NM_THREADS = 256, NM_WARPS = NM_THREADS / 32;
 // align.rs:896 `multiscale_align` of one frame: the NmJob's whole coarse-to-fine search.
-__global__ void __launch_bounds__(NM_THREADS) nm_search_kernel(const NmJob J) {
-    __shared__ NmState S;
+// The simplex is in warp 0's registers, as in nm_cluster_kernel: in shared memory, each step by a chain of accesses, a
+// batch took 2 us more (516 x 344 pair 1.10 ms -> 1.01, 2048 x 1536 x 16 17.7 -> 17.25). 2 CTAs an SM: held to 64 or 80
+// registers (4 or 3) the state spills into the pixel loop (1.15 and 1.09).
+template <int N>
+__global__ void __launch_bounds__(NM_THREADS, 2) nm_search_kernel(const NmJob J) {
+    __shared__ double pts[MAX_CAND][8], cur[8];
     __shared__ double cand[MAX_CAND][9];
     __shared__ double wred[MAX_CAND][3][NM_WARPS];
     __shared__ double gred[NM_THREADS];
-    __shared__ double cost[MAX_CAND];
     __shared__ int pending;
     __shared__ int s_ok;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (tid == 0) {
-        for (int q = 0; q < 8; q++) S.cur[q] = J.init_dev ? J.init_dev[q] : J.init[q];
-        for (int q = 0; q < J.nfree; q++) {
-            S.lo[q] = __dsub_rn(S.cur[J.free_idx[q]], c_span[J.free_idx[q]]);
-            S.hi[q] = __dadd_rn(S.cur[J.free_idx[q]], c_span[J.free_idx[q]]);
-        }
-        S.evals = 0;
+    NmWarp<N> S;  // warp 0's
+    if (wid == 0) {
+        if (lane < 8) cur[lane] = J.init_dev ? J.init_dev[lane] : J.init[lane];
+        __syncwarp();
+        S.begin(J, cur, lane);
+        __syncwarp();
         if (J.nlv_cluster > 0) {  // the cluster's levels are done: on from their result, in the box of the start
-            for (int q = 0; q < 8; q++) S.cur[q] = J.mid[q];
+            if (lane < 8) cur[lane] = J.mid[lane];
             S.evals = (int)J.mid[8];
+            __syncwarp();
         }
     }
     int batch = 0;
@@ -1080,7 +1079,11 @@ __global__ void __launch_bounds__(NM_THREADS) nm_search_kernel(const NmJob J) {
     for (int L = J.nlv_cluster; L < J.nlv; L++) {
         const NmLevel lv = J.lv[L];
         __syncthreads();
-        if (tid == 0) pending = J.nfree > 0 ? nm_level_start(J, S, L) : 0;
+        if (wid == 0) {
+            const int nc = S.level(J, lv, pts, cur);
+            S.matrices(nc, lv, pts, cand);
+            if (lane == 0) pending = nc;
+        }
         __syncthreads();
         const double xmax = (double)(lv.w - 1), ymax = (double)(lv.h - 1);
         const unsigned npx = (unsigned)lv.w * lv.h;  // < 2^32 (the host checks)
@@ -1089,17 +1092,8 @@ __global__ void __launch_bounds__(NM_THREADS) nm_search_kernel(const NmJob J) {
         const unsigned sdy = stride / (unsigned)lv.w, sdx = stride - sdy * (unsigned)lv.w;
         const unsigned i0 = blockIdx.x * NM_THREADS + tid;
         const int y0s = (int)(i0 / (unsigned)lv.w), x0s = (int)(i0 - (unsigned)y0s * lv.w);
-        int passes = 0;
         while (pending > 0) {
             const int nc = pending;
-            if (tid < nc) {
-                double v[8], m[9];
-                for (int q = 0; q < 8; q++) v[q] = S.snap[q];
-                for (int q = 0; q < J.nfree; q++) v[J.free_idx[q]] = S.pts[tid][q];
-                dev_sim_matrix(v, lv.w, lv.h, m);
-                dev_mat_inverse(m, cand[tid]);
-            }
-            __syncthreads();
             // the batch's candidates three at a time in one pass over this block's pixels: the
             // reference value and the pixel's coordinates are shared, the three chains interleave
             for (int k0 = 0; k0 < nc; k0 += 3) {
@@ -1227,35 +1221,28 @@ __global__ void __launch_bounds__(NM_THREADS) nm_search_kernel(const NmJob J) {
                 }
                 gred[tid] = sv;
                 __syncthreads();
-                if (tid < nc) {
-                    double v3[3];
-                    for (int q = 0; q < 3; q++) {
-                        const double* g = gred + (size_t)(tid * 3 + q) * gsz;
-                        double a = 0.0;
-                        for (int i = 0; i < gsz; i++) a += g[i];
-                        v3[q] = a;
+                if (wid == 0) {
+                    double cost = 0.0;
+                    if (lane < nc) {
+                        double v3[3];
+                        for (int q = 0; q < 3; q++) {
+                            const double* g = gred + (size_t)(lane * 3 + q) * gsz;
+                            double a = 0.0;
+                            for (int i = 0; i < gsz; i++) a += g[i];
+                            v3[q] = a;
+                        }
+                        cost = nm_cost(v3[0], v3[1], v3[2]);
                     }
-                    const double sdv = v3[0], sd2v = v3[1], cn = v3[2];
-                    cost[tid] = cn < 16.0 ? 1e9 : sqrt(fmax(__ddiv_rn(__dsub_rn(sd2v, __ddiv_rn(__dmul_rn(sdv, sdv), cn)), cn), 0.0));
-                }
-            }
-            __syncthreads();
-            if (wid == 0) {
-                int nx = nm_advance_warp(J, S, cost, lane);
-                // <= 200 iterations of at most two batches each, plus the first simplex
-                if (lane == 0) {
-                    if (++passes > 402 && nx > 0) {
-                        nx = 0;
-                        if (blockIdx.x == 0) atomicCAS(J.ctl, 0, 2);
-                    }
-                    pending = nx;
+                    const int nx = S.advance(cost, pts, cur, J.ctl, blockIdx.x == 0);
+                    S.matrices(nx, lv, pts, cand);
+                    if (lane == 0) pending = nx;
                 }
             }
             batch++;
             __syncthreads();
         }
     }
-    if (blockIdx.x == 0 && tid == 0) nm_publish(J, S.cur, S.evals);
+    if (blockIdx.x == 0 && tid == 0) nm_publish(J, cur, S.evals);
 }
 
 // How a level is shared out: strips of 32 columns x `rows` rows, one warp at a time.
@@ -1417,9 +1404,9 @@ __device__ __forceinline__ void nm_eval(const NmLevel& lv, const double (*cand)[
 // the finer ones. What bounds a batch there is latency, and most of it was the hand-off between 296 CTAs through
 // global memory (4 us), their partial sums (2.5) and the Nelder-Mead step in shared memory (2.5): here every CTA's
 // sums go straight into every other's shared memory, one cluster barrier hands them over, and warp 0 of each CTA keeps
-// the sorted simplex in registers (lane q: parameter q of every vertex; the costs in every lane). N: the number of
-// free parameters. The search is align.rs:796's, step for step, as in nm_search_kernel; the f64 sums are added in
-// another order. A batch of the coarsest levels of 2048 x 1536: 14 us there, 6 here.
+// the sorted simplex in registers (NmWarp). N: the number of free parameters. The search is align.rs:796's, step for
+// step, as in nm_search_kernel; the f64 sums are added in another order. A batch of the coarsest levels of 2048 x 1536:
+// 14 us there, 6 here.
 // Where the line lies: 16 SMs evaluate a larger level more slowly than the grid does, and the grid pays its hand-off
 // only once per batch. A 516 x 344 pair, a 2048 x 1536 stack of 16 and an 8256 x 5504 one of 10, ms: no cluster 1.24 /
 // 22.7 / 80.2, levels of up to 4096 pixels 1.13 / 20.0 / -, 16384 1.11 / 18.4 / 77.9, 65536 1.37 / 20.7 / 78.1.
@@ -1436,105 +1423,19 @@ __global__ void __launch_bounds__(NMC_THREADS) nm_cluster_kernel(const NmJob J) 
     __shared__ int pending;
     cg::cluster_group cl = cg::this_cluster();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, rank = (int)cl.block_rank(), nb = (int)cl.num_blocks();
-    const bool lq = lane < N;
-    // warp 0's copy of the search: this lane's parameter of the vertices (sorted by cost), its box, step and tolerance
-    double col[N + 1], f[N + 1], lo = 0.0, hi = 0.0, tol = 0.0, xr = 0.0, xe = 0.0, xc = 0.0;
-    int it = 0, phase = NM_INIT, evals = 0, passes = 0;
+    NmWarp<N> S;  // warp 0's copy of the search
     if (tid < 8) cur[tid] = J.init_dev ? J.init_dev[tid] : J.init[tid];
     __syncthreads();
-    int fi = 0;
-#pragma unroll
-    for (int q = 0; q < N; q++)
-        if (lane == q) fi = J.free_idx[q];
-    if (lq) {
-        lo = __dsub_rn(cur[fi], c_span[fi]);
-        hi = __dadd_rn(cur[fi], c_span[fi]);
-    }
-    auto clampq = [&](double v) { return fmin(fmax(v, lo), hi); };
-    auto put = [&](int k, double v) {
-        if (lq) pts[k][fi] = v;
-    };
-    // align.rs:815's loop from its top: stable sort, convergence, the next candidates. Returns how many are pending.
-    auto iterate = [&]() -> int {
-        bool done = it >= 200;
-        // insertion from the back; strictly smaller moves forward, so equal costs keep their order
-#pragma unroll
-        for (int i = 1; i <= N; i++)
-#pragma unroll
-            for (int j = i; j > 0; j--)
-                if (f[j] < f[j - 1]) {
-                    const double tf = f[j], tc = col[j];
-                    f[j] = f[j - 1], col[j] = col[j - 1];
-                    f[j - 1] = tf, col[j - 1] = tc;
-                }
-        if (!done) {
-            it++;
-            // align.rs:888 `converged`
-            const bool conv = fabs(__dsub_rn(f[N], f[0])) <= __dmul_rn(1e-4, __dadd_rn(1.0, fabs(f[0])));
-            bool mine = true;
-            if (lq)
-#pragma unroll
-                for (int i = 1; i <= N; i++) mine = mine && fabs(__dsub_rn(col[i], col[0])) <= tol;
-            done = conv && __all_sync(0xffffffffu, mine);
-        }
-        if (done) {
-            if (lq) cur[fi] = col[0];
-            return 0;
-        }
-        double c = 0.0;
-#pragma unroll
-        for (int i = 0; i < N; i++) c = __dadd_rn(c, col[i]);
-        c = __ddiv_rn(c, (double)N);
-        xr = clampq(__dadd_rn(c, __dmul_rn(1.0, __dsub_rn(c, col[N]))));
-        xe = clampq(__dadd_rn(c, __dmul_rn(2.0, __dsub_rn(xr, c))));
-        xc = clampq(__dadd_rn(c, __dmul_rn(0.5, __dsub_rn(col[N], c))));
-        put(0, xr);
-        put(1, xe);
-        put(2, xc);
-        phase = NM_RXC;
-        return 3;
-    };
+    S.begin(J, cur, lane);
+    __syncthreads();
     int batch = 0;
     for (int L = 0; L < J.nlv_cluster; L++) {
         const NmLevel lv = J.lv[L];
         const NmStrips S_ = nm_strips(lv, nb * NMC_WARPS);
-        // the pending candidates' matrices, by warp 0 (their parameters that are not free: the level's start)
-        auto matrices = [&](int nc) {
-            __syncwarp();
-            if (lane < nc) {
-                double v[8], m[9];
-#pragma unroll
-                for (int q = 0; q < 8; q++) v[q] = pts[lane][q];
-                dev_sim_matrix(v, lv.w, lv.h, m);
-                dev_mat_inverse(m, cand[lane]);
-            }
+        if (wid == 0) {
+            const int nc = S.level(J, lv, pts, cur);
+            S.matrices(nc, lv, pts, cand);
             if (lane == 0) pending = nc;
-        };
-        if (wid == 0) {  // align.rs:784 `level_steps`, align.rs:806-813 the first simplex
-            double step = 0.0;
-            if (lq) {
-                const double wf = J.W, hf = J.H, r = fmax(wf, hf) / 2.0;
-                const double gain[8] = {wf, hf, r, r, hf / 2.0, hf / 2.0, wf / 4.0, hf / 4.0};
-                const double px = (double)(1ull << lv.lvl);
-                double g = 1.0;
-#pragma unroll
-                for (int q = 0; q < 8; q++)
-                    if (q == fi) g = gain[q];
-                step = __ddiv_rn(__dmul_rn(1.0, px), g);
-                tol = __ddiv_rn(__dmul_rn(0.1, px), g);
-            }
-            const double x0 = lq ? cur[fi] : 0.0;
-            for (int e = lane; e < MAX_CAND * 8; e += 32) pts[e / 8][e % 8] = cur[e % 8];
-            __syncwarp();
-            col[0] = x0;
-#pragma unroll
-            for (int k = 0; k < N; k++) col[k + 1] = clampq(k == lane ? __dadd_rn(x0, step) : x0);
-#pragma unroll
-            for (int k = 0; k <= N; k++) put(k, col[k]);
-            phase = NM_INIT;
-            it = 0;
-            passes = 0;
-            matrices(N + 1);
         }
         __syncthreads();
         while (pending > 0) {
@@ -1572,51 +1473,9 @@ __global__ void __launch_bounds__(NMC_THREADS) nm_cluster_kernel(const NmJob J) 
                     for (int i = 0; i < nb; i++) t += slot[par][lane][i];
                 const int src = min(3 * lane, 29);
                 const double sdv = __shfl_sync(0xffffffffu, t, src), sd2v = __shfl_sync(0xffffffffu, t, src + 1), cn = __shfl_sync(0xffffffffu, t, src + 2);
-                const double cost = cn < 16.0 ? 1e9 : sqrt(fmax(__ddiv_rn(__dsub_rn(sd2v, __ddiv_rn(__dmul_rn(sdv, sdv), cn)), cn), 0.0));
-                int nx;
-                if (phase == NM_INIT) {
-#pragma unroll
-                    for (int k = 0; k <= N; k++) f[k] = __shfl_sync(0xffffffffu, cost, k);
-                    evals += N + 1;
-                    nx = iterate();
-                } else if (phase == NM_SHRINK) {
-#pragma unroll
-                    for (int k = 1; k <= N; k++) f[k] = __shfl_sync(0xffffffffu, cost, k - 1);
-                    evals += N;
-                    nx = iterate();
-                } else {
-                    const double fr = __shfl_sync(0xffffffffu, cost, 0), fe = __shfl_sync(0xffffffffu, cost, 1), fc = __shfl_sync(0xffffffffu, cost, 2);
-                    evals++;
-                    int take;  // 0 xr, 1 xe, 2 xc, 3 shrink
-                    if (fr < f[0]) {
-                        evals++;
-                        take = fe < fr ? 1 : 0;
-                    } else if (fr < f[N - 1]) {
-                        take = 0;
-                    } else {
-                        evals++;
-                        take = fc < f[N] ? 2 : 3;
-                    }
-                    if (take < 3) {
-                        col[N] = take == 0 ? xr : take == 1 ? xe : xc;
-                        f[N] = take == 0 ? fr : take == 1 ? fe : fc;
-                        nx = iterate();
-                    } else {
-#pragma unroll
-                        for (int i = 1; i <= N; i++) {
-                            col[i] = clampq(__dadd_rn(col[0], __dmul_rn(0.5, __dsub_rn(col[i], col[0]))));
-                            put(i - 1, col[i]);
-                        }
-                        phase = NM_SHRINK;
-                        nx = N;
-                    }
-                }
-                // <= 200 iterations of at most two batches each, plus the first simplex
-                if (++passes > 402 && nx > 0) {
-                    nx = 0;
-                    if (rank == 0 && lane == 0) atomicCAS(J.ctl, 0, 2);
-                }
-                matrices(nx);
+                const int nx = S.advance(nm_cost(sdv, sd2v, cn), pts, cur, J.ctl, rank == 0);
+                S.matrices(nx, lv, pts, cand);
+                if (lane == 0) pending = nx;
             }
             batch++;
             __syncthreads();
@@ -1624,10 +1483,10 @@ __global__ void __launch_bounds__(NMC_THREADS) nm_cluster_kernel(const NmJob J) 
     }
     if (rank == 0 && tid == 0) {
         if (J.nlv_cluster == J.nlv) {
-            nm_publish(J, cur, evals);
+            nm_publish(J, cur, S.evals);
         } else {
             for (int q = 0; q < 8; q++) J.mid[q] = cur[q];
-            J.mid[8] = (double)evals;
+            J.mid[8] = (double)S.evals;
         }
     }
     cl.sync();
@@ -1660,7 +1519,7 @@ static cudaError_t nm_job(AlignCtx& C, const float* rf, const std::vector<float*
         int dev = 0, sms = 0, per = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, nm_search_kernel, NM_THREADS, 0);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, nm_search_kernel<8>, NM_THREADS, 0);
         if (e != cudaSuccess) return e;
         if (per < 1) return cudaErrorCooperativeLaunchTooLarge;
         int want = 2;  // CTAs per SM: more warps hide the gathers, more CTAs make every barrier dearer
@@ -1746,7 +1605,10 @@ static cudaError_t nm_launch(AlignCtx& C, NmJob& J) {
     void* args[] = {(void*)&J};
     lsb_launched();
     const int blocks = C.max_blocks > 0 ? std::min(g_nm_blocks.load(), C.max_blocks) : g_nm_blocks.load();
-    return cudaLaunchCooperativeKernel((void*)nm_search_kernel, dim3(blocks), dim3(NM_THREADS), args, 0, C.s);
+    static void* const kernels[] = {(void*)nm_search_kernel<1>, (void*)nm_search_kernel<2>, (void*)nm_search_kernel<3>, (void*)nm_search_kernel<4>,
+                                    (void*)nm_search_kernel<5>, (void*)nm_search_kernel<6>, (void*)nm_search_kernel<7>, (void*)nm_search_kernel<8>};
+    if (J.nfree == 0) J.nlv = 0;  // nothing to search: the start is the result
+    return cudaLaunchCooperativeKernel(kernels[std::max(J.nfree, 1) - 1], dim3(blocks), dim3(NM_THREADS), args, 0, C.s);
 }
 
 static cudaError_t multiscale_align_dev(AlignCtx& C, const float* rf, const std::vector<float*>& pr, const float* tg,

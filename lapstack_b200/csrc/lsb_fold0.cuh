@@ -1,7 +1,7 @@
 // The level-0 fold in ONE kernel (included by lsb_fold.cu inside namespace
 // lsb, after lsb_level.cuh).
 //
-// reduce_level_kernel + select_level_kernel read every level-0 frame from HBM
+// reduce_level_kernel + select_strip_kernel read every level-0 frame from HBM
 // twice (once to REDUCE it to G_1 and take its focus slice, once to select
 // its Laplacian coefficients). fold0_kernel does both from one staged copy of
 // the frame: a CTA owns a 64x32 tile of level 0 and walks the frames in
