@@ -2,12 +2,12 @@
 // inside namespace lsb.
 //
 // Level l of the fold runs as two kernels:
-//  * reduce_level_kernel, one CTA per (frame, 32x16 tile of G_{l+1}): stages
-//    the tile's G_l window, REDUCEs rows then columns (pyramid.rs:86) and
-//    writes G_{l+1} once; at level 0 it also takes the frame's focus slice
-//    (depth.rs:1097: luma -> ring difference filter -> block mean) from the
-//    same staged window. Parallel over frames, so even the coarse levels fill
-//    the GPU.
+//  * the REDUCE (pyramid.rs:86). reduce_level_kernel, of 16-bit frames and with
+//    a focus slice, one CTA per (frame, 32x16 tile of G_{l+1}): stages the
+//    tile's G_l window, REDUCEs rows then columns, writes G_{l+1} once and takes
+//    the focus slice (depth.rs:1097: luma -> ring difference filter -> block
+//    mean) from the same window. reduce_strip_kernel, of planar sources without
+//    a focus slice: register strips.
 //  * select_strip_kernel (lsb_select.cuh) selects from G_l and G_{l+1}.
 // Tiles whose windows never reach the border index without reflect-101
 // (IN = true); border tiles reflect as pyramid.rs:51 does. Every float op is
