@@ -1437,7 +1437,7 @@ __global__ void __launch_bounds__(NMC_THREADS) nm_cluster_kernel(const NmJob J) 
     if (tid < 8) cur[tid] = J.init_dev ? J.init_dev[tid] : J.init[tid];
     __syncthreads();
     S.begin(J, cur, lane);
-    __syncthreads();
+    cl.sync();  // every CTA runs: only from here on may the others write into its shared memory
     int batch = 0;
     for (int L = 0; L < J.nlv_cluster; L++) {
         const NmLevel lv = J.lv[L];
