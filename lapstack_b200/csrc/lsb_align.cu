@@ -1442,6 +1442,7 @@ __global__ void __launch_bounds__(NMC_THREADS) nm_cluster_kernel(const NmJob J) 
     for (int L = 0; L < J.nlv_cluster; L++) {
         const NmLevel lv = J.lv[L];
         const NmStrips S_ = nm_strips(lv, nb * NMC_WARPS);
+        __syncthreads();  // every warp has read the last level's `pending`
         if (wid == 0) {
             const int nc = S.level(J, lv, pts, cur);
             S.matrices(nc, lv, pts, cand);

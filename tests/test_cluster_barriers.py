@@ -52,3 +52,18 @@ def test_a_cluster_barrier_comes_before_the_first_remote_access(kernel):
     body = _body(_code(name), kernel)
     first = re.search(FIRST_REMOTE[kernel], body).start()
     assert "cl.sync()" in body[:first], "another CTA's shared memory is written before the cluster is known to run"
+
+
+def _after_level_loop_starts(kernel):
+    body = _body(_code("lsb_align.cu"), kernel)
+    loop = re.search(r"for \(int L = [^)]*\)", body)
+    return body[loop.end():]
+
+
+@pytest.mark.parametrize("kernel", ["nm_search_kernel", "nm_cluster_kernel"])
+def test_a_search_level_begins_behind_a_barrier(kernel):
+    """Warp 0 writes `pending` for the next level; every other warp has left the loop before, which reads it, only behind
+    a barrier of the CTA."""
+    rest = _after_level_loop_starts(kernel)
+    assert "while (pending > 0)" in rest
+    assert "__syncthreads();" in rest[:rest.index("pending =")], "a warp may still be reading the last level's count"
