@@ -1286,7 +1286,7 @@ __global__ void __launch_bounds__(CH_THREADS) coarse_h_kernel(uint16_t* __restri
         if (r == 0 && up[q]) up[q][i] = u;
         if (r == nr - 1 && down[q]) down[q][i] = u;
     };
-    __syncthreads();
+    cl.sync();  // this band is loaded, and every CTA runs: its neighbours may write into its halo rows
     for (int r = warp; r < nr; r += CH_THREADS / 32)
         for (int i = lane; i < w; i += 32) put(0, r, i, MG_OMEGA * ldh(sdi, r * w + i) * ldh(sb, r * w + i));
     cl.sync();

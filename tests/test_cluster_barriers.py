@@ -39,14 +39,14 @@ def _kernels_with_remote_memory():
 
 
 def test_the_cluster_kernels_are_found():
-    assert ("lsb_align.cu", "nm_cluster_kernel") in _kernels_with_remote_memory()
+    assert _kernels_with_remote_memory() == [("lsb_align.cu", "nm_cluster_kernel"), ("lsb_wls.cu", "coarse_h_kernel")]
 
 
 # where each kernel first touches another CTA's shared memory
 FIRST_REMOTE = {"nm_cluster_kernel": r"\*cl\.map_shared_rank\(", "coarse_h_kernel": r"\bput\(0,"}
 
 
-@pytest.mark.parametrize("kernel", ["nm_cluster_kernel"])
+@pytest.mark.parametrize("kernel", sorted(FIRST_REMOTE))
 def test_a_cluster_barrier_comes_before_the_first_remote_access(kernel):
     name = {k: n for n, k in _kernels_with_remote_memory()}[kernel]
     body = _body(_code(name), kernel)
