@@ -126,20 +126,22 @@ __device__ __forceinline__ void ss_frames(const FoldArgs& a, int k0, int k1, int
         float2 up[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) up[c] = odd ? exp_odd2(E1[c], E2[c]) : exp_even2(E0[c], E1[c], E2[c]);
-        if (EDGE && (y < 0 || y >= H)) {  // the reflected row's own neighbours
+        if (EDGE && (y < 0 || y >= H)) {
+            // the reflected row's own neighbours and parity: y's, except in a level one row high, all of whose rows are row 0
             const int cy = lsb_reflect(y, H) >> 1;
+            const bool from_odd = odd && H > 1;
             float t0[3], t1[3], t2[3];
             load_g1(k, sc, cy - 1, t0);
             load_g1(k, sc, cy, t1);
             load_g1(k, sc, cy + 1, t2);
             float2 D[3];
-            if (!odd) expand(t0, up);
+            if (!from_odd) expand(t0, up);
             expand(t1, D);
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 const float l = __shfl_up_sync(ALL, t2[c], 1), r = __shfl_down_sync(ALL, t2[c], 1);
                 const float2 F = make_float2(lsb_exp_even(l, t2[c], r), lsb_exp_odd(t2[c], r));
-                up[c] = odd ? exp_odd2(D[c], F) : exp_even2(up[c], D[c], F);
+                up[c] = from_odd ? exp_odd2(D[c], F) : exp_even2(up[c], D[c], F);
             }
         }
 #pragma unroll
