@@ -665,8 +665,11 @@ __global__ void out_grad_kernel(const float* __restrict__ dy0, __nv_bfloat16* __
 
 // dW[tap][co][ci] = sum over pixels of dZ[p][co] X[p + off(tap)][ci], and db[co] = sum of dZ, on the
 // 5th-generation tensor cores: a GEMM whose K is the pixels. A CTA owns CO couts x 32 cins and every
-// splits-th 16 x 8 pixel tile; the sums of all its tiles stay in TMEM (D: a lane per cout, a column per
-// (tap, cin)) and go out once, as vector reductions. Both operands are MN-major (the channel is
+// splits-th 16 x 8 pixel tile. A tile's sums are made in TMEM (D: a lane per cout, a column per (tap, cin)) and
+// added, tile by tile, to FP32 registers, rounded to nearest; a CTA's sums go out once, as vector reductions. (The
+// tensor core's own accumulator drops what lies below its last place at every step, so sums of positive products left in
+// it over all of a CTA's tiles fell short in proportion to their number: by 7.8e-6 on 8 crops of 256 x 256 and 2.4e-5
+// on 1024 x 1024; here by less than 5e-8, for 0.1 ms a step of those crops.) Both operands are MN-major (the channel is
 // contiguous in a pixel): A = dZ as [c8][pixel][8 channels], B = X's halo in three copies, one per kx,
 // as [kx][c8][18 rows][8 pixels][8 channels], so that one MMA takes the three kx of a ky (N = 96) and ky
 // is a start address one row further down. db is one more column block whose B is all ones.
@@ -676,7 +679,7 @@ __global__ void out_grad_kernel(const float* __restrict__ dy0, __nv_bfloat16* __
 // Couts below 128 leave lanes that hold products of whatever lies behind A's planes (in bounds; a
 // lane's sums never mix with another's); they are not read.
 // Measured over the 15 layers of a step of 8 crops of 256 x 256: 13.4 ms as register sums on the CUDA
-// cores, 0.79 ms here (0.17 TFLOP: 215 TFLOP/s).
+// cores, 0.90 ms here (0.17 TFLOP: 190 TFLOP/s), of which the reads of the TMEM 0.10.
 constexpr int DW_THREADS = 256;
 constexpr int DW_XROWS = TC_HP * TC_TW;                     // 144 pixels of one copy of X
 constexpr int DW_XPLANE = DW_XROWS * 16 + 32;               // bytes of 8 channels of one copy (+32: bank spread)
@@ -689,6 +692,7 @@ __host__ __device__ constexpr size_t dw_smem_bytes(int co) { return (size_t)2 * 
 static_assert(dw_stage(32) >= 16 * dw_zplane(32) && dw_stage(64) >= 16 * dw_zplane(64) && dw_stage(128) >= 16 * dw_zplane(128),
               "A's planes stay inside the stage");
 constexpr uint32_t DW_COLS = 512, DW_DB_COL = 288;
+constexpr int DW_BLOCKS = DW_DB_COL / 16 / 2;  // blocks of 16 columns a warp reads
 
 __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
     asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
@@ -702,7 +706,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv_dw_kernel(const ConvArgs a
     constexpr int XU = TC_PIX * 4, XQ = (XU + DW_THREADS - 1) / DW_THREADS;
     unsigned char* ones = dw_smem + 2 * STAGE;
     uint64_t* mbar = reinterpret_cast<uint64_t*>(ones + 512);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 2);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int c0 = blockIdx.y * UN_CH, co0 = blockIdx.z * CO, splits = gridDim.x;
     const int tiles_x = (a.W + TC_TW - 1) / TC_TW, tiles_y = (a.H + TC_TH - 1) / TC_TH, ntiles = tiles_x * tiles_y * a.B;
@@ -715,7 +719,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv_dw_kernel(const ConvArgs a
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        for (int q = 0; q < 2; q++) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mbar + q)), "r"(1));
+        mbar_init(smem_u32(mbar), 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     if (tid < 128) reinterpret_cast<uint32_t*>(ones)[tid] = 0x3F803F80u;  // bf16 ones, 16 columns x 16 pixels
@@ -744,14 +748,48 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv_dw_kernel(const ConvArgs a
             if (i < XU && yy >= 0 && yy < a.H && xx >= 0 && xx < a.W) xr[q] = load8(src, cs, mode, b, yy, xx, a.H, a.W, cb + 8 * v);
         }
     };
+    // a warp's sums: its lane quarter's couts, every other 16 of the 288 columns (the quarter's other warp has the rest)
+    const bool reads = 32 * (warp & 3) < CO;
+    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    float sum[DW_BLOCKS][16], dbs = 0.f;
+#pragma unroll
+    for (int h = 0; h < DW_BLOCKS; h++)
+#pragma unroll
+        for (int q = 0; q < 16; q++) sum[h][q] = 0.f;
+    // tile n's MMAs are done: its sums out of the TMEM, before the next tile's take their place
+    auto take = [&](int n) {
+        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(mbar), (uint32_t)(n & 1)))) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        if (reads) {
+#pragma unroll
+            for (int h = 0; h < DW_BLOCKS; h++) {
+                uint32_t r[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                      "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                    : "r"(tq + (uint32_t)((2 * h + (warp >> 2)) * 16)));
+                asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+                for (int q = 0; q < 16; q++) sum[h][q] += __uint_as_float(r[q]);
+            }
+            if (bias && warp < 4) {
+                uint32_t r;
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(tq + DW_DB_COL));
+                asm volatile("tcgen05.wait::ld.sync.aligned;");
+                dbs += __uint_as_float(r);
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        return true;
+    };
     bool ok = true;
     int it = 0;
     fetch(blockIdx.x);
     for (int tile = blockIdx.x; tile < ntiles; tile += splits, it++) {
+        // two stages in turn: the MMAs of two tiles ago, which read this one, were done before those of the last tile began
         unsigned char* Z = dw_smem + (it & 1) * STAGE;
         unsigned char* X = Z + ZV * ZP;
-        // the MMAs of two tiles ago have read this stage
-        if (it >= 2) ok = mbar_wait(smem_u32(mbar + (it & 1)), (uint32_t)(((it >> 1) - 1) & 1));
 #pragma unroll
         for (int q = 0; q < ZQ; q++) {
             const int i = tid + q * DW_THREADS, pix = i / ZV, v = i % ZV;
@@ -767,6 +805,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv_dw_kernel(const ConvArgs a
         }
         if (tile + splits < ntiles) fetch(tile + splits);  // in flight across the barrier and the MMAs
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (it > 0) ok = take(it - 1);
         if (!__syncthreads_and(ok)) {
             ok = false;
             break;
@@ -777,51 +816,30 @@ __global__ void __launch_bounds__(DW_THREADS, 1) conv_dw_kernel(const ConvArgs a
 #pragma unroll 1
             for (int j = 0; j < 8; j++) {  // 16 pixels (two tile rows) per K-step
                 const uint64_t da = umma_desc(zb + j * 256, 128, ZP);
-                const uint32_t acc = (it > 0 || j > 0) ? 1u : 0u;
+                const uint32_t acc = j > 0 ? 1u : 0u;
 #pragma unroll
                 for (int ky = 0; ky < 3; ky++) umma_bf16(tmem + ky * 96, da, umma_desc(xb + (2 * j + ky) * 128, 128, DW_XPLANE), IDESC, acc);
                 if (bias) umma_bf16(tmem + DW_DB_COL, da, umma_desc(smem_u32(ones), 128, 256), IDESC1, acc);
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar + (it & 1)))
-                         : "memory");
+            umma_commit(smem_u32(mbar));
         }
     }
-    // the last commit covers every MMA before it
-    if (ok) ok = mbar_wait(smem_u32(mbar + ((it - 1) & 1)), (uint32_t)(((it - 1) >> 1) & 1));
+    if (ok) ok = take(it - 1);
     ok = __syncthreads_and(ok) != 0;
     if (!ok) {
         // a wait ran out: flag it, give the MMAs in flight a second bounded wait, free the TMEM, return
         if (tid == 0) atomicOr(status, 0x200);
-        mbar_wait(smem_u32(mbar + ((it - 1) & 1)), (uint32_t)(((it - 1) >> 1) & 1));
-    } else {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const int m = 32 * (warp & 3) + lane;  // this lane's cout; the two warps of a lane quarter share the taps
-        if (32 * (warp & 3) < CO) {
-#pragma unroll 1
-            for (int t = warp >> 2; t < 9; t += 2)
+        mbar_wait(smem_u32(mbar), (uint32_t)((it - 1) & 1));
+    } else if (reads) {
+        const int m = 32 * (warp & 3) + lane;  // this lane's cout
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    uint32_t r[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                        : "r"(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(t * 32 + h * 16)));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;");
-                    float* o = dw + ((size_t)t * a.cout + co0 + m) * a.cin + c0 + h * 16;
+        for (int h = 0; h < DW_BLOCKS; h++) {
+            const int col = (2 * h + (warp >> 2)) * 16;
+            float* o = dw + ((size_t)(col / 32) * a.cout + co0 + m) * a.cin + c0 + col % 32;
 #pragma unroll
-                    for (int q = 0; q < 16; q += 4)
-                        red_add4(o + q, __uint_as_float(r[q]), __uint_as_float(r[q + 1]), __uint_as_float(r[q + 2]), __uint_as_float(r[q + 3]));
-                }
-            if (bias && warp < 4) {
-                uint32_t r;
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];"
-                             : "=r"(r)
-                             : "r"(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + DW_DB_COL));
-                asm volatile("tcgen05.wait::ld.sync.aligned;");
-                atomicAdd(&db[co0 + m], __uint_as_float(r));
-            }
+            for (int q = 0; q < 16; q += 4) red_add4(o + q, sum[h][q], sum[h][q + 1], sum[h][q + 2], sum[h][q + 3]);
         }
+        if (bias && warp < 4) atomicAdd(&db[co0 + m], dbs);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
