@@ -268,6 +268,9 @@ char* lsb_stack_run(lsb_stack* s, double* ms_out12);
 void lsb_stack_destroy(lsb_stack* s);
 void lsb_result_free(lsb_result* r);
 
+/* The engine keeps the device workspaces of lsb_depth_from_slices, lsb_wls_solve and lsb_align_pair for its next call of
+   the same kind and size: at most 8 of them and 4 GB. They are given back when any allocation of this library on the
+   engine's device finds no room beside them, and by lsb_engine_destroy. */
 /* gpu.rs:1327 depth_from_slices: slices [n][dh][dw] f32, fused [3][h][w] f32 (host pointers).
    On an error *out is left empty. */
 char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint32_t n, const float* fused, uint32_t w, uint32_t h,

@@ -25,6 +25,7 @@
 
 #include "lapstack_b200.h"
 #include "lsb_align.h"
+#include "lsb_common.cuh"
 #include "lsb_depth.h"
 #include "lsb_internal.h"
 #include "lsb_prep.h"
@@ -62,7 +63,7 @@ struct DevPool {
     template <class T>
     cudaError_t get(T** p, size_t n) {
         void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
+        cudaError_t e = lsb_dev_alloc(&q, std::max<size_t>(n, 1) * sizeof(T));
         if (e == cudaSuccess) ptrs.push_back(q), bytes += std::max<size_t>(n, 1) * sizeof(T);
         *p = (T*)q;
         return e;
@@ -119,7 +120,7 @@ struct HostStage {
 // for the next call of the same kind and size: allocating and freeing it (and the solver's captured graphs) cost
 // 25 to 40 ms a call, the solve of a 3 Mpx grid 6. A call takes its entry out of the list while it runs, so that no two
 // calls share one; the engine keeps at most SOLO_MAX entries and SOLO_BYTES, newest first, and frees all of them when
-// an allocation fails and when it is destroyed.
+// any allocation of the library on its device finds no room (lsb_dev_alloc) and when it is destroyed.
 struct Solo {
     int kind = 0;
     uint32_t key[4] = {};
@@ -284,13 +285,33 @@ Solo::~Solo() {
 }
 size_t Solo::bytes() const { return pool.bytes + wls_bytes(ws) + (st ? st->pool.bytes + wls_bytes(st->ws) : 0); }
 
-static void solo_flush(lsb_engine* e) {
+// Frees an engine's idle workspaces; whether there were any.
+static bool solo_flush(lsb_engine* e) {
     std::list<Solo*> all;
     {
         std::lock_guard<std::mutex> lk(e->solo_mu);
         all.swap(e->solos);
     }
     for (Solo* s : all) delete s;
+    return !all.empty();
+}
+// The engines there are, from the end of their creation to the start of their destruction.
+static std::mutex g_engines_mu;
+static std::vector<lsb_engine*> g_engines;
+cudaError_t lsb_dev_alloc(void** p, size_t bytes) {
+    *p = nullptr;
+    cudaError_t r = cudaMalloc(p, bytes);
+    int dev = 0;
+    if (r != cudaErrorMemoryAllocation || cudaGetDevice(&dev) != cudaSuccess) return r;
+    bool freed = false;
+    {
+        std::lock_guard<std::mutex> lk(g_engines_mu);
+        for (lsb_engine* e : g_engines)
+            if (e->device == dev && solo_flush(e)) freed = true;
+    }
+    if (!freed) return r;
+    cudaGetLastError();
+    return cudaMalloc(p, bytes);
 }
 // The workspace of one call, out of the engine's list (or a new one: fresh) and back into it when the call is done.
 struct SoloHold {
@@ -335,15 +356,6 @@ struct SoloHold {
         for (Solo* q : out) delete q;
     }
 };
-// f(), and once more without the idle workspaces if the device has no room for it beside them.
-template <class F>
-static cudaError_t with_room(lsb_engine* e, F f) {
-    cudaError_t r = f();
-    if (r != cudaErrorMemoryAllocation) return r;
-    cudaGetLastError();
-    solo_flush(e);
-    return f();
-}
 
 static bool pageable(const void* p) {
     cudaPointerAttributes a;
@@ -425,7 +437,7 @@ static cudaError_t warm_start(lsb_stack* s, int dw, int dh, int n, cudaStream_t 
         if (s->x0) cudaFree(s->x0);
         s->x0 = nullptr;
         s->x0_cells = 0;
-        cudaError_t e = cudaMalloc(&s->x0, m * sizeof(float));
+        cudaError_t e = lsb_dev_alloc(&s->x0, m * sizeof(float));
         if (e != cudaSuccess) return e;
         s->x0_cells = m;
     }
@@ -515,12 +527,18 @@ char* lsb_engine_create(const lsb_config* cfg, lsb_engine** out) {
         lsb_engine_destroy(e);
         return err;
     }
+    std::lock_guard<std::mutex> lk(g_engines_mu);
+    g_engines.push_back(e);
     *out = e;
     return nullptr;
 }
 
 void lsb_engine_destroy(lsb_engine* e) {
     if (!e) return;
+    {
+        std::lock_guard<std::mutex> lk(g_engines_mu);
+        g_engines.erase(std::remove(g_engines.begin(), g_engines.end(), e), g_engines.end());
+    }
     if (e->s) cudaStreamSynchronize(e->s);
     for (auto& v : e->ev)
         if (v) cudaEventDestroy(v);
@@ -579,7 +597,7 @@ static char* stack_alloc(lsb_stack* s, bool depth_only) {
     s->best.assign(s->levels, nullptr);
     for (int l = 1; l <= s->levels; l++) {
         void* p = nullptr;
-        TRY(cudaMalloc(&p, N * 3 * (size_t)s->lw[l] * s->lh[l] * gs_bytes(s) + 64));
+        TRY(lsb_dev_alloc(&p, N * 3 * (size_t)s->lw[l] * s->lh[l] * gs_bytes(s) + 64));
         P.ptrs.push_back(p);
         s->g[l] = p;
     }
@@ -622,7 +640,7 @@ static char* stack_alloc(lsb_stack* s, bool depth_only) {
     if (s->ap.enabled && N > 1) {
         {
             void* p = nullptr;
-            TRY(cudaMalloc(&p, N * W * H * (s->storage == STORE_F32 ? 3 * sizeof(float) : 3 * sizeof(uint16_t)) + 64));
+            TRY(lsb_dev_alloc(&p, N * W * H * (s->storage == STORE_F32 ? 3 * sizeof(float) : 3 * sizeof(uint16_t)) + 64));
             P.ptrs.push_back(p);
             s->warped = p;
         }
@@ -781,16 +799,6 @@ extern "C" char* lsb_stack_begin(lsb_engine* e, uint32_t w, uint32_t h, uint32_t
                                  lsb_stack** out) {
     *out = nullptr;
     if (!e) return dup_err("no engine");
-    char* err = stack_make(e, w, h, n_frames, fuse, align, depth, brightness, crop, e->cfg.storage, false, out);
-    if (!err || cudaGetLastError() != cudaErrorMemoryAllocation) return err;
-    bool idle;
-    {
-        std::lock_guard<std::mutex> lk(e->solo_mu);
-        idle = !e->solos.empty();
-    }
-    if (!idle) return err;
-    lsb_free_str(err);  // again without the idle workspaces of standalone calls
-    solo_flush(e);
     return stack_make(e, w, h, n_frames, fuse, align, depth, brightness, crop, e->cfg.storage, false, out);
 }
 
@@ -870,7 +878,7 @@ static cudaError_t grow_u16(uint16_t** buf, size_t* have, size_t px, cudaStream_
     if (*buf) cudaFree(*buf);
     *buf = nullptr;
     *have = 0;
-    e = cudaMalloc(buf, sizeof(uint16_t) * 3 * px);
+    e = lsb_dev_alloc(buf, sizeof(uint16_t) * 3 * px);
     if (e == cudaSuccess) *have = px;
     return e;
 }
@@ -959,9 +967,9 @@ extern "C" char* lsb_prep_frame_u16(lsb_engine* e, const lsb_frame_prep* p, cons
     }
     cudaStream_t cs = e->cs;
     uint16_t *raw = nullptr, *mid = nullptr, *res = nullptr;
-    cudaError_t ce = cudaMalloc(&raw, sizeof(uint16_t) * 3 * (size_t)w * h);
-    if (ce == cudaSuccess) ce = cudaMalloc(&mid, sizeof(uint16_t) * 3 * (size_t)pw * ph);
-    if (ce == cudaSuccess) ce = cudaMalloc(&res, sizeof(uint16_t) * 3 * (size_t)ow * oh);
+    cudaError_t ce = lsb_dev_alloc(&raw, sizeof(uint16_t) * 3 * (size_t)w * h);
+    if (ce == cudaSuccess) ce = lsb_dev_alloc(&mid, sizeof(uint16_t) * 3 * (size_t)pw * ph);
+    if (ce == cudaSuccess) ce = lsb_dev_alloc(&res, sizeof(uint16_t) * 3 * (size_t)ow * oh);
     const size_t bi = sizeof(uint16_t) * 3 * (size_t)w * h, bo = sizeof(uint16_t) * 3 * (size_t)ow * oh;
     if (ce == cudaSuccess) ce = is_device_ptr(in) ? cudaMemcpyAsync(raw, in, bi, cudaMemcpyDeviceToDevice, cs) : host_in(e, raw, in, bi, cs);
     if (ce == cudaSuccess && d && (int)w == d->W && (int)h == d->H) ce = dust_apply_rgb16(d, raw, cs);
@@ -988,7 +996,7 @@ extern "C" char* lsb_stack_push_f32(lsb_stack* s, const float* const planes[3]) 
     if (!s->frames_f32) {
         if (s->count > 0) return dup_err("this stack takes u16 frames");
         void* p = nullptr;
-        TRY(cudaMalloc(&p, sizeof(float) * 3 * (size_t)s->n * s->w * s->h));
+        TRY(lsb_dev_alloc(&p, sizeof(float) * 3 * (size_t)s->n * s->w * s->h));
         s->pool.ptrs.push_back(p);
         s->frames_f32 = (float*)p;
         s->f32src = true;
@@ -1897,13 +1905,7 @@ extern "C" char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint3
     if (const char* bad = params_error(&fp, nullptr, &dp)) return dup_err(bad);
     SoloHold hold(e, SOLO_DEPTH, w, h, n, dp.scale);
     if (hold.fresh) {
-        char* err = stack_make(e, w, h, n, &fp, nullptr, &dp, 0, 0, STORE_F32, true, &hold.s->st);
-        if (err && cudaGetLastError() == cudaErrorMemoryAllocation) {
-            lsb_free_str(err);
-            solo_flush(e);
-            err = stack_make(e, w, h, n, &fp, nullptr, &dp, 0, 0, STORE_F32, true, &hold.s->st);
-        }
-        if (err) return err;
+        if (char* err = stack_make(e, w, h, n, &fp, nullptr, &dp, 0, 0, STORE_F32, true, &hold.s->st)) return err;
     }
     lsb_stack* s = hold.s->st;
     s->dp = dp;
@@ -1941,8 +1943,7 @@ extern "C" char* lsb_depth_from_slices(lsb_engine* e, const float* slices, uint3
     double rel64 = 0.0;
     if (dp.lambda > 0.f) {
         cudaError_t ce;
-        WlsSolver* ws = nullptr;
-        with_room(e, [&] { return ws = stack_solver(s, dw, dh, dp, st, &ce), ce; });
+        WlsSolver* ws = stack_solver(s, dw, dh, dp, st, &ce);
         if (ce == cudaSuccess) ce = wls_set_weights(ws, s->conf, (int)s->dp.vcycle_mode, st);
         if (ce == cudaSuccess) ce = wls_solve(ws, s->dmed, (int)dp.cg_iters, s->u, &rel, &it, st, (int)dp.vcycle_mode, false, &rel64);
         it1 = it;
@@ -2000,13 +2001,10 @@ extern "C" char* lsb_wls_solve(lsb_engine* e, const float* d, const float* conf,
     Solo& S = *hold.s;
     if (hold.fresh) {
         S.planes.assign(4, nullptr);
-        for (float*& q : S.planes) TRY(with_room(e, [&] { return S.pool.get(&q, m); }));
-        TRY(with_room(e, [&] {  // planes first: the timed part is the solve
-            cudaError_t ce;
-            wls_destroy(S.ws);
-            S.ws = wls_alloc((int)w, (int)h, &ce);
-            return ce;
-        }));
+        for (float*& q : S.planes) TRY(S.pool.get(&q, m));
+        cudaError_t ce;
+        S.ws = wls_alloc((int)w, (int)h, &ce);
+        TRY(ce);
     }
     float *dd = S.planes[0], *cc = S.planes[1], *gg = S.planes[2], *uu = S.planes[3];
     TRY(host_in(e, dd, d, sizeof(float) * m, st));
@@ -2043,7 +2041,7 @@ extern "C" char* lsb_align_pair(lsb_engine* e, const float* rf, const float* tg,
         S.planes.assign(2 + 2 * dims.size(), nullptr);
         for (size_t q = 0; q < S.planes.size(); q++) {
             const size_t cells = q < 2 ? (size_t)w * h : (size_t)dims[q / 2 - 1].first * dims[q / 2 - 1].second;
-            TRY(with_room(e, [&] { return S.pool.get(&S.planes[q], cells); }));
+            TRY(S.pool.get(&S.planes[q], cells));
         }
     }
     float *a = S.planes[0], *b = S.planes[1];
@@ -2093,7 +2091,7 @@ extern "C" char* lsb_stack_weighted_average(lsb_stack* s, const lsb_wav_params* 
         if (s->wav_w) cudaFree(s->wav_w);
         s->wav_w = nullptr;
         s->wav_frames = 0;
-        TRY(cudaMalloc(&s->wav_w, sizeof(float) * m * n));
+        TRY(lsb_dev_alloc(&s->wav_w, sizeof(float) * m * n));
         s->wav_frames = n;
     }
     // the guided filter's statistics for radius `smooth` on the depth pass's guide (the fused luma's block mean)
@@ -2237,7 +2235,7 @@ extern "C" char* lsb_stack_fuse_range(lsb_stack* s, uint32_t lo, uint32_t hi, co
         if (s->slab_out) cudaFree(s->slab_out);
         s->slab_out = nullptr;
         s->slab_out_floats = 0;
-        TRY(cudaMalloc(&s->slab_out, sizeof(float) * of));
+        TRY(lsb_dev_alloc(&s->slab_out, sizeof(float) * of));
         s->slab_out_floats = of;
     }
     TRY(resize_planes(s->slab_img, s->w, (size_t)s->w * s->h, 3, (int)r[0], (int)r[1], (int)r[2], (int)r[3], (int)ow, (int)oh, (int)interp,
@@ -2260,8 +2258,8 @@ extern "C" char* lsb_resize(lsb_engine* e, const float* src, uint32_t planes, ui
     if (const char* why = size_error(w, h)) return dup_err(fmt("resize output: %s", why));
     const size_t ni = (size_t)planes * pw * ph, no = (size_t)planes * w * h;
     float *di = nullptr, *dout = nullptr;
-    cudaError_t ce = cudaMalloc(&di, sizeof(float) * ni);
-    if (ce == cudaSuccess) ce = cudaMalloc(&dout, sizeof(float) * no);
+    cudaError_t ce = lsb_dev_alloc(&di, sizeof(float) * ni);
+    if (ce == cudaSuccess) ce = lsb_dev_alloc(&dout, sizeof(float) * no);
     if (ce == cudaSuccess) ce = host_in(e, di, src, sizeof(float) * ni, e->s);
     if (ce == cudaSuccess) ce = resize_planes(di, pw, (size_t)pw * ph, (int)planes, 0, 0, (int)pw, (int)ph, (int)w, (int)h, (int)interp, dout, e->s);
     if (ce == cudaSuccess) ce = host_out(e, out, dout, sizeof(float) * no, e->s);

@@ -16,6 +16,16 @@ void lsb_launched();
 // Graph replays count the kernels they hold; a capture takes back the counts its launches added.
 void lsb_launched_add(long long k);
 uint64_t lsb_launched_now();
+// Every device allocation of the library: cudaMalloc, and once more without the engines' idle workspaces if the device
+// has no room beside them (lsb_api.cu).
+cudaError_t lsb_dev_alloc(void** p, size_t bytes);
+template <class T>
+cudaError_t lsb_dev_alloc(T** p, size_t bytes) {
+    void* q = nullptr;
+    const cudaError_t e = lsb_dev_alloc(&q, bytes);
+    *p = (T*)q;
+    return e;
+}
 
 // Reflect-101 into [0, n) (pyramid.rs:51 `reflect`): period 2(n-1); n == 1 maps to 0.
 LSB_HD int lsb_reflect(int i, int n) {

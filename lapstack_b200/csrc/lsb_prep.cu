@@ -268,7 +268,7 @@ static bool masks_meet(const lsb_dust_spot& a, const lsb_dust_spot& b) {
 
 template <class T>
 static cudaError_t upload(T** dst, const std::vector<T>& v) {
-    cudaError_t e = cudaMalloc(dst, sizeof(T) * std::max<size_t>(v.size(), 1));
+    cudaError_t e = lsb_dev_alloc(dst, sizeof(T) * std::max<size_t>(v.size(), 1));
     if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
     return e;
 }
@@ -347,13 +347,13 @@ std::string dust_create(const lsb_dust_map* m, DustDev** out) {
         d->layer_off.push_back((int)list.size());
     }
     d->scratch_bytes = (size_t)soff * sizeof(float);
-    cudaError_t e = cudaMalloc(&d->spots, sizeof(DSpot) * std::max(n, 1));
+    cudaError_t e = lsb_dev_alloc(&d->spots, sizeof(DSpot) * std::max(n, 1));
     if (e == cudaSuccess && n) e = cudaMemcpy(d->spots, tab.data(), sizeof(DSpot) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = upload(&d->masks, masks);
     if (e == cudaSuccess) e = upload(&d->wzero, wzero);
     if (e == cudaSuccess) e = upload(&d->gains, gains);
     if (e == cudaSuccess) e = upload(&d->list, list);
-    if (e == cudaSuccess) e = cudaMalloc(&d->scratch, std::max<size_t>(d->scratch_bytes, 4));
+    if (e == cudaSuccess) e = lsb_dev_alloc(&d->scratch, std::max<size_t>(d->scratch_bytes, 4));
     if (e != cudaSuccess) {
         delete d;
         return std::string("dust map upload: ") + cudaGetErrorString(e);

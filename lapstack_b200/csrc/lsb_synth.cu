@@ -257,9 +257,9 @@ const char* lsb_synth_stack_device(const lsb_synth_desc* d, uint16_t* out_dev, d
     float *z = nullptr, *t = nullptr, *B = nullptr;
     unsigned* mm = nullptr;
     const char* err = nullptr;
-    if (cudaMalloc(&dp, sizeof(SynthPlan)) != cudaSuccess || cudaMalloc(&z, n * 4) != cudaSuccess ||
-        cudaMalloc(&t, 3 * n * 4) != cudaSuccess || cudaMalloc(&B, (size_t)hp->nb * 3 * n * 4) != cudaSuccess ||
-        cudaMalloc(&mm, 8) != cudaSuccess) {
+    if (lsb_dev_alloc(&dp, sizeof(SynthPlan)) != cudaSuccess || lsb_dev_alloc(&z, n * 4) != cudaSuccess ||
+        lsb_dev_alloc(&t, 3 * n * 4) != cudaSuccess || lsb_dev_alloc(&B, (size_t)hp->nb * 3 * n * 4) != cudaSuccess ||
+        lsb_dev_alloc(&mm, 8) != cudaSuccess) {
         err = "synth: device allocation failed";
     } else {
         cudaMemcpyAsync(dp, hp, sizeof(SynthPlan), cudaMemcpyHostToDevice, s);

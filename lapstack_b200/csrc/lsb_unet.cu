@@ -1033,7 +1033,7 @@ static cudaError_t ensure_shape(lsb_unet* u, int B, int H, int W, bool train) {
     if (u->B == B && u->H == H && u->W == W && (!train || !u->dx.empty())) return cudaSuccess;
     free_shape(u);
     auto get = [&](size_t bytes, void** p) {
-        cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+        cudaError_t e = lsb_dev_alloc(p, std::max<size_t>(bytes, 16));
         if (e == cudaSuccess) u->shape_allocs.push_back(*p);
         return e;
     };
@@ -1216,7 +1216,7 @@ extern "C" char* lsb_unet_create(int32_t device, uint64_t seed, lsb_unet** out) 
         for (int co = 0; co < l.cout; co++) bm[l.boff + co] = li + 1 != u->layers.size() || co == 0;
     }
     auto alloc = [&](void** p, size_t bytes) -> bool {
-        if (cudaMalloc(p, bytes) != cudaSuccess) return false;
+        if (lsb_dev_alloc(p, bytes) != cudaSuccess) return false;
         return cudaMemset(*p, 0, bytes) == cudaSuccess;
     };
     bool ok = alloc((void**)&u->w, u->nw * 4) && alloc((void**)&u->gw, u->nw * 4) && alloc((void**)&u->mw, u->nw * 4) &&

@@ -1348,7 +1348,7 @@ WlsSolver* wls_alloc(int w, int h, cudaError_t* err) {
         put(&S->ctl, 4);
         if (pass == 0) {
             S->bytes = at;
-            *err = cudaMalloc(&S->slab, at);
+            *err = lsb_dev_alloc(&S->slab, at);
             if (*err != cudaSuccess) return S;
         }
     }
