@@ -1592,8 +1592,9 @@ static char* run_pipeline_once(lsb_stack* s) {
                 r1 = robust_weights(s->conf, s->dmed, s->u, s->dp.robust, s->w2, m, st);
                 if (r1 == cudaSuccess) r1 = wls_set_weights(ws, s->w2, (int)s->dp.vcycle_mode, st);
                 // with a given start the reweighted solve goes on from the first one's solution (in u), which is nearer
-                // than the prediction (a 2048 x 1536 stack: 0 iterations to the same residual against 7); the plain
-                // solve starts from its sweeps again, as the reference does
+                // than the prediction (a 2048 x 1536 stack whose weights the robust threshold leaves as they are: 0
+                // iterations against 7, 1.73 -> 1.20 ms for both solves), to the same residual of the reweighted
+                // system; the plain solve starts from its sweeps again, as the reference does
                 if (r1 == cudaSuccess) r1 = wls_solve(ws, s->dmed, (int)s->dp.cg_iters, s->u, &rel, &it, st, (int)s->dp.vcycle_mode, given, &s->rel64);
             }
             if (r1 != cudaSuccess) return dup_err(fmt("wls: %s", cudaGetErrorString(r1)));
