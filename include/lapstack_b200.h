@@ -62,8 +62,8 @@ typedef struct {
     int32_t device;        /* CUDA device ordinal */
     int32_t storage;       /* Gaussian levels >= 1 and focus slices: 0 FP32 (bit-exact with the reference
                               FP32 path); 1 16-bit: UNORM16 levels, FP16 slices; 2 FP16 levels and slices */
-    int32_t grid_limit;    /* CTAs of the persistent kernels and of the device registration search;
-                              0 = 2 x the SM count */
+    int32_t grid_limit;    /* CTAs of the persistent kernels, of the fold's selection and of the device
+                              registration search; 0 = 2 x the SM count (the selection: no limit) */
     int32_t flags;         /* LSB_FLAG_* bits; 0 for the defaults */
     lsb_log_fn log;        /* optional progress lines (stack.rs:1014 `log`) */
     void* user;
@@ -340,7 +340,7 @@ char* lsb_unet_forward_ms(lsb_unet* u, float* ms);
 char* lsb_unet_train_step(lsb_unet* u, const void* in_dev, const float* d_in_dev, const float* target_dev, uint32_t B, uint32_t H,
                           uint32_t W, float lr, double* loss_out);
 /* The autotuner (no counterpart in the reference): the persistent kernels' grid
- * sizes (the fold's select kernel, the depth aggregation) timed on this stack's
+ * sizes (the fold's fused level-0 kernel, the depth aggregation) timed on this stack's
  * frames (two full runs per candidate), the fastest kept by the engine for every
  * later run. The grid size changes no result. */
 typedef struct {

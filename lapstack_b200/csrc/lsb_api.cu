@@ -1121,6 +1121,7 @@ static FoldArgs level_args(const lsb_stack* s, int l, bool warped, bool depth_on
     a.H = s->lh[l];
     a.W1 = s->lw[l + 1];
     a.H1 = s->lh[l + 1];
+    a.cta_limit = std::max(0, s->e->cfg.grid_limit);
     a.src_u16 = warped && s->storage != STORE_F32 ? (const uint16_t*)s->warped : s->frames;
     a.src_f32 = warped && s->storage == STORE_F32 ? (const float*)s->warped : s->frames_f32;
     a.xf = s->xf_dev;
@@ -2341,8 +2342,8 @@ extern "C" char* lsb_batch_run(lsb_stack* const* stacks, uint32_t n_stacks, lsb_
     return nullptr;
 }
 
-// The project's autotuner: the persistent kernels' grid sizes (the fold's select
-// kernel and the depth aggregation; CTAs walk tiles, so any grid gives the same
+// The project's autotuner: the persistent kernels' grid sizes (the fold's fused
+// level-0 kernel and the depth aggregation; CTAs walk tiles, so any grid gives the same
 // results) timed on this stack's own frames, one full run per candidate, the
 // fastest kept in the engine for every later run.
 extern "C" char* lsb_stack_autotune(lsb_stack* s, lsb_tuning* out) {

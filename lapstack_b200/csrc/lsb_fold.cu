@@ -100,10 +100,9 @@ static void fold0_border_rects(int W, int H, const Fold0Range& rg, SelBatch& T) 
 // take a share of the frames each of one tile (not with halo control, which adds the frames up in order).
 template <int SRC, class GS, int R>
 static cudaError_t launch_select(SelBatch& T, cudaStream_t s) {
-    auto k = select_strip_kernel<SRC, GS, R>;
     auto tiles = [](const SelBatch::Rect& r) { return (long)((r.x1 - r.x0 + SS_W - 1) / SS_W) * ((r.y1 - r.y0 + SS_H - 1) / SS_H); };
     constexpr long WANT = 148 * SS_CTAS * SS_WARPS;
-    int ctas = 0;
+    int ctas = 0, limit = 0;
     bool beside = false;
     for (int i = 0; i < T.n; i++) {
         auto& r = T.r[i];
@@ -122,11 +121,15 @@ static cudaError_t launch_select(SelBatch& T, cudaStream_t s) {
         r.cta0 = ctas;
         ctas += r.ntx * ((r.y1 - r.y0 + per - 1) / per);
         beside = beside || a.beside;
+        limit = a.cta_limit;
     }
+    T.ctas = ctas;
     const size_t smem = beside ? std::max(SS_SMEM, BESIDE_SMEM) : SS_SMEM;  // one CTA per SM beside the registration chain
+    const bool turns = limit > 0 && limit < ctas;
+    auto k = turns ? select_strip_kernel<SRC, GS, R, true> : select_strip_kernel<SRC, GS, R, false>;
     cudaError_t e = with_smem(k, smem);
     if (e != cudaSuccess) return e;
-    lsb_launched(), k<<<ctas, SS_WARPS * 32, smem, s>>>(T);
+    lsb_launched(), k<<<turns ? limit : ctas, SS_WARPS * 32, smem, s>>>(T);
     return cudaGetLastError();
 }
 template <class GS>

@@ -63,6 +63,7 @@ struct FoldArgs {
     // level 0 only: fused0 set, the interior tiles (fold0_range(W, H, f0r)) are the fused kernel's, and
     // the two other kernels take the border's (fold0_border_tile, fold0_border_rects)
     int fused0, f0r;
+    int cta_limit;  // CTAs of the selection at most (lsb_config.grid_limit), 0: as many as there is work for
     int no_fused;  // 1: level 0 runs the two kernels on every tile (the fused kernel's cross-check)
     // 1: the level runs beside the registration chain: its persistent kernels take at most one CTA per
     // SM (they ask for BESIDE_SMEM of shared memory), so the chain's cooperative search keeps room

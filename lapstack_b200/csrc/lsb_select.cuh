@@ -23,7 +23,7 @@ constexpr int SS_W = 56, SS_H = 8, SS_WARPS = 6, SS_CTAS = 3;
 // What a launch selects: rectangles of tiles of one or more levels, one after another in the grid.
 constexpr int SS_MAX = 16;
 struct SelBatch {
-    int n;
+    int n, ctas;  // rectangles; CTAs of work, which the launched ones take in turn
     struct Rect {
         int lv;                        // its level's arguments
         int x0, y0, x1, y1, ntx, cta0;  // cta0: the first CTA's index
@@ -269,16 +269,16 @@ __device__ __forceinline__ void ss_frames(const FoldArgs& a, int k0, int k1, int
 constexpr int SS_STATE = SS_H * 9;  // words of a lane's state
 constexpr size_t SS_SMEM = sizeof(float) * SS_WARPS * SS_STATE * 32;
 
+// One CTA's tiles.
 template <int SRC, class GS, int R>
-__global__ void __launch_bounds__(SS_WARPS * 32, SS_CTAS) select_strip_kernel(const __grid_constant__ SelBatch T) {
-    extern __shared__ float sm[];
+__device__ __forceinline__ void select_cta(const SelBatch& T, int cta, float* sm) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int ri = 0;
-    while (ri + 1 < T.n && (int)blockIdx.x >= T.r[ri + 1].cta0) ri++;
+    while (ri + 1 < T.n && cta >= T.r[ri + 1].cta0) ri++;
     const SelBatch::Rect& rc = T.r[ri];
     const FoldArgs& a = T.a[rc.lv];
     const int G = rc.groups, per = SS_WARPS / G, g = wid % G, sub = wid / G;  // a CTA: `per` tiles one above the other
-    const int ci = (int)blockIdx.x - rc.cta0, by = ci / rc.ntx, bx = ci - by * rc.ntx;
+    const int ci = cta - rc.cta0, by = ci / rc.ntx, bx = ci - by * rc.ntx;
     const int x0 = rc.x0 + bx * SS_W, y0 = rc.y0 + (by * per + sub) * SS_H;
     const int W = a.W, H = a.H;
     const size_t np = (size_t)W * H;
@@ -335,5 +335,19 @@ __global__ void __launch_bounds__(SS_WARPS * 32, SS_CTAS) select_strip_kernel(co
             for (int c = 0; c < 3; c++) a.acc[c * np + o + l] = p[(2 * c + l) * 32];
             if (a.winner) a.winner[o + l] = ((const uint16_t*)(p + 8 * 32))[l];
         }
+    }
+}
+
+// TURNS: a launch bounded to fewer CTAs than there is work for, which they take in turn. A kernel of its own, because
+// with the loop around them the strips keep more in registers and spill their window for it (R = 2: 460 to 850 bytes
+// a thread instead of 210 to 310).
+template <int SRC, class GS, int R, bool TURNS>
+__global__ void __launch_bounds__(SS_WARPS * 32, SS_CTAS) select_strip_kernel(const __grid_constant__ SelBatch T) {
+    extern __shared__ float sm[];
+    if (!TURNS) return select_cta<SRC, GS, R>(T, blockIdx.x, sm);
+#pragma unroll 1
+    for (int cta = blockIdx.x; cta < T.ctas; cta += gridDim.x) {
+        select_cta<SRC, GS, R>(T, cta, sm);
+        __syncthreads();  // the groups' states are merged
     }
 }
