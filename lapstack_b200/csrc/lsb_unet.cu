@@ -530,6 +530,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) conv3x3_tc_kernel(const ConvArg
             const size_t pix = ((size_t)at.b * a.H + y) * a.W + x;
 #pragma unroll 1
             for (int c = 0; c < N; c += 32) {
+                __syncwarp();  // lanes outside the image skip the stores below; the read is the whole warp's
                 uint32_t r[32];
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
