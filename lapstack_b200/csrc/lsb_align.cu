@@ -1593,11 +1593,11 @@ static cudaError_t nm_cluster_launch(AlignCtx& C, NmJob& J, int limit) {
 static cudaError_t nm_launch(AlignCtx& C, NmJob& J) {
     cudaError_t e = cudaMemsetAsync(C.nm_ctl + 2, 0, sizeof(int) * 2, C.s);  // the barrier; the error word stays sticky
     if (e != cudaSuccess) return e;
-    // the small levels first, in one cluster (not with the spin limit overridden: that is for the grid-wide hand-off's
-    // wait, which a cluster barrier does not have)
+    // the small levels first, in one cluster (with the spin limit overridden the finest is left to the grid-wide kernel:
+    // the limit is for its hand-off's wait, which a cluster barrier does not have)
     J.nlv_cluster = 0;
-    if (!getenv("LSB_NM_SPIN_LIMIT"))
-        while (J.nlv_cluster < J.nlv && (unsigned)J.lv[J.nlv_cluster].w * J.lv[J.nlv_cluster].h <= NM_CLUSTER_PX) J.nlv_cluster++;
+    const int most = getenv("LSB_NM_SPIN_LIMIT") ? J.nlv - 1 : J.nlv;
+    while (J.nlv_cluster < most && (unsigned)J.lv[J.nlv_cluster].w * J.lv[J.nlv_cluster].h <= NM_CLUSTER_PX) J.nlv_cluster++;
     if (J.nlv_cluster > 0) {
         switch (J.nfree) {
             case 1: e = nm_cluster_launch<1>(C, J, C.max_blocks); break;
