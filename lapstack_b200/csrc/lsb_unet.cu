@@ -1165,9 +1165,8 @@ static cudaError_t unet_forward(lsb_unet* u) {
     for (int i = 0; i < N_LAYERS; i++) {
         ConvArgs a = layer_args(u, i);
         const bool last = i == N_LAYERS - 1;
-        a.out = last ? nullptr : u->act[i + 1];
+        a.out = u->act[i + 1];
         a.out_c0 = last ? u->out0 : nullptr;
-        if (last) a.out = u->act[i + 1];
         cudaError_t e = conv_launch(a, u->s, u->status, u->tc);
         if (e != cudaSuccess) return e;
     }

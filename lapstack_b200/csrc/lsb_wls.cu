@@ -1448,7 +1448,7 @@ static void vcycle(WlsSolver* S, size_t l, const float* bin, float* xout, cudaSt
 }
 
 // A damped Jacobi sweep on level L (zero: the zero-start one) against its BF16 right-hand side:
-// the coarsest level's sweeps when it does not fit one CTA's shared memory.
+// the coarsest level's sweeps when its bands do not fit the shared memory of coarse_h_kernel's cluster.
 static void jacobi_h(WlsLevel& L, bool zero, cudaStream_t s) {
     if (zero) {
         lsb_launched(), jac0_h_kernel<uint16_t><<<g1((size_t)L.w * L.h), 256, 0, s>>>(L.hb, L.hdinv, L.hx, (size_t)L.w * L.h);
