@@ -1311,9 +1311,9 @@ __device__ __forceinline__ bool nm_split(double v, int& i, double& frac) {
 // What bounds it: instructions issued (about half of the SM's slots over the whole kernel, 8 % of the f64 unit), f64 and
 // conversions the dearest. The affine source point is (m1 y + m2) + m0 x in that order (align.rs:485), so the row's
 // part comes from a table the warp makes per strip and the column's is the thread's own for the strip: 2 f64 additions
-// a sample instead of 8 operations, and 11 f64 operations and 3 conversions in all instead of 17 and 7. It takes all 128
-// registers: nm_search_kernel, whose two CTAs an SM leave room for the frames' warps and the fold beside them, keeps the
-// plain loop (with this one 8256 x 5504 x 10 is 80.2 -> 83.2 ms). rt: the warp's table, [rows][3 candidates x 2 axes].
+// a sample instead of 8 operations, and 11 f64 operations and 3 conversions in all instead of 17 and 7. nm_search_kernel,
+// on the larger levels and with the frames' warps on the SMs beside it, keeps the plain loop (with this one
+// 8256 x 5504 x 10 was 83.2 ms instead of 80.2). rt: the warp's table, [rows][3 candidates x 2 axes].
 __device__ __forceinline__ void nm_eval(const NmLevel& lv, const double (*cand)[9], int k0, int kn, const NmStrips& S, int gw, int warps,
                                         double (*rt)[6], double (&sd)[3], double (&sd2)[3], int (&cnt)[3]) {
     const int lane = threadIdx.x & 31;

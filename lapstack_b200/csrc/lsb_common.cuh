@@ -132,4 +132,4 @@ __device__ __forceinline__ float bil(const float* g, int dw, int x0, int x1, int
     return __fadd_rn(top, __fmul_rn(__fsub_rn(bot, top), ty));
 }
 // Error flag bits a kernel may raise in the engine's device status word.
-enum { LSB_ERR_BOUNDS = 1, LSB_ERR_TIMEOUT = 2 };
+enum { LSB_ERR_TIMEOUT = 2 };

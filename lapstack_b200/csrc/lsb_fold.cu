@@ -1,5 +1,5 @@
 // The fold: Burt-Adelson Laplacian pyramid + Wang-Chang region-energy
-// selection over ALL frames of a stack, one launch per pyramid level.
+// selection over ALL frames of a stack.
 //
 // Reference semantics (crates/lapstack-core/src): per frame, pyramid.rs:203
 // `build` (REDUCE pyramid.rs:86, EXPAND pyramid.rs:143, L = G - EXPAND),
@@ -7,17 +7,16 @@
 // window of fuse.rs:168) and the strict-> winner-take-all of fuse.rs:414-451
 // (ties to the earlier frame), frames folded in order.
 //
-// B200 layout: level-major instead of frame-major. A CTA owns a 64x32 tile of
-// level l and walks the frames k = 0..n-1; for each it stages the G_l window
-// (tile + halo) in shared memory, REDUCEs it to G_{l+1} (written once to HBM
-// for the next level's pass), EXPANDs back, forms L_l, the luma energy and
-// its window sum, and keeps the running best energy, the winning L_l
-// coefficients and the winner index in registers. The accumulator is written
-// once per level instead of read-modified-written once per frame. At level 0
-// the source is the interleaved u16 frame itself (gains and, for aligned
-// stacks, the Spline4x4 warp applied on load), and the depth pass's focus
-// slice (depth.rs:1097: luma -> ring difference filter -> block mean) is
-// taken from the same staged tile.
+// B200 layout: level-major instead of frame-major. Whoever owns a tile of level
+// l walks the frames k = 0..n-1: L_l = G_l - EXPAND(G_{l+1}), the luma energy
+// and its window sum, and the running best energy, winning coefficients and
+// winner index stay on the SM. The accumulator is written once per level instead
+// of read-modified-written once per frame. Level 0 of 16-bit frames is one kernel
+// (lsb_fold0.cuh): REDUCE to G_1, the selection and the depth pass's focus slice
+// (depth.rs:1097: luma -> ring difference filter -> block mean) from one staged
+// copy of the interleaved u16 frame, its gains applied on load. The other levels
+// are REDUCEd one after another (lsb_level.cuh), then selected together in one
+// launch (lsb_select.cuh).
 //
 // Every float op on the selection path is an explicit round-to-nearest
 // intrinsic in the reference's association order, so selection maps and
